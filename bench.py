@@ -43,23 +43,26 @@ WORKLOAD = "wall-RPY M_UF.F, 256 shells x 42 blobs = 10,752 blobs (FP64-accurate
 NF_EXACT_R = 6.0
 NF_CUTOFF_R = 9.0
 NF_ALL_EXACT_R = NF_CUTOFF_R
-# Issued thread instructions per ordered pair of the df64 UF kernels (all
-# pipes, 80-85 % of them on the FMA pipe), from ncu's smsp__inst_executed.sum
-# on the 10,752-blob product: symmetric kernel (each unordered pair once),
-# 1,705,420,652 warp instructions * 32 / 10752^2 = 472.1; one-sided kernel
-# (source split 15) 2,719,541,740 * 32 / 10752^2 = 752.8.  The FP32 pipe
-# issues at most one thread instruction per lane per clock, the rate the
-# FMA-chain probe measures (FLOP/s / 2), so achieved / peak is the fraction of
-# issue capacity used.  The constants hold for the kernel sources whose hash is
+# FP32-issue slots per ordered pair of the df64 UF kernels, from ncu on the
+# 10,752-blob product: thread instructions of all pipes, a packed (f32x2)
+# instruction counted as the two lanes' operations it does on the FMA pipe
+# (which takes it two clocks).  Symmetric kernel (each unordered pair once,
+# two targets per thread in packed lanes): smsp__inst_executed.sum
+# 572,086,998 + packed (pipe_fmaheavy + pipe_fmalite - pipe_fma) 515,134,737
+# = 1,087,221,735 warp instructions * 32 / 10752^2 = 301.0; one-sided kernel
+# (source split 15) 1,804,026,278 * 32 / 10752^2 = 499.4.  The FP32 pipe takes
+# at most one thread instruction per lane per clock, the rate the FMA-chain
+# probe measures (FLOP/s / 2), so achieved / peak is the fraction of that
+# capacity used.  The constants hold for the kernel sources whose hash is
 # DF64_UF_KERNEL_SOURCE_SHA (tests/test_bench_constants.py fails when the
 # kernel changes without a new capture).
-DF64_UF_INST_PER_PAIR = {"symmetric": 1705420652.0 * 32 / 10752 ** 2, "standard": 2719541740.0 * 32 / 10752 ** 2}
+DF64_UF_INST_PER_PAIR = {"symmetric": 1087221735.0 * 32 / 10752 ** 2, "standard": 1804026278.0 * 32 / 10752 ** 2}
 # dram__bytes_read.sum + dram__bytes_write.sum per launch, same captures
-DF64_UF_TRAFFIC_BYTES = {"symmetric": 736000, "standard": 718848}
+DF64_UF_TRAFFIC_BYTES = {"symmetric": 765696, "standard": 710400}
 # issued thread instructions per pair and right-hand side of the 16-wide multi-RHS M_UF kernel
 # (smsp__inst_executed.sum * 32 / (N^2 * 16), 60,000 blobs)
 MULTI16_INST_PER_PAIR_RHS = 17.4
-DF64_UF_KERNEL_SOURCE_SHA = "89b6f0fd4303f7413dd2bee1784d821e0f30340b3afe8b244a7c7d322d3f7b63"
+DF64_UF_KERNEL_SOURCE_SHA = "1a6871ae31f7d8272fe6483bef4749eafe9e57a46a7344c3bc2e0ee06b7933d0"
 
 
 def df64_uf_kernel_source_sha():
@@ -73,7 +76,7 @@ def df64_uf_kernel_source_sha():
     beg = src.index("namespace rmw {")
     end = src.index("// The rotation blocks (UT, WF, WT) on the same grid")
     h.update(src[beg:end].encode())
-    for name in ("pair_math_df.cuh", "dfloat.cuh"):
+    for name in ("pair_math_df.cuh", "dfloat.cuh", "f32x2.cuh"):
         with open(os.path.join(d, name)) as fh:
             h.update(fh.read().encode())
     with open(os.path.join(d, "rmw_common.cuh")) as fh:

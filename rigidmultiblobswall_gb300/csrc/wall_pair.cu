@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kThreads) wall_pair_df_kernel(const SrcDF *__r
                             for (int bz = -pz; bz <= pz; ++bz) {
                                 const bool self = (j == i) && bx == 0 && by == 0 && bz == 0;
                                 const df kx = ux, ky = uy, kz = uz;
-                                pair_acc_df<KIND>(df_of_double(rx + bx * P.Lx), df_of_double(ry + by * P.Ly),
+                                pair_acc_df<KIND, true>(df_of_double(rx + bx * P.Lx), df_of_double(ry + by * P.Ly),
                                                   df_of_double(rz + bz * P.Lz), Rz, zi, zj, vx, vy, vz, ux, uy, uz);
                                 if (self) {
                                     ux = kx;
@@ -342,9 +342,6 @@ __device__ __forceinline__ void df_sym_body(const SrcDF *__restrict__ src, int n
         // square a double-float product drops); the sum of two heights cannot cancel
         if constexpr (NOWALL)
             pair_rpy_sym_df<KIND>(xi - xj, yi - yj, zi - zj, vx, vy, vz, qx, qy, qz, ux, uy, uz, wx, wy, wz);
-        else if constexpr (KIND == RMW_UF)
-            pair_uf_sym_df(xi - xj, yi - yj, zi - zj, add_u(zi, zj), zi, zj, vx, vy, vz, qx, qy, qz, ux, uy, uz, wx,
-                           wy, wz);
         else
             pair_rot_sym_df<KIND>(xi - xj, yi - yj, zi - zj, add_u(zi, zj), zi, zj, vx, vy, vz, qx, qy, qz, ux, uy,
                                   uz, wx, wy, wz);
@@ -413,12 +410,214 @@ __device__ __forceinline__ void df_sym_body(const SrcDF *__restrict__ src, int n
     }
 }
 
-template <bool SEG>
-__global__ void __launch_bounds__(kThreads) wall_uf_df_sym_kernel(const SrcDF *__restrict__ src, int n, int nt,
-                                                                   double *__restrict__ partial,
-                                                                   const SymJob *__restrict__ jobs)
+// The UF kernel of that grid with two targets per thread in packed FP32 lanes
+// (f32x2.cuh): a CTA is 64 threads, thread t owns targets t (lane x) and
+// t + 64 (lane y) of tile T, and a step evaluates the same source for both
+// (on a diagonal tile the two sources at the same offset, so the skip test
+// goes too).  The FMA pipe bounds the kernel; packing takes the loads, the
+// shared-memory sums and the near test to half the issue slots per pair, and
+// the explicit block (uf_block_df) takes 30 % of the arithmetic.  The
+// source-side sums are float4 (hi x, hi y, lo x, lo y) per warp, component
+// and source; the target-side ones are renormalised every kF2Group steps and
+// stay on the FP32 pipe.
+// Measured (pair kernel): 10,752 blobs 1.63 -> 0.99 ms, FMA pipe 86 % active,
+// issue 48 %; the product at 172,032 blobs 400 -> 240 ms.  128 registers (8 CTAs per SM) are
+// 2 % faster than the 158 that one CTA takes unbounded.
+// gridDim.y = nsplit CTAs share a tile pair, each a contiguous range of its
+// steps with its own slots (slot = tile * nsplit + split), so that few tiles
+// still fill the GPU.
+constexpr int kF2Threads = kTile / 2;
+constexpr int kF2Group = 8;
+
+struct F2Target {
+    df2 x, y, z, h4, qx, qy, qz;  // positions, 4 z, b v of both targets
+};
+
+// one step: sources ja (lane x) and jb (lane y); DIAG false: ja = jb
+template <bool DIAG>
+__device__ __forceinline__ void uf_f2_step(const F2Target &me, int ja, int jb, const float4 *thi, const float4 *tlo,
+                                           const float4 *tvh, const float4 *tvl, float4 (*sacc)[kTile], df2 &ux,
+                                           df2 &uy, df2 &uz)
 {
-    df_sym_body<SEG, RMW_UF>(src, n, nt, partial, jobs);
+    const float4 sh = thi[ja], sl = tlo[ja], vh = tvh[ja], vl = tvl[ja];
+    float4 sh1 = sh, sl1 = sl, vh1 = vh, vl1 = vl;
+    float4 w0, w1, w2;
+    if (DIAG) {
+        sh1 = thi[jb]; sl1 = tlo[jb]; vh1 = tvh[jb]; vl1 = tvl[jb];
+        auto at = [&](int c) {
+            const float4 p = sacc[c][ja], q = sacc[c][jb];
+            return make_float4(p.x, q.y, p.z, q.w);
+        };
+        w0 = at(0); w1 = at(1); w2 = at(2);
+    } else {
+        w0 = sacc[0][ja]; w1 = sacc[1][ja]; w2 = sacc[2][ja];
+    }
+    const df2 xj = {make_float2(sh.x, sh1.x), make_float2(sl.x, sl1.x)};
+    const df2 yj = {make_float2(sh.y, sh1.y), make_float2(sl.y, sl1.y)};
+    const df2 zj = {make_float2(sh.z, sh1.z), make_float2(sl.z, sl1.z)};
+    const df2 vx = {make_float2(vh.x, vh1.x), make_float2(vl.x, vl1.x)};
+    const df2 vy = {make_float2(vh.y, vh1.y), make_float2(vl.y, vl1.y)};
+    const df2 vz = {make_float2(vh.z, vh1.z), make_float2(vl.z, vl1.z)};
+    df2 wx = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w)};
+    df2 wy = {make_float2(w1.x, w1.y), make_float2(w1.z, w1.w)};
+    df2 wz = {make_float2(w2.x, w2.y), make_float2(w2.z, w2.w)};
+    // differences renormalised (a cancelled high part must not leave the value in the low part, whose
+    // square a double-float product drops); the sum of two heights cannot cancel
+    const df2 dx = me.x - xj, dy = me.y - yj;
+    const UFBlockDF<df2> m = uf_block_df<df2>(dx, dy, me.z - zj, add_u(me.z, zj), me.h4, zj);
+    uf_block_acc_df(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);                // M_ij v_j
+    uf_block_acc_df(m, m.t4, m.t3, dx, dy, me.qx, me.qy, me.qz, wx, wy, wz);       // M_ij^T v_i
+    if (DIAG) {
+        float *s = reinterpret_cast<float *>(sacc);
+        auto put = [&](int c, const df2 &w) {
+            float *a = s + 4 * (c * kTile + ja), *b = s + 4 * (c * kTile + jb);
+            a[0] = w.hi.x; a[2] = w.lo.x;
+            b[1] = w.hi.y; b[3] = w.lo.y;
+        };
+        put(0, wx); put(1, wy); put(2, wz);
+    } else {
+        sacc[0][ja] = make_float4(wx.hi.x, wx.hi.y, wx.lo.x, wx.lo.y);
+        sacc[1][ja] = make_float4(wy.hi.x, wy.hi.y, wy.lo.x, wy.lo.y);
+        sacc[2][ja] = make_float4(wz.hi.x, wz.hi.y, wz.lo.x, wz.lo.y);
+    }
+}
+
+template <bool SEG, bool BAND>
+__device__ __forceinline__ void uf_f2_body(const SrcDF *__restrict__ src, int n, int nt, double *__restrict__ partial,
+                                           const SymJob *__restrict__ jobs,
+                                           const SymBand bd = SymBand{0, 0, nullptr, nullptr})
+{
+    __shared__ float4 thi[kTile], tlo[kTile], tvh[kTile], tvl[kTile];
+    __shared__ float4 sacc[kF2Threads / 32][3][kTile];
+    int T, S;
+    if constexpr (BAND) sym_band_pair(blockIdx.x, nt, bd, T, S);
+    else sym_cta<SEG>(jobs, n, nt, T, S, src, partial);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool diag = (T == S);
+    const int i0 = T * kTile + tid, i1 = i0 + kF2Threads;
+    // a target or source past the end is a dummy far above the wall with a zero vector
+    const SrcDF dummy = {make_float4(1.0e6f, 1.0e6f, 1.0e6f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f),
+                         make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+    F2Target me;
+    {
+        const SrcDF a = i0 < n ? src[i0] : dummy, b = i1 < n ? src[i1] : dummy;
+        me.x = df2_pack({a.hi.x, a.lo.x}, {b.hi.x, b.lo.x});
+        me.y = df2_pack({a.hi.y, a.lo.y}, {b.hi.y, b.lo.y});
+        me.z = df2_pack({a.hi.z, a.lo.z}, {b.hi.z, b.lo.z});
+        me.h4 = scale2(me.z, 4.0f);
+        me.qx = df2_pack({a.vhi.x, a.vlo.x}, {b.vhi.x, b.vlo.x});
+        me.qy = df2_pack({a.vhi.y, a.vlo.y}, {b.vhi.y, b.vlo.y});
+        me.qz = df2_pack({a.vhi.z, a.vlo.z}, {b.vhi.z, b.vlo.z});
+    }
+    for (int k = tid; k < kTile; k += kF2Threads) {
+        const int j = S * kTile + k;
+        const SrcDF sj = (j < n) ? src[j] : dummy;
+        thi[k] = sj.hi;
+        tlo[k] = sj.lo;
+        tvh[k] = sj.vhi;
+        tvl[k] = sj.vlo;
+    }
+    for (int c = 0; c < 3; ++c)
+        for (int k = lane; k < kTile; k += 32) sacc[warp][c][k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    df2 ux = df2_zero(), uy = df2_zero(), uz = df2_zero();
+    // a power of two at most kF2MaxSplit: every CTA's range of steps is a multiple of kF2Group / 2
+    const int nsplit = (SEG || BAND) ? 1 : gridDim.y, split = (SEG || BAND) ? 0 : blockIdx.y;
+    if (diag) {
+        // offsets 1..64 (source - target): each unordered pair once; 64 pairs up targets 0..63 with
+        // 64..127, so there lane y, whose pairs lane x has, works with zero vectors
+        const int m = kTile / 2 / nsplit;
+        for (int o = 1 + split * m; o < 1 + split * m + m; ++o) {
+            __syncwarp();
+            const int ja = (tid + o) & (kTile - 1), jb = (tid + kF2Threads + o) & (kTile - 1);
+            if (o < kTile / 2) {
+                uf_f2_step<true>(me, ja, jb, thi, tlo, tvh, tvl, sacc[warp], ux, uy, uz);
+            } else {
+                F2Target half = me;
+                half.qx.hi.y = half.qx.lo.y = half.qy.hi.y = half.qy.lo.y = half.qz.hi.y = half.qz.lo.y = 0.f;
+                df2 vx = ux, vy = uy, vz = uz;
+                uf_f2_step<true>(half, ja, jb, thi, tlo, tvh, tvl, sacc[warp], vx, vy, vz);
+                ux.hi.x = vx.hi.x; ux.lo.x = vx.lo.x;
+                uy.hi.x = vy.hi.x; uy.lo.x = vy.lo.x;
+                uz.hi.x = vz.hi.x; uz.lo.x = vz.lo.x;
+            }
+            if (!(o & (kF2Group - 1))) { ux = norm(ux); uy = norm(uy); uz = norm(uz); }
+        }
+    } else {
+        const int m = kTile / nsplit;
+        for (int g = split * m; g < split * m + m;) {
+            const int e = min(g + kF2Group, split * m + m);
+#pragma unroll 1
+            for (; g < e; ++g) {
+                __syncwarp();
+                const int j = (lane + g) & (kTile - 1);
+                uf_f2_step<false>(me, j, j, thi, tlo, tvh, tvl, sacc[warp], ux, uy, uz);
+            }
+            ux = norm(ux);
+            uy = norm(uy);
+            uz = norm(uz);
+        }
+    }
+    __syncthreads();
+    const size_t stride = 3 * (size_t)n;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const int l = tid + half * kF2Threads;  // blob l of the tile
+        auto lane_sum = [half](const df2 &u) {
+            return half ? (double)u.hi.y + (double)u.lo.y : (double)u.hi.x + (double)u.lo.x;
+        };
+        const double ax = lane_sum(ux), ay = lane_sum(uy), az = lane_sum(uz);
+        // source role of blob S*128 + l (dummy pairs contributed exact zeros)
+        double s[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            s[c] = 0.0;
+            for (int w = 0; w < kF2Threads / 32; ++w) {
+                const float4 q = sacc[w][c][l];
+                s[c] += ((double)q.x + (double)q.z) + ((double)q.y + (double)q.w);
+            }
+        }
+        if constexpr (BAND) {
+            const int W = nt - bd.t0, C = bd.t1 - bd.t0;
+            double *o = bd.bt + ((size_t)(T - bd.t0) * W + (S - bd.t0)) * (3 * kTile) + 3 * l;
+            o[0] = diag ? ax + s[0] : ax;
+            o[1] = diag ? ay + s[1] : ay;
+            o[2] = diag ? az + s[2] : az;
+            if (!diag) {
+                double *q = bd.bs + ((size_t)(S - bd.t0) * C + (T - bd.t0)) * (3 * kTile) + 3 * l;
+                q[0] = s[0]; q[1] = s[1]; q[2] = s[2];
+            }
+        } else {
+            const int i = T * kTile + l, j = S * kTile + l;
+            const int st = S * nsplit + split, ss = T * nsplit + split;
+            if (i < n) {
+                double *o = partial + (size_t)st * stride + 3 * (size_t)i;
+                o[0] = diag ? ax + s[0] : ax;
+                o[1] = diag ? ay + s[1] : ay;
+                o[2] = diag ? az + s[2] : az;
+            }
+            if (!diag && j < n) {
+                double *o = partial + (size_t)ss * stride + 3 * (size_t)j;
+                o[0] = s[0]; o[1] = s[1]; o[2] = s[2];
+            }
+        }
+    }
+}
+
+template <bool SEG>
+__global__ void __launch_bounds__(kF2Threads, 8) wall_uf_df_sym_kernel(const SrcDF *__restrict__ src, int n, int nt,
+                                                                     double *__restrict__ partial,
+                                                                     const SymJob *__restrict__ jobs)
+{
+    uf_f2_body<SEG, false>(src, n, nt, partial, jobs);
+}
+
+// the same over one band of tile rows (SymBand): products whose per-tile
+// partial sums would not fit in the scratch budget
+__global__ void __launch_bounds__(kF2Threads, 8) wall_uf_df_sym_band_kernel(const SrcDF *__restrict__ src, int n, int nt,
+                                                                          const SymBand bd)
+{
+    uf_f2_body<false, true>(src, n, nt, nullptr, nullptr, bd);
 }
 
 // The rotation blocks (UT, WF, WT) on the same grid: pair_rot_sym_df.
@@ -1312,8 +1511,8 @@ static void launch_sym(bool seg, int mode, const void *src, int n, int nt, unsig
     } else if (mode == RMW_MODE_DF64) {
         const SrcDF *s = (const SrcDF *)src;
         if (KIND == RMW_UF) {
-            if (seg) wall_uf_df_sym_kernel<true><<<ncta, kThreads, 0, st>>>(s, n, nt, partial, jobs);
-            else wall_uf_df_sym_kernel<false><<<ncta, kThreads, 0, st>>>(s, n, nt, partial, jobs);
+            if (seg) wall_uf_df_sym_kernel<true><<<ncta, kF2Threads, 0, st>>>(s, n, nt, partial, jobs);
+            else wall_uf_df_sym_kernel<false><<<ncta, kF2Threads, 0, st>>>(s, n, nt, partial, jobs);
         } else {
             if (seg) wall_rot_df_sym_kernel<true, KIND><<<ncta, kThreads, 0, st>>>(s, n, nt, partial, jobs);
             else wall_rot_df_sym_kernel<false, KIND><<<ncta, kThreads, 0, st>>>(s, n, nt, partial, jobs);
@@ -1447,7 +1646,7 @@ static int sym_band_product(int kind, const double *r, const double *v, double *
         const SymBand bd{t0, t1, bt, bs};
         const SrcDF *src = (const SrcDF *)base;
         switch (kind) {
-        case RMW_UF: wall_df_sym_band_kernel<RMW_UF><<<(unsigned)ncta, kThreads, 0, st>>>(src, n, nt, bd); break;
+        case RMW_UF: wall_uf_df_sym_band_kernel<<<(unsigned)ncta, kF2Threads, 0, st>>>(src, n, nt, bd); break;
         case RMW_UT: wall_df_sym_band_kernel<RMW_UT><<<(unsigned)ncta, kThreads, 0, st>>>(src, n, nt, bd); break;
         case RMW_WF: wall_df_sym_band_kernel<RMW_WF><<<(unsigned)ncta, kThreads, 0, st>>>(src, n, nt, bd); break;
         default: wall_df_sym_band_kernel<RMW_WT><<<(unsigned)ncta, kThreads, 0, st>>>(src, n, nt, bd); break;
