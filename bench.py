@@ -48,21 +48,21 @@ NF_ALL_EXACT_R = NF_CUTOFF_R
 # instruction counted as the two lanes' operations it does on the FMA pipe
 # (which takes it two clocks).  Symmetric kernel (each unordered pair once,
 # two targets per thread in packed lanes): smsp__inst_executed.sum
-# 572,086,998 + packed (pipe_fmaheavy + pipe_fmalite - pipe_fma) 515,134,737
-# = 1,087,221,735 warp instructions * 32 / 10752^2 = 301.0; one-sided kernel
+# 575,836,506 + packed (pipe_fmaheavy + pipe_fmalite - pipe_fma) 512,338,797
+# = 1,088,175,303 warp instructions * 32 / 10752^2 = 301.2; one-sided kernel
 # (source split 15) 1,804,026,278 * 32 / 10752^2 = 499.4.  The FP32 pipe takes
 # at most one thread instruction per lane per clock, the rate the FMA-chain
 # probe measures (FLOP/s / 2), so achieved / peak is the fraction of that
 # capacity used.  The constants hold for the kernel sources whose hash is
 # DF64_UF_KERNEL_SOURCE_SHA (tests/test_bench_constants.py fails when the
 # kernel changes without a new capture).
-DF64_UF_INST_PER_PAIR = {"symmetric": 1087221735.0 * 32 / 10752 ** 2, "standard": 1804026278.0 * 32 / 10752 ** 2}
+DF64_UF_INST_PER_PAIR = {"symmetric": 1088175303.0 * 32 / 10752 ** 2, "standard": 1804026278.0 * 32 / 10752 ** 2}
 # dram__bytes_read.sum + dram__bytes_write.sum per launch, same captures
-DF64_UF_TRAFFIC_BYTES = {"symmetric": 765696, "standard": 710400}
+DF64_UF_TRAFFIC_BYTES = {"symmetric": 745984, "standard": 710400}
 # issued thread instructions per pair and right-hand side of the 16-wide multi-RHS M_UF kernel
 # (smsp__inst_executed.sum * 32 / (N^2 * 16), 60,000 blobs)
 MULTI16_INST_PER_PAIR_RHS = 17.4
-DF64_UF_KERNEL_SOURCE_SHA = "1a6871ae31f7d8272fe6483bef4749eafe9e57a46a7344c3bc2e0ee06b7933d0"
+DF64_UF_KERNEL_SOURCE_SHA = "096f6c6225bad29d3e319cf2687b42159783d90f2bd028164d24570c0a4a7064"
 
 
 def df64_uf_kernel_source_sha():

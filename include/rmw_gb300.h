@@ -198,6 +198,10 @@ int rmw_wall_force_torque(const double *r, const double *F, const double *T, dou
  * the built-in rule's. */
 int rmw_wall_autotune(int kind, int mode, int64_t n, int reps, void *stream, int *best_nchunks, double *best_ms,
                       double *default_ms);
+/* The choice for (kind, mode, n): -1 the symmetric kernel, else the one-sided
+ * kernel's source split (*tuned = 0: the built-in rule's).  Untuned FP64 and
+ * df64 products of 256 to 4,095 blobs report the one-sided split but take the
+ * symmetric kernel where it applies (rmw_wall_product_route). */
 int rmw_wall_autotune_lookup(int kind, int mode, int64_t n, int *nchunks, int *tuned);
 /* Pin a choice instead of measuring: nchunks in [1, 64], or -1 for the
  * symmetric kernel of any block and precision mode (each unordered pair
@@ -210,7 +214,8 @@ int rmw_wall_autotune_lookup(int kind, int mode, int64_t n, int *nchunks, int *t
 int rmw_wall_autotune_set(int kind, int mode, int64_t n, int nchunks);
 /* Library-only (no reference counterpart): how a product of (kind, mode, n)
  * runs on the current device - 0 the one-sided kernel, 1 the symmetric kernel
- * (each unordered pair once; ceil(n/128) x 3n doubles of partial sums), 2 the
+ * (each unordered pair once; ceil(n/128) x 3n doubles of partial sums, times
+ * the CTAs that share a tile pair below a few thousand blobs), 2 the
  * symmetric df64 kernel band by band of tile rows, when those partial sums
  * exceed the budget (an eighth of the device memory, or the scratch cap):
  * about 3 x 128 doubles per blob and tile row of a band, bands summed in a

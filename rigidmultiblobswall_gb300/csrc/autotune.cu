@@ -83,11 +83,21 @@ int wall_chunks(int kind, int mode, int n)
             return std::max(1, std::min(it->second, max_chunks(n)));
         }
     }
-    // untuned: the symmetric kernel from 4,096 blobs in FP64 and df64 and from
-    // 8,192 in mixed precision (measured faster at every size from there; the
-    // caller falls back where it does not apply)
+    // untuned: whole tile pairs of the symmetric kernel from 4,096 blobs in FP64 and df64 and from 8,192 in
+    // mixed precision; below, the one-sided kernel's split (which FP64 and df64 products from 256 blobs take
+    // only where the symmetric kernel does not apply, wall_prefers_sym)
     if ((mode != RMW_MODE_MIXED && n >= 4096) || (mode == RMW_MODE_MIXED && n >= 8192)) return kSymChunks;
-    return wall_default_chunks(n);
+    return wall_default_chunks(mode, n);
+}
+
+bool wall_prefers_sym(int kind, int mode, int n)
+{
+    {
+        std::lock_guard<std::mutex> lk(g_tune_mu);
+        auto it = g_tuned.find(key_of(kind, mode, n));
+        if (it != g_tuned.end()) return it->second == kSymChunks;
+    }
+    return n >= (mode == RMW_MODE_MIXED ? 8192 : 256);
 }
 
 }  // namespace rmw
@@ -109,11 +119,12 @@ int rmw_wall_autotune(int kind, int mode, int64_t n, int reps, void *stream, int
     std::vector<int> cand;
     for (int c : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64})
         if (c <= rmw::max_chunks(N)) cand.push_back(c);
-    const int def = rmw::wall_default_chunks(N);
+    const int def = rmw::wall_default_chunks(mode, N);
     if (std::find(cand.begin(), cand.end(), def) == cand.end()) cand.push_back(def);
     const bool try_sym = rmw::wall_sym_applicable(kind, mode, N, nullptr);
     if (try_sym) cand.push_back(rmw::kSymChunks);
-    const int cmax = std::max(*std::max_element(cand.begin(), cand.end()), try_sym ? rmw::wall_sym_slots(N) : 1);
+    const int nsplit = try_sym ? rmw::wall_sym_split(mode, N) : 1;
+    const int cmax = std::max(*std::max_element(cand.begin(), cand.end()), try_sym ? rmw::wall_sym_slots(N, nsplit) : 1);
     const size_t vec = sizeof(double) * 3 * (size_t)N;
     const size_t ws_bytes = rmw::wall_scratch_bytes(N, mode, cmax);
     // events first: nothing to release if their creation fails
@@ -136,7 +147,7 @@ int rmw_wall_autotune(int kind, int mode, int64_t n, int reps, void *stream, int
     float tbest = 0.f, tdef = 0.f;
     auto run = [&](int c) {
         if (c == rmw::kSymChunks)
-            return rmw::wall_product_sym_with_scratch(kind, r, v, out, N, 1.0, 1.0, mode, st, ws);
+            return rmw::wall_product_sym_with_scratch(kind, r, v, out, N, 1.0, 1.0, mode, st, ws, nsplit);
         return rmw::wall_product_with_scratch(kind, r, v, out, N, 1.0, 1.0, nullptr, mode, st, ws, c);
     };
     for (int c : cand) {

@@ -240,15 +240,19 @@ __global__ void __launch_bounds__(kNwThreads) nw_pair_df_kernel(const NwSrcDF *_
     }
 }
 
-// DF2: double-float slots of the mixed symmetric kernels, added on the FP32 pipe
+// DF2: double-float slots of the mixed symmetric kernels, added on the FP32
+// pipe by one thread per blob.  FP64 slots: kNwFinGroup threads per blob
+// (their loads in flight together), added by a fixed shuffle tree.
+constexpr int kNwFinGroup = 16;
 template <bool DF2 = false>
 __global__ void nw_finalize_kernel(const double *__restrict__ v, const double *__restrict__ partial, int nchunks,
                                    double *__restrict__ out, int n, double self_coef, double nf)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (int)(DF2 ? gt : gt / kNwFinGroup), g = DF2 ? 0 : (int)(gt % kNwFinGroup);
     double u[3] = {0.0, 0.0, 0.0};
     if constexpr (DF2) {
+        if (i >= n) return;
         const float2 *p2 = reinterpret_cast<const float2 *>(partial);
         df s3[3] = {df_from(0.f), df_from(0.f), df_from(0.f)};
         for (int s = 0; s < nchunks; ++s)
@@ -258,8 +262,14 @@ __global__ void nw_finalize_kernel(const double *__restrict__ v, const double *_
             }
         for (int c = 0; c < 3; ++c) u[c] = (double)s3[c].hi + (double)s3[c].lo;
     } else {
-        for (int s = 0; s < nchunks; ++s)
-            for (int c = 0; c < 3; ++c) u[c] += partial[(size_t)s * 3 * n + 3 * (size_t)i + c];
+        if (i < n)
+#pragma unroll 4
+            for (int s = g; s < nchunks; s += kNwFinGroup)
+                for (int c = 0; c < 3; ++c) u[c] += partial[(size_t)s * 3 * n + 3 * (size_t)i + c];
+#pragma unroll
+        for (int o = kNwFinGroup / 2; o > 0; o >>= 1)  // every lane of the warp takes part
+            for (int c = 0; c < 3; ++c) u[c] += __shfl_down_sync(0xffffffffu, u[c], o, kNwFinGroup);
+        if (i >= n || g != 0) return;
     }
     for (int c = 0; c < 3; ++c) out[3 * i + c] = nf * (u[c] + self_coef * v[3 * i + c]);
 }
@@ -292,17 +302,18 @@ int nowall_product(int kind, const double *r, const double *v, double *out, int6
     if (n == 0) return RMW_OK;
     const int N = (int)n;
     const bool per = L && (L[0] > 0 || L[1] > 0 || L[2] > 0);
-    // the symmetric kernel (each unordered pair once, both ways) from 4,096 blobs
+    // the symmetric kernel (each unordered pair once, both ways) from 256 blobs
     // in FP64 and df64 and 8,192 in mixed, as the wall products' untuned rule
-    bool sym = !per && N >= (mode == RMW_MODE_MIXED ? 8192 : 4096) &&
+    bool sym = !per && N >= (mode == RMW_MODE_MIXED ? 8192 : 256) &&
                wall_sym_applicable(kind, mode, N, nullptr);
-    int nchunks = sym ? wall_sym_slots(N) : wall_default_chunks(N);
+    const int nsplit = sym ? wall_sym_split(mode, N) : 1;
+    int nchunks = sym ? wall_sym_slots(N, nsplit) : wall_default_chunks(mode, N);
     const size_t rec = (mode == RMW_MODE_FP64) ? sizeof(NwSrcD) : (mode == RMW_MODE_DF64 ? sizeof(NwSrcDF)
                                                                                           : sizeof(NwSrcF));
     const size_t packed = ((rec * (size_t)N + 255) / 256) * 256;
     void *ws = nullptr;
     int src = scratch(SCRATCH_PAIR, packed + sizeof(double) * 3 * (size_t)N * nchunks, &ws, st);
-    if (src && sym) {
+    if (src && (sym || nchunks > wall_default_chunks(N))) {
         // the symmetric partial sums did not fit next to the caller's
         // allocations (or above rmw_set_scratch_limit): the one-sided kernels
         // need far less scratch
@@ -325,7 +336,7 @@ int nowall_product(int kind, const double *r, const double *v, double *out, int6
     if (int rc = trace_begin(TRACE_PAIR, st, &tok)) return rc;
     if (sym) {
         // the sym slots have the chunk layout (slot s of blob i at s * 3n + 3i)
-        if (int rc = nowall_sym_launch(kind, mode, ws, N, partial, st)) return rc;
+        if (int rc = nowall_sym_launch(kind, mode, ws, N, partial, st, nsplit)) return rc;
     } else {
         switch (kind) {
         case RMW_UF: nw_dispatch<RMW_UF>(per, mode, grid, st, ws, N, chunk, P, partial); break;
@@ -340,7 +351,8 @@ int nowall_product(int kind, const double *r, const double *v, double *out, int6
     if (sym && mode == RMW_MODE_MIXED)
         nw_finalize_kernel<true><<<pg, pb, 0, st>>>(v, partial, nchunks, out, N, self_coef, 1.0 / (8.0 * kPi * eta * p));
     else
-        nw_finalize_kernel<false><<<pg, pb, 0, st>>>(v, partial, nchunks, out, N, self_coef,
+        nw_finalize_kernel<false><<<(unsigned)(((long long)kNwFinGroup * N + pb - 1) / pb), pb, 0, st>>>(
+            v, partial, nchunks, out, N, self_coef,
                                                      1.0 / (8.0 * kPi * eta * p));
     RMW_CHECK_LAUNCH("free-space product kernels");
     return RMW_OK;

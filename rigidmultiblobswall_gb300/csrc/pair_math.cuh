@@ -251,6 +251,84 @@ __device__ __forceinline__ void uf_apply<float>(const UFCoeffs<float> &c, float 
     uz = fmaf(c.Af5, vz, fmaf(G, dz, fmaf(Gw, h2, fmaf(c.c4, W, uz))));
 }
 
+// 1/sqrt(x) in FP64: the hardware's estimate (relative error below 2^-20) and
+// one third-order Householder step, y + y e (1/2 + 3 e / 8) with
+// e = 1 - x y^2: five FP64 instructions and no special-case branch (zero,
+// infinite and subnormal x give non-finite values; no pair of distinct blobs
+// has one).
+__device__ __forceinline__ double rsqrt64(double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y * y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// The explicit M_UF block in FP64, times 3/2: the formulas of uf_block_df
+// (pair_math_df.cuh), where they are derived.  73 FP64 instructions a pair,
+// both ways, against 93 of uf_coeffs / uf_apply: the FP64 pipe bounds the
+// kernels that use it (1/64 of the FP32 rate).  ZPER: dz is an image's and
+// not h_i - h_j.
+struct UFBlockD {
+    double Af, b2, t3, t4, zz;
+};
+template <bool ZPER>
+__device__ __forceinline__ UFBlockD uf_block_d(double dx, double dy, double dz, double Rz, double hi, double hj)
+{
+    const double rho2 = fma(dx, dx, dy * dy);
+    const double r2 = fma(dz, dz, rho2);
+    const double k = hi * hj;
+    const double invr = rsqrt64(r2);
+    const double z2 = Rz * Rz;
+    const double s = rsqrt64(ZPER ? rho2 + z2 : fma(4.0, k, r2));
+    const double i2 = invr * invr;
+    double ia = invr, a3 = i2 * invr;
+    double Bc = fma(-3.0, i2, 1.5) * a3;
+    const bool near = !(r2 > 4.0);  // r <= 2
+    if (__any_sync(__activemask(), near)) {
+        if (near) {
+            ia = 0.0;
+            a3 = fma(-0.5625, r2 * invr, 2.0);
+            Bc = 0.1875 * invr;
+        }
+    }
+    const double u = s * s, t = u * s, p = t * u;
+    const double E = z2 * u;
+    const double b1 = fma(3.0, z2, 1.0);
+    const double w5 = fma(-5.0, E, b1), w7 = fma(-7.0, E, b1);
+    const double Y = fma(-5.0, u * w7, fma(9.0, k, 3.0));
+    const double Y10 = fma(-10.0, u, Y);
+    const double Z = fma(z2, fma(-20.0, u, Y10) + 6.0, 4.0);
+    const double X = Rz * p * Y10;
+    UFBlockD m;
+    m.Af = fma(p, w5, fma(-fma(3.0, k, 1.0), t, fma(1.5, ia - s, a3)));
+    const double F = fma(-1.5, t, Bc);
+    m.b2 = fma(p, Y, F);
+    double G, dG;  // dz F, dz^2 F
+    if constexpr (ZPER) {
+        const double dw = hi - hj, g = dz * Bc, w = -1.5 * t * dw;
+        G = g + w;
+        dG = fma(dz, g, dw * w);
+    } else {
+        G = dz * F;
+        dG = dz * G;
+    }
+    m.t3 = G - X;
+    m.t4 = G + X;
+    m.zz = fma(-p, Z, m.Af + dG);
+    return m;
+}
+// (ux, uy, uz) += (3/2) M v; with t3 and t4 exchanged, the transposed block
+__device__ __forceinline__ void uf_block_acc_d(const UFBlockD &m, double t3, double t4, double dx, double dy,
+                                               double vx, double vy, double vz, double &ux, double &uy, double &uz)
+{
+    const double P = fma(dy, vy, dx * vx);
+    const double G = fma(t3, vz, m.b2 * P);
+    ux = fma(G, dx, fma(m.Af, vx, ux));
+    uy = fma(G, dy, fma(m.Af, vy, uy));
+    uz = fma(t4, P, fma(m.zz, vz, uz));
+}
+
 // ---------------------------------------------------------------------------
 // Symmetric forms of the rotation blocks in FP32 and FP64 (the double-float
 // forms are pair_rot_sym_df): M_ji is the M_ij formula with d -> -d and

@@ -72,7 +72,7 @@ extern "C" int rmw_wall_product_noalloc(int kind, const double *r, const double 
     if (rc) return rc;
     // Same source-chunk split as the standard entry point when it fits,
     // otherwise as many chunks as the fixed array holds (at least one).
-    int nchunks = rmw::wall_default_chunks((int)n);
+    int nchunks = rmw::wall_default_chunks(mode, (int)n);
     while (nchunks > 1 && rmw::wall_scratch_bytes((int)n, mode, nchunks) > rmw::kNoallocScratchBytes) --nchunks;
     // Every scratch byte a call reads was written earlier in the same call
     // (pack writes all n records, the pair kernel writes every partial slot),

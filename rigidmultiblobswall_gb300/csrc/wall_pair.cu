@@ -244,6 +244,19 @@ __global__ void __launch_bounds__(kThreads) wall_pair_df_kernel(const SrcDF *__r
 // sums ntiles slots in fixed order and the result is deterministic.
 constexpr int kSymWarps = kThreads / 32;
 
+// The steps of this CTA's tile pair: all of them, or (FP64 and df64 products
+// of few tiles) one of gridDim.y equal ranges, each with its own slots.
+struct SymSteps {
+    int k0, k1, nsplit, split;
+    __device__ __forceinline__ int slot(int tile) const { return tile * nsplit + split; }
+};
+template <bool WHOLE>
+__device__ __forceinline__ SymSteps sym_steps()
+{
+    if (WHOLE) return {0, kTile, 1, 0};
+    const int m = kTile / gridDim.y, s = blockIdx.y;
+    return {s * m, (s + 1) * m, (int)gridDim.y, s};
+}
 
 // The CTA's tile pair: from blockIdx.x over the upper triangle of nt tiles, or
 // (SEG) from its job, which also moves src and partial to its suspension.
@@ -349,20 +362,22 @@ __device__ __forceinline__ void df_sym_body(const SrcDF *__restrict__ src, int n
         sacc[warp][1][jl] = make_float2(wy.hi, wy.lo);
         sacc[warp][2][jl] = make_float2(wz.hi, wz.lo);
     };
+    const SymSteps sp = sym_steps<SEG || BAND>();
     if (diag) {
-        for (int k = 0; k < kTile; ++k) {
+        for (int k = sp.k0; k < sp.k1; ++k) {
             __syncwarp();
-            if (k && !(k & 31)) fold();
+            if (k > sp.k0 && !(k & 31)) fold();
             const int off = (k - 32 * warp) & (kTile - 1);  // (source - target) mod 128, warp-uniform
             if (off == 0 || off > kTile / 2 || (off == kTile / 2 && warp >= kSymWarps / 2)) continue;
             step(k);
         }
     } else {
         // off-diagonal tiles: no per-step skip test (unrolling measured slower here)
-        for (int g = 0; g < kTile; g += 32) {
-            if (g) fold();
+        for (int g = sp.k0; g < sp.k1; g += 32) {
+            if (g > sp.k0) fold();
+            const int e = min(g + 32, sp.k1);
 #pragma unroll 1
-            for (int k = g; k < g + 32; ++k) {
+            for (int k = g; k < e; ++k) {
                 __syncwarp();
                 step(k);
             }
@@ -394,17 +409,17 @@ __device__ __forceinline__ void df_sym_body(const SrcDF *__restrict__ src, int n
     const size_t stride = 3 * (size_t)n;
     if (diag) {
         if (valid_i) {
-            double *o = partial + (size_t)T * stride + 3 * (size_t)i;
+            double *o = partial + (size_t)sp.slot(T) * stride + 3 * (size_t)i;
             o[0] = ax + sx; o[1] = ay + sy; o[2] = az + sz;
         }
     } else {
         if (valid_i) {
-            double *o = partial + (size_t)S * stride + 3 * (size_t)i;
+            double *o = partial + (size_t)sp.slot(S) * stride + 3 * (size_t)i;
             o[0] = ax; o[1] = ay; o[2] = az;
         }
         const int j = S * kTile + tid;
         if (j < n) {
-            double *o = partial + (size_t)T * stride + 3 * (size_t)j;
+            double *o = partial + (size_t)sp.slot(T) * stride + 3 * (size_t)j;
             o[0] = sx; o[1] = sy; o[2] = sz;
         }
     }
@@ -423,9 +438,6 @@ __device__ __forceinline__ void df_sym_body(const SrcDF *__restrict__ src, int n
 // Measured (pair kernel): 10,752 blobs 1.63 -> 0.99 ms, FMA pipe 86 % active,
 // issue 48 %; the product at 172,032 blobs 400 -> 240 ms.  128 registers (8 CTAs per SM) are
 // 2 % faster than the 158 that one CTA takes unbounded.
-// gridDim.y = nsplit CTAs share a tile pair, each a contiguous range of its
-// steps with its own slots (slot = tile * nsplit + split), so that few tiles
-// still fill the GPU.
 constexpr int kF2Threads = kTile / 2;
 constexpr int kF2Group = 8;
 
@@ -482,7 +494,7 @@ __device__ __forceinline__ void uf_f2_step(const F2Target &me, int ja, int jb, c
     }
 }
 
-template <bool SEG, bool BAND>
+template <bool WHOLE, bool SEG, bool BAND>
 __device__ __forceinline__ void uf_f2_body(const SrcDF *__restrict__ src, int n, int nt, double *__restrict__ partial,
                                            const SymJob *__restrict__ jobs,
                                            const SymBand bd = SymBand{0, 0, nullptr, nullptr})
@@ -521,13 +533,11 @@ __device__ __forceinline__ void uf_f2_body(const SrcDF *__restrict__ src, int n,
         for (int k = lane; k < kTile; k += 32) sacc[warp][c][k] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
     df2 ux = df2_zero(), uy = df2_zero(), uz = df2_zero();
-    // a power of two at most kF2MaxSplit: every CTA's range of steps is a multiple of kF2Group / 2
-    const int nsplit = (SEG || BAND) ? 1 : gridDim.y, split = (SEG || BAND) ? 0 : blockIdx.y;
+    const SymSteps sp = sym_steps<WHOLE>();
     if (diag) {
         // offsets 1..64 (source - target): each unordered pair once; 64 pairs up targets 0..63 with
         // 64..127, so there lane y, whose pairs lane x has, works with zero vectors
-        const int m = kTile / 2 / nsplit;
-        for (int o = 1 + split * m; o < 1 + split * m + m; ++o) {
+        for (int o = 1 + sp.k0 / 2; o < 1 + sp.k1 / 2; ++o) {
             __syncwarp();
             const int ja = (tid + o) & (kTile - 1), jb = (tid + kF2Threads + o) & (kTile - 1);
             if (o < kTile / 2) {
@@ -544,9 +554,8 @@ __device__ __forceinline__ void uf_f2_body(const SrcDF *__restrict__ src, int n,
             if (!(o & (kF2Group - 1))) { ux = norm(ux); uy = norm(uy); uz = norm(uz); }
         }
     } else {
-        const int m = kTile / nsplit;
-        for (int g = split * m; g < split * m + m;) {
-            const int e = min(g + kF2Group, split * m + m);
+        for (int g = sp.k0; g < sp.k1;) {
+            const int e = min(g + kF2Group, sp.k1);
 #pragma unroll 1
             for (; g < e; ++g) {
                 __syncwarp();
@@ -563,53 +572,55 @@ __device__ __forceinline__ void uf_f2_body(const SrcDF *__restrict__ src, int n,
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         const int l = tid + half * kF2Threads;  // blob l of the tile
-        auto lane_sum = [half](const df2 &u) {
-            return half ? (double)u.hi.y + (double)u.lo.y : (double)u.hi.x + (double)u.lo.x;
-        };
-        const double ax = lane_sum(ux), ay = lane_sum(uy), az = lane_sum(uz);
-        // source role of blob S*128 + l (dummy pairs contributed exact zeros)
-        double s[3];
+        // source role of blob S*128 + l (dummy pairs contributed exact zeros): four double-float sums, on the
+        // FP32 pipe (an FP64 add costs as much as 64 FP32 ones), one FP64 value per component at the end
+        const df2 uu[3] = {ux, uy, uz};
+        double own[3], s[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            s[c] = 0.0;
+            const df t = half ? df{uu[c].hi.y, uu[c].lo.y} : df{uu[c].hi.x, uu[c].lo.x};
+            df q = df_from(0.f);
+#pragma unroll
             for (int w = 0; w < kF2Threads / 32; ++w) {
-                const float4 q = sacc[w][c][l];
-                s[c] += ((double)q.x + (double)q.z) + ((double)q.y + (double)q.w);
+                const float4 f = sacc[w][c][l];
+                q = q + (df{f.x, f.z} + df{f.y, f.w});
             }
+            own[c] = to_double(diag ? t + q : t);
+            s[c] = diag ? 0.0 : to_double(q);
         }
         if constexpr (BAND) {
             const int W = nt - bd.t0, C = bd.t1 - bd.t0;
             double *o = bd.bt + ((size_t)(T - bd.t0) * W + (S - bd.t0)) * (3 * kTile) + 3 * l;
-            o[0] = diag ? ax + s[0] : ax;
-            o[1] = diag ? ay + s[1] : ay;
-            o[2] = diag ? az + s[2] : az;
+            o[0] = own[0];
+            o[1] = own[1];
+            o[2] = own[2];
             if (!diag) {
                 double *q = bd.bs + ((size_t)(S - bd.t0) * C + (T - bd.t0)) * (3 * kTile) + 3 * l;
                 q[0] = s[0]; q[1] = s[1]; q[2] = s[2];
             }
         } else {
             const int i = T * kTile + l, j = S * kTile + l;
-            const int st = S * nsplit + split, ss = T * nsplit + split;
             if (i < n) {
-                double *o = partial + (size_t)st * stride + 3 * (size_t)i;
-                o[0] = diag ? ax + s[0] : ax;
-                o[1] = diag ? ay + s[1] : ay;
-                o[2] = diag ? az + s[2] : az;
+                double *o = partial + (size_t)sp.slot(S) * stride + 3 * (size_t)i;
+                o[0] = own[0];
+                o[1] = own[1];
+                o[2] = own[2];
             }
             if (!diag && j < n) {
-                double *o = partial + (size_t)ss * stride + 3 * (size_t)j;
+                double *o = partial + (size_t)sp.slot(T) * stride + 3 * (size_t)j;
                 o[0] = s[0]; o[1] = s[1]; o[2] = s[2];
             }
         }
     }
 }
 
-template <bool SEG>
+// WHOLE: one CTA per tile pair (constant loop bounds: 2 % at 10,752 blobs)
+template <bool SEG, bool WHOLE>
 __global__ void __launch_bounds__(kF2Threads, 8) wall_uf_df_sym_kernel(const SrcDF *__restrict__ src, int n, int nt,
                                                                      double *__restrict__ partial,
                                                                      const SymJob *__restrict__ jobs)
 {
-    uf_f2_body<SEG, false>(src, n, nt, partial, jobs);
+    uf_f2_body<WHOLE, SEG, false>(src, n, nt, partial, jobs);
 }
 
 // the same over one band of tile rows (SymBand): products whose per-tile
@@ -617,7 +628,7 @@ __global__ void __launch_bounds__(kF2Threads, 8) wall_uf_df_sym_kernel(const Src
 __global__ void __launch_bounds__(kF2Threads, 8) wall_uf_df_sym_band_kernel(const SrcDF *__restrict__ src, int n, int nt,
                                                                           const SymBand bd)
 {
-    uf_f2_body<false, true>(src, n, nt, nullptr, nullptr, bd);
+    uf_f2_body<true, false, true>(src, n, nt, nullptr, nullptr, bd);
 }
 
 // The rotation blocks (UT, WF, WT) on the same grid: pair_rot_sym_df.
@@ -785,7 +796,9 @@ __global__ void __launch_bounds__(kThreads) wall_rot_mixed_sym_kernel(const SrcF
 // Symmetric FP64 kernel of any kind: the same grid, pairing and partial-sum
 // slots, FP64 pair arithmetic (the FP64 pipe bounds it, so halving the
 // coefficient work per ordered pair is the gain); source-side sums per warp
-// in FP64 shared memory.
+// in FP64 shared memory.  UF through the explicit block of uf_block_d: the
+// 10,752-blob product 11.6 -> 8.1 ms, 73 FP64 instructions per pair at 98 %
+// of the pipe's measured rate (0.53 T instructions/s).
 template <bool SEG, int KIND, bool NOWALL = false>
 __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int n, int nt, double inva,
                                               double *__restrict__ partial, const SymJob *__restrict__ jobs)
@@ -825,10 +838,9 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
         if constexpr (NOWALL) {
             pair_rpy_sym<double, KIND>(dx, dy, dz, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
         } else if constexpr (KIND == RMW_UF) {
-            const UFCoeffs<double> c = uf_coeffs<double>(dx, dy, dz, Rz, zi, zj);
-            uf_apply<double>(c, dx, dy, dz, Rz, vx, vy, vz, ux, uy, uz);
-            const UFCoeffs<double> ct = {c.Af, c.Bc, c.c2, c.c4, c.c3, c.Af5};  // M^T: f3 and f4 trade places
-            uf_apply<double>(ct, dx, dy, dz, Rz, me.vx, me.vy, me.vz, wx, wy, wz);
+            const UFBlockD m = uf_block_d<false>(dx, dy, dz, Rz, zi, zj);
+            uf_block_acc_d(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
+            uf_block_acc_d(m, m.t4, m.t3, dx, dy, me.vx, me.vy, me.vz, wx, wy, wz);
         } else {
             pair_rot_sym<double, KIND>(dx, dy, dz, Rz, zi, zj, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy,
                                        wz);
@@ -837,15 +849,16 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
         sacc[warp][1][jl] = wy;
         sacc[warp][2][jl] = wz;
     };
+    const SymSteps sp = sym_steps<SEG>();
     if (diag) {
-        for (int k = 0; k < kTile; ++k) {
+        for (int k = sp.k0; k < sp.k1; ++k) {
             __syncwarp();
             const int off = (k - 32 * warp) & (kTile - 1);
             if (off == 0 || off > kTile / 2 || (off == kTile / 2 && warp >= kSymWarps / 2)) continue;
             step(k);
         }
     } else {
-        for (int k = 0; k < kTile; ++k) {
+        for (int k = sp.k0; k < sp.k1; ++k) {
             __syncwarp();
             step(k);
         }
@@ -860,17 +873,17 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
     const size_t stride = 3 * (size_t)n;
     if (diag) {
         if (valid_i) {
-            double *o = partial + (size_t)T * stride + 3 * (size_t)i;
+            double *o = partial + (size_t)sp.slot(T) * stride + 3 * (size_t)i;
             o[0] = ux + qx; o[1] = uy + qy; o[2] = uz + qz;
         }
     } else {
         if (valid_i) {
-            double *o = partial + (size_t)S * stride + 3 * (size_t)i;
+            double *o = partial + (size_t)sp.slot(S) * stride + 3 * (size_t)i;
             o[0] = ux; o[1] = uy; o[2] = uz;
         }
         const int j = S * kTile + tid;
         if (j < n) {
-            double *o = partial + (size_t)T * stride + 3 * (size_t)j;
+            double *o = partial + (size_t)sp.slot(T) * stride + 3 * (size_t)j;
             o[0] = qx; o[1] = qy; o[2] = qz;
         }
     }
@@ -906,33 +919,48 @@ __global__ void __launch_bounds__(kThreads) nowall_fp64_sym_kernel(const SrcD *_
     fp64_sym_body<false, KIND, true>(src, n, nt, 1.0, partial, nullptr);
 }
 
+static int sym_tiles(int n) { return (n + kTile - 1) / kTile; }
+
 template <int KIND>
-static void nowall_sym_launch_kind(int mode, const void *src, int n, int nt, double *partial, cudaStream_t st)
+static void nowall_sym_launch_kind(int mode, const void *src, int n, int nt, double *partial, cudaStream_t st,
+                                   int nsplit)
 {
-    const unsigned ncta = (unsigned)((long long)nt * (nt + 1) / 2);
+    const unsigned npair = (unsigned)((long long)nt * (nt + 1) / 2);
+    const dim3 ncta(npair, nsplit);
     if (mode == RMW_MODE_FP64)
         nowall_fp64_sym_kernel<KIND><<<ncta, kThreads, 0, st>>>((const SrcD *)src, n, nt, partial);
     else if (mode == RMW_MODE_DF64)
         nowall_df_sym_kernel<KIND><<<ncta, kThreads, 0, st>>>((const SrcDF *)src, n, nt, partial);
     else
-        nowall_mixed_sym_kernel<KIND><<<ncta, kThreads, 0, st>>>((const SrcF *)src, n, nt, partial);
+        nowall_mixed_sym_kernel<KIND><<<npair, kThreads, 0, st>>>((const SrcF *)src, n, nt, partial);
 }
 
-int nowall_sym_launch(int kind, int mode, const void *src, int n, double *partial, cudaStream_t st)
+int nowall_sym_launch(int kind, int mode, const void *src, int n, double *partial, cudaStream_t st, int nsplit)
 {
-    const int nt = wall_sym_slots(n);
+    const int nt = sym_tiles(n);
     switch (kind) {
-    case RMW_UF: nowall_sym_launch_kind<RMW_UF>(mode, src, n, nt, partial, st); break;
-    case RMW_UT: nowall_sym_launch_kind<RMW_UT>(mode, src, n, nt, partial, st); break;
-    case RMW_WF: nowall_sym_launch_kind<RMW_WF>(mode, src, n, nt, partial, st); break;
-    default: nowall_sym_launch_kind<RMW_WT>(mode, src, n, nt, partial, st); break;
+    case RMW_UF: nowall_sym_launch_kind<RMW_UF>(mode, src, n, nt, partial, st, nsplit); break;
+    case RMW_UT: nowall_sym_launch_kind<RMW_UT>(mode, src, n, nt, partial, st, nsplit); break;
+    case RMW_WF: nowall_sym_launch_kind<RMW_WF>(mode, src, n, nt, partial, st, nsplit); break;
+    default: nowall_sym_launch_kind<RMW_WT>(mode, src, n, nt, partial, st, nsplit); break;
     }
     RMW_CHECK_LAUNCH("symmetric free-space product");
     return RMW_OK;
 }
 
 // ---------------------------------------------------------------------------
-// FP64 pair kernel
+// FP64 pair kernel (UF: (3/2) M v through the explicit block)
+template <int KIND, bool ZPER>
+__device__ __forceinline__ void pair_acc_d(double dx, double dy, double dz, double Rz, double hi, double hj, double vx,
+                                           double vy, double vz, double &ux, double &uy, double &uz)
+{
+    if constexpr (KIND == RMW_UF) {
+        const UFBlockD m = uf_block_d<ZPER>(dx, dy, dz, Rz, hi, hj);
+        uf_block_acc_d(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
+    } else {
+        pair_contrib<KIND, double>(dx, dy, dz, Rz, hi, hj, vx, vy, vz, ux, uy, uz);
+    }
+}
 template <int KIND, bool PER, bool SEG>
 __global__ void __launch_bounds__(kThreads) wall_pair_fp64_kernel(const SrcD *__restrict__ src, int n, int chunk,
                                                                    double inva, Periodic P,
@@ -961,10 +989,10 @@ __global__ void __launch_bounds__(kThreads) wall_pair_fp64_kernel(const SrcD *__
             const double hj = s.z * inva;
             const double Rz = (me.z + s.z) * inva;
             if (!PER) {
-                double cx = 0.0, cy = 0.0, cz = 0.0;
-                pair_contrib<KIND, double>((me.x - s.x) * inva, (me.y - s.y) * inva, (me.z - s.z) * inva, Rz, hi, hj,
-                                           s.vx, s.vy, s.vz, cx, cy, cz);
-                if (j != i) { ux += cx; uy += cy; uz += cz; }
+                double cx = ux, cy = uy, cz = uz;
+                pair_acc_d<KIND, false>((me.x - s.x) * inva, (me.y - s.y) * inva, (me.z - s.z) * inva, Rz, hi, hj,
+                                        s.vx, s.vy, s.vz, cx, cy, cz);
+                if (j != i) { ux = cx; uy = cy; uz = cz; }
             } else {
                 double rx = me.x - s.x, ry = me.y - s.y, rz = me.z - s.z;
                 if (P.Lx > 0) rx = project(rx, P.Lx);
@@ -974,12 +1002,11 @@ __global__ void __launch_bounds__(kThreads) wall_pair_fp64_kernel(const SrcD *__
                 for (int bx = -px; bx <= px; ++bx)
                     for (int by = -py; by <= py; ++by)
                         for (int bz = -pz; bz <= pz; ++bz) {
-                            double cx = 0.0, cy = 0.0, cz = 0.0;
-                            pair_contrib<KIND, double>((rx + bx * P.Lx) * inva, (ry + by * P.Ly) * inva,
-                                                       (rz + bz * P.Lz) * inva, Rz, hi, hj, s.vx, s.vy, s.vz, cx, cy,
-                                                       cz);
+                            double cx = ux, cy = uy, cz = uz;
+                            pair_acc_d<KIND, true>((rx + bx * P.Lx) * inva, (ry + by * P.Ly) * inva,
+                                                   (rz + bz * P.Lz) * inva, Rz, hi, hj, s.vx, s.vy, s.vz, cx, cy, cz);
                             const bool self = (j == i) && bx == 0 && by == 0 && bz == 0;
-                            if (!self) { ux += cx; uy += cy; uz += cz; }
+                            if (!self) { ux = cx; uy = cy; uz = cz; }
                         }
             }
         }
@@ -1276,12 +1303,17 @@ __global__ void wall_finalize_multi_kernel(const double *__restrict__ r, const d
 // kFinGroup consecutive threads share a blob: thread g of the group sums slots
 // g, g + kFinGroup, ... and a fixed shuffle tree adds the group's sums, so the
 // order is fixed (deterministic) and the slot loads run kFinGroup-wide.
-constexpr int kFinGroup = 4;
-inline unsigned finalize_blocks(int n, int pb) { return (unsigned)(((long long)kFinGroup * n + pb - 1) / pb); }
+// Products of few blobs and many slots (split tile pairs) use kFinGroupWide
+// threads, which keeps more of a blob's slot loads in flight.
+constexpr int kFinGroup = 4, kFinGroupWide = 16;
+inline unsigned finalize_blocks(int n, int pb, int group = kFinGroup)
+{
+    return (unsigned)(((long long)group * n + pb - 1) / pb);
+}
 
 // DF2: the slots hold double-float values (the mixed symmetric kernels), added
 // in double-float on the FP32 pipe
-template <int KIND, bool DF2 = false>
+template <int KIND, bool DF2 = false, int G = kFinGroup>
 __global__ void wall_finalize_kernel(const double *__restrict__ r, const double *__restrict__ v,
                                      const double *__restrict__ partial, int nchunks, double *__restrict__ out,
                                      int n, double a, double nf, const int *__restrict__ blob_nchunks,
@@ -1289,7 +1321,7 @@ __global__ void wall_finalize_kernel(const double *__restrict__ r, const double 
                                      const int *__restrict__ pstride = nullptr, double pair_scale = 1.0)
 {
     const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = (int)(gt / kFinGroup), g = (int)(gt % kFinGroup);
+    const int i = (int)(gt / G), g = (int)(gt % G);
     double ux = 0.0, uy = 0.0, uz = 0.0;
     if constexpr (DF2) {
         df sx = df_from(0.f), sy = df_from(0.f), sz = df_from(0.f);
@@ -1298,7 +1330,7 @@ __global__ void wall_finalize_kernel(const double *__restrict__ r, const double 
             const float2 *p0 = reinterpret_cast<const float2 *>(partial) + (pbase ? pbase[i] : 3 * (long long)i);
             const size_t ps = pstride ? (size_t)pstride[i] : 3 * (size_t)n;
 #pragma unroll 4
-            for (int s = g; s < nc; s += kFinGroup) {
+            for (int s = g; s < nc; s += G) {
                 const float2 *p = p0 + (size_t)s * ps;
                 const float2 px = p[0], py = p[1], pz = p[2];
                 sx = sx + df{px.x, px.y};
@@ -1307,13 +1339,13 @@ __global__ void wall_finalize_kernel(const double *__restrict__ r, const double 
             }
         }
 #pragma unroll
-        for (int o = kFinGroup / 2; o > 0; o >>= 1) {  // every lane of the warp takes part
-            sx = sx + df{__shfl_down_sync(0xffffffffu, sx.hi, o, kFinGroup),
-                         __shfl_down_sync(0xffffffffu, sx.lo, o, kFinGroup)};
-            sy = sy + df{__shfl_down_sync(0xffffffffu, sy.hi, o, kFinGroup),
-                         __shfl_down_sync(0xffffffffu, sy.lo, o, kFinGroup)};
-            sz = sz + df{__shfl_down_sync(0xffffffffu, sz.hi, o, kFinGroup),
-                         __shfl_down_sync(0xffffffffu, sz.lo, o, kFinGroup)};
+        for (int o = G / 2; o > 0; o >>= 1) {  // every lane of the warp takes part
+            sx = sx + df{__shfl_down_sync(0xffffffffu, sx.hi, o, G),
+                         __shfl_down_sync(0xffffffffu, sx.lo, o, G)};
+            sy = sy + df{__shfl_down_sync(0xffffffffu, sy.hi, o, G),
+                         __shfl_down_sync(0xffffffffu, sy.lo, o, G)};
+            sz = sz + df{__shfl_down_sync(0xffffffffu, sz.hi, o, G),
+                         __shfl_down_sync(0xffffffffu, sz.lo, o, G)};
         }
         ux = (double)sx.hi + (double)sx.lo;
         uy = (double)sy.hi + (double)sy.lo;
@@ -1324,16 +1356,16 @@ __global__ void wall_finalize_kernel(const double *__restrict__ r, const double 
             const double *p0 = pbase ? partial + pbase[i] : partial + 3 * (size_t)i;
             const size_t ps = pstride ? (size_t)pstride[i] : 3 * (size_t)n;
 #pragma unroll 4
-            for (int s = g; s < nc; s += kFinGroup) {  // unrolled: loads of several slots in flight
+            for (int s = g; s < nc; s += G) {  // unrolled: loads of several slots in flight
                 const double *p = p0 + (size_t)s * ps;
                 ux += p[0]; uy += p[1]; uz += p[2];
             }
         }
 #pragma unroll
-        for (int o = kFinGroup / 2; o > 0; o >>= 1) {  // every lane of the warp takes part
-            ux += __shfl_down_sync(0xffffffffu, ux, o, kFinGroup);
-            uy += __shfl_down_sync(0xffffffffu, uy, o, kFinGroup);
-            uz += __shfl_down_sync(0xffffffffu, uz, o, kFinGroup);
+        for (int o = G / 2; o > 0; o >>= 1) {  // every lane of the warp takes part
+            ux += __shfl_down_sync(0xffffffffu, ux, o, G);
+            uy += __shfl_down_sync(0xffffffffu, uy, o, G);
+            uz += __shfl_down_sync(0xffffffffu, uz, o, G);
         }
     }
     if (i >= n || g != 0) return;
@@ -1376,6 +1408,32 @@ static int choose_chunks(int n)
 }
 
 int wall_default_chunks(int n) { return choose_chunks(n); }
+
+// The one-sided kernels' source split in FP64 and df64 (periodic products,
+// fewer than 256 blobs): the split whose busiest SM has the least to do,
+// counting a tile's staging as two sources; an SM needs about two FP64 or
+// four df64 CTAs to keep its pipe busy.  choose_chunks keeps 256 sources per
+// chunk, which left 1,500 periodic blobs on 60 CTAs.  Where the partial sums
+// of the finer split would exceed the scratch limit, the coarser one stands.
+int wall_default_chunks(int mode, int n)
+{
+    const int base = choose_chunks(n);
+    if (mode == RMW_MODE_MIXED) return base;
+    const int tiles = (n + kThreads - 1) / kThreads, fill = mode == RMW_MODE_FP64 ? 2 : 4;
+    const size_t cap = scratch_limit();
+    int best = base;
+    long long cost = -1;
+    for (int c = 1; c <= 64 && c <= std::max(base, n / 8); ++c) {
+        if (c > base && cap && wall_scratch_bytes(n, mode, c) > cap) break;
+        const long long ctas = ((long long)tiles * c + 151) / 152;
+        const long long t = std::max<long long>(ctas, fill) * ((n + c - 1) / c + 2);
+        if (cost < 0 || t < cost) {
+            cost = t;
+            best = c;
+        }
+    }
+    return best;
+}
 
 size_t wall_scratch_bytes(int n, int mode, int nchunks)
 {
@@ -1428,8 +1486,8 @@ static int launch_kind(const double *r, const double *v, double *out, int n, dou
         else wall_pair_mixed_kernel<KIND, false, false><<<grid, kThreads, 0, st>>>(src, n, chunk, Ps, partial, jobs);
     }
     if (int rc = trace_end(tok, st)) return rc;
-    // the df64 UF pair kernel sums (3/2) M v
-    const double scale = (KIND == RMW_UF && mode == RMW_MODE_DF64) ? kUFCoeffScale : 1.0;
+    // the FP64 and df64 UF pair kernels sum (3/2) M v
+    const double scale = (KIND == RMW_UF && mode != RMW_MODE_MIXED) ? kUFCoeffScale : 1.0;
     wall_finalize_kernel<KIND><<<finalize_blocks(n, pb), pb, 0, st>>>(r, v, partial, nchunks, out, n, a, nf,
                                                                        B ? B->blob_nch : nullptr, nullptr, nullptr,
                                                                        scale);
@@ -1486,6 +1544,9 @@ size_t wall_sym_partial_budget()
     return cap ? std::min(b, cap) : b;
 }
 
+constexpr int kSplitMax = 32;
+constexpr int kSplitCtasFp64 = 24, kSplitCtasDf64 = 12;
+
 bool wall_sym_applicable(int kind, int mode, int n, const double *L)
 {
     if (kind < RMW_UF || kind > RMW_WT ||
@@ -1497,11 +1558,33 @@ bool wall_sym_applicable(int kind, int mode, int n, const double *L)
     return nt * 3.0 * (double)n * sizeof(double) <= (double)wall_sym_partial_budget();
 }
 
-int wall_sym_slots(int n) { return (n + kTile - 1) / kTile; }
+// How many CTAs share the steps of a tile pair (a power of two).  Below about
+// 4,000 blobs the tile pairs alone leave SMs idle (2,048 blobs: 136 of them);
+// the split fills the GPU with the symmetric kernel's work per pair where the
+// one-sided kernel used to do each pair twice (2,048 blobs: FP64 UF 961 ->
+// 364 us, df64 181 -> 74).  Measured by CTAs per SM wanted: df64 UF, 2,048
+// blobs 6: 72, 12: 74, 24: 81 us, 5,003 blobs 6: 287, 12: 269, 24: 279; FP64
+// UF, 2,048 blobs 3: 365, 12: 357, 24: 364 us, 10,752 blobs, where the six
+// CTAs that share an SM's FP64 pipe end together, 12: 8.24, 24: 8.10 ms.
+// Mixed products keep whole tile pairs: their FP32 sums would change with the
+// split.
+int wall_sym_split(int mode, int n)
+{
+    if (mode == RMW_MODE_MIXED) return 1;
+    const double nt = (double)sym_tiles(n), pairs = 0.5 * nt * (nt + 1);
+    const double want = 152.0 * (mode == RMW_MODE_FP64 ? kSplitCtasFp64 : kSplitCtasDf64);
+    int s = 1;
+    while (s < kSplitMax && pairs * s < want &&
+           nt * (2 * s) * 3.0 * (double)n * sizeof(double) <= (double)wall_sym_partial_budget())
+        s *= 2;
+    return s;
+}
+
+int wall_sym_slots(int n, int nsplit) { return sym_tiles(n) * nsplit; }
 
 // the symmetric kernel and finalize of one kind: the UF kernels sum (3/2) M v
 template <int KIND>
-static void launch_sym(bool seg, int mode, const void *src, int n, int nt, unsigned ncta, double *partial,
+static void launch_sym(bool seg, int mode, const void *src, int n, int nt, dim3 ncta, double *partial,
                        const SymJob *jobs, cudaStream_t st, double inva)
 {
     if (mode == RMW_MODE_FP64) {
@@ -1511,8 +1594,9 @@ static void launch_sym(bool seg, int mode, const void *src, int n, int nt, unsig
     } else if (mode == RMW_MODE_DF64) {
         const SrcDF *s = (const SrcDF *)src;
         if (KIND == RMW_UF) {
-            if (seg) wall_uf_df_sym_kernel<true><<<ncta, kF2Threads, 0, st>>>(s, n, nt, partial, jobs);
-            else wall_uf_df_sym_kernel<false><<<ncta, kF2Threads, 0, st>>>(s, n, nt, partial, jobs);
+            if (seg) wall_uf_df_sym_kernel<true, true><<<ncta, kF2Threads, 0, st>>>(s, n, nt, partial, jobs);
+            else if (ncta.y == 1) wall_uf_df_sym_kernel<false, true><<<ncta, kF2Threads, 0, st>>>(s, n, nt, partial, jobs);
+            else wall_uf_df_sym_kernel<false, false><<<ncta, kF2Threads, 0, st>>>(s, n, nt, partial, jobs);
         } else {
             if (seg) wall_rot_df_sym_kernel<true, KIND><<<ncta, kThreads, 0, st>>>(s, n, nt, partial, jobs);
             else wall_rot_df_sym_kernel<false, KIND><<<ncta, kThreads, 0, st>>>(s, n, nt, partial, jobs);
@@ -1542,7 +1626,10 @@ static void launch_sym_finalize_t(const double *r, const double *v, const double
 {
     const int pb = 256;
     const double scale = (KIND == RMW_UF) ? kUFCoeffScale : 1.0;
-    if (B)
+    if (!B && !DF2 && nt >= 32 && n < 6144)
+        wall_finalize_kernel<KIND, DF2, kFinGroupWide><<<finalize_blocks(n, pb, kFinGroupWide), pb, 0, st>>>(
+            r, v, partial, nt, out, n, a, nf, nullptr, nullptr, nullptr, scale);
+    else if (B)
         wall_finalize_kernel<KIND, DF2><<<finalize_blocks(n, pb), pb, 0, st>>>(r, v, partial, 0, out, n, a, nf,
                                                                                B->blob_nslots, B->blob_pbase,
                                                                                B->blob_pstride, scale);
@@ -1562,15 +1649,15 @@ static void launch_sym_finalize(const double *r, const double *v, const double *
 
 // pack, symmetric pair kernel and finalize of any kind (B: segmented over its suspensions)
 static int sym_product(int kind, const double *r, const double *v, double *out, int n, double eta, double a,
-                       int mode, cudaStream_t st, void *scratch_ptr, const WallBatch *B)
+                       int mode, cudaStream_t st, void *scratch_ptr, const WallBatch *B, int nsplit)
 {
-    const int nt = B ? 0 : wall_sym_slots(n);
+    const int nt = B ? 0 : sym_tiles(n);
     const size_t rec = (mode == RMW_MODE_FP64) ? sizeof(SrcD) : (mode == RMW_MODE_DF64 ? sizeof(SrcDF) : sizeof(SrcF));
     const size_t packed = ((rec * (size_t)n + 255) / 256) * 256;
     char *base = (char *)scratch_ptr;
     double *partial = (double *)(base + packed);
     const int pb = 256, pg = (n + pb - 1) / pb;
-    const unsigned ncta = B ? (unsigned)B->nsym : (unsigned)((long long)nt * (nt + 1) / 2);
+    const dim3 ncta(B ? (unsigned)B->nsym : (unsigned)((long long)nt * (nt + 1) / 2), nsplit);
     const SymJob *jobs = B ? B->sym_jobs : nullptr;
     if (mode == RMW_MODE_FP64) pack_fp64_kernel<<<pg, pb, 0, st>>>(r, v, (SrcD *)base, n, a);
     else if (mode == RMW_MODE_DF64) pack_df_kernel<<<pg, pb, 0, st>>>(r, v, (SrcDF *)base, n, a);
@@ -1587,19 +1674,19 @@ static int sym_product(int kind, const double *r, const double *v, double *out, 
     if (int rc = trace_end(tok, st)) return rc;
     const double nf = kind_norm(kind, eta, a);
     switch (kind) {
-    case RMW_UF: launch_sym_finalize<RMW_UF>(r, v, partial, nt, out, n, a, nf, B, st, mode == RMW_MODE_MIXED); break;
-    case RMW_UT: launch_sym_finalize<RMW_UT>(r, v, partial, nt, out, n, a, nf, B, st, mode == RMW_MODE_MIXED); break;
-    case RMW_WF: launch_sym_finalize<RMW_WF>(r, v, partial, nt, out, n, a, nf, B, st, mode == RMW_MODE_MIXED); break;
-    default: launch_sym_finalize<RMW_WT>(r, v, partial, nt, out, n, a, nf, B, st, mode == RMW_MODE_MIXED); break;
+    case RMW_UF: launch_sym_finalize<RMW_UF>(r, v, partial, nt * nsplit, out, n, a, nf, B, st, mode == RMW_MODE_MIXED); break;
+    case RMW_UT: launch_sym_finalize<RMW_UT>(r, v, partial, nt * nsplit, out, n, a, nf, B, st, mode == RMW_MODE_MIXED); break;
+    case RMW_WF: launch_sym_finalize<RMW_WF>(r, v, partial, nt * nsplit, out, n, a, nf, B, st, mode == RMW_MODE_MIXED); break;
+    default: launch_sym_finalize<RMW_WT>(r, v, partial, nt * nsplit, out, n, a, nf, B, st, mode == RMW_MODE_MIXED); break;
     }
     RMW_CHECK_LAUNCH("symmetric wall product kernels");
     return RMW_OK;
 }
 
 int wall_product_sym_with_scratch(int kind, const double *r, const double *v, double *out, int n, double eta,
-                                  double a, int mode, cudaStream_t st, void *scratch_ptr)
+                                  double a, int mode, cudaStream_t st, void *scratch_ptr, int nsplit)
 {
-    return sym_product(kind, r, v, out, n, eta, a, mode, st, scratch_ptr, nullptr);
+    return sym_product(kind, r, v, out, n, eta, a, mode, st, scratch_ptr, nullptr, nsplit);
 }
 
 // Tile rows per band of the banded symmetric product: the band's two partial
@@ -1671,8 +1758,9 @@ int wall_product(int kind, const double *r, const double *v, double *out, int64_
     int rc = validate_product_args(kind, r, v, out, n, eta, a, mode);
     if (rc) return rc;
     if (n == 0) return RMW_OK;
-    int nchunks = wall_chunks(kind, mode, (int)n);
+    int nchunks = wall_prefers_sym(kind, mode, (int)n) ? kSymChunks : wall_chunks(kind, mode, (int)n);
     bool sym = nchunks == kSymChunks && wall_sym_applicable(kind, mode, (int)n, L);
+    const int nsplit = sym ? wall_sym_split(mode, (int)n) : 1;
     const bool periodic = L && (L[0] > 0 || L[1] > 0 || L[2] > 0);
     void *ws = nullptr;
     if (nchunks == kSymChunks && !sym && mode == RMW_MODE_DF64 && !periodic && n >= 2 * kTile) {
@@ -1681,8 +1769,9 @@ int wall_product(int kind, const double *r, const double *v, double *out, int64_
             return sym_band_product(kind, r, v, out, (int)n, eta, a, st, ws);
         cudaGetLastError();
     }
-    if (nchunks == kSymChunks && !sym) nchunks = wall_default_chunks((int)n);
-    rc = scratch(SCRATCH_PAIR, wall_scratch_bytes((int)n, mode, sym ? wall_sym_slots((int)n) : nchunks), &ws, st);
+    if (nchunks == kSymChunks && !sym) nchunks = wall_default_chunks(mode, (int)n);
+    rc = scratch(SCRATCH_PAIR, wall_scratch_bytes((int)n, mode, sym ? wall_sym_slots((int)n, nsplit) : nchunks), &ws,
+                 st);
     if (rc && sym) {
         // the symmetric kernel's partial sums did not fit next to the caller's
         // allocations: the standard kernel needs far less scratch
@@ -1690,9 +1779,13 @@ int wall_product(int kind, const double *r, const double *v, double *out, int64_
         sym = false;
         nchunks = wall_default_chunks((int)n);
         rc = scratch(SCRATCH_PAIR, wall_scratch_bytes((int)n, mode, nchunks), &ws, st);
+    } else if (rc && nchunks > wall_default_chunks((int)n)) {
+        cudaGetLastError();
+        nchunks = wall_default_chunks((int)n);
+        rc = scratch(SCRATCH_PAIR, wall_scratch_bytes((int)n, mode, nchunks), &ws, st);
     }
     if (rc) return rc;
-    if (sym) return wall_product_sym_with_scratch(kind, r, v, out, (int)n, eta, a, mode, st, ws);
+    if (sym) return wall_product_sym_with_scratch(kind, r, v, out, (int)n, eta, a, mode, st, ws, nsplit);
     return wall_product_with_scratch(kind, r, v, out, (int)n, eta, a, L, mode, st, ws, nchunks);
 }
 
@@ -1808,7 +1901,7 @@ int wall_product_batched(const WallBatch &B, int kind, const double *r, const do
         const size_t packed = ((rec * (size_t)B.n + 255) / 256) * 256;
         rc = scratch(SCRATCH_PAIR, packed + sizeof(double) * (size_t)B.sym_doubles, &ws, st);
         if (rc) return rc;
-        return sym_product(kind, r, v, out, B.n, eta, a, mode, st, ws, &B);
+        return sym_product(kind, r, v, out, B.n, eta, a, mode, st, ws, &B, 1);
     }
     rc = scratch(SCRATCH_PAIR, wall_scratch_bytes(B.n, mode, B.max_slots), &ws, st);
     if (rc) return rc;
@@ -1888,9 +1981,8 @@ int rmw_wall_product_route(int kind, int mode, int64_t n, const double *L_host, 
     if (int rc = rmw::validate_product_args(kind, (void *)1, (void *)1, (void *)1, n, 1.0, 1.0, mode)) return rc;
     const int N = (int)n;
     const bool periodic = L_host && (L_host[0] > 0 || L_host[1] > 0 || L_host[2] > 0);
-    const int c = rmw::wall_chunks(kind, mode, N);
     int route = 0;
-    if (c == rmw::kSymChunks) {
+    if (rmw::wall_prefers_sym(kind, mode, N)) {
         if (rmw::wall_sym_applicable(kind, mode, N, L_host)) route = 1;
         else if (mode == RMW_MODE_DF64 && !periodic && N >= 2 * rmw::kTile) route = 2;
     }

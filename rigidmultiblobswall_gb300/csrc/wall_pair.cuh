@@ -71,11 +71,13 @@ int wall_product_batched(const WallBatch &B, int kind, const double *r, const do
 
 // Source-chunk count of the built-in rule for n blobs.
 int wall_default_chunks(int n);
+// the same for a precision mode: finer in FP64 and df64 where few tiles would leave SMs idle
+int wall_default_chunks(int mode, int n);
 // Symmetric product of any kind (each unordered pair once, applied both ways),
 // df64 or mixed: selected when wall_chunks returns kSymChunks and
 // wall_sym_applicable holds (df64 or mixed, not periodic, n >= 256, ntiles x
 // 3n doubles of partial sums within wall_sym_partial_budget()).  Its scratch is
-// wall_scratch_bytes(n, mode, wall_sym_slots(n)).
+// wall_scratch_bytes(n, mode, wall_sym_slots(n, nsplit)).
 constexpr int kSymChunks = -1;
 constexpr size_t kSymMaxPartialBytes = size_t(6) << 30;  // up to ~185,000 blobs (5.5 GB at 172,032)
 // The partial-sum budget of the current device: kSymMaxPartialBytes, or an
@@ -84,20 +86,27 @@ constexpr size_t kSymMaxPartialBytes = size_t(6) << 30;  // up to ~185,000 blobs
 // given n does not depend on what else is allocated.
 size_t wall_sym_partial_budget();
 bool wall_sym_applicable(int kind, int mode, int n, const double *L);
-int wall_sym_slots(int n);
+// CTAs per tile pair of the symmetric kernels, and their partial-sum slots
+int wall_sym_split(int mode, int n);
+int wall_sym_slots(int n, int nsplit);
 // banded symmetric df64 product (above the partial-sum budget): tile rows per band, its scratch
 int wall_sym_band_rows(int n);
 size_t wall_sym_band_scratch_bytes(int n);
 int wall_product_sym_with_scratch(int kind, const double *r, const double *v, double *out, int n, double eta,
-                                  double a, int mode, cudaStream_t st, void *scratch_ptr);
+                                  double a, int mode, cudaStream_t st, void *scratch_ptr, int nsplit);
 // The symmetric free-space pair kernel of `kind` on records packed by the
 // no-wall product (layouts of SrcD / SrcDF / SrcF, positions over a); writes
-// wall_sym_slots(n) partial-sum slots of 3n doubles.
-int nowall_sym_launch(int kind, int mode, const void *src, int n, double *partial, cudaStream_t st);
+// wall_sym_slots(n, nsplit) partial-sum slots of 3n doubles.
+int nowall_sym_launch(int kind, int mode, const void *src, int n, double *partial, cudaStream_t st, int nsplit);
 // Source-chunk count the standard entry points use: the autotuned choice of
 // (kind, mode, n's size bucket) on the current device if there is one
 // (autotune.cu; kSymChunks = the symmetric kernel), else the built-in rule.
 int wall_chunks(int kind, int mode, int n);
+// Whether the standard entry points take the symmetric kernel where it
+// applies: the autotuned choice if there is one, else from 256 blobs in FP64
+// and df64 (its tile pairs split over several CTAs, wall_sym_split) and from
+// 8,192 in mixed.
+bool wall_prefers_sym(int kind, int mode, int n);
 // Scratch bytes needed for n blobs in `mode` split into `nchunks` source chunks:
 // packed sources (64 B/blob FP64, 48 B/blob mixed, rounded up to 256 B) plus
 // nchunks * 3n doubles of partial sums.
