@@ -2,6 +2,7 @@
 // all-pairs product kernels and the dense per-body mobility of the
 // preconditioner).
 #pragma once
+#include "f32x2.cuh"
 #include "rmw_common.cuh"
 
 namespace rmw {
@@ -194,6 +195,77 @@ __device__ __forceinline__ void uf_apply(const UFCoeffs<T> &c, T dx, T dy, T dz,
     ux += c.Af * vx + G * dx;
     uy += c.Af * vy + G * dy;
     uz += c.Af5 * vz + Gr * dz + Gw * Rz + c.c4 * W;
+}
+
+// uf_coeffs<float> for two pairs in packed lanes: every operation written out
+// with the contractions the compiler gives the scalar form (products that
+// feed a sum fused into it, the operands of other products rounded), so a
+// mixed product is the same to the bit whichever form forms its blocks.
+// FUSED_R2: R^2 = fma(Rz, Rz, rho^2) instead of rho^2 + Rz^2 rounded, which
+// the scalar form came out as in every second step of an unrolled loop.
+struct UFCoeffs2 {
+    f2 Af, Bc, c2, c3, c4, Af5;
+};
+__device__ __forceinline__ f2 f2_c(float a, f2 b, f2 c) { return f2_fma(f2_dup(a), b, c); }  // a b + c
+__device__ __forceinline__ f2 f2_c(float a, f2 b, float c) { return f2_fma(f2_dup(a), b, f2_dup(c)); }
+__device__ __forceinline__ f2 f2_s(float a, f2 b) { return f2_mul(f2_dup(a), b); }
+
+template <bool FUSED_R2>
+__device__ __forceinline__ UFCoeffs2 uf_coeffs_f2(f2 dx, f2 dy, f2 dz, f2 Rz, f2 hi, f2 hj)
+{
+    const f2 rho2 = f2_fma(dx, dx, f2_mul(dy, dy));
+    const f2 r2 = f2_fma(dz, dz, rho2);
+    const f2 invr = make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
+    const f2 Rz2 = f2_mulr(Rz, Rz);
+    const f2 R2 = FUSED_R2 ? f2_fma(Rz, Rz, rho2) : f2_add(rho2, Rz2);
+    const f2 s = make_float2(rsqrt_approx(R2.x), rsqrt_approx(R2.y));
+    const f2 u = f2_mul(s, s), t = f2_mul(u, s), p = f2_mul(t, u), E = f2_mul(Rz2, u);
+    const f2 invr2 = f2_mul(invr, invr), invr3 = f2_mul(invr2, invr);
+    f2 A = f2_c(1.5f, invr, invr3);
+    f2 Bc = f2_mul(f2_c(-3.0f, invr2, 1.5f), invr3);
+    const bool na = !(r2.x > 4.0f), nb = !(r2.y > 4.0f);  // r <= 2
+    if (__any_sync(__activemask(), na || nb)) {
+        if (na) {
+            A.x = fmaf(-0.5625f, __fmul_rn(r2.x, invr.x), 2.0f);
+            Bc.x = __fmul_rn(0.1875f, invr.x);
+        }
+        if (nb) {
+            A.y = fmaf(-0.5625f, __fmul_rn(r2.y, invr.y), 2.0f);
+            Bc.y = __fmul_rn(0.1875f, invr.y);
+        }
+    }
+    const f2 hh = f2_mul(f2_mul(hi, hj), u);
+    const f2 q5 = f2_mul(f2_c(-5.0f, E, 1.0f), t);
+    const f2 Ru = f2_mul(Rz, u);
+    const f2 hjt3 = f2_mul(f2_s(3.0f, hj), t);
+    const f2 e7 = f2_c(-7.0f, E, 1.0f);
+    // -f1
+    const f2 g1 = f2_fma(f2_c(3.0f, hh, 1.5f), s, f2_fma(f2_c(-3.0f, E, 1.0f), t, f2_neg(f2_mul(q5, u))));
+    const f2 x2 = f2_c(3.0f, q5, f2_neg(f2_mul(f2_c(-9.0f, hh, 1.5f), s)));
+    const f2 f2c = f2_fma(f2_neg(f2_s(5.0f, e7)), p, x2);
+    const f2 in = f2_fma(f2_s(10.0f, f2_c(-7.0f, E, 2.0f)), p, f2_neg(f2_s(6.0f, q5)));
+    const f2 f5 = f2_fma(f2_s(3.0f, f2_fma(hj, hj, E)), t, f2_mul(f2_c(-15.0f, E, 2.0f), p));
+    UFCoeffs2 c;
+    c.Af = f2_sub(A, g1);
+    c.Bc = Bc;
+    c.c2 = f2_mul(f2c, u);
+    c.c3 = f2_fma(Ru, in, f2_fma(f2_neg(f2_mul(f2_s(18.0f, hh), Rz)), t, hjt3));
+    c.c4 = f2_fma(f2_neg(f2_s(10.0f, Ru)), p, hjt3);
+    c.Af5 = f2_c(-2.0f, f5, c.Af);
+    return c;
+}
+
+// uf_apply<float> in packed lanes
+__device__ __forceinline__ void uf_apply_f2(const UFCoeffs2 &c, f2 c3, f2 c4, f2 dx, f2 dy, f2 dz, f2 h2, f2 vx, f2 vy,
+                                            f2 vz, f2 &ux, f2 &uy, f2 &uz)
+{
+    const f2 dv = f2_fma(dz, vz, f2_fma(dy, vy, f2_mul(dx, vx)));
+    const f2 W = f2_fma(h2, vz, dv);
+    const f2 Gw = f2_fma(c.c2, W, f2_mul(c3, vz));
+    const f2 G = f2_fma(c.Bc, dv, Gw);
+    ux = f2_fma(c.Af, vx, f2_fma(G, dx, ux));
+    uy = f2_fma(c.Af, vy, f2_fma(G, dy, uy));
+    uz = f2_fma(c.Af5, vz, f2_fma(G, dz, f2_fma(Gw, h2, f2_fma(c4, W, uz))));
 }
 
 // The explicit 3x3 block of uf_coeffs, for products with several right-hand

@@ -721,11 +721,6 @@ __device__ __forceinline__ void mixed_sym_body(const SrcF *__restrict__ src, int
         float wx = sacc[warp][0][jl], wy = sacc[warp][1][jl], wz = sacc[warp][2][jl];
         if constexpr (NOWALL) {
             pair_rpy_sym<float, KIND>(dx, dy, dz, sv.x, sv.y, sv.z, me.v.x, me.v.y, me.v.z, ux, uy, uz, wx, wy, wz);
-        } else if constexpr (KIND == RMW_UF) {
-            const UFCoeffs<float> c = uf_coeffs<float>(dx, dy, dz, Rz, hi, hj);
-            uf_apply<float>(c, dx, dy, dz, Rz, sv.x, sv.y, sv.z, ux, uy, uz);
-            const UFCoeffs<float> ct = {c.Af, c.Bc, c.c2, c.c4, c.c3, c.Af5};  // M^T: f3 and f4 trade places
-            uf_apply<float>(ct, dx, dy, dz, Rz, me.v.x, me.v.y, me.v.z, wx, wy, wz);
         } else {
             pair_rot_sym<float, KIND>(dx, dy, dz, Rz, hi, hj, sv.x, sv.y, sv.z, me.v.x, me.v.y, me.v.z, ux, uy, uz, wx,
                                       wy, wz);
@@ -777,12 +772,155 @@ __device__ __forceinline__ void mixed_sym_body(const SrcF *__restrict__ src, int
     }
 }
 
-template <bool SEG>
-__global__ void __launch_bounds__(kThreads) wall_uf_mixed_sym_kernel(const SrcF *__restrict__ src, int n, int nt,
-                                                                      double *__restrict__ partial,
-                                                                      const SymJob *__restrict__ jobs)
+// The UF kernel of that grid with two targets per thread in packed FP32 lanes
+// (as wall_uf_df_sym_kernel: thread t owns targets t and t + 64).  Issue slots
+// bounded the one-target form (134 instructions per pair, 95 of them on the
+// FMA pipe, issue 81 %); packed, a step of two pairs is 95 packed FMA-pipe
+// instructions and 41 others, and the pipe (73 % active: three distinct
+// 64-bit operands are more than the register ports deliver every time)
+// bounds it: 245 -> 190 us at 10,752 blobs, the product 271 -> 212; 60,000
+// blobs 5.47 ms with 14 CTAs per SM, 5.62 unbounded.  Same operations in the same order
+// per target and per source-side sum as mixed_sym_body with its four warps
+// (lane x of warp w is its warp w, lane y its warp w + 2), so the products
+// are the same to the bit.
+struct MixTarget {
+    f2 hx, hy, hz, lx, ly, lz, h, qx, qy, qz;
+};
+
+template <bool DIAG, bool FUSED_R2>
+__device__ __forceinline__ void uf_mixed_f2_step(const MixTarget &me, int ja, int jb, bool two, const float4 *thi,
+                                                 const float4 *tlo, const float4 *tv, float2 (*sacc)[kTile], f2 &ux,
+                                                 f2 &uy, f2 &uz)
 {
-    mixed_sym_body<SEG, RMW_UF>(src, n, nt, partial, jobs);
+    const float4 sh = thi[ja], sl = tlo[ja], sv = tv[ja];
+    float4 sh1 = sh, sl1 = sl, sv1 = sv;
+    f2 wx, wy, wz;
+    if (DIAG) {
+        sh1 = thi[jb]; sl1 = tlo[jb]; sv1 = tv[jb];
+        wx = make_float2(sacc[0][ja].x, sacc[0][jb].y);
+        wy = make_float2(sacc[1][ja].x, sacc[1][jb].y);
+        wz = make_float2(sacc[2][ja].x, sacc[2][jb].y);
+    } else {
+        wx = sacc[0][ja];
+        wy = sacc[1][ja];
+        wz = sacc[2][ja];
+    }
+    const f2 dx = f2_add(f2_sub(me.hx, make_float2(sh.x, sh1.x)), f2_sub(me.lx, make_float2(sl.x, sl1.x)));
+    const f2 dy = f2_add(f2_sub(me.hy, make_float2(sh.y, sh1.y)), f2_sub(me.ly, make_float2(sl.y, sl1.y)));
+    const f2 dz = f2_add(f2_sub(me.hz, make_float2(sh.z, sh1.z)), f2_sub(me.lz, make_float2(sl.z, sl1.z)));
+    const f2 hj = make_float2(sh.w, sh1.w);  // sh.z + sl.z
+    const f2 Rz = f2_add(me.h, hj);
+    const f2 vx = make_float2(sv.x, sv1.x), vy = make_float2(sv.y, sv1.y), vz = make_float2(sv.z, sv1.z);
+    const UFCoeffs2 c = uf_coeffs_f2<FUSED_R2>(dx, dy, dz, Rz, me.h, hj);
+    const f2 h2 = f2_sub(Rz, dz);
+    f2 tx = ux, ty = uy, tz = uz;
+    uf_apply_f2(c, c.c3, c.c4, dx, dy, dz, h2, vx, vy, vz, tx, ty, tz);
+    uf_apply_f2(c, c.c4, c.c3, dx, dy, dz, h2, me.qx, me.qy, me.qz, wx, wy, wz);  // M^T: f3 and f4 trade places
+    if (DIAG) {
+        ux.x = tx.x; uy.x = ty.x; uz.x = tz.x;
+        sacc[0][ja].x = wx.x;
+        sacc[1][ja].x = wy.x;
+        sacc[2][ja].x = wz.x;
+        if (two) {
+            ux.y = tx.y; uy.y = ty.y; uz.y = tz.y;
+            sacc[0][jb].y = wx.y;
+            sacc[1][jb].y = wy.y;
+            sacc[2][jb].y = wz.y;
+        }
+    } else {
+        ux = tx; uy = ty; uz = tz;
+        sacc[0][ja] = wx;
+        sacc[1][ja] = wy;
+        sacc[2][ja] = wz;
+    }
+}
+
+template <bool SEG>
+__global__ void __launch_bounds__(kF2Threads, 14) wall_uf_mixed_sym_kernel(const SrcF *__restrict__ src, int n, int nt,
+                                                                        double *__restrict__ partial,
+                                                                        const SymJob *__restrict__ jobs)
+{
+    __shared__ float4 thi[kTile], tlo[kTile], tv[kTile];  // thi.w: the source's height in one float
+    __shared__ float2 sacc[kF2Threads / 32][3][kTile];
+    int T, S;
+    sym_cta<SEG>(jobs, n, nt, T, S, src, partial);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool diag = (T == S);
+    const int i0 = T * kTile + tid, i1 = i0 + kF2Threads;
+    const SrcF dummy = {make_float4(1.0e6f, 1.0e6f, 1.0e6f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f),
+                        make_float4(0.f, 0.f, 0.f, 0.f)};
+    MixTarget me;
+    {
+        const SrcF a = i0 < n ? src[i0] : dummy, b = i1 < n ? src[i1] : dummy;
+        me.hx = make_float2(a.hi.x, b.hi.x);
+        me.hy = make_float2(a.hi.y, b.hi.y);
+        me.hz = make_float2(a.hi.z, b.hi.z);
+        me.lx = make_float2(a.lo.x, b.lo.x);
+        me.ly = make_float2(a.lo.y, b.lo.y);
+        me.lz = make_float2(a.lo.z, b.lo.z);
+        me.h = f2_add(me.hz, me.lz);
+        me.qx = make_float2(a.v.x, b.v.x);
+        me.qy = make_float2(a.v.y, b.v.y);
+        me.qz = make_float2(a.v.z, b.v.z);
+    }
+    for (int k = tid; k < kTile; k += kF2Threads) {
+        const int j = S * kTile + k;
+        SrcF sj = (j < n) ? src[j] : dummy;
+        sj.hi.w = sj.hi.z + sj.lo.z;
+        thi[k] = sj.hi;
+        tlo[k] = sj.lo;
+        tv[k] = sj.v;
+    }
+    for (int c = 0; c < 3; ++c)
+        for (int k = lane; k < kTile; k += 32) sacc[warp][c][k] = make_float2(0.f, 0.f);
+    __syncthreads();
+    f2 ux = f2_dup(0.f), uy = ux, uz = ux;
+    if (diag) {
+        // offsets (source - target) mod 128 from 1 to 63, and 64 for targets 0..63; targets 96..127 take
+        // 32..63 first, the order in which the rotation over all sources meets them
+        for (int o = 1; o <= kTile / 2; ++o) {
+            __syncwarp();
+            const int ob = warp == 0 ? o : (o <= 32 ? o + 31 : o - 32);
+            const bool two = o < kTile / 2;
+            const int ja = (tid + o) & (kTile - 1), jb = (tid + kF2Threads + (two ? ob : o)) & (kTile - 1);
+            uf_mixed_f2_step<true, SEG>(me, ja, jb, two, thi, tlo, tv, sacc[warp], ux, uy, uz);
+        }
+    } else {
+#pragma unroll 1
+        for (int k = 0; k < kTile; k += 2) {
+            __syncwarp();
+            const int j = (lane + k) & (kTile - 1), j1 = (j + 1) & (kTile - 1);
+            uf_mixed_f2_step<false, SEG>(me, j, j, true, thi, tlo, tv, sacc[warp], ux, uy, uz);
+            __syncwarp();
+            uf_mixed_f2_step<false, true>(me, j1, j1, true, thi, tlo, tv, sacc[warp], ux, uy, uz);
+        }
+    }
+    __syncthreads();
+    float2 *part2 = reinterpret_cast<float2 *>(partial);
+    const size_t stride = 3 * (size_t)n;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const int l = tid + half * kF2Threads, i = T * kTile + l, j = S * kTile + l;
+        const f2 uu[3] = {ux, uy, uz};
+        df t[3], q[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            t[c] = df_from(half ? uu[c].y : uu[c].x);
+            q[c] = df_from(sacc[0][c][l].x);
+            q[c] = q[c] + sacc[1][c][l].x;
+            q[c] = q[c] + sacc[0][c][l].y;
+            q[c] = q[c] + sacc[1][c][l].y;
+            if (diag) t[c] = t[c] + q[c];
+        }
+        if (i < n) {
+            float2 *o = part2 + (size_t)(diag ? T : S) * stride + 3 * (size_t)i;
+            for (int c = 0; c < 3; ++c) o[c] = make_float2(t[c].hi, t[c].lo);
+        }
+        if (!diag && j < n) {
+            float2 *o = part2 + (size_t)T * stride + 3 * (size_t)j;
+            for (int c = 0; c < 3; ++c) o[c] = make_float2(q[c].hi, q[c].lo);
+        }
+    }
 }
 
 template <bool SEG, int KIND>
@@ -1604,8 +1742,8 @@ static void launch_sym(bool seg, int mode, const void *src, int n, int nt, dim3 
     } else {
         const SrcF *s = (const SrcF *)src;
         if (KIND == RMW_UF) {
-            if (seg) wall_uf_mixed_sym_kernel<true><<<ncta, kThreads, 0, st>>>(s, n, nt, partial, jobs);
-            else wall_uf_mixed_sym_kernel<false><<<ncta, kThreads, 0, st>>>(s, n, nt, partial, jobs);
+            if (seg) wall_uf_mixed_sym_kernel<true><<<ncta, kF2Threads, 0, st>>>(s, n, nt, partial, jobs);
+            else wall_uf_mixed_sym_kernel<false><<<ncta, kF2Threads, 0, st>>>(s, n, nt, partial, jobs);
         } else {
             if (seg) wall_rot_mixed_sym_kernel<true, KIND><<<ncta, kThreads, 0, st>>>(s, n, nt, partial, jobs);
             else wall_rot_mixed_sym_kernel<false, KIND><<<ncta, kThreads, 0, st>>>(s, n, nt, partial, jobs);
