@@ -5,18 +5,25 @@
 //   U(r) = U0 exp(-(r - 2a)/b) for r > 2a (linear below), the force on blob i
 //   is  f_i = -sum_{j != i} (eps/b) g(r_ij) (r_j - r_i) / r_ij  with
 //   g = exp(-(r - 2a)/b) beyond 2a and 1 inside, minimum periodic image.
-//   All pairs in FP64, as the reference.  Exact screening: exp(-(r - 2a)/b)
-//   is exactly 0 in FP64 once (r - 2a)/b > 746, so such pairs contribute
-//   nothing; a conservative FP32 distance test (coordinates relative to the
-//   CTA's first target) skips them before any FP64 work.  It is used only
-//   where the CTA's spatial extent bounds the FP32 error below the test's
-//   margin, so no contributing pair is ever skipped; elsewhere the FP64
-//   distance decides.  An optional cutoff restricts the sum to pairs within
-//   it (the reference's neighbour-list variant uses 2a + 30 b,
-//   multi_bodies/forces_numba.py:228-270).
+//   Pairs that can matter are evaluated in FP64, as the reference does; FP32
+//   distances decide which.  A pair adds exactly 0 once (r - 2a)/b > 746, and
+//   less than 2^-65 / n of the blob's largest term once
+//     r > max(2a, r_min) + b (65 ln 2 + ln n),
+//   r_min the distance to the nearest blob: all such pairs together change no
+//   bit of the sum (the largest term's own rounding is 2^-53).  An optional
+//   cutoff restricts the sum to pairs within it (the reference's
+//   neighbour-list variant uses 2a + 30 b, multi_bodies/forces_numba.py:228-270).
+//   Two FP32 passes over all pairs (nearest blob, candidates; about 10
+//   instructions a pair, the floor of 12,288 blobs 90 us) and the FP64 work of
+//   the candidates, several source chunks per target tile so that the GPU is
+//   full.  1,024 shells of 12 blobs with the wall and body reduction, Debye
+//   length 0.1a: 19.2 -> 0.33 ms (FP64 for a fifth of all pairs on 96 CTAs
+//   before); 0.5a 25.4 -> 1.7 ms; 1a 24.6 -> 4.1 ms; 172,032 blobs, 0.1a
+//   195 -> 33 ms, 1a 2,818 -> 99 ms.
 // * external blob forces (multi_bodies_functions.py:153-189): gravity
 //   -g m e_z and the wall repulsion (e/b) exp(-(h - a)/b) (e/b for h <= a).
 // The body reduction [F_b, T_b] = K^T f is rmw_rigid_KT_mult.
+#include <algorithm>
 #include <cmath>
 
 #include "pair_math.cuh"
@@ -28,69 +35,147 @@ namespace {
 
 constexpr int kFThreads = 128;
 
-struct __align__(16) BlobPos {
-    double x, y, z, pad;
+// Pair lists of the FP64 work: kPend candidates per thread in shared memory,
+// evaluated together when some lane's list is full, so the lanes of a warp
+// work on different pairs instead of waiting for each other's.
+constexpr int kPend = 16;
+
+// FP32 coordinates relative to the CTA's first target (absolute if that is not
+// finite) in units of 2a + b, and the error bound of a distance to them: with
+// m = |x_i| + |x_j| + L, rounding coordinates, differences and image shifts
+// loses at most 6 2^-24 m per component, 6.2e-7 m in the distance, its sum and
+// root 1.6e-7 m, and an image chosen differently next to L/2 6.2e-7 m.
+constexpr float kErr = 2e-6f;
+
+struct Box {
+    double x, y, z;  // periodic lengths, 0 = none
+    float fx, fy, fz, ix, iy, iz, big;  // in units of 2a + b: the same, their inverses, the largest
+    float unit;      // 1 / (2a + b)
 };
 
-__global__ void __launch_bounds__(kFThreads) blob_blob_kernel(const double *__restrict__ r, double *__restrict__ f,
-                                                               int n, double eps_over_b, double inv_b,
-                                                               double two_a, double rc, double margin, double Lx,
-                                                               double Ly, double Lz, int accumulate)
+__device__ __forceinline__ float image_f(float d, float L, float inv) { return L > 0.f ? d - L * rintf(d * inv) : d; }
+
+struct Screen {
+    double x0[3];
+    float x, y, z;  // this thread's target
+    float ext;      // largest |coordinate| of the CTA's targets
+};
+
+__device__ __forceinline__ Screen screen_setup(const double *__restrict__ r, int n, const Box &L, unsigned *bits)
 {
-    __shared__ BlobPos tile[kFThreads];
-    __shared__ float4 tilef[kFThreads];
-    __shared__ double x0[3];
-    __shared__ unsigned ext_bits;
-    const int i = blockIdx.x * kFThreads + threadIdx.x;
-    const bool valid = i < n;
-    if (threadIdx.x == 0) {
-        const int i0 = blockIdx.x * kFThreads;
-        x0[0] = r[3 * i0];
-        x0[1] = r[3 * i0 + 1];
-        x0[2] = r[3 * i0 + 2];
-        ext_bits = 0u;
+    Screen s;
+    const int i0 = blockIdx.x * kFThreads, i = min(i0 + (int)threadIdx.x, n - 1);
+    if (threadIdx.x == 0) *bits = 0u;
+    for (int c = 0; c < 3; ++c) {
+        s.x0[c] = r[3 * i0 + c];
+        if (!isfinite(s.x0[c])) s.x0[c] = 0.0;
     }
     __syncthreads();
-    const double xi = valid ? r[3 * i] : x0[0], yi = valid ? r[3 * i + 1] : x0[1], zi = valid ? r[3 * i + 2] : x0[2];
-    // target coordinates relative to the CTA's first target, in FP32
-    const float xf = (float)(xi - x0[0]), yf = (float)(yi - x0[1]), zf = (float)(zi - x0[2]);
-    atomicMax(&ext_bits, __float_as_uint(fmaxf(fabsf(xf), fmaxf(fabsf(yf), fabsf(zf)))));
+    s.x = (float)(r[3 * i] - s.x0[0]) * L.unit;
+    s.y = (float)(r[3 * i + 1] - s.x0[1]) * L.unit;
+    s.z = (float)(r[3 * i + 2] - s.x0[2]) * L.unit;
+    atomicMax(bits, __float_as_uint(fmaxf(fabsf(s.x), fmaxf(fabsf(s.y), fabsf(s.z)))));
     __syncthreads();
-    // FP32 screen only where its error provably stays below the margin:
-    // |error of the FP32 distance| <= 2^-22 sqrt(3) (rc + 2 extent + max L)
-    const double ext = (double)__uint_as_float(ext_bits);
-    const double Lm = fmax(Lx, fmax(Ly, Lz));
-    const bool screen32 = 4.2e-7 * (rc + 2.0 * ext + Lm) < margin;
-    const float cut2 = (float)((rc + margin) * (rc + margin));
-    const float Lxf = (float)Lx, Lyf = (float)Ly, Lzf = (float)Lz;
-    double fx = 0.0, fy = 0.0, fz = 0.0;
-    for (int t0 = 0; t0 < n; t0 += kFThreads) {
-        const int cnt = min(kFThreads, n - t0);
+    s.ext = __uint_as_float(*bits);
+    return s;
+}
+
+// source tile: FP32 coordinates and the error bound of distances to them (w)
+__device__ __forceinline__ void screen_tile(const double *__restrict__ r, const Screen &s, const Box &L, int j, int j1,
+                                            float4 *tile)
+{
+    if (j < j1) {
+        const float x = (float)(r[3 * (size_t)j] - s.x0[0]) * L.unit,
+                    y = (float)(r[3 * (size_t)j + 1] - s.x0[1]) * L.unit,
+                    z = (float)(r[3 * (size_t)j + 2] - s.x0[2]) * L.unit;
+        tile[threadIdx.x] =
+            make_float4(x, y, z, kErr * (fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z))) + s.ext + L.big));
+    }
+}
+
+template <bool PER>
+__device__ __forceinline__ float screen_r2(const Screen &s, const Box &L, float4 q)
+{
+    float ex = q.x - s.x, ey = q.y - s.y, ez = q.z - s.z;
+    if (PER) {
+        ex = image_f(ex, L.fx, L.ix);
+        ey = image_f(ey, L.fy, L.iy);
+        ez = image_f(ez, L.fz, L.iz);
+    }
+    return fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+}
+
+// nearest[i] = min over this CTA's sources of an upper bound on the distance
+// to blob i (bit pattern of a positive float: atomicMin keeps it independent
+// of the order); blobs that may coincide with i, which exert no force, do not
+// count.
+template <bool PER>
+__global__ void __launch_bounds__(kFThreads) nearest_kernel(const double *__restrict__ r, int n, int chunk, Box L,
+                                                             unsigned *__restrict__ nearest)
+{
+    __shared__ float4 tile[kFThreads];
+    __shared__ unsigned bits;
+    const Screen s = screen_setup(r, n, L, &bits);
+    const int i = blockIdx.x * kFThreads + threadIdx.x;
+    const int j0 = blockIdx.y * chunk, j1 = min(n, j0 + chunk);
+    float best = 3.0e38f, err = 0.f;
+    for (int t0 = j0; t0 < j1; t0 += kFThreads) {
         __syncthreads();
-        if (threadIdx.x < cnt) {
-            const int j = t0 + threadIdx.x;
-            const BlobPos p = {r[3 * j], r[3 * j + 1], r[3 * j + 2], 0.0};
-            tile[threadIdx.x] = p;
-            tilef[threadIdx.x] =
-                make_float4((float)(p.x - x0[0]), (float)(p.y - x0[1]), (float)(p.z - x0[2]), 0.f);
-        }
+        screen_tile(r, s, L, t0 + threadIdx.x, j1, tile);
         __syncthreads();
-        if (!valid) continue;
+        const int cnt = min(kFThreads, j1 - t0);
+#pragma unroll 4
         for (int k = 0; k < cnt; ++k) {
-            const int j = t0 + k;
-            if (screen32) {
-                const float4 q = tilef[k];
-                float ex = q.x - xf, ey = q.y - yf, ez = q.z - zf;
-                if (Lxf > 0.f) ex = project(ex, Lxf);
-                if (Lyf > 0.f) ey = project(ey, Lyf);
-                if (Lzf > 0.f) ez = project(ez, Lzf);
-                if (ex * ex + ey * ey + ez * ez >= cut2) continue;
+            const float4 q = tile[k];
+            const float r2 = screen_r2<PER>(s, L, q);
+            if (r2 < best && r2 > q.w * q.w) {
+                best = r2;
+                err = q.w;
             }
-            if (j == i) continue;
-            double dx = tile[k].x - xi, dy = tile[k].y - yi, dz = tile[k].z - zi;
-            if (Lx > 0) dx = project(dx, Lx);
-            if (Ly > 0) dy = project(dy, Ly);
-            if (Lz > 0) dz = project(dz, Lz);
+        }
+    }
+    if (i < n && best < 3.0e38f) atomicMin(&nearest[i], __float_as_uint(fmaf(sqrtf(best), 1.0f + 1e-6f, err)));
+}
+
+// f_i over this CTA's sources: FP32 distances pick the candidates (nearest !=
+// NULL: within max(2a, r_min) + reach; always within rc = rcut units), FP64
+// evaluates them.
+// Partial sums to part[blockIdx.y][3n], or (part = NULL, one chunk) straight to f.
+template <bool PER>
+__global__ void __launch_bounds__(kFThreads) blob_blob_kernel(const double *__restrict__ r, double *__restrict__ f,
+                                                               double *__restrict__ part, int n, int chunk,
+                                                               double eps_over_b, double inv_b, double two_a,
+                                                               double rc, float rcut,
+                                                               const unsigned *__restrict__ nearest, float reach,
+                                                               Box L, int accumulate)
+{
+    __shared__ float4 tile[kFThreads];
+    __shared__ int pend[kPend][kFThreads];
+    __shared__ unsigned bits;
+    const Screen s = screen_setup(r, n, L, &bits);
+    const int tid = threadIdx.x, i = blockIdx.x * kFThreads + tid;
+    const bool valid = i < n;
+    const int ii = valid ? i : n - 1;
+    const double xi = r[3 * (size_t)ii], yi = r[3 * (size_t)ii + 1], zi = r[3 * (size_t)ii + 2];
+    // (a bound FP32 cannot hold: no screen, every pair is a candidate)
+    float cut = rcut < 1e15f ? rcut : __int_as_float(0x7fffffff);
+    if (nearest) {
+        const float near = __uint_as_float(nearest[ii]);
+        if (near < 1e15f) cut = fminf(cut, (fmaxf((float)two_a * L.unit, near) + reach) * (1.0f + 1e-6f));
+    }
+    if (!valid) cut = -1e30f;  // no candidate
+    double fx = 0.0, fy = 0.0, fz = 0.0;
+    int np = 0;
+    auto drain = [&]() {  // every lane works off its list
+        for (int k = 0; __any_sync(0xffffffffu, k < np); ++k) {
+            if (k >= np) continue;
+            const size_t j = pend[k][tid];
+            double dx = r[3 * j] - xi, dy = r[3 * j + 1] - yi, dz = r[3 * j + 2] - zi;
+            if (PER) {
+                if (L.x > 0) dx = project(dx, L.x);
+                if (L.y > 0) dy = project(dy, L.y);
+                if (L.z > 0) dz = project(dz, L.z);
+            }
             const double rn = sqrt(dx * dx + dy * dy + dz * dz);
             if (!(rn > 0.0) || rn > rc) continue;  // coincident: no direction; beyond rc: exactly zero
             const double g = (rn > two_a) ? exp(-(rn - two_a) * inv_b) : 1.0;
@@ -99,18 +184,49 @@ __global__ void __launch_bounds__(kFThreads) blob_blob_kernel(const double *__re
             fy -= m * dy;
             fz -= m * dz;
         }
-    }
-    if (valid) {
-        if (accumulate) {
-            f[3 * i] += fx;
-            f[3 * i + 1] += fy;
-            f[3 * i + 2] += fz;
-        } else {
-            f[3 * i] = fx;
-            f[3 * i + 1] = fy;
-            f[3 * i + 2] = fz;
+        np = 0;
+    };
+    const int j0 = blockIdx.y * chunk, j1 = min(n, j0 + chunk);
+    for (int t0 = j0; t0 < j1; t0 += kFThreads) {
+        __syncthreads();
+        screen_tile(r, s, L, t0 + tid, j1, tile);
+        __syncthreads();
+        const int cnt = min(kFThreads, j1 - t0);
+        for (int k0 = 0; k0 < cnt; k0 += kPend / 2) {
+            const int k1 = min(cnt, k0 + kPend / 2);
+            for (int k = k0; k < k1; ++k) {
+                const float4 q = tile[k];
+                const float t = cut + q.w;
+                if (!(screen_r2<PER>(s, L, q) >= t * fabsf(t)) && t0 + k != i) pend[np++][tid] = t0 + k;
+            }
+            if (__any_sync(0xffffffffu, np > kPend / 2)) drain();
         }
     }
+    drain();
+    if (!valid) return;
+    if (part) {
+        double *o = part + ((size_t)blockIdx.y * n + i) * 3;
+        o[0] = fx; o[1] = fy; o[2] = fz;
+    } else if (accumulate) {
+        f[3 * (size_t)i] += fx;
+        f[3 * (size_t)i + 1] += fy;
+        f[3 * (size_t)i + 2] += fz;
+    } else {
+        f[3 * (size_t)i] = fx;
+        f[3 * (size_t)i + 1] = fy;
+        f[3 * (size_t)i + 2] = fz;
+    }
+}
+
+__global__ void force_sum_kernel(const double *__restrict__ part, double *__restrict__ f, int m, int nchunks,
+                                 int accumulate)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= m) return;
+    double v = 0.0;
+#pragma unroll 8
+    for (int c = 0; c < nchunks; ++c) v += part[(size_t)c * m + k];
+    f[k] = accumulate ? f[k] + v : v;
 }
 
 __global__ void external_force_kernel(const double *__restrict__ r, double *__restrict__ f, int n, double weight,
@@ -129,7 +245,55 @@ __global__ void external_force_kernel(const double *__restrict__ r, double *__re
     }
 }
 
+template <bool PER>
+int blob_blob_launch(const double *r, double *f, int n, double eps_over_b, double b, double two_a, double rc,
+                     const Box &L, int accumulate, cudaStream_t st)
+{
+    const int tiles = (n + kFThreads - 1) / kFThreads;
+    // enough CTAs for eight per SM, no chunk below two tiles of sources
+    const int want = std::min((152 * 8 + tiles - 1) / tiles, std::max(1, n / (2 * kFThreads)));
+    const int chunk = (((n + want - 1) / want + kFThreads - 1) / kFThreads) * kFThreads;
+    const int nchunks = (n + chunk - 1) / chunk;
+    const size_t head = ((sizeof(unsigned) * (size_t)n + 255) / 256) * 256;
+    const size_t bytes = head + (nchunks > 1 ? sizeof(double) * 3 * (size_t)n * nchunks : 0);
+    // Without scratch (a capture must not allocate; a scratch limit; memory
+    // pressure) one chunk and the fixed radius: same pairs to rounding, slower.
+    const float rcut = (float)(rc / (two_a + b) * 1.000001);
+    void *ws = nullptr;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
+        scratch(SCRATCH_FORCES, bytes, &ws, st) != RMW_OK) {
+        cudaGetLastError();
+        blob_blob_kernel<PER><<<tiles, kFThreads, 0, st>>>(r, f, nullptr, n, n, eps_over_b, 1.0 / b, two_a, rc, rcut,
+                                                           nullptr, 0.f, L, accumulate);
+        RMW_CHECK_LAUNCH("blob-blob forces");
+        return RMW_OK;
+    }
+    unsigned *nearest = (unsigned *)ws;
+    double *part = nchunks > 1 ? (double *)((char *)ws + head) : nullptr;
+    const dim3 grid(tiles, nchunks);
+    RMW_CUDA(cudaMemsetAsync(nearest, 0x7f, sizeof(unsigned) * (size_t)n, st));  // 3.4e38
+    nearest_kernel<PER><<<grid, kFThreads, 0, st>>>(r, n, chunk, L, nearest);
+    const float reach = (float)(b / (two_a + b) * (65.0 * 0.69314718055994531 + std::log((double)n)) * 1.000001);
+    blob_blob_kernel<PER><<<grid, kFThreads, 0, st>>>(r, f, part, n, chunk, eps_over_b, 1.0 / b, two_a, rc, rcut,
+                                                      nearest, reach, L, accumulate);
+    if (part) force_sum_kernel<<<(3 * n + 255) / 256, 256, 0, st>>>(part, f, 3 * n, nchunks, accumulate);
+    RMW_CHECK_LAUNCH("blob-blob forces");
+    return RMW_OK;
+}
+
 }  // namespace
+
+static int blob_blob(const double *r, double *f, int n, double eps_over_b, double b, double two_a, double rc, double Lx,
+                     double Ly, double Lz, int accumulate, cudaStream_t st)
+{
+    const double unit = 1.0 / (two_a + b);
+    auto inv = [unit](double L) { return L > 0 ? (float)(1.0 / (L * unit)) : 0.f; };
+    const Box L = {Lx, Ly, Lz, (float)(Lx * unit), (float)(Ly * unit), (float)(Lz * unit), inv(Lx), inv(Ly), inv(Lz),
+                   (float)(unit * std::max(0.0, std::max(Lx, std::max(Ly, Lz)))), (float)unit};
+    if (Lx > 0 || Ly > 0 || Lz > 0) return blob_blob_launch<true>(r, f, n, eps_over_b, b, two_a, rc, L, accumulate, st);
+    return blob_blob_launch<false>(r, f, n, eps_over_b, b, two_a, rc, L, accumulate, st);
+}
 
 }  // namespace rmw
 
@@ -148,18 +312,12 @@ int rmw_blob_blob_forces(const double *r, double *f, int64_t n, double repulsion
     const double Lx = L_host ? L_host[0] : 0.0, Ly = L_host ? L_host[1] : 0.0, Lz = L_host ? L_host[2] : 0.0;
     // beyond 2a + 746 b the FP64 exponential is exactly zero: such pairs
     // contribute nothing; a positive cutoff truncates earlier (pairs farther
-    // than it are left out, as the reference's neighbour-list variant does);
-    // the FP32 screen tests against rc + margin
+    // than it are left out, as the reference's neighbour-list variant does)
     const double rexact = 2.0 * blob_radius + 746.0 * debye_length;
     const double rc = (cutoff > 0.0) ? fmin(cutoff, rexact) : rexact;
-    const double margin = 1e-3 * rc + 1e-6;
     const int N = (int)n;
-    cudaStream_t st = rmw::as_stream(stream);
-    rmw::blob_blob_kernel<<<(N + rmw::kFThreads - 1) / rmw::kFThreads, rmw::kFThreads, 0, st>>>(
-        r, f, N, repulsion_strength / debye_length, 1.0 / debye_length, 2.0 * blob_radius, rc, margin, Lx, Ly, Lz,
-        accumulate);
-    RMW_CHECK_LAUNCH("blob-blob forces");
-    return RMW_OK;
+    return rmw::blob_blob(r, f, N, repulsion_strength / debye_length, debye_length, 2.0 * blob_radius, rc, Lx, Ly, Lz,
+                          accumulate, rmw::as_stream(stream));
 }
 
 // f (+)= gravity and wall repulsion of n blobs (device arrays, 3n doubles).

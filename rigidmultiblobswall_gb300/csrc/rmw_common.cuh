@@ -30,7 +30,7 @@ int cuda_fail(cudaError_t e, const char *where);
 // device, stream and slot share it (they are ordered by the stream); a call that
 // needs more frees the old buffer (cudaFree synchronises the device, so no
 // kernel still reads it) and allocates anew.
-enum ScratchSlot { SCRATCH_PAIR = 0, SCRATCH_HOST_STAGING = 1, SCRATCH_FT_TERM = 2, SCRATCH_SLOTS = 3 };
+enum ScratchSlot { SCRATCH_PAIR = 0, SCRATCH_HOST_STAGING = 1, SCRATCH_FT_TERM = 2, SCRATCH_FORCES = 3, SCRATCH_SLOTS = 4 };
 int scratch(ScratchSlot slot, size_t bytes, void **ptr, cudaStream_t st);
 // frees the current device's scratch buffers (deferred while graphs are alive)
 int scratch_release_all();
