@@ -205,6 +205,7 @@ __device__ __forceinline__ void uf_apply(const UFCoeffs<T> &c, T dx, T dy, T dz,
 // the scalar form came out as in every second step of an unrolled loop.
 struct UFCoeffs2 {
     f2 Af, Bc, c2, c3, c4, Af5;
+    f2 g, u;  // c2 = g u
 };
 __device__ __forceinline__ f2 f2_c(float a, f2 b, f2 c) { return f2_fma(f2_dup(a), b, c); }  // a b + c
 __device__ __forceinline__ f2 f2_c(float a, f2 b, float c) { return f2_fma(f2_dup(a), b, f2_dup(c)); }
@@ -252,6 +253,8 @@ __device__ __forceinline__ UFCoeffs2 uf_coeffs_f2(f2 dx, f2 dy, f2 dz, f2 Rz, f2
     c.c3 = f2_fma(Ru, in, f2_fma(f2_neg(f2_mul(f2_s(18.0f, hh), Rz)), t, hjt3));
     c.c4 = f2_fma(f2_neg(f2_s(10.0f, Ru)), p, hjt3);
     c.Af5 = f2_c(-2.0f, f5, c.Af);
+    c.g = f2c;
+    c.u = u;
     return c;
 }
 
@@ -274,35 +277,28 @@ __device__ __forceinline__ void uf_apply_f2(const UFCoeffs2 &c, f2 c3, f2 c4, f2
 //   M = Af I + Bc d d^T + c2 e e^T + c3 e z^T + c4 z e^T + f5 z z^T,
 // so M_xy = M_yx = (Bc + c2) dx dy, M_xz = dx t3, M_zx = dx t4 with
 // t3,4 = Bc dz + c2 Rz + c3,4, and M_zz = Af + f5 + Bc dz^2 + (c2 Rz + c3 + c4) Rz.
-struct UFBlock {
-    float xx, xy, xz, yy, yz, zx, zy, zz;  // M_yx = M_xy
+// Two pairs (sources) in packed lanes; Bc + c2 with c2's product fused into it.
+struct UFBlock2 {
+    f2 xx, xy, xz, yy, yz, zx, zy, zz;  // M_yx = M_xy
 };
 
-__device__ __forceinline__ UFBlock uf_block_f(const UFCoeffs<float> &c, float dx, float dy, float dz, float Rz)
+template <bool FUSED_B>
+__device__ __forceinline__ UFBlock2 uf_block_f2(const UFCoeffs2 &c, f2 dx, f2 dy, f2 dz, f2 Rz)
 {
-    const float b2 = c.Bc + c.c2;
-    const float t = fmaf(c.Bc, dz, c.c2 * Rz);
-    const float t3 = t + c.c3, t4 = t + c.c4;
-    const float px = b2 * dx;
-    UFBlock m;
-    m.xx = fmaf(px, dx, c.Af);
-    m.xy = px * dy;
-    m.yy = fmaf(b2 * dy, dy, c.Af);
-    m.xz = dx * t3;
-    m.yz = dy * t3;
-    m.zx = dx * t4;
-    m.zy = dy * t4;
-    m.zz = fmaf(fmaf(c.c2, Rz, c.c3 + c.c4), Rz, fmaf(c.Bc * dz, dz, c.Af5));
+    const f2 b2 = FUSED_B ? f2_fma(c.g, c.u, c.Bc) : f2_add(c.Bc, f2_mulr(c.g, c.u));
+    const f2 t = f2_fma(c.Bc, dz, f2_mul(c.c2, Rz));
+    const f2 t3 = f2_add(t, c.c3), t4 = f2_add(t, c.c4);
+    const f2 px = f2_mul(b2, dx);
+    UFBlock2 m;
+    m.xx = f2_fma(px, dx, c.Af);
+    m.xy = f2_mul(px, dy);
+    m.yy = f2_fma(f2_mul(b2, dy), dy, c.Af);
+    m.xz = f2_mul(dx, t3);
+    m.yz = f2_mul(dy, t3);
+    m.zx = f2_mul(dx, t4);
+    m.zy = f2_mul(dy, t4);
+    m.zz = f2_fma(f2_fma(c.c2, Rz, f2_add(c.c3, c.c4)), Rz, f2_fma(f2_mul(c.Bc, dz), dz, c.Af5));
     return m;
-}
-
-// (ux, uy, uz) += M v
-__device__ __forceinline__ void uf_block_apply(const UFBlock &m, float vx, float vy, float vz, float &ux, float &uy,
-                                               float &uz)
-{
-    ux = fmaf(m.xx, vx, fmaf(m.xy, vy, fmaf(m.xz, vz, ux)));
-    uy = fmaf(m.xy, vx, fmaf(m.yy, vy, fmaf(m.yz, vz, uy)));
-    uz = fmaf(m.zx, vx, fmaf(m.zy, vy, fmaf(m.zz, vz, uz)));
 }
 
 // FP32: every term chained into the accumulator by an FMA (two plain
