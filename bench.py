@@ -58,12 +58,12 @@ NF_ALL_EXACT_R = NF_CUTOFF_R
 # kernel changes without a new capture).
 DF64_UF_INST_PER_PAIR = {"symmetric": 1088175303.0 * 32 / 10752 ** 2, "standard": 1804026278.0 * 32 / 10752 ** 2}
 # dram__bytes_read.sum + dram__bytes_write.sum per launch, same captures
-DF64_UF_TRAFFIC_BYTES = {"symmetric": 745984, "standard": 710400}
+DF64_UF_TRAFFIC_BYTES = {"symmetric": 745472, "standard": 794624}
 # FP32-issue slots per pair and right-hand side of the 16-wide multi-RHS M_UF kernel, packed instructions
 # counted twice as above ((smsp__inst_executed.sum 17,258,189,476 + packed 12,838,677,918) * 32 / (N^2 * 16),
 # 60,000 blobs)
 MULTI16_INST_PER_PAIR_RHS = 16.72
-DF64_UF_KERNEL_SOURCE_SHA = "096f6c6225bad29d3e319cf2687b42159783d90f2bd028164d24570c0a4a7064"
+DF64_UF_KERNEL_SOURCE_SHA = "9f4e60b55215de2cf1365c2b6d03868d0daabff7b6ec8eab58923e465a7eae13"
 
 
 def df64_uf_kernel_source_sha():

@@ -150,6 +150,25 @@ __device__ __forceinline__ void acc_dot2(df2 &acc, df2 a, df2 b, df2 c, df2 d)
     acc.lo = f2_add(acc.lo, f2_add(f2_add(t1.lo, t2.lo), f2_add(p.lo, q.lo)));
 }
 
+// acc += a b (+ c d + e f) without renormalising acc
+__device__ __forceinline__ void acc_dot1(df2 &acc, df2 a, df2 b)
+{
+    const df2 p = mul_u(a, b);
+    const df2 t = two_sum_df(acc.hi, p.hi);
+    acc.hi = t.hi;
+    acc.lo = f2_add(acc.lo, f2_add(t.lo, p.lo));
+}
+__device__ __forceinline__ void acc_dot3(df2 &acc, df2 a, df2 b, df2 c, df2 d, df2 e, df2 f)
+{
+    const df2 p = mul_u(a, b), q = mul_u(c, d), r = mul_u(e, f);
+    const df2 t1 = two_sum_df(acc.hi, p.hi);
+    const df2 t2 = two_sum_df(t1.hi, q.hi);
+    const df2 t3 = two_sum_df(t2.hi, r.hi);
+    acc.hi = t3.hi;
+    const f2 lo = f2_add(f2_add(t1.lo, t2.lo), t3.lo);
+    acc.lo = f2_add(acc.lo, f2_add(lo, f2_add(f2_add(p.lo, q.lo), r.lo)));
+}
+
 // 1/sqrt(x) from the estimate y, as rsqrt_df
 __device__ __forceinline__ df2 rsqrt_df(df2 x, f2 y)
 {

@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(kNwThreads) nw_pair_df_kernel(const NwSrcDF *_
 constexpr int kNwFinGroup = 16;
 template <bool DF2 = false>
 __global__ void nw_finalize_kernel(const double *__restrict__ v, const double *__restrict__ partial, int nchunks,
-                                   double *__restrict__ out, int n, double self_coef, double nf)
+                                   double *__restrict__ out, int n, double self_coef, double nf, double pair_scale)
 {
     const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int i = (int)(DF2 ? gt : gt / kNwFinGroup), g = DF2 ? 0 : (int)(gt % kNwFinGroup);
@@ -271,7 +271,7 @@ __global__ void nw_finalize_kernel(const double *__restrict__ v, const double *_
             for (int c = 0; c < 3; ++c) u[c] += __shfl_down_sync(0xffffffffu, u[c], o, kNwFinGroup);
         if (i >= n || g != 0) return;
     }
-    for (int c = 0; c < 3; ++c) out[3 * i + c] = nf * (u[c] + self_coef * v[3 * i + c]);
+    for (int c = 0; c < 3; ++c) out[3 * i + c] = nf * (pair_scale * u[c] + self_coef * v[3 * i + c]);
 }
 
 template <int KIND, bool PER>
@@ -349,11 +349,13 @@ int nowall_product(int kind, const double *r, const double *v, double *out, int6
     const double p = (kind == RMW_UF) ? a : (kind == RMW_WT ? a * a * a : a * a);
     const double self_coef = (kind == RMW_UF) ? 4.0 / 3.0 : (kind == RMW_WT ? 1.0 : 0.0);
     if (sym && mode == RMW_MODE_MIXED)
-        nw_finalize_kernel<true><<<pg, pb, 0, st>>>(v, partial, nchunks, out, N, self_coef, 1.0 / (8.0 * kPi * eta * p));
+        nw_finalize_kernel<true><<<pg, pb, 0, st>>>(v, partial, nchunks, out, N, self_coef, 1.0 / (8.0 * kPi * eta * p),
+                                                    1.0);
     else
         nw_finalize_kernel<false><<<(unsigned)(((long long)kNwFinGroup * N + pb - 1) / pb), pb, 0, st>>>(
-            v, partial, nchunks, out, N, self_coef,
-                                                     1.0 / (8.0 * kPi * eta * p));
+            v, partial, nchunks, out, N, self_coef, 1.0 / (8.0 * kPi * eta * p),
+            // the symmetric df64 UF kernel sums (3/2) M v
+            sym && mode == RMW_MODE_DF64 && kind == RMW_UF ? 2.0 / 3.0 : 1.0);
     RMW_CHECK_LAUNCH("free-space product kernels");
     return RMW_OK;
 }

@@ -7,9 +7,22 @@
 
 namespace rmw {
 
+// 1/sqrt(x) in FP64: the hardware's estimate (relative error below 2^-20) and
+// one third-order Householder step, y + y e (1/2 + 3 e / 8) with
+// e = 1 - x y^2: five FP64 instructions and no special-case branch (zero,
+// infinite and subnormal x give non-finite values; no pair of distinct blobs
+// has one).
+__device__ __forceinline__ double rsqrt64(double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y * y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
 // pair math.  (dx,dy,dz) = (r_i - r_j)/a; Rz = (z_i + z_j)/a; hi = z_i/a; hj = z_j/a.
 template <typename T> __device__ __forceinline__ T rsq(T x);
-template <> __device__ __forceinline__ double rsq<double>(double x) { return rsqrt(x); }
+template <> __device__ __forceinline__ double rsq<double>(double x) { return rsqrt64(x); }
 template <> __device__ __forceinline__ float rsq<float>(float x) { return rsqrt_approx(x); }
 
 // The reference builds each 3x3 block from unit vectors e = (dx, dy, Rz)/R and
@@ -319,19 +332,6 @@ __device__ __forceinline__ void uf_apply<float>(const UFCoeffs<float> &c, float 
     uz = fmaf(c.Af5, vz, fmaf(G, dz, fmaf(Gw, h2, fmaf(c.c4, W, uz))));
 }
 
-// 1/sqrt(x) in FP64: the hardware's estimate (relative error below 2^-20) and
-// one third-order Householder step, y + y e (1/2 + 3 e / 8) with
-// e = 1 - x y^2: five FP64 instructions and no special-case branch (zero,
-// infinite and subnormal x give non-finite values; no pair of distinct blobs
-// has one).
-__device__ __forceinline__ double rsqrt64(double x)
-{
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y * y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
 // The explicit M_UF block in FP64, times 3/2: the formulas of uf_block_df
 // (pair_math_df.cuh), where they are derived.  73 FP64 instructions a pair,
 // both ways, against 93 of uf_coeffs / uf_apply: the FP64 pipe bounds the
@@ -397,12 +397,75 @@ __device__ __forceinline__ void uf_block_acc_d(const UFBlockD &m, double t3, dou
     uz = fma(t4, P, fma(m.zz, vz, uz));
 }
 
+// UT, WF and WT for both orders of a pair in FP64, the formulas of
+// rot_block_df and wt_block_df (pair_math_df.cuh), where they are derived: 64
+// (UT, WF) and 62 (WT) FP64 instructions a pair against 91 and 74 of the
+// tensor forms.  10,752 blobs: UT 9.82 -> 7.01 ms, WF 9.97 -> 7.01, WT 8.08 ->
+// 7.06.
+template <int KIND>
+__device__ __forceinline__ void pair_rot_sym_d(double dx, double dy, double dz, double Rz, double hi, double hj,
+                                               double vx, double vy, double vz, double qx, double qy, double qz,
+                                               double &ux, double &uy, double &uz, double &wx, double &wy, double &wz)
+{
+    const double r2 = fma(dz, dz, fma(dx, dx, dy * dy));
+    const double invr = rsqrt64(r2);
+    const double s = rsqrt64(fma(4.0 * hi, hj, r2));
+    const double i2 = invr * invr, u = s * s, t = u * s, p = t * u;
+    const bool near = !(r2 >= 4.0);  // r < 2
+    if constexpr (KIND == RMW_WT) {
+        const double i3 = i2 * invr;
+        double A = -0.5 * i3, Bc = 1.5 * i2 * i3;
+        if (__any_sync(__activemask(), near)) {
+            if (near) {
+                const double r = r2 * invr;
+                A = fma(fma(0.078125, r2, -0.84375), r, 1.0);
+                Bc = fma(-0.046875, r, 0.28125 * invr);
+            }
+        }
+        const double Et = Rz * Rz * u * t, D = Bc * dz, X = 1.5 * p * Rz;
+        UFBlockD m;
+        m.Af = fma(-6.0, Et, fma(3.5, t, A));
+        m.b2 = fma(-4.5, p, Bc);
+        m.t3 = D - X;
+        m.t4 = D + X;
+        m.zz = fma(D, dz, fma(-1.5, Et, fma(0.5, t, A)));
+        uf_block_acc_d(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
+        uf_block_acc_d(m, m.t4, m.t3, dx, dy, qx, qy, qz, wx, wy, wz);
+    } else {
+        double c = i2 * invr;
+        if (__any_sync(__activemask(), near)) {
+            if (near) c = fma(-0.1875, r2 * invr, 0.5);
+        }
+        const double b = t - c, m = dz * b, Rp = Rz * p, a = fma(2.0, Rp, -m), ar = fma(2.0, Rp, m);
+        const double Ru = Rz * u, R10 = 10.0 * Ru, R6 = 6.0 * Rz, y = fma(-10.0 * Rz, Ru, 2.0);
+        const double ei = p * fma(-6.0, hi, R10), ej = p * fma(-6.0, hj, R10);
+        const double wi = fma(p, fma(R6, hi, y), b), wj = fma(p, fma(R6, hj, y), b);
+        const double Q = fma(dy, vx, -dx * vy), Qq = fma(dy, qx, -dx * qy);
+        if constexpr (KIND == RMW_UT) {
+            const double bv = b * vz, eQ = ei * Q, bq = b * qz, eq = ej * Qq;
+            ux = fma(a, vy, fma(bv, dy, fma(eQ, dx, ux)));
+            uy = fma(-a, vx, fma(-bv, dx, fma(eQ, dy, uy)));
+            uz = fma(-wi, Q, uz);
+            wx = fma(ar, qy, fma(-bq, dy, fma(eq, dx, wx)));
+            wy = fma(-ar, qx, fma(bq, dx, fma(eq, dy, wy)));
+            wz = fma(wj, Qq, wz);
+        } else {
+            const double H = fma(ej, fma(dy, vy, dx * vx), wj * vz), Hq = fma(ei, fma(dy, qy, dx * qx), -wi * qz);
+            ux = fma(-ar, vy, fma(H, dy, ux));
+            uy = fma(ar, vx, fma(-H, dx, uy));
+            uz = fma(-b, Q, uz);
+            wx = fma(-a, qy, fma(Hq, dy, wx));
+            wy = fma(a, qx, fma(-Hq, dx, wy));
+            wz = fma(b, Qq, wz);
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
-// Symmetric forms of the rotation blocks in FP32 and FP64 (the double-float
-// forms are pair_rot_sym_df): M_ji is the M_ij formula with d -> -d and
-// h_i <-> h_j, so one pair evaluation serves both targets.  WT has no height
-// dependence; UT and WF form the height-dependent coefficients for both
-// heights.
+// Symmetric forms of the rotation blocks in FP32: M_ji is the M_ij formula
+// with d -> -d and h_i <-> h_j, so one pair evaluation serves both targets.
+// WT has no height dependence; UT and WF form the height-dependent
+// coefficients for both heights.
 template <typename T> __device__ __forceinline__ T fm(T a, T b, T c);
 template <> __device__ __forceinline__ float fm<float>(float a, float b, float c) { return fmaf(a, b, c); }
 template <> __device__ __forceinline__ double fm<double>(double a, double b, double c) { return fma(a, b, c); }

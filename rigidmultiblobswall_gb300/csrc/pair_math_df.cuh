@@ -368,57 +368,183 @@ __device__ __forceinline__ void wt_apply_df(df Af, df Bc, df s5, df dx, df dy, d
     acc_dot3(uz, Af, vz, Gr, dz, Gw, -Rz);
 }
 
-// UT, WF or WT for both orders of one pair: (ux, uy, uz) += M_ij v_j for
-// target i, (wx, wy, wz) += M_ji v_i for target j.
-template <int KIND>
-__device__ __forceinline__ void pair_rot_sym_df(df dx, df dy, df dz, df Rz, df hi, df hj, df vx, df vy, df vz,
-                                                df qx, df qy, df qz, df &ux, df &uy, df &uz, df &wx, df &wy,
-                                                df &wz)
+// UT, WF and WT for both orders of a pair, two pairs in packed lanes.  With
+// t = s^3, p = s^5, c the RPY factor (1/r^3, or (1 - 3r/8)/2 below 2),
+// b = t - c, m = dz b, n = 2 Rz p and the two heights' coefficients
+//   e_h = p (10 Rz u - 6 h),  W_h = b + p (2 - 10 E + 6 h Rz),
+// the wall terms fold into a = n - m and a' = n + m (the heights' parts of
+// s^2 ez + f4 are -dz t and +dz t, because Rz - 2 h_i = -dz), so that
+//   UT_ij v = (a vy + b vz dy + e_i Q dx, -a vx - b vz dx + e_i Q dy, -W_i Q)
+//   WF_ij v = (-a' vy + H dy, a' vx - H dx, -b Q),  H = e_j P + W_j vz
+// with P = dx vx + dy vy, Q = dy vx - dx vy; the reverse blocks take the other
+// height and a <-> a' with the signs of d.  WT, with the identity
+// rho rho^T + rho' rho'^T = rho^2 I, has the five scalars of a UF block:
+//   Af = A + 7t/2 - 6 E t,  b2 = Bc - 9p/2,  t3,4 = Bc dz -+ 3/2 p Rz,
+//   zz = A + t/2 - 3/2 E t + Bc dz^2     (A = -1/(2 r^3), Bc = 3/(2 r^5)).
+// About 500 FP32-pipe operations a pair against 720 (WT) and 840 (UT, WF) of
+// the tensor forms below.
+struct RotBlockDF2 {
+    df2 a, ar, b, ei, ej, wi, wj;
+};
+
+__device__ __forceinline__ void rot_near_c(df2 r2, df2 invr, df2 &c)
 {
-    const df rho2 = mad_u(dx, dx, sqr_u(dy));
-    const df r2 = mad(dz, dz, rho2);
-    const df invr = rsqrt_df(r2);
-    const df Rz2 = sqr(Rz);
-    const df s = rsqrt_df(rho2 + Rz2);
-    const df s2 = sqr(s);
-    const df s3 = s2 * s;
-    const df E = Rz2 * s2;
-    const bool near = !(r2 >= 4.0f);  // r < 2
-    if (KIND == RMW_WT) {
-        const df invr2 = sqr(invr);
-        const df invr3 = invr2 * invr;
-        df A = invr3 * -0.5f;
-        df Bc = (invr2 * invr3) * 1.5f;
-        if (__any_sync(__activemask(), near)) {
-            if (near) {
-                const df r = r2 * invr;
-                A = (1.0f - r * 0.84375f) + (r * r2) * 0.078125f;
-                Bc = invr * 0.28125f - r * 0.046875f;
-            }
+    const df xa = {r2.hi.x, r2.lo.x}, xb = {r2.hi.y, r2.lo.y};
+    const bool na = !(xa >= 4.0f), nb = !(xb >= 4.0f);  // r < 2
+    if (__any_sync(__activemask(), na || nb)) {
+        if (na) {
+            const df v = scale2(1.0f - (xa * df{invr.hi.x, invr.lo.x}) * 0.375f, 0.5f);
+            c.hi.x = v.hi; c.lo.x = v.lo;
         }
-        const df s5 = s3 * s2;
-        const df Af = A + scale2((1.0f - E * 6.0f) * s3, 0.5f);
-        wt_apply_df(Af, Bc, s5, dx, dy, dz, Rz, vx, vy, vz, ux, uy, uz);
-        wt_apply_df(Af, Bc, s5, -dx, -dy, -dz, Rz, qx, qy, qz, wx, wy, wz);
-    } else {
-        df c = sqr(invr) * invr;
-        if (__any_sync(__activemask(), near)) {
-            if (near) c = scale2(1.0f - (r2 * invr) * 0.375f, 0.5f);
-        }
-        const df s4 = sqr(s2);
-        const df ez = Rz * s;
-        const df ezs4 = ez * s4;
-        const df K = mul_u(1.0f - mul_u(E, 10.0f), s4);
-        const RotHDF Hi = rot_h_df(hi, s, s2, s3, ez, ezs4, K);
-        const RotHDF Hj = rot_h_df(hj, s, s2, s3, ez, ezs4, K);
-        if (KIND == RMW_UT) {
-            ut_apply_df(c, Hi, s3, dx, dy, dz, vx, vy, vz, ux, uy, uz);
-            ut_apply_df(c, Hj, s3, -dx, -dy, -dz, qx, qy, qz, wx, wy, wz);
-        } else {
-            wf_apply_df(c, Hj, s3, dx, dy, dz, vx, vy, vz, ux, uy, uz);
-            wf_apply_df(c, Hi, s3, -dx, -dy, -dz, qx, qy, qz, wx, wy, wz);
+        if (nb) {
+            const df v = scale2(1.0f - (xb * df{invr.hi.y, invr.lo.y}) * 0.375f, 0.5f);
+            c.hi.y = v.hi; c.lo.y = v.lo;
         }
     }
+}
+// r < 2: A = 1 - 27 r/32 + 5 r^3/64, Bc = 9/(32 r) - 3 r/64
+__device__ __forceinline__ void wt_near(df2 r2, df2 invr, df2 &A, df2 &Bc)
+{
+    const df xa = {r2.hi.x, r2.lo.x}, xb = {r2.hi.y, r2.lo.y};
+    const bool na = !(xa >= 4.0f), nb = !(xb >= 4.0f);
+    if (__any_sync(__activemask(), na || nb)) {
+        if (na) {
+            const df v = {invr.hi.x, invr.lo.x}, r = xa * v;
+            const df f = (1.0f - r * 0.84375f) + (r * xa) * 0.078125f, g = v * 0.28125f - r * 0.046875f;
+            A.hi.x = f.hi; A.lo.x = f.lo;
+            Bc.hi.x = g.hi; Bc.lo.x = g.lo;
+        }
+        if (nb) {
+            const df v = {invr.hi.y, invr.lo.y}, r = xb * v;
+            const df f = (1.0f - r * 0.84375f) + (r * xb) * 0.078125f, g = v * 0.28125f - r * 0.046875f;
+            A.hi.y = f.hi; A.lo.y = f.lo;
+            Bc.hi.y = g.hi; Bc.lo.y = g.lo;
+        }
+    }
+}
+
+// hi4 = 4 h_i
+__device__ __forceinline__ RotBlockDF2 rot_block_df(df2 dx, df2 dy, df2 dz, df2 Rz, df2 hi, df2 hi4, df2 hj)
+{
+    const df2 r2 = norm(add_u(sqr_u(dz), add_u(sqr_u(dx), sqr_u(dy))));
+    const df2 invr = rsqrt_df(r2);
+    const df2 s = rsqrt_far_df(norm(add_u(r2, mul_u(hi4, hj))));
+    df2 c = mul_u(sqr(invr), invr);
+    rot_near_c(r2, invr, c);
+    const df2 u = sqr(s);
+    const df2 t = mul_u(u, s);
+    const df2 p = mul_u(t, u);
+    const df2 Ru = mul_u(Rz, u);
+    const df2 y = add_u(mul_u(mul_u(Rz, Ru), -10.0f), df2_dup(df_from(2.0f)));
+    RotBlockDF2 k;
+    k.b = t - c;
+    const df2 m = mul_u(dz, k.b), n = scale2(mul_u(Rz, p), 2.0f);
+    k.a = sub_u(n, m);
+    k.ar = add_u(n, m);
+    const df2 R10 = mul_u(Ru, 10.0f), R6 = mul_u(Rz, 6.0f);
+    k.ei = mul_u(p, sub_u(R10, mul_u(hi, 6.0f)));
+    k.ej = mul_u(p, sub_u(R10, mul_u(hj, 6.0f)));
+    k.wi = add_u(k.b, mul_u(p, add_u(y, mul_u(R6, hi))));
+    k.wj = add_u(k.b, mul_u(p, add_u(y, mul_u(R6, hj))));
+    return k;
+}
+
+__device__ __forceinline__ UFBlockDF<df2> wt_block_df(df2 dx, df2 dy, df2 dz, df2 Rz, df2 hi4, df2 hj)
+{
+    const df2 r2 = norm(add_u(sqr_u(dz), add_u(sqr_u(dx), sqr_u(dy))));
+    const df2 invr = rsqrt_df(r2);
+    const df2 s = rsqrt_far_df(norm(add_u(r2, mul_u(hi4, hj))));
+    const df2 i2 = sqr(invr);
+    const df2 i3 = mul_u(i2, invr);
+    df2 A = scale2(i3, -0.5f), Bc = mul_u(mul_u(i2, i3), 1.5f);
+    wt_near(r2, invr, A, Bc);
+    const df2 u = sqr(s);
+    const df2 t = mul_u(u, s);
+    const df2 p = mul_u(t, u);
+    const df2 Et = mul_u(mul_u(sqr_u(Rz), u), t);
+    UFBlockDF<df2> m;
+    m.Af = add_u(add_u(A, mul_u(t, 3.5f)), mul_u(Et, -6.0f));
+    m.b2 = add_u(Bc, mul_u(p, -4.5f));
+    const df2 D = mul_u(Bc, dz), X = mul_u(mul_u(p, Rz), 1.5f);
+    m.t3 = sub_u(D, X);
+    m.t4 = add_u(D, X);
+    m.zz = add_u(add_u(A, scale2(t, 0.5f)), add_u(mul_u(Et, -1.5f), mul_u(D, dz)));
+    return m;
+}
+
+// u += UT v / WF v of the pair (i, j); w += the reverse block times q
+__device__ __forceinline__ void ut_acc_df(const RotBlockDF2 &k, df2 dx, df2 dy, df2 vx, df2 vy, df2 vz, df2 qx, df2 qy,
+                                          df2 qz, df2 &ux, df2 &uy, df2 &uz, df2 &wx, df2 &wy, df2 &wz)
+{
+    const df2 nx = -dx;
+    {
+        const df2 Q = mad2_u(dy, vx, nx, vy), bv = mul_u(k.b, vz), eQ = mul_u(k.ei, Q);
+        acc_dot3(ux, k.a, vy, bv, dy, eQ, dx);
+        acc_dot3(uy, -k.a, vx, bv, nx, eQ, dy);
+        acc_dot1(uz, -k.wi, Q);
+    }
+    const df2 Q = mad2_u(dy, qx, nx, qy), bv = mul_u(k.b, qz), eQ = mul_u(k.ej, Q);
+    acc_dot3(wx, k.ar, qy, -bv, dy, eQ, dx);
+    acc_dot3(wy, -k.ar, qx, bv, dx, eQ, dy);
+    acc_dot1(wz, k.wj, Q);
+}
+__device__ __forceinline__ void wf_acc_df(const RotBlockDF2 &k, df2 dx, df2 dy, df2 vx, df2 vy, df2 vz, df2 qx, df2 qy,
+                                          df2 qz, df2 &ux, df2 &uy, df2 &uz, df2 &wx, df2 &wy, df2 &wz)
+{
+    const df2 nx = -dx;
+    {
+        const df2 P = mad2_u(dx, vx, dy, vy), Q = mad2_u(dy, vx, nx, vy), H = mad2_u(k.ej, P, k.wj, vz);
+        acc_dot2(ux, -k.ar, vy, H, dy);
+        acc_dot2(uy, k.ar, vx, H, nx);
+        acc_dot1(uz, -k.b, Q);
+    }
+    const df2 P = mad2_u(dx, qx, dy, qy), Q = mad2_u(dy, qx, nx, qy), H = mad2_u(k.ei, P, -k.wi, qz);
+    acc_dot2(wx, -k.a, qy, H, dy);
+    acc_dot2(wy, k.a, qx, H, nx);
+    acc_dot1(wz, k.b, Q);
+}
+
+// Free-space blocks for both orders of a pair: UF (times 3/2, as with the
+// wall) and WT, even in d, A I + B d d^T; UT and WF, odd, c (v x d).
+template <int KIND>
+__device__ __forceinline__ void rpy_acc_df(df2 dx, df2 dy, df2 dz, df2 vx, df2 vy, df2 vz, df2 qx, df2 qy, df2 qz,
+                                           df2 &ux, df2 &uy, df2 &uz, df2 &wx, df2 &wy, df2 &wz)
+{
+    const df2 r2 = norm(add_u(sqr_u(dz), add_u(sqr_u(dx), sqr_u(dy))));
+    const df2 invr = rsqrt_df(r2);
+    const df2 i2 = sqr(invr);
+    if constexpr (KIND == RMW_UT || KIND == RMW_WF) {
+        df2 c = mul_u(i2, invr);
+        rot_near_c(r2, invr, c);
+        const df2 nx = -dx, ny = -dy, nz = -dz;
+        acc_dot1(ux, c, mad2_u(vy, dz, vz, ny));
+        acc_dot1(uy, c, mad2_u(vz, dx, vx, nz));
+        acc_dot1(uz, c, mad2_u(dy, vx, nx, vy));
+        acc_dot1(wx, c, mad2_u(qz, dy, qy, nz));
+        acc_dot1(wy, c, mad2_u(qx, dz, qz, nx));
+        acc_dot1(wz, c, mad2_u(qy, dx, qx, ny));
+        return;
+    }
+    df2 A, B;
+    if constexpr (KIND == RMW_UF) {
+        df2 ia = invr, a3 = mul_u(i2, invr);
+        B = mul_u(add_fast_u(1.5f, mul_u(i2, -3.0f)), a3);
+        uf_near_df(r2, invr, ia, a3, B);
+        A = add_u(mul_u(ia, 1.5f), a3);
+    } else {
+        const df2 i3 = mul_u(i2, invr);
+        A = scale2(i3, -0.5f);
+        B = mul_u(mul_u(i2, i3), 1.5f);
+        wt_near(r2, invr, A, B);
+    }
+    const df2 G = mul_u(B, add_u(mad2_u(dx, vx, dy, vy), mul_u(dz, vz)));
+    const df2 Gq = mul_u(B, add_u(mad2_u(dx, qx, dy, qy), mul_u(dz, qz)));
+    acc_dot2(ux, A, vx, G, dx);
+    acc_dot2(uy, A, vy, G, dy);
+    acc_dot2(uz, A, vz, G, dz);
+    acc_dot2(wx, A, qx, Gq, dx);
+    acc_dot2(wy, A, qy, Gq, dy);
+    acc_dot2(wz, A, qz, Gq, dz);
 }
 
 // ---------------------------------------------------------------------------
@@ -469,66 +595,6 @@ __device__ __forceinline__ void pair_acc_df(df dx, df dy, df dz, df Rz, df hi, d
         if (KIND == RMW_UT) ut_apply_df(c, rot_h_df(hi, s, s2, s3, ez, ezs4, K), s3, dx, dy, dz, vx, vy, vz, ux, uy, uz);
         else wf_apply_df(c, rot_h_df(hj, s, s2, s3, ez, ezs4, K), s3, dx, dy, dz, vx, vy, vz, ux, uy, uz);
     }
-}
-
-// Double-float form of pair_rpy_sym (free space, both orders of one pair).
-template <int KIND>
-__device__ __forceinline__ void pair_rpy_sym_df(df dx, df dy, df dz, df vx, df vy, df vz, df qx, df qy, df qz,
-                                                df &ux, df &uy, df &uz, df &wx, df &wy, df &wz)
-{
-    constexpr df TWO_THIRDS = dfc::make(2.0 / 3.0);
-    constexpr df FOUR_THIRDS = dfc::make(4.0 / 3.0);
-    const df r2 = mad(dz, dz, mad_u(dx, dx, sqr_u(dy)));
-    const df invr = rsqrt_df(r2);
-    if (KIND == RMW_UT || KIND == RMW_WF) {
-        df c = sqr(invr) * invr;
-        const bool near = !(r2 >= 4.0f);  // r < 2
-        if (__any_sync(__activemask(), near)) {
-            if (near) c = scale2(1.0f - (r2 * invr) * 0.375f, 0.5f);
-        }
-        // c (v x d) for target i, -c (q x d) for target j
-        acc_add(ux, c * mad2(vy, dz, -vz, dy));
-        acc_add(uy, c * mad2(vz, dx, -vx, dz));
-        acc_add(uz, c * mad2(dy, vx, -dx, vy));
-        acc_add(wx, -(c * mad2(qy, dz, -qz, dy)));
-        acc_add(wy, -(c * mad2(qz, dx, -qx, dz)));
-        acc_add(wz, -(c * mad2(dy, qx, -dx, qy)));
-        return;
-    }
-    const df invr2 = sqr(invr);
-    df A, Bc;
-    if (KIND == RMW_UF) {
-        A = mad(TWO_THIRDS, invr2, df_from(1.0f)) * invr;
-        Bc = (1.0f - scale2(invr2, 2.0f)) * invr2 * invr;
-        const bool near = !(r2 > 4.0f);  // r <= 2
-        if (__any_sync(__activemask(), near)) {
-            if (near) {
-                const df r = r2 * invr;
-                A = FOUR_THIRDS * (1.0f - r * 0.28125f);
-                Bc = scale2(invr, 0.125f);
-            }
-        }
-    } else {  // RMW_WT
-        const df invr3 = invr2 * invr;
-        A = invr3 * -0.5f;
-        Bc = (invr2 * invr3) * 1.5f;
-        const bool near = !(r2 >= 4.0f);
-        if (__any_sync(__activemask(), near)) {
-            if (near) {
-                const df r = r2 * invr;
-                A = (1.0f - r * 0.84375f) + (r * r2) * 0.078125f;
-                Bc = invr * 0.28125f - r * 0.046875f;
-            }
-        }
-    }
-    const df G = Bc * dot3(dx, vx, dy, vy, dz, vz);
-    const df Gq = Bc * dot3(dx, qx, dy, qy, dz, qz);
-    acc_dot2(ux, A, vx, G, dx);
-    acc_dot2(uy, A, vy, G, dy);
-    acc_dot2(uz, A, vz, G, dz);
-    acc_dot2(wx, A, qx, Gq, dx);
-    acc_dot2(wy, A, qy, Gq, dy);
-    acc_dot2(wz, A, qz, Gq, dz);
 }
 
 }  // namespace rmw

@@ -300,131 +300,6 @@ __device__ __forceinline__ void sym_band_pair(long long b, int nt, const SymBand
     S = t + (int)b;
 }
 
-template <bool SEG, int KIND, bool NOWALL = false, bool BAND = false>
-__device__ __forceinline__ void df_sym_body(const SrcDF *__restrict__ src, int n, int nt,
-                                            double *__restrict__ partial, const SymJob *__restrict__ jobs,
-                                            const SymBand bd = SymBand{0, 0, nullptr, nullptr})
-{
-    // structure-of-arrays source tile: the rotated reads of a warp hit 32
-    // consecutive 16-byte entries (no bank conflicts)
-    __shared__ float4 thi[kTile], tlo[kTile], tvh[kTile], tvl[kTile];
-    __shared__ float2 sacc[kSymWarps][3][kTile];  // per-warp source-side double-float sums (hi, lo)
-    int T, S;
-    if constexpr (BAND) sym_band_pair(blockIdx.x, nt, bd, T, S);
-    else sym_cta<SEG>(jobs, n, nt, T, S, src, partial);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const bool diag = (T == S);
-    const int i = T * kTile + tid;
-    const bool valid_i = i < n;
-    // a target or source past the end is a dummy far above the wall with a zero vector
-    const SrcDF dummy = {make_float4(1.0e6f, 1.0e6f, 1.0e6f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f),
-                         make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-    const SrcDF me = valid_i ? src[i] : dummy;
-    const df xi = {me.hi.x, me.lo.x}, yi = {me.hi.y, me.lo.y}, zi = {me.hi.z, me.lo.z};
-    const df qx = {me.vhi.x, me.vlo.x}, qy = {me.vhi.y, me.vlo.y}, qz = {me.vhi.z, me.vlo.z};
-    {
-        const int j = S * kTile + tid;
-        const SrcDF sj = (j < n) ? src[j] : dummy;
-        thi[tid] = sj.hi;
-        tlo[tid] = sj.lo;
-        tvh[tid] = sj.vhi;
-        tvl[tid] = sj.vlo;
-    }
-    for (int c = 0; c < 3; ++c)
-        for (int k = lane; k < kTile; k += 32) sacc[warp][c][k] = make_float2(0.f, 0.f);
-    __syncthreads();
-    double ax = 0.0, ay = 0.0, az = 0.0;
-    df ux = df_from(0.f), uy = df_from(0.f), uz = df_from(0.f);
-    auto fold = [&]() {  // fold each group of 32 double-float sums into FP64
-        ax += to_double(ux);
-        ay += to_double(uy);
-        az += to_double(uz);
-        ux = df_from(0.f);
-        uy = df_from(0.f);
-        uz = df_from(0.f);
-    };
-    auto step = [&](int k) {
-        const int jl = (lane + k) & (kTile - 1);
-        const float4 sh = thi[jl], sl = tlo[jl], svh = tvh[jl], svl = tvl[jl];
-        const df xj = {sh.x, sl.x}, yj = {sh.y, sl.y}, zj = {sh.z, sl.z};
-        const df vx = {svh.x, svl.x}, vy = {svh.y, svl.y}, vz = {svh.z, svl.z};
-        // double-float accumulation on the FP32 pipe (no FP64 conversions per pair)
-        const float2 a0 = sacc[warp][0][jl], a1 = sacc[warp][1][jl], a2 = sacc[warp][2][jl];
-        df wx = {a0.x, a0.y}, wy = {a1.x, a1.y}, wz = {a2.x, a2.y};
-        // differences renormalised (a cancelled high part must not leave the value in the low part, whose
-        // square a double-float product drops); the sum of two heights cannot cancel
-        if constexpr (NOWALL)
-            pair_rpy_sym_df<KIND>(xi - xj, yi - yj, zi - zj, vx, vy, vz, qx, qy, qz, ux, uy, uz, wx, wy, wz);
-        else
-            pair_rot_sym_df<KIND>(xi - xj, yi - yj, zi - zj, add_u(zi, zj), zi, zj, vx, vy, vz, qx, qy, qz, ux, uy,
-                                  uz, wx, wy, wz);
-        sacc[warp][0][jl] = make_float2(wx.hi, wx.lo);
-        sacc[warp][1][jl] = make_float2(wy.hi, wy.lo);
-        sacc[warp][2][jl] = make_float2(wz.hi, wz.lo);
-    };
-    const SymSteps sp = sym_steps<SEG || BAND>();
-    if (diag) {
-        for (int k = sp.k0; k < sp.k1; ++k) {
-            __syncwarp();
-            if (k > sp.k0 && !(k & 31)) fold();
-            const int off = (k - 32 * warp) & (kTile - 1);  // (source - target) mod 128, warp-uniform
-            if (off == 0 || off > kTile / 2 || (off == kTile / 2 && warp >= kSymWarps / 2)) continue;
-            step(k);
-        }
-    } else {
-        // off-diagonal tiles: no per-step skip test (unrolling measured slower here)
-        for (int g = sp.k0; g < sp.k1; g += 32) {
-            if (g > sp.k0) fold();
-            const int e = min(g + 32, sp.k1);
-#pragma unroll 1
-            for (int k = g; k < e; ++k) {
-                __syncwarp();
-                step(k);
-            }
-        }
-    }
-    ax += to_double(ux);
-    ay += to_double(uy);
-    az += to_double(uz);
-    __syncthreads();
-    // source role of blob S*128 + tid (dummy pairs contributed exact zeros)
-    double sx = 0.0, sy = 0.0, sz = 0.0;
-    for (int w = 0; w < kSymWarps; ++w) {
-        sx += (double)sacc[w][0][tid].x + (double)sacc[w][0][tid].y;
-        sy += (double)sacc[w][1][tid].x + (double)sacc[w][1][tid].y;
-        sz += (double)sacc[w][2][tid].x + (double)sacc[w][2][tid].y;
-    }
-    if constexpr (BAND) {
-        const int W = nt - bd.t0, C = bd.t1 - bd.t0;
-        double *o = bd.bt + ((size_t)(T - bd.t0) * W + (S - bd.t0)) * (3 * kTile) + 3 * tid;
-        o[0] = diag ? ax + sx : ax;
-        o[1] = diag ? ay + sy : ay;
-        o[2] = diag ? az + sz : az;
-        if (!diag) {
-            double *q = bd.bs + ((size_t)(S - bd.t0) * C + (T - bd.t0)) * (3 * kTile) + 3 * tid;
-            q[0] = sx; q[1] = sy; q[2] = sz;
-        }
-        return;
-    }
-    const size_t stride = 3 * (size_t)n;
-    if (diag) {
-        if (valid_i) {
-            double *o = partial + (size_t)sp.slot(T) * stride + 3 * (size_t)i;
-            o[0] = ax + sx; o[1] = ay + sy; o[2] = az + sz;
-        }
-    } else {
-        if (valid_i) {
-            double *o = partial + (size_t)sp.slot(S) * stride + 3 * (size_t)i;
-            o[0] = ax; o[1] = ay; o[2] = az;
-        }
-        const int j = S * kTile + tid;
-        if (j < n) {
-            double *o = partial + (size_t)sp.slot(T) * stride + 3 * (size_t)j;
-            o[0] = sx; o[1] = sy; o[2] = sz;
-        }
-    }
-}
-
 // The UF kernel of that grid with two targets per thread in packed FP32 lanes
 // (f32x2.cuh): a CTA is 64 threads, thread t owns targets t (lane x) and
 // t + 64 (lane y) of tile T, and a step evaluates the same source for both
@@ -446,8 +321,8 @@ struct F2Target {
 };
 
 // one step: sources ja (lane x) and jb (lane y); DIAG false: ja = jb
-template <bool DIAG>
-__device__ __forceinline__ void uf_f2_step(const F2Target &me, int ja, int jb, const float4 *thi, const float4 *tlo,
+template <int KIND, bool NOWALL, bool DIAG>
+__device__ __forceinline__ void df_f2_step(const F2Target &me, int ja, int jb, const float4 *thi, const float4 *tlo,
                                            const float4 *tvh, const float4 *tvl, float4 (*sacc)[kTile], df2 &ux,
                                            df2 &uy, df2 &uz)
 {
@@ -475,10 +350,22 @@ __device__ __forceinline__ void uf_f2_step(const F2Target &me, int ja, int jb, c
     df2 wz = {make_float2(w2.x, w2.y), make_float2(w2.z, w2.w)};
     // differences renormalised (a cancelled high part must not leave the value in the low part, whose
     // square a double-float product drops); the sum of two heights cannot cancel
-    const df2 dx = me.x - xj, dy = me.y - yj;
-    const UFBlockDF<df2> m = uf_block_df<df2>(dx, dy, me.z - zj, add_u(me.z, zj), me.h4, zj);
-    uf_block_acc_df(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);                // M_ij v_j
-    uf_block_acc_df(m, m.t4, m.t3, dx, dy, me.qx, me.qy, me.qz, wx, wy, wz);       // M_ij^T v_i
+    const df2 dx = me.x - xj, dy = me.y - yj, dz = me.z - zj;
+    if constexpr (NOWALL) {
+        rpy_acc_df<KIND>(dx, dy, dz, vx, vy, vz, me.qx, me.qy, me.qz, ux, uy, uz, wx, wy, wz);
+    } else if constexpr (KIND == RMW_UF || KIND == RMW_WT) {
+        const df2 Rz = add_u(me.z, zj);
+        UFBlockDF<df2> m;
+        if constexpr (KIND == RMW_UF) m = uf_block_df<df2>(dx, dy, dz, Rz, me.h4, zj);
+        else m = wt_block_df(dx, dy, dz, Rz, me.h4, zj);
+        uf_block_acc_df(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);           // M_ij v_j
+        uf_block_acc_df(m, m.t4, m.t3, dx, dy, me.qx, me.qy, me.qz, wx, wy, wz);  // M_ij^T v_i
+    } else {
+        const RotBlockDF2 k = rot_block_df(dx, dy, dz, add_u(me.z, zj), me.z, me.h4, zj);
+        if constexpr (KIND == RMW_UT)
+            ut_acc_df(k, dx, dy, vx, vy, vz, me.qx, me.qy, me.qz, ux, uy, uz, wx, wy, wz);
+        else wf_acc_df(k, dx, dy, vx, vy, vz, me.qx, me.qy, me.qz, ux, uy, uz, wx, wy, wz);
+    }
     if (DIAG) {
         float *s = reinterpret_cast<float *>(sacc);
         auto put = [&](int c, const df2 &w) {
@@ -494,8 +381,8 @@ __device__ __forceinline__ void uf_f2_step(const F2Target &me, int ja, int jb, c
     }
 }
 
-template <bool WHOLE, bool SEG, bool BAND>
-__device__ __forceinline__ void uf_f2_body(const SrcDF *__restrict__ src, int n, int nt, double *__restrict__ partial,
+template <int KIND, bool NOWALL, bool WHOLE, bool SEG, bool BAND>
+__device__ __forceinline__ void df_f2_body(const SrcDF *__restrict__ src, int n, int nt, double *__restrict__ partial,
                                            const SymJob *__restrict__ jobs,
                                            const SymBand bd = SymBand{0, 0, nullptr, nullptr})
 {
@@ -541,12 +428,12 @@ __device__ __forceinline__ void uf_f2_body(const SrcDF *__restrict__ src, int n,
             __syncwarp();
             const int ja = (tid + o) & (kTile - 1), jb = (tid + kF2Threads + o) & (kTile - 1);
             if (o < kTile / 2) {
-                uf_f2_step<true>(me, ja, jb, thi, tlo, tvh, tvl, sacc[warp], ux, uy, uz);
+                df_f2_step<KIND, NOWALL, true>(me, ja, jb, thi, tlo, tvh, tvl, sacc[warp], ux, uy, uz);
             } else {
                 F2Target half = me;
                 half.qx.hi.y = half.qx.lo.y = half.qy.hi.y = half.qy.lo.y = half.qz.hi.y = half.qz.lo.y = 0.f;
                 df2 vx = ux, vy = uy, vz = uz;
-                uf_f2_step<true>(half, ja, jb, thi, tlo, tvh, tvl, sacc[warp], vx, vy, vz);
+                df_f2_step<KIND, NOWALL, true>(half, ja, jb, thi, tlo, tvh, tvl, sacc[warp], vx, vy, vz);
                 ux.hi.x = vx.hi.x; ux.lo.x = vx.lo.x;
                 uy.hi.x = vy.hi.x; uy.lo.x = vy.lo.x;
                 uz.hi.x = vz.hi.x; uz.lo.x = vz.lo.x;
@@ -560,7 +447,7 @@ __device__ __forceinline__ void uf_f2_body(const SrcDF *__restrict__ src, int n,
             for (; g < e; ++g) {
                 __syncwarp();
                 const int j = (lane + g) & (kTile - 1);
-                uf_f2_step<false>(me, j, j, thi, tlo, tvh, tvl, sacc[warp], ux, uy, uz);
+                df_f2_step<KIND, NOWALL, false>(me, j, j, thi, tlo, tvh, tvl, sacc[warp], ux, uy, uz);
             }
             ux = norm(ux);
             uy = norm(uy);
@@ -620,7 +507,7 @@ __global__ void __launch_bounds__(kF2Threads, 8) wall_uf_df_sym_kernel(const Src
                                                                      double *__restrict__ partial,
                                                                      const SymJob *__restrict__ jobs)
 {
-    uf_f2_body<WHOLE, SEG, false>(src, n, nt, partial, jobs);
+    df_f2_body<RMW_UF, false, WHOLE, SEG, false>(src, n, nt, partial, jobs);
 }
 
 // the same over one band of tile rows (SymBand): products whose per-tile
@@ -628,25 +515,26 @@ __global__ void __launch_bounds__(kF2Threads, 8) wall_uf_df_sym_kernel(const Src
 __global__ void __launch_bounds__(kF2Threads, 8) wall_uf_df_sym_band_kernel(const SrcDF *__restrict__ src, int n, int nt,
                                                                           const SymBand bd)
 {
-    uf_f2_body<true, false, true>(src, n, nt, nullptr, nullptr, bd);
+    df_f2_body<RMW_UF, false, true, false, true>(src, n, nt, nullptr, nullptr, bd);
 }
 
-// The rotation blocks (UT, WF, WT) on the same grid: pair_rot_sym_df.
-template <bool SEG, int KIND>
-__global__ void __launch_bounds__(kThreads) wall_rot_df_sym_kernel(const SrcDF *__restrict__ src, int n, int nt,
-                                                                    double *__restrict__ partial,
-                                                                    const SymJob *__restrict__ jobs)
+// The rotation blocks (UT, WF, WT) on the same grid: rot_block_df, wt_block_df
+// (about 500 FP32-pipe operations a pair against 842, 842 and 720 issued by
+// the one-target tensor forms).  Products at 10,752 blobs: UT 1.47 -> 0.91 ms,
+// WF 1.53 -> 0.91, WT 1.28 -> 0.85; 5,003 blobs WF 408 -> 240 us.
+template <bool SEG, bool WHOLE, int KIND>
+__global__ void __launch_bounds__(kF2Threads, 8) wall_rot_df_sym_kernel(const SrcDF *__restrict__ src, int n, int nt,
+                                                                         double *__restrict__ partial,
+                                                                         const SymJob *__restrict__ jobs)
 {
-    df_sym_body<SEG, KIND>(src, n, nt, partial, jobs);
+    df_f2_body<KIND, false, WHOLE, SEG, false>(src, n, nt, partial, jobs);
 }
 
-// The same kernels over one band of tile rows (SymBand): products whose
-// per-tile partial sums would not fit in the scratch budget.
 template <int KIND>
-__global__ void __launch_bounds__(kThreads) wall_df_sym_band_kernel(const SrcDF *__restrict__ src, int n, int nt,
-                                                                     const SymBand bd)
+__global__ void __launch_bounds__(kF2Threads, 8) wall_df_sym_band_kernel(const SrcDF *__restrict__ src, int n, int nt,
+                                                                          const SymBand bd)
 {
-    df_sym_body<false, KIND, false, true>(src, n, nt, nullptr, nullptr, bd);
+    df_f2_body<KIND, false, true, false, true>(src, n, nt, nullptr, nullptr, bd);
 }
 
 // acc (3n doubles, FP64) += the band's contributions to every blob of tiles
@@ -980,8 +868,7 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
             uf_block_acc_d(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
             uf_block_acc_d(m, m.t4, m.t3, dx, dy, me.vx, me.vy, me.vz, wx, wy, wz);
         } else {
-            pair_rot_sym<double, KIND>(dx, dy, dz, Rz, zi, zj, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy,
-                                       wz);
+            pair_rot_sym_d<KIND>(dx, dy, dz, Rz, zi, zj, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
         }
         sacc[warp][0][jl] = wx;
         sacc[warp][1][jl] = wy;
@@ -1038,11 +925,11 @@ __global__ void __launch_bounds__(kThreads) wall_fp64_sym_kernel(const SrcD *__r
 // Free-space (no wall) symmetric kernels: the same bodies with pair_rpy_sym;
 // the no-wall pack writes records of the same layouts (positions over a, no
 // height shift or damping), so the FP64 body takes inva = 1.
-template <int KIND>
-__global__ void __launch_bounds__(kThreads) nowall_df_sym_kernel(const SrcDF *__restrict__ src, int n, int nt,
-                                                                  double *__restrict__ partial)
+template <int KIND, bool WHOLE>
+__global__ void __launch_bounds__(kF2Threads, 8) nowall_df_sym_kernel(const SrcDF *__restrict__ src, int n, int nt,
+                                                                       double *__restrict__ partial)
 {
-    df_sym_body<false, KIND, true>(src, n, nt, partial, nullptr);
+    df_f2_body<KIND, true, WHOLE, false, false>(src, n, nt, partial, nullptr);
 }
 template <int KIND>
 __global__ void __launch_bounds__(kThreads) nowall_mixed_sym_kernel(const SrcF *__restrict__ src, int n, int nt,
@@ -1067,8 +954,10 @@ static void nowall_sym_launch_kind(int mode, const void *src, int n, int nt, dou
     const dim3 ncta(npair, nsplit);
     if (mode == RMW_MODE_FP64)
         nowall_fp64_sym_kernel<KIND><<<ncta, kThreads, 0, st>>>((const SrcD *)src, n, nt, partial);
+    else if (mode == RMW_MODE_DF64 && nsplit == 1)
+        nowall_df_sym_kernel<KIND, true><<<ncta, kF2Threads, 0, st>>>((const SrcDF *)src, n, nt, partial);
     else if (mode == RMW_MODE_DF64)
-        nowall_df_sym_kernel<KIND><<<ncta, kThreads, 0, st>>>((const SrcDF *)src, n, nt, partial);
+        nowall_df_sym_kernel<KIND, false><<<ncta, kF2Threads, 0, st>>>((const SrcDF *)src, n, nt, partial);
     else
         nowall_mixed_sym_kernel<KIND><<<npair, kThreads, 0, st>>>((const SrcF *)src, n, nt, partial);
 }
@@ -1766,17 +1655,19 @@ static void launch_sym(bool seg, int mode, const void *src, int n, int nt, dim3 
         else wall_fp64_sym_kernel<false, KIND><<<ncta, kThreads, 0, st>>>(s, n, nt, inva, partial, jobs);
     } else if (mode == RMW_MODE_DF64) {
         const SrcDF *s = (const SrcDF *)src;
-        if (KIND == RMW_UF) {
+        if constexpr (KIND == RMW_UF) {
             if (seg) wall_uf_df_sym_kernel<true, true><<<ncta, kF2Threads, 0, st>>>(s, n, nt, partial, jobs);
             else if (ncta.y == 1) wall_uf_df_sym_kernel<false, true><<<ncta, kF2Threads, 0, st>>>(s, n, nt, partial, jobs);
             else wall_uf_df_sym_kernel<false, false><<<ncta, kF2Threads, 0, st>>>(s, n, nt, partial, jobs);
         } else {
-            if (seg) wall_rot_df_sym_kernel<true, KIND><<<ncta, kThreads, 0, st>>>(s, n, nt, partial, jobs);
-            else wall_rot_df_sym_kernel<false, KIND><<<ncta, kThreads, 0, st>>>(s, n, nt, partial, jobs);
+            if (seg) wall_rot_df_sym_kernel<true, true, KIND><<<ncta, kF2Threads, 0, st>>>(s, n, nt, partial, jobs);
+            else if (ncta.y == 1)
+                wall_rot_df_sym_kernel<false, true, KIND><<<ncta, kF2Threads, 0, st>>>(s, n, nt, partial, jobs);
+            else wall_rot_df_sym_kernel<false, false, KIND><<<ncta, kF2Threads, 0, st>>>(s, n, nt, partial, jobs);
         }
     } else {
         const SrcF *s = (const SrcF *)src;
-        if (KIND == RMW_UF) {
+        if constexpr (KIND == RMW_UF) {
             if (seg) wall_uf_mixed_sym_kernel<true><<<ncta, kF2Threads, 0, st>>>(s, n, nt, partial, jobs);
             else wall_uf_mixed_sym_kernel<false><<<ncta, kF2Threads, 0, st>>>(s, n, nt, partial, jobs);
         } else {
@@ -1907,9 +1798,9 @@ static int sym_band_product(int kind, const double *r, const double *v, double *
         const SrcDF *src = (const SrcDF *)base;
         switch (kind) {
         case RMW_UF: wall_uf_df_sym_band_kernel<<<(unsigned)ncta, kF2Threads, 0, st>>>(src, n, nt, bd); break;
-        case RMW_UT: wall_df_sym_band_kernel<RMW_UT><<<(unsigned)ncta, kThreads, 0, st>>>(src, n, nt, bd); break;
-        case RMW_WF: wall_df_sym_band_kernel<RMW_WF><<<(unsigned)ncta, kThreads, 0, st>>>(src, n, nt, bd); break;
-        default: wall_df_sym_band_kernel<RMW_WT><<<(unsigned)ncta, kThreads, 0, st>>>(src, n, nt, bd); break;
+        case RMW_UT: wall_df_sym_band_kernel<RMW_UT><<<(unsigned)ncta, kF2Threads, 0, st>>>(src, n, nt, bd); break;
+        case RMW_WF: wall_df_sym_band_kernel<RMW_WF><<<(unsigned)ncta, kF2Threads, 0, st>>>(src, n, nt, bd); break;
+        default: wall_df_sym_band_kernel<RMW_WT><<<(unsigned)ncta, kF2Threads, 0, st>>>(src, n, nt, bd); break;
         }
         sym_band_accum_kernel<<<pg, pb, 0, st>>>(bd, n, nt, acc);
     }
