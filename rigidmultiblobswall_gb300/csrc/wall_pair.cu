@@ -83,7 +83,11 @@ __device__ __forceinline__ PairRange pair_range(const TileJob *jobs, int n, int 
 }
 
 // ---------------------------------------------------------------------------
-// pack
+// pack: one blob per thread, few threads per CTA (latency, not bandwidth,
+// bounds it: 10,752 blobs are 344 warps); inva = 1 / a from the host, the
+// damping's division only where a blob overlaps the wall
+constexpr int kPackThreads = 64;
+inline unsigned pack_blocks(int n) { return (unsigned)((n + kPackThreads - 1) / kPackThreads); }
 __global__ void pack_fp64_kernel(const double *__restrict__ r, const double *__restrict__ v, SrcD *__restrict__ src,
                                  int n, double a)
 {
@@ -99,11 +103,10 @@ __global__ void pack_fp64_kernel(const double *__restrict__ r, const double *__r
 }
 
 __global__ void pack_mixed_kernel(const double *__restrict__ r, const double *__restrict__ v, SrcF *__restrict__ src,
-                                  int n, double a)
+                                  int n, double a, double inva)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    double inva = 1.0 / a;
     double x = r[3 * i], y = r[3 * i + 1], z = r[3 * i + 2];
     double b = (z < a) ? z / a : 1.0;
     double ze = (z <= a) ? a : z;
@@ -117,11 +120,10 @@ __global__ void pack_mixed_kernel(const double *__restrict__ r, const double *__
 }
 
 __global__ void pack_df_kernel(const double *__restrict__ r, const double *__restrict__ v, SrcDF *__restrict__ src,
-                               int n, double a)
+                               int n, double a, double inva)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const double inva = 1.0 / a;
     const double z = r[3 * i + 2];
     const double b = (z < a) ? z / a : 1.0;
     const double ze = (z <= a) ? a : z;
@@ -1362,75 +1364,67 @@ __global__ void wall_finalize_multi_kernel(const double *__restrict__ r, const d
 // finalize: fixed-order chunk sum + FP64 self term + b_i * norm factor.
 // With pbase / pstride (segmented symmetric layout) blob i's slot s is at
 // partial + pbase[i] + s * pstride[i]; otherwise at partial + s * 3n + 3i.
-// kFinGroup consecutive threads share a blob: thread g of the group sums slots
-// g, g + kFinGroup, ... and a fixed shuffle tree adds the group's sums, so the
-// order is fixed (deterministic) and the slot loads run kFinGroup-wide.
-// Products of few blobs and many slots (split tile pairs) use kFinGroupWide
-// threads, which keeps more of a blob's slot loads in flight.
-constexpr int kFinGroup = 4, kFinGroupWide = 16;
-inline unsigned finalize_blocks(int n, int pb, int group = kFinGroup)
-{
-    return (unsigned)(((long long)group * n + pb - 1) / pb);
-}
+// A CTA takes kFinBlobs blobs: 96 x G threads, thread (x, g) the sum of slots
+// g, g + G, ... of component x of those blobs (a warp reads 32 consecutive
+// values of a slot, and three times as many threads keep loads in flight as
+// with a thread per blob and group), then one thread per blob adds the G sums
+// in order.  The sum of 84 slots of 10,752 blobs is a read of 21.7 MB from L2.
+constexpr int kFinBlobs = 32;
+// few blobs with many slots (split tile pairs): more groups
+inline int finalize_groups(int n, int slots) { return slots >= 32 && n < 6144 ? 8 : 4; }
+inline unsigned finalize_blocks(int n) { return (unsigned)((n + kFinBlobs - 1) / kFinBlobs); }
 
 // DF2: the slots hold double-float values (the mixed symmetric kernels), added
 // in double-float on the FP32 pipe
-template <int KIND, bool DF2 = false, int G = kFinGroup>
-__global__ void wall_finalize_kernel(const double *__restrict__ r, const double *__restrict__ v,
-                                     const double *__restrict__ partial, int nchunks, double *__restrict__ out,
-                                     int n, double a, double nf, const int *__restrict__ blob_nchunks,
-                                     const long long *__restrict__ pbase = nullptr,
-                                     const int *__restrict__ pstride = nullptr, double pair_scale = 1.0)
+template <int KIND, bool DF2 = false>
+__global__ void __launch_bounds__(3 * kFinBlobs * 8) wall_finalize_kernel(
+    const double *__restrict__ r, const double *__restrict__ v, const double *__restrict__ partial, int nchunks,
+    double *__restrict__ out, int n, double a, double nf, const int *__restrict__ blob_nchunks,
+    const long long *__restrict__ pbase = nullptr, const int *__restrict__ pstride = nullptr, double pair_scale = 1.0)
 {
-    const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = (int)(gt / G), g = (int)(gt % G);
-    double ux = 0.0, uy = 0.0, uz = 0.0;
-    if constexpr (DF2) {
-        df sx = df_from(0.f), sy = df_from(0.f), sz = df_from(0.f);
-        if (i < n) {
-            const int nc = blob_nchunks ? blob_nchunks[i] : nchunks;
-            const float2 *p0 = reinterpret_cast<const float2 *>(partial) + (pbase ? pbase[i] : 3 * (long long)i);
-            const size_t ps = pstride ? (size_t)pstride[i] : 3 * (size_t)n;
-#pragma unroll 4
+    __shared__ double red[8][3 * kFinBlobs];
+    const int x = threadIdx.x, g = threadIdx.y, G = blockDim.y;
+    const int ib = blockIdx.x * kFinBlobs + x / 3;
+    if (ib < n) {
+        const int nc = blob_nchunks ? blob_nchunks[ib] : nchunks;
+        const long long p0 = (pbase ? pbase[ib] : 3 * (long long)ib) + x % 3;
+        const size_t ps = pstride ? (size_t)pstride[ib] : 3 * (size_t)n;
+        if constexpr (DF2) {
+            const float2 *p = reinterpret_cast<const float2 *>(partial) + p0;
+            df sum = df_from(0.f);
+#pragma unroll 8
             for (int s = g; s < nc; s += G) {
-                const float2 *p = p0 + (size_t)s * ps;
-                const float2 px = p[0], py = p[1], pz = p[2];
-                sx = sx + df{px.x, px.y};
-                sy = sy + df{py.x, py.y};
-                sz = sz + df{pz.x, pz.y};
+                const float2 q = p[(size_t)s * ps];
+                sum = sum + df{q.x, q.y};
             }
-        }
-#pragma unroll
-        for (int o = G / 2; o > 0; o >>= 1) {  // every lane of the warp takes part
-            sx = sx + df{__shfl_down_sync(0xffffffffu, sx.hi, o, G),
-                         __shfl_down_sync(0xffffffffu, sx.lo, o, G)};
-            sy = sy + df{__shfl_down_sync(0xffffffffu, sy.hi, o, G),
-                         __shfl_down_sync(0xffffffffu, sy.lo, o, G)};
-            sz = sz + df{__shfl_down_sync(0xffffffffu, sz.hi, o, G),
-                         __shfl_down_sync(0xffffffffu, sz.lo, o, G)};
-        }
-        ux = (double)sx.hi + (double)sx.lo;
-        uy = (double)sy.hi + (double)sy.lo;
-        uz = (double)sz.hi + (double)sz.lo;
-    } else {
-        if (i < n) {
-            const int nc = blob_nchunks ? blob_nchunks[i] : nchunks;
-            const double *p0 = pbase ? partial + pbase[i] : partial + 3 * (size_t)i;
-            const size_t ps = pstride ? (size_t)pstride[i] : 3 * (size_t)n;
-#pragma unroll 4
-            for (int s = g; s < nc; s += G) {  // unrolled: loads of several slots in flight
-                const double *p = p0 + (size_t)s * ps;
-                ux += p[0]; uy += p[1]; uz += p[2];
-            }
-        }
-#pragma unroll
-        for (int o = G / 2; o > 0; o >>= 1) {  // every lane of the warp takes part
-            ux += __shfl_down_sync(0xffffffffu, ux, o, G);
-            uy += __shfl_down_sync(0xffffffffu, uy, o, G);
-            uz += __shfl_down_sync(0xffffffffu, uz, o, G);
+            reinterpret_cast<float2 *>(red[g])[x] = make_float2(sum.hi, sum.lo);
+        } else {
+            const double *p = partial + p0;
+            double sum = 0.0;
+#pragma unroll 8
+            for (int s = g; s < nc; s += G) sum += p[(size_t)s * ps];
+            red[g][x] = sum;
         }
     }
-    if (i >= n || g != 0) return;
+    __syncthreads();
+    const int i = blockIdx.x * kFinBlobs + x;
+    if (g != 0 || x >= kFinBlobs || i >= n) return;
+    double u[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        if constexpr (DF2) {
+            df sum = df_from(0.f);
+            for (int k = 0; k < G; ++k) {
+                const float2 q = reinterpret_cast<const float2 *>(red[k])[3 * x + c];
+                sum = sum + df{q.x, q.y};
+            }
+            u[c] = to_double(sum);
+        } else {
+            u[c] = 0.0;
+            for (int k = 0; k < G; ++k) u[c] += red[k][3 * x + c];
+        }
+    }
+    double ux = u[0], uy = u[1], uz = u[2];
     ux *= pair_scale; uy *= pair_scale; uz *= pair_scale;
     const double z = r[3 * i + 2];
     const double b = (z < a) ? z / a : 1.0;
@@ -1521,18 +1515,17 @@ static int launch_kind(const double *r, const double *v, double *out, int n, dou
     const int chunk = (n + nchunks - 1) / nchunks;
     const dim3 grid = B ? dim3(B->njobs) : dim3((n + kThreads - 1) / kThreads, nchunks);
     const TileJob *jobs = B ? B->jobs : nullptr;
-    const int pb = 256, pg = (n + pb - 1) / pb;
     void *tok = nullptr;
     if (mode == RMW_MODE_FP64) {
         SrcD *src = (SrcD *)base;
-        pack_fp64_kernel<<<pg, pb, 0, st>>>(r, v, src, n, a);
+        pack_fp64_kernel<<<pack_blocks(n), kPackThreads, 0, st>>>(r, v, src, n, a);
         if (int rc = trace_begin(TRACE_PAIR, st, &tok)) return rc;
         if (B) wall_pair_fp64_kernel<KIND, false, true><<<grid, kThreads, 0, st>>>(src, n, chunk, inva, P, partial, jobs);
         else if (per) wall_pair_fp64_kernel<KIND, true, false><<<grid, kThreads, 0, st>>>(src, n, chunk, inva, P, partial, jobs);
         else wall_pair_fp64_kernel<KIND, false, false><<<grid, kThreads, 0, st>>>(src, n, chunk, inva, P, partial, jobs);
     } else if (mode == RMW_MODE_DF64) {
         SrcDF *src = (SrcDF *)base;
-        pack_df_kernel<<<pg, pb, 0, st>>>(r, v, src, n, a);
+        pack_df_kernel<<<pack_blocks(n), kPackThreads, 0, st>>>(r, v, src, n, a, 1.0 / a);
         Periodic Ps{P.Lx * inva, P.Ly * inva, P.Lz * inva};
         if (int rc = trace_begin(TRACE_PAIR, st, &tok)) return rc;
         if (B) wall_pair_df_kernel<KIND, false, true><<<grid, kThreads, 0, st>>>(src, n, chunk, Ps, partial, jobs);
@@ -1540,7 +1533,7 @@ static int launch_kind(const double *r, const double *v, double *out, int n, dou
         else wall_pair_df_kernel<KIND, false, false><<<grid, kThreads, 0, st>>>(src, n, chunk, Ps, partial, jobs);
     } else {
         SrcF *src = (SrcF *)base;
-        pack_mixed_kernel<<<pg, pb, 0, st>>>(r, v, src, n, a);
+        pack_mixed_kernel<<<pack_blocks(n), kPackThreads, 0, st>>>(r, v, src, n, a, 1.0 / a);
         Periodic Ps{P.Lx * inva, P.Ly * inva, P.Lz * inva};
         if (int rc = trace_begin(TRACE_PAIR, st, &tok)) return rc;
         if (B) wall_pair_mixed_kernel<KIND, false, true><<<grid, kThreads, 0, st>>>(src, n, chunk, Ps, partial, jobs);
@@ -1550,9 +1543,8 @@ static int launch_kind(const double *r, const double *v, double *out, int n, dou
     if (int rc = trace_end(tok, st)) return rc;
     // the FP64 and df64 UF pair kernels sum (3/2) M v
     const double scale = (KIND == RMW_UF && mode != RMW_MODE_MIXED) ? kUFCoeffScale : 1.0;
-    wall_finalize_kernel<KIND><<<finalize_blocks(n, pb), pb, 0, st>>>(r, v, partial, nchunks, out, n, a, nf,
-                                                                       B ? B->blob_nch : nullptr, nullptr, nullptr,
-                                                                       scale);
+    wall_finalize_kernel<KIND><<<finalize_blocks(n), dim3(3 * kFinBlobs, finalize_groups(n, nchunks)), 0, st>>>(
+        r, v, partial, nchunks, out, n, a, nf, B ? B->blob_nch : nullptr, nullptr, nullptr, scale);
     RMW_CHECK_LAUNCH("wall product kernels");
     return RMW_OK;
 }
@@ -1688,18 +1680,11 @@ template <int KIND, bool DF2>
 static void launch_sym_finalize_t(const double *r, const double *v, const double *partial, int nt, double *out,
                                   int n, double a, double nf, const WallBatch *B, cudaStream_t st)
 {
-    const int pb = 256;
     const double scale = (KIND == RMW_UF) ? kUFCoeffScale : 1.0;
-    if (!B && !DF2 && nt >= 32 && n < 6144)
-        wall_finalize_kernel<KIND, DF2, kFinGroupWide><<<finalize_blocks(n, pb, kFinGroupWide), pb, 0, st>>>(
-            r, v, partial, nt, out, n, a, nf, nullptr, nullptr, nullptr, scale);
-    else if (B)
-        wall_finalize_kernel<KIND, DF2><<<finalize_blocks(n, pb), pb, 0, st>>>(r, v, partial, 0, out, n, a, nf,
-                                                                               B->blob_nslots, B->blob_pbase,
-                                                                               B->blob_pstride, scale);
-    else
-        wall_finalize_kernel<KIND, DF2><<<finalize_blocks(n, pb), pb, 0, st>>>(r, v, partial, nt, out, n, a, nf,
-                                                                               nullptr, nullptr, nullptr, scale);
+    const dim3 threads(3 * kFinBlobs, B ? 4 : finalize_groups(n, nt));
+    wall_finalize_kernel<KIND, DF2><<<finalize_blocks(n), threads, 0, st>>>(
+        r, v, partial, nt, out, n, a, nf, B ? B->blob_nslots : nullptr, B ? B->blob_pbase : nullptr,
+        B ? B->blob_pstride : nullptr, scale);
 }
 
 // mixed: the symmetric kernels' slots hold double-float values
@@ -1720,12 +1705,11 @@ static int sym_product(int kind, const double *r, const double *v, double *out, 
     const size_t packed = ((rec * (size_t)n + 255) / 256) * 256;
     char *base = (char *)scratch_ptr;
     double *partial = (double *)(base + packed);
-    const int pb = 256, pg = (n + pb - 1) / pb;
     const dim3 ncta(B ? (unsigned)B->nsym : (unsigned)((long long)nt * (nt + 1) / 2), nsplit);
     const SymJob *jobs = B ? B->sym_jobs : nullptr;
-    if (mode == RMW_MODE_FP64) pack_fp64_kernel<<<pg, pb, 0, st>>>(r, v, (SrcD *)base, n, a);
-    else if (mode == RMW_MODE_DF64) pack_df_kernel<<<pg, pb, 0, st>>>(r, v, (SrcDF *)base, n, a);
-    else pack_mixed_kernel<<<pg, pb, 0, st>>>(r, v, (SrcF *)base, n, a);
+    if (mode == RMW_MODE_FP64) pack_fp64_kernel<<<pack_blocks(n), kPackThreads, 0, st>>>(r, v, (SrcD *)base, n, a);
+    else if (mode == RMW_MODE_DF64) pack_df_kernel<<<pack_blocks(n), kPackThreads, 0, st>>>(r, v, (SrcDF *)base, n, a, 1.0 / a);
+    else pack_mixed_kernel<<<pack_blocks(n), kPackThreads, 0, st>>>(r, v, (SrcF *)base, n, a, 1.0 / a);
     const double inva = 1.0 / a;
     void *tok = nullptr;
     if (int rc = trace_begin(TRACE_PAIR, st, &tok)) return rc;
@@ -1786,7 +1770,7 @@ static int sym_band_product(int kind, const double *r, const double *v, double *
     double *bt = (double *)(base + packed + accb);
     double *bs = bt + (size_t)C * nt * 3 * kTile;
     const int pb = 256, pg = (n + pb - 1) / pb;
-    pack_df_kernel<<<pg, pb, 0, st>>>(r, v, (SrcDF *)base, n, a);
+    pack_df_kernel<<<pack_blocks(n), kPackThreads, 0, st>>>(r, v, (SrcDF *)base, n, a, 1.0 / a);
     RMW_CUDA(cudaMemsetAsync(acc, 0, sizeof(double) * 3 * (size_t)n, st));
     void *tok = nullptr;
     if (int rc = trace_begin(TRACE_PAIR, st, &tok)) return rc;
