@@ -13,13 +13,14 @@
 //   bit of the sum (the largest term's own rounding is 2^-53).  An optional
 //   cutoff restricts the sum to pairs within it (the reference's
 //   neighbour-list variant uses 2a + 30 b, multi_bodies/forces_numba.py:228-270).
-//   Two FP32 passes over all pairs (nearest blob, candidates; about 10
-//   instructions a pair, the floor of 12,288 blobs 90 us) and the FP64 work of
-//   the candidates, several source chunks per target tile so that the GPU is
-//   full.  1,024 shells of 12 blobs with the wall and body reduction, Debye
-//   length 0.1a: 19.2 -> 0.33 ms (FP64 for a fifth of all pairs on 96 CTAs
-//   before); 0.5a 25.4 -> 1.7 ms; 1a 24.6 -> 4.1 ms; 172,032 blobs, 0.1a
-//   195 -> 33 ms, 1a 2,818 -> 99 ms.
+//   Two FP32 passes over all pairs (nearest blob, candidates; two sources in
+//   packed lanes, 60 us each at 12,288 blobs) and the FP64 work of about 25
+//   candidates per blob (150 us: lanes of a warp have lists of different
+//   lengths), several source chunks per target tile so that the GPU is full.
+//   1,024 shells of 12 blobs with the wall and body reduction, Debye length
+//   0.1a: 19.2 -> 0.29 ms (before: FP64 for a fifth of all pairs, lanes waiting
+//   for each other's, on 96 CTAs); 0.5a 25.4 -> 1.5 ms; 1a 24.6 -> 3.6 ms;
+//   172,032 blobs, 0.1a 195 -> 29 ms, 1a 2,818 -> 74 ms.
 // * external blob forces (multi_bodies_functions.py:153-189): gravity
 //   -g m e_z and the wall repulsion (e/b) exp(-(h - a)/b) (e/b for h <= a).
 // The body reduction [F_b, T_b] = K^T f is rmw_rigid_KT_mult.
@@ -53,8 +54,6 @@ struct Box {
     float unit;      // 1 / (2a + b)
 };
 
-__device__ __forceinline__ float image_f(float d, float L, float inv) { return L > 0.f ? d - L * rintf(d * inv) : d; }
-
 struct Screen {
     double x0[3];
     float x, y, z;  // this thread's target
@@ -80,29 +79,45 @@ __device__ __forceinline__ Screen screen_setup(const double *__restrict__ r, int
     return s;
 }
 
-// source tile: FP32 coordinates and the error bound of distances to them (w)
+// source tile: FP32 coordinates and the error bound w of distances to them,
+// two sources side by side (x x' y y', z z' w w'), so that a scan works on
+// packed pairs; a source past the end is out of every reach
 __device__ __forceinline__ void screen_tile(const double *__restrict__ r, const Screen &s, const Box &L, int j, int j1,
                                             float4 *tile)
 {
-    if (j < j1) {
+    float *o = (float *)(tile + 2 * (threadIdx.x >> 1)) + (threadIdx.x & 1);
+    if (j >= j1) {
+        o[0] = o[2] = o[4] = 3.0e18f;
+        o[6] = 0.f;
+    } else {
         const float x = (float)(r[3 * (size_t)j] - s.x0[0]) * L.unit,
                     y = (float)(r[3 * (size_t)j + 1] - s.x0[1]) * L.unit,
                     z = (float)(r[3 * (size_t)j + 2] - s.x0[2]) * L.unit;
-        tile[threadIdx.x] =
-            make_float4(x, y, z, kErr * (fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z))) + s.ext + L.big));
+        o[0] = x;
+        o[2] = y;
+        o[4] = z;
+        o[6] = kErr * (fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z))) + s.ext + L.big);
     }
 }
 
-template <bool PER>
-__device__ __forceinline__ float screen_r2(const Screen &s, const Box &L, float4 q)
+__device__ __forceinline__ f2 image_f2(f2 d, float L, float inv)
 {
-    float ex = q.x - s.x, ey = q.y - s.y, ez = q.z - s.z;
+    if (!(L > 0.f)) return d;
+    const f2 t = f2_mul(d, f2_dup(inv));
+    return f2_fma(f2_dup(-L), make_float2(rintf(t.x), rintf(t.y)), d);
+}
+
+template <bool PER>
+__device__ __forceinline__ f2 screen_r2(const Screen &s, const Box &L, float4 a, float4 b)
+{
+    f2 ex = f2_sub(make_float2(a.x, a.y), f2_dup(s.x)), ey = f2_sub(make_float2(a.z, a.w), f2_dup(s.y)),
+       ez = f2_sub(make_float2(b.x, b.y), f2_dup(s.z));
     if (PER) {
-        ex = image_f(ex, L.fx, L.ix);
-        ey = image_f(ey, L.fy, L.iy);
-        ez = image_f(ez, L.fz, L.iz);
+        ex = image_f2(ex, L.fx, L.ix);
+        ey = image_f2(ey, L.fy, L.iy);
+        ez = image_f2(ez, L.fz, L.iz);
     }
-    return fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+    return f2_fma(ex, ex, f2_fma(ey, ey, f2_mul(ez, ez)));
 }
 
 // nearest[i] = min over this CTA's sources of an upper bound on the distance
@@ -125,12 +140,16 @@ __global__ void __launch_bounds__(kFThreads) nearest_kernel(const double *__rest
         __syncthreads();
         const int cnt = min(kFThreads, j1 - t0);
 #pragma unroll 4
-        for (int k = 0; k < cnt; ++k) {
-            const float4 q = tile[k];
-            const float r2 = screen_r2<PER>(s, L, q);
-            if (r2 < best && r2 > q.w * q.w) {
-                best = r2;
-                err = q.w;
+        for (int k = 0; k < cnt; k += 2) {
+            const float4 a = tile[k], b = tile[k + 1];
+            const f2 r2 = screen_r2<PER>(s, L, a, b), w2 = f2_mul(make_float2(b.z, b.w), make_float2(b.z, b.w));
+            if (r2.x < best && r2.x > w2.x) {
+                best = r2.x;
+                err = b.z;
+            }
+            if (r2.y < best && r2.y > w2.y) {
+                best = r2.y;
+                err = b.w;
             }
         }
     }
@@ -176,10 +195,13 @@ __global__ void __launch_bounds__(kFThreads) blob_blob_kernel(const double *__re
                 if (L.y > 0) dy = project(dy, L.y);
                 if (L.z > 0) dz = project(dz, L.z);
             }
-            const double rn = sqrt(dx * dx + dy * dy + dz * dz);
+            // 1/r by rsqrt64, r = r^2 / r with one Newton correction (nine FP64 instructions instead of
+            // the library's square root and division, about 35)
+            const double r2 = dx * dx + dy * dy + dz * dz, invr = rsqrt64(r2), r0 = r2 * invr;
+            const double rn = fma(fma(-r0, r0, r2), 0.5 * invr, r0);
             if (!(rn > 0.0) || rn > rc) continue;  // coincident: no direction; beyond rc: exactly zero
             const double g = (rn > two_a) ? exp(-(rn - two_a) * inv_b) : 1.0;
-            const double m = eps_over_b * g / rn;
+            const double m = eps_over_b * g * invr;
             fx -= m * dx;
             fy -= m * dy;
             fz -= m * dz;
@@ -194,10 +216,12 @@ __global__ void __launch_bounds__(kFThreads) blob_blob_kernel(const double *__re
         const int cnt = min(kFThreads, j1 - t0);
         for (int k0 = 0; k0 < cnt; k0 += kPend / 2) {
             const int k1 = min(cnt, k0 + kPend / 2);
-            for (int k = k0; k < k1; ++k) {
-                const float4 q = tile[k];
-                const float t = cut + q.w;
-                if (!(screen_r2<PER>(s, L, q) >= t * fabsf(t)) && t0 + k != i) pend[np++][tid] = t0 + k;
+            for (int k = k0; k < k1; k += 2) {
+                const float4 a = tile[k], b = tile[k + 1];
+                const f2 r2 = screen_r2<PER>(s, L, a, b), t = f2_add(f2_dup(cut), make_float2(b.z, b.w));
+                const f2 t2 = f2_mul(t, make_float2(fabsf(t.x), fabsf(t.y)));
+                if (!(r2.x >= t2.x) && t0 + k != i) pend[np++][tid] = t0 + k;
+                if (!(r2.y >= t2.y) && t0 + k + 1 != i && k + 1 < cnt) pend[np++][tid] = t0 + k + 1;
             }
             if (__any_sync(0xffffffffu, np > kPend / 2)) drain();
         }
