@@ -63,7 +63,7 @@ DF64_UF_TRAFFIC_BYTES = {"symmetric": 745472, "standard": 794624}
 # counted twice as above ((smsp__inst_executed.sum 17,258,189,476 + packed 12,838,677,918) * 32 / (N^2 * 16),
 # 60,000 blobs)
 MULTI16_INST_PER_PAIR_RHS = 16.72
-DF64_UF_KERNEL_SOURCE_SHA = "9f4e60b55215de2cf1365c2b6d03868d0daabff7b6ec8eab58923e465a7eae13"
+DF64_UF_KERNEL_SOURCE_SHA = "aafb1ddcb05cb24774fcf881ec791450c48536f10890bfa6fb9fb2a39e6e6b05"
 
 
 def df64_uf_kernel_source_sha():

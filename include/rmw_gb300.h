@@ -209,8 +209,8 @@ int rmw_wall_autotune_lookup(int kind, int mode, int64_t n, int *nchunks, int *t
  * deterministic partial sums take ceil(n/128) x 3n doubles, 5.5 GB at
  * 172,032 blobs, within an eighth of the device memory and at least 6 GiB:
  * about 430,000 blobs on a 284 GB device).  Without a tuned or pinned
- * choice the products use the symmetric kernel from 4,096 blobs in FP64 and
- * df64 and from 8,192 in mixed precision. */
+ * choice the products use the symmetric kernel from 256 blobs in FP64 (also
+ * periodic in x and / or y) and df64 and from 8,192 in mixed precision. */
 int rmw_wall_autotune_set(int kind, int mode, int64_t n, int nchunks);
 /* Library-only (no reference counterpart): how a product of (kind, mode, n)
  * runs on the current device - 0 the one-sided kernel, 1 the symmetric kernel

@@ -27,6 +27,7 @@
 //                 b_i and the 1/(8 pi eta a^p) factor.
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstdio>
 #include <mutex>
 #include <vector>
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(kThreads) wall_pair_df_kernel(const SrcDF *__r
 constexpr int kSymWarps = kThreads / 32;
 
 // The steps of this CTA's tile pair: all of them, or (FP64 and df64 products
-// of few tiles) one of gridDim.y equal ranges, each with its own slots.
+// of few tiles) one of gridDim.y contiguous ranges, each with its own slots.
 struct SymSteps {
     int k0, k1, nsplit, split;
     __device__ __forceinline__ int slot(int tile) const { return tile * nsplit + split; }
@@ -256,8 +257,8 @@ template <bool WHOLE>
 __device__ __forceinline__ SymSteps sym_steps()
 {
     if (WHOLE) return {0, kTile, 1, 0};
-    const int m = kTile / gridDim.y, s = blockIdx.y;
-    return {s * m, (s + 1) * m, (int)gridDim.y, s};
+    const int m = gridDim.y, s = blockIdx.y;
+    return {kTile * s / m, kTile * (s + 1) / m, m, s};
 }
 
 // The CTA's tile pair: from blockIdx.x over the upper triangle of nt tiles, or
@@ -821,15 +822,34 @@ __global__ void __launch_bounds__(kThreads) wall_rot_mixed_sym_kernel(const SrcF
     mixed_sym_body<SEG, KIND>(src, n, nt, partial, jobs);
 }
 
+// One ordered pair in FP64, accumulated (UF: (3/2) M v through the explicit
+// block).
+template <int KIND, bool ZPER>
+__device__ __forceinline__ void pair_acc_d(double dx, double dy, double dz, double Rz, double hi, double hj, double vx,
+                                           double vy, double vz, double &ux, double &uy, double &uz)
+{
+    if constexpr (KIND == RMW_UF) {
+        const UFBlockD m = uf_block_d<ZPER>(dx, dy, dz, Rz, hi, hj);
+        uf_block_acc_d(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
+    } else {
+        pair_contrib<KIND, double>(dx, dy, dz, Rz, hi, hj, vx, vy, vz, ux, uy, uz);
+    }
+}
 // Symmetric FP64 kernel of any kind: the same grid, pairing and partial-sum
 // slots, FP64 pair arithmetic (the FP64 pipe bounds it, so halving the
 // coefficient work per ordered pair is the gain); source-side sums per warp
 // in FP64 shared memory.  UF through the explicit block of uf_block_d: the
 // 10,752-blob product 11.6 -> 8.1 ms, 73 FP64 instructions per pair at 98 %
 // of the pipe's measured rate (0.53 T instructions/s).
-template <bool SEG, int KIND, bool NOWALL = false>
+// PER (periodic in x and / or y): a pair is its minimum image and the
+// neighbour boxes' images, each both ways (the reverse separations are the
+// negatives of the same set); a blob's own images are added once, to the
+// diagonal tile's first split.  Separations in the one-sided kernel's order of
+// operations, so both kernels choose the same images.
+template <bool SEG, int KIND, bool NOWALL = false, bool PER = false>
 __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int n, int nt, double inva,
-                                              double *__restrict__ partial, const SymJob *__restrict__ jobs)
+                                              double *__restrict__ partial, const SymJob *__restrict__ jobs,
+                                              const Periodic P = Periodic{0.0, 0.0, 0.0})
 {
     __shared__ double tx[kTile], ty[kTile], tz[kTile], tvx[kTile], tvy[kTile], tvz[kTile];
     __shared__ double sacc[kSymWarps][3][kTile];
@@ -842,12 +862,13 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
     // a target or source past the end is a dummy far above the wall with a zero vector
     const SrcD dummy = {1.0e6, 1.0e6, 1.0e6, 0.0, 0.0, 0.0, 0.0, 0.0};
     const SrcD me = valid_i ? src[i] : dummy;
-    const double xi = me.x * inva, yi = me.y * inva, zi = me.z * inva;
+    // in radii; PER: x and y as given, scaled after the image shift
+    const double xi = PER ? me.x : me.x * inva, yi = PER ? me.y : me.y * inva, zi = me.z * inva;
     {
         const int j = S * kTile + tid;
         const SrcD sj = (j < n) ? src[j] : dummy;
-        tx[tid] = sj.x * inva;
-        ty[tid] = sj.y * inva;
+        tx[tid] = PER ? sj.x : sj.x * inva;
+        ty[tid] = PER ? sj.y : sj.y * inva;
         tz[tid] = sj.z * inva;
         tvx[tid] = sj.vx;
         tvy[tid] = sj.vy;
@@ -860,17 +881,30 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
     auto step = [&](int k) {
         const int jl = (lane + k) & (kTile - 1);
         const double zj = tz[jl];
-        const double dx = xi - tx[jl], dy = yi - ty[jl], dz = zi - zj, Rz = zi + zj;
         const double vx = tvx[jl], vy = tvy[jl], vz = tvz[jl];
         double wx = sacc[warp][0][jl], wy = sacc[warp][1][jl], wz = sacc[warp][2][jl];
-        if constexpr (NOWALL) {
-            pair_rpy_sym<double, KIND>(dx, dy, dz, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
-        } else if constexpr (KIND == RMW_UF) {
-            const UFBlockD m = uf_block_d<false>(dx, dy, dz, Rz, zi, zj);
-            uf_block_acc_d(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
-            uf_block_acc_d(m, m.t4, m.t3, dx, dy, me.vx, me.vy, me.vz, wx, wy, wz);
+        auto pair = [&](double dx, double dy) {
+            const double dz = zi - zj, Rz = zi + zj;
+            if constexpr (NOWALL) {
+                pair_rpy_sym<double, KIND>(dx, dy, dz, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
+            } else if constexpr (KIND == RMW_UF) {
+                const UFBlockD m = uf_block_d<false>(dx, dy, dz, Rz, zi, zj);
+                uf_block_acc_d(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
+                uf_block_acc_d(m, m.t4, m.t3, dx, dy, me.vx, me.vy, me.vz, wx, wy, wz);
+            } else {
+                pair_rot_sym_d<KIND>(dx, dy, dz, Rz, zi, zj, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy,
+                                     wz);
+            }
+        };
+        if constexpr (PER) {
+            double rx = xi - tx[jl], ry = yi - ty[jl];
+            if (P.Lx > 0) rx = project(rx, P.Lx);
+            if (P.Ly > 0) ry = project(ry, P.Ly);
+            const int px = P.Lx > 0, py = P.Ly > 0;
+            for (int bx = -px; bx <= px; ++bx)
+                for (int by = -py; by <= py; ++by) pair((rx + bx * P.Lx) * inva, (ry + by * P.Ly) * inva);
         } else {
-            pair_rot_sym_d<KIND>(dx, dy, dz, Rz, zi, zj, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
+            pair(xi - tx[jl], yi - ty[jl]);
         }
         sacc[warp][0][jl] = wx;
         sacc[warp][1][jl] = wy;
@@ -883,6 +917,16 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
             const int off = (k - 32 * warp) & (kTile - 1);
             if (off == 0 || off > kTile / 2 || (off == kTile / 2 && warp >= kSymWarps / 2)) continue;
             step(k);
+        }
+        if constexpr (PER) {
+            if (sp.split == 0) {  // the blob's own images, each of them once
+                const int px = P.Lx > 0, py = P.Ly > 0;
+                for (int bx = -px; bx <= px; ++bx)
+                    for (int by = -py; by <= py; ++by)
+                        if (bx || by)
+                            pair_acc_d<KIND, true>(bx * P.Lx * inva, by * P.Ly * inva, 0.0, 2.0 * zi, zi, zi, me.vx,
+                                                   me.vy, me.vz, ux, uy, uz);
+            }
         }
     } else {
         for (int k = sp.k0; k < sp.k1; ++k) {
@@ -922,6 +966,14 @@ __global__ void __launch_bounds__(kThreads) wall_fp64_sym_kernel(const SrcD *__r
                                                                   const SymJob *__restrict__ jobs)
 {
     fp64_sym_body<SEG, KIND>(src, n, nt, inva, partial, jobs);
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(kThreads) wall_fp64_per_sym_kernel(const SrcD *__restrict__ src, int n, int nt,
+                                                                      double inva, Periodic P,
+                                                                      double *__restrict__ partial)
+{
+    fp64_sym_body<false, KIND, false, true>(src, n, nt, inva, partial, nullptr, P);
 }
 
 // Free-space (no wall) symmetric kernels: the same bodies with pair_rpy_sym;
@@ -978,18 +1030,7 @@ int nowall_sym_launch(int kind, int mode, const void *src, int n, double *partia
 }
 
 // ---------------------------------------------------------------------------
-// FP64 pair kernel (UF: (3/2) M v through the explicit block)
-template <int KIND, bool ZPER>
-__device__ __forceinline__ void pair_acc_d(double dx, double dy, double dz, double Rz, double hi, double hj, double vx,
-                                           double vy, double vz, double &ux, double &uy, double &uz)
-{
-    if constexpr (KIND == RMW_UF) {
-        const UFBlockD m = uf_block_d<ZPER>(dx, dy, dz, Rz, hi, hj);
-        uf_block_acc_d(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
-    } else {
-        pair_contrib<KIND, double>(dx, dy, dz, Rz, hi, hj, vx, vy, vz, ux, uy, uz);
-    }
-}
+// FP64 pair kernel
 template <int KIND, bool PER, bool SEG>
 __global__ void __launch_bounds__(kThreads) wall_pair_fp64_kernel(const SrcD *__restrict__ src, int n, int chunk,
                                                                    double inva, Periodic P,
@@ -1598,40 +1639,64 @@ size_t wall_sym_partial_budget()
     return cap ? std::min(b, cap) : b;
 }
 
-constexpr int kSplitMax = 32;
-constexpr int kSplitCtasFp64 = 24, kSplitCtasDf64 = 12;
+constexpr int kSplitMax = 64;
+constexpr double kSplitBytes = 64e6;  // partial sums of a split product: they stay in L2
+
+// periodic in x and / or y only: the FP64 kernel has a symmetric form
+static bool per_sym(int mode, const double *L)
+{
+    return mode == RMW_MODE_FP64 && L && (L[0] > 0 || L[1] > 0) && !(L[2] > 0);
+}
 
 bool wall_sym_applicable(int kind, int mode, int n, const double *L)
 {
     if (kind < RMW_UF || kind > RMW_WT ||
         (mode != RMW_MODE_FP64 && mode != RMW_MODE_DF64 && mode != RMW_MODE_MIXED))
         return false;
-    if (L && (L[0] > 0 || L[1] > 0 || L[2] > 0)) return false;
+    if (L && (L[0] > 0 || L[1] > 0 || L[2] > 0) && !per_sym(mode, L)) return false;
     if (n < 2 * kTile) return false;
     const double nt = (double)((n + kTile - 1) / kTile);
     return nt * 3.0 * (double)n * sizeof(double) <= (double)wall_sym_partial_budget();
 }
 
-// How many CTAs share the steps of a tile pair (a power of two).  Below about
-// 4,000 blobs the tile pairs alone leave SMs idle (2,048 blobs: 136 of them);
-// the split fills the GPU with the symmetric kernel's work per pair where the
-// one-sided kernel used to do each pair twice (2,048 blobs: FP64 UF 961 ->
-// 364 us, df64 181 -> 74).  Measured by CTAs per SM wanted: df64 UF, 2,048
-// blobs 6: 72, 12: 74, 24: 81 us, 5,003 blobs 6: 287, 12: 269, 24: 279; FP64
-// UF, 2,048 blobs 3: 365, 12: 357, 24: 364 us, 10,752 blobs, where the six
-// CTAs that share an SM's FP64 pipe end together, 12: 8.24, 24: 8.10 ms.
-// Mixed products keep whole tile pairs: their FP32 sums would change with the
-// split.
-int wall_sym_split(int mode, int n)
+// How many CTAs share the steps of a tile pair.  Below about 4,000 blobs the
+// tile pairs alone leave SMs idle (2,048 blobs: 136 of them); the split fills
+// the GPU with the symmetric kernel's work per pair where the one-sided kernel
+// used to do each pair twice (2,048 blobs: FP64 UF 961 -> 364 us, df64 181 ->
+// 70).  With P tile pairs, s CTAs each and a CTA's start and end worth e steps,
+// an SM takes (P s / 152 + d)(128 / s + e) step times, d the uneven end of the
+// grid: least at s = sqrt(152 * 128 d / (e P)).  Measured by s: df64 UF 2,048
+// blobs 8: 72, 16: 74, 32: 81 us; 5,003 blobs 2: 275, 4: 259, 8: 279 us; FP64
+// UF 10,752 blobs 1: 8.24, 2: 8.08 ms; FP64 periodic 4,800 blobs 2: 15.2,
+// 8: 14.8 ms, which K = 13,000 (df64), 40,000 (FP64) and 160,000 (periodic
+// FP64, whose steps are nine times as long) in s = sqrt(K / P) reproduce.
+// Where even 64 CTAs per pair are fewer than 16 per SM, the split whose
+// busiest SM has least to do (504 blobs FP64: 43, 48 us; 32: 54 us).  Mixed
+// products keep whole tile pairs: their FP32 sums would change with the split.
+int wall_sym_split(int mode, int n, bool periodic)
 {
     if (mode == RMW_MODE_MIXED) return 1;
+    const bool fp64 = mode == RMW_MODE_FP64;
     const double nt = (double)sym_tiles(n), pairs = 0.5 * nt * (nt + 1);
-    const double want = 152.0 * (mode == RMW_MODE_FP64 ? kSplitCtasFp64 : kSplitCtasDf64);
+    const double slot = nt * 3.0 * (double)n * sizeof(double);
+    const double bytes = std::min((double)wall_sym_partial_budget(), kSplitBytes);
     int s = 1;
-    while (s < kSplitMax && pairs * s < want &&
-           nt * (2 * s) * 3.0 * (double)n * sizeof(double) <= (double)wall_sym_partial_budget())
-        s *= 2;
-    return s;
+    if (pairs * kSplitMax < 16 * 152.0) {
+        const double ends = periodic ? 0.05 : fp64 ? 0.4 : 1.2, fill = fp64 ? 2.0 : 6.0;
+        double cost = 0.0;
+        for (int c = 1; c <= kSplitMax; ++c) {
+            const double t = std::max(std::ceil(pairs * c / 152.0), fill) * (std::ceil((double)kTile / c) + ends);
+            if (c == 1 || t < 0.99 * cost) {
+                cost = t;
+                s = c;
+            }
+        }
+    } else {
+        s = (int)std::min((double)kSplitMax, std::sqrt((periodic ? 160000.0 : fp64 ? 40000.0 : 13000.0) / pairs) +
+                                                     (fp64 ? 0.5 : 0.05));  // whole df64 pairs have constant bounds
+    }
+    while (s > 1 && slot * s > bytes) --s;
+    return std::max(1, s);
 }
 
 int wall_sym_slots(int n, int nsplit) { return sym_tiles(n) * nsplit; }
@@ -1694,6 +1759,28 @@ static void launch_sym_finalize(const double *r, const double *v, const double *
 {
     if (mixed) launch_sym_finalize_t<KIND, true>(r, v, partial, nt, out, n, a, nf, B, st);
     else launch_sym_finalize_t<KIND, false>(r, v, partial, nt, out, n, a, nf, B, st);
+}
+
+// The FP64 product periodic in x and / or y through the symmetric kernel.
+// Measured, M_UF of 1,500 blobs in a square box: one-sided 2.94, symmetric
+// 1.62 ms (FP64 pipe floor 1.5); the images of a pair share its minimum-image division.
+template <int KIND>
+static int per_sym_product(const double *r, const double *v, double *out, int n, double a, double nf, const double *L,
+                           cudaStream_t st, void *scratch_ptr, int nsplit)
+{
+    const int nt = sym_tiles(n);
+    const size_t packed = ((sizeof(SrcD) * (size_t)n + 255) / 256) * 256;
+    SrcD *src = (SrcD *)scratch_ptr;
+    double *partial = (double *)((char *)scratch_ptr + packed);
+    pack_fp64_kernel<<<pack_blocks(n), kPackThreads, 0, st>>>(r, v, src, n, a);
+    const dim3 ncta((unsigned)((long long)nt * (nt + 1) / 2), nsplit);
+    void *tok = nullptr;
+    if (int rc = trace_begin(TRACE_PAIR, st, &tok)) return rc;
+    wall_fp64_per_sym_kernel<KIND><<<ncta, kThreads, 0, st>>>(src, n, nt, 1.0 / a, Periodic{L[0], L[1], 0.0}, partial);
+    if (int rc = trace_end(tok, st)) return rc;
+    launch_sym_finalize<KIND>(r, v, partial, nt * nsplit, out, n, a, nf, nullptr, st);
+    RMW_CHECK_LAUNCH("symmetric periodic wall product kernels");
+    return RMW_OK;
 }
 
 // pack, symmetric pair kernel and finalize of any kind (B: segmented over its suspensions)
@@ -1808,8 +1895,8 @@ int wall_product(int kind, const double *r, const double *v, double *out, int64_
     if (n == 0) return RMW_OK;
     int nchunks = wall_prefers_sym(kind, mode, (int)n) ? kSymChunks : wall_chunks(kind, mode, (int)n);
     bool sym = nchunks == kSymChunks && wall_sym_applicable(kind, mode, (int)n, L);
-    const int nsplit = sym ? wall_sym_split(mode, (int)n) : 1;
     const bool periodic = L && (L[0] > 0 || L[1] > 0 || L[2] > 0);
+    const int nsplit = sym ? wall_sym_split(mode, (int)n, periodic) : 1;
     void *ws = nullptr;
     if (nchunks == kSymChunks && !sym && mode == RMW_MODE_DF64 && !periodic && n >= 2 * kTile) {
         // too many tiles for one partial-sum slot per tile: the symmetric kernel band by band
@@ -1833,6 +1920,15 @@ int wall_product(int kind, const double *r, const double *v, double *out, int64_
         rc = scratch(SCRATCH_PAIR, wall_scratch_bytes((int)n, mode, nchunks), &ws, st);
     }
     if (rc) return rc;
+    if (sym && periodic) {
+        const double nf = kind_norm(kind, eta, a);
+        switch (kind) {
+        case RMW_UF: return per_sym_product<RMW_UF>(r, v, out, (int)n, a, nf, L, st, ws, nsplit);
+        case RMW_UT: return per_sym_product<RMW_UT>(r, v, out, (int)n, a, nf, L, st, ws, nsplit);
+        case RMW_WF: return per_sym_product<RMW_WF>(r, v, out, (int)n, a, nf, L, st, ws, nsplit);
+        default: return per_sym_product<RMW_WT>(r, v, out, (int)n, a, nf, L, st, ws, nsplit);
+        }
+    }
     if (sym) return wall_product_sym_with_scratch(kind, r, v, out, (int)n, eta, a, mode, st, ws, nsplit);
     return wall_product_with_scratch(kind, r, v, out, (int)n, eta, a, L, mode, st, ws, nchunks);
 }

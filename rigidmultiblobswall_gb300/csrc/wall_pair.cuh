@@ -87,7 +87,7 @@ constexpr size_t kSymMaxPartialBytes = size_t(6) << 30;  // up to ~185,000 blobs
 size_t wall_sym_partial_budget();
 bool wall_sym_applicable(int kind, int mode, int n, const double *L);
 // CTAs per tile pair of the symmetric kernels, and their partial-sum slots
-int wall_sym_split(int mode, int n);
+int wall_sym_split(int mode, int n, bool periodic = false);
 int wall_sym_slots(int n, int nsplit);
 // banded symmetric df64 product (above the partial-sum budget): tile rows per band, its scratch
 int wall_sym_band_rows(int n);
