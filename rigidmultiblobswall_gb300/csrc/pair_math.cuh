@@ -337,30 +337,41 @@ __device__ __forceinline__ void uf_apply<float>(const UFCoeffs<float> &c, float 
 // both ways, against 93 of uf_coeffs / uf_apply: the FP64 pipe bounds the
 // kernels that use it (1/64 of the FP32 rate).  ZPER: dz is an image's and
 // not h_i - h_j.
+struct PairGeoD {
+    double r2, invr, i2, u, s, t, p;
+};
+template <bool ZPER>
+__device__ __forceinline__ PairGeoD pair_geo_d(double dx, double dy, double dz, double Rz, double hi, double hj)
+{
+    PairGeoD g;
+    const double rho2 = fma(dx, dx, dy * dy);
+    g.r2 = fma(dz, dz, rho2);
+    g.invr = rsqrt64(g.r2);
+    g.s = rsqrt64(ZPER ? fma(Rz, Rz, rho2) : fma(4.0 * hi, hj, g.r2));
+    g.i2 = g.invr * g.invr;
+    g.u = g.s * g.s;
+    g.t = g.u * g.s;
+    g.p = g.t * g.u;
+    return g;
+}
 struct UFBlockD {
     double Af, b2, t3, t4, zz;
 };
 template <bool ZPER>
-__device__ __forceinline__ UFBlockD uf_block_d(double dx, double dy, double dz, double Rz, double hi, double hj)
+__device__ __forceinline__ UFBlockD uf_block_d(const PairGeoD &g, double dz, double Rz, double hi, double hj)
 {
-    const double rho2 = fma(dx, dx, dy * dy);
-    const double r2 = fma(dz, dz, rho2);
-    const double k = hi * hj;
-    const double invr = rsqrt64(r2);
-    const double z2 = Rz * Rz;
-    const double s = rsqrt64(ZPER ? rho2 + z2 : fma(4.0, k, r2));
-    const double i2 = invr * invr;
-    double ia = invr, a3 = i2 * invr;
-    double Bc = fma(-3.0, i2, 1.5) * a3;
-    const bool near = !(r2 > 4.0);  // r <= 2
+    const double k = hi * hj, z2 = Rz * Rz;
+    double ia = g.invr, a3 = g.i2 * g.invr;
+    double Bc = fma(-3.0, g.i2, 1.5) * a3;
+    const bool near = !(g.r2 > 4.0);  // r <= 2
     if (__any_sync(__activemask(), near)) {
         if (near) {
             ia = 0.0;
-            a3 = fma(-0.5625, r2 * invr, 2.0);
-            Bc = 0.1875 * invr;
+            a3 = fma(-0.5625, g.r2 * g.invr, 2.0);
+            Bc = 0.1875 * g.invr;
         }
     }
-    const double u = s * s, t = u * s, p = t * u;
+    const double s = g.s, u = g.u, t = g.t, p = g.p;
     const double E = z2 * u;
     const double b1 = fma(3.0, z2, 1.0);
     const double w5 = fma(-5.0, E, b1), w7 = fma(-7.0, E, b1);
@@ -374,9 +385,9 @@ __device__ __forceinline__ UFBlockD uf_block_d(double dx, double dy, double dz, 
     m.b2 = fma(p, Y, F);
     double G, dG;  // dz F, dz^2 F
     if constexpr (ZPER) {
-        const double dw = hi - hj, g = dz * Bc, w = -1.5 * t * dw;
-        G = g + w;
-        dG = fma(dz, g, dw * w);
+        const double dw = hi - hj, x = dz * Bc, w = -1.5 * t * dw;
+        G = x + w;
+        dG = fma(dz, x, dw * w);
     } else {
         G = dz * F;
         dG = dz * G;
@@ -401,64 +412,79 @@ __device__ __forceinline__ void uf_block_acc_d(const UFBlockD &m, double t3, dou
 // rot_block_df and wt_block_df (pair_math_df.cuh), where they are derived: 64
 // (UT, WF) and 62 (WT) FP64 instructions a pair against 91 and 74 of the
 // tensor forms.  10,752 blobs: UT 9.82 -> 7.01 ms, WF 9.97 -> 7.01, WT 8.08 ->
-// 7.06.
-template <int KIND>
-__device__ __forceinline__ void pair_rot_sym_d(double dx, double dy, double dz, double Rz, double hi, double hj,
-                                               double vx, double vy, double vz, double qx, double qy, double qz,
-                                               double &ux, double &uy, double &uz, double &wx, double &wy, double &wz)
+// 7.06.  UF32: the blocks times 3/2, as the UF block (for sums of both).
+struct RotBlockD {
+    double a, ar, b, ei, ej, wi, wj;
+};
+template <bool UF32 = false>
+__device__ __forceinline__ RotBlockD rot_block_d(const PairGeoD &g, double dz, double Rz, double hi, double hj)
 {
-    const double r2 = fma(dz, dz, fma(dx, dx, dy * dy));
-    const double invr = rsqrt64(r2);
-    const double s = rsqrt64(fma(4.0 * hi, hj, r2));
-    const double i2 = invr * invr, u = s * s, t = u * s, p = t * u;
-    const bool near = !(r2 >= 4.0);  // r < 2
-    if constexpr (KIND == RMW_WT) {
-        const double i3 = i2 * invr;
-        double A = -0.5 * i3, Bc = 1.5 * i2 * i3;
-        if (__any_sync(__activemask(), near)) {
-            if (near) {
-                const double r = r2 * invr;
-                A = fma(fma(0.078125, r2, -0.84375), r, 1.0);
-                Bc = fma(-0.046875, r, 0.28125 * invr);
-            }
-        }
-        const double Et = Rz * Rz * u * t, D = Bc * dz, X = 1.5 * p * Rz;
-        UFBlockD m;
-        m.Af = fma(-6.0, Et, fma(3.5, t, A));
-        m.b2 = fma(-4.5, p, Bc);
-        m.t3 = D - X;
-        m.t4 = D + X;
-        m.zz = fma(D, dz, fma(-1.5, Et, fma(0.5, t, A)));
-        uf_block_acc_d(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
-        uf_block_acc_d(m, m.t4, m.t3, dx, dy, qx, qy, qz, wx, wy, wz);
-    } else {
-        double c = i2 * invr;
-        if (__any_sync(__activemask(), near)) {
-            if (near) c = fma(-0.1875, r2 * invr, 0.5);
-        }
-        const double b = t - c, m = dz * b, Rp = Rz * p, a = fma(2.0, Rp, -m), ar = fma(2.0, Rp, m);
-        const double Ru = Rz * u, R10 = 10.0 * Ru, R6 = 6.0 * Rz, y = fma(-10.0 * Rz, Ru, 2.0);
-        const double ei = p * fma(-6.0, hi, R10), ej = p * fma(-6.0, hj, R10);
-        const double wi = fma(p, fma(R6, hi, y), b), wj = fma(p, fma(R6, hj, y), b);
-        const double Q = fma(dy, vx, -dx * vy), Qq = fma(dy, qx, -dx * qy);
-        if constexpr (KIND == RMW_UT) {
-            const double bv = b * vz, eQ = ei * Q, bq = b * qz, eq = ej * Qq;
-            ux = fma(a, vy, fma(bv, dy, fma(eQ, dx, ux)));
-            uy = fma(-a, vx, fma(-bv, dx, fma(eQ, dy, uy)));
-            uz = fma(-wi, Q, uz);
-            wx = fma(ar, qy, fma(-bq, dy, fma(eq, dx, wx)));
-            wy = fma(-ar, qx, fma(bq, dx, fma(eq, dy, wy)));
-            wz = fma(wj, Qq, wz);
-        } else {
-            const double H = fma(ej, fma(dy, vy, dx * vx), wj * vz), Hq = fma(ei, fma(dy, qy, dx * qx), -wi * qz);
-            ux = fma(-ar, vy, fma(H, dy, ux));
-            uy = fma(ar, vx, fma(-H, dx, uy));
-            uz = fma(-b, Q, uz);
-            wx = fma(-a, qy, fma(Hq, dy, wx));
-            wy = fma(a, qx, fma(-Hq, dx, wy));
-            wz = fma(b, Qq, wz);
+    constexpr double f = UF32 ? 1.5 : 1.0;
+    double c = g.i2 * g.invr;
+    const bool near = !(g.r2 >= 4.0);  // r < 2
+    if (__any_sync(__activemask(), near)) {
+        if (near) c = fma(-0.1875, g.r2 * g.invr, 0.5);
+    }
+    RotBlockD k;
+    k.b = UF32 ? 1.5 * (g.t - c) : g.t - c;
+    const double m = dz * k.b, Rp = Rz * g.p, Ru = Rz * g.u;
+    k.a = fma(2.0 * f, Rp, -m);
+    k.ar = fma(2.0 * f, Rp, m);
+    const double R10 = 10.0 * f * Ru, R6 = 6.0 * f * Rz, y = fma(-10.0 * f * Rz, Ru, 2.0 * f);
+    k.ei = g.p * fma(-6.0 * f, hi, R10);
+    k.ej = g.p * fma(-6.0 * f, hj, R10);
+    k.wi = fma(g.p, fma(R6, hi, y), k.b);
+    k.wj = fma(g.p, fma(R6, hj, y), k.b);
+    return k;
+}
+template <bool UF32 = false>
+__device__ __forceinline__ UFBlockD wt_block_d(const PairGeoD &g, double dz, double Rz)
+{
+    constexpr double f = UF32 ? 1.5 : 1.0;
+    const double i3 = g.i2 * g.invr;
+    double A = -0.5 * f * i3, Bc = 1.5 * f * g.i2 * i3;
+    const bool near = !(g.r2 >= 4.0);
+    if (__any_sync(__activemask(), near)) {
+        if (near) {
+            const double r = g.r2 * g.invr;
+            A = f * fma(fma(0.078125, g.r2, -0.84375), r, 1.0);
+            Bc = f * fma(-0.046875, r, 0.28125 * g.invr);
         }
     }
+    const double Et = Rz * Rz * g.u * g.t, D = Bc * dz, X = 1.5 * f * g.p * Rz;
+    UFBlockD m;
+    m.Af = fma(-6.0 * f, Et, fma(3.5 * f, g.t, A));
+    m.b2 = fma(-4.5 * f, g.p, Bc);
+    m.t3 = D - X;
+    m.t4 = D + X;
+    m.zz = fma(D, dz, fma(-1.5 * f, Et, fma(0.5 * f, g.t, A)));
+    return m;
+}
+__device__ __forceinline__ void ut_acc_d(const RotBlockD &k, double dx, double dy, double vx, double vy, double vz,
+                                         double qx, double qy, double qz, double &ux, double &uy, double &uz,
+                                         double &wx, double &wy, double &wz)
+{
+    const double Q = fma(dy, vx, -dx * vy), Qq = fma(dy, qx, -dx * qy);
+    const double bv = k.b * vz, eQ = k.ei * Q, bq = k.b * qz, eq = k.ej * Qq;
+    ux = fma(k.a, vy, fma(bv, dy, fma(eQ, dx, ux)));
+    uy = fma(-k.a, vx, fma(-bv, dx, fma(eQ, dy, uy)));
+    uz = fma(-k.wi, Q, uz);
+    wx = fma(k.ar, qy, fma(-bq, dy, fma(eq, dx, wx)));
+    wy = fma(-k.ar, qx, fma(bq, dx, fma(eq, dy, wy)));
+    wz = fma(k.wj, Qq, wz);
+}
+__device__ __forceinline__ void wf_acc_d(const RotBlockD &k, double dx, double dy, double vx, double vy, double vz,
+                                         double qx, double qy, double qz, double &ux, double &uy, double &uz,
+                                         double &wx, double &wy, double &wz)
+{
+    const double Q = fma(dy, vx, -dx * vy), Qq = fma(dy, qx, -dx * qy);
+    const double H = fma(k.ej, fma(dy, vy, dx * vx), k.wj * vz), Hq = fma(k.ei, fma(dy, qy, dx * qx), -k.wi * qz);
+    ux = fma(-k.ar, vy, fma(H, dy, ux));
+    uy = fma(k.ar, vx, fma(-H, dx, uy));
+    uz = fma(-k.b, Q, uz);
+    wx = fma(-k.a, qy, fma(Hq, dy, wx));
+    wy = fma(k.a, qx, fma(-Hq, dx, wy));
+    wz = fma(k.b, Qq, wz);
 }
 
 // ---------------------------------------------------------------------------

@@ -245,24 +245,35 @@ __device__ __forceinline__ void uf_near_df(df2 r2, df2 invr, df2 &ia, df2 &a3, d
     }
 }
 
+// What the blocks of a pair share: r^2, 1/r, 1/r^2 and the powers of s = 1/R.
 // h4 = 4 h_i, hj, Rz = h_i + h_j (may be unnormalised).  ZPER: dz is an
 // image's and not h_i - h_j (= dw), so R^2 and the wall parts of G and zz are
 // formed from the heights.
+template <class D> struct PairGeoDF {
+    D r2, invr, i2, s, u, t, p;
+};
 template <class D, bool ZPER = false>
-__device__ __forceinline__ UFBlockDF<D> uf_block_df(D dx, D dy, D dz, D Rz, D h4, D hj, D dw = D{})
+__device__ __forceinline__ PairGeoDF<D> pair_geo_df(D dx, D dy, D dz, D Rz, D h4, D hj)
 {
+    PairGeoDF<D> g;
     const D rho2 = add_u(sqr_u(dx), sqr_u(dy));
-    const D r2 = norm(add_u(sqr_u(dz), rho2));
-    const D invr = rsqrt_df(r2);
-    const D k4 = mul_u(h4, hj);
-    const D s = rsqrt_far_df(norm(ZPER ? add_u(rho2, sqr_u(Rz)) : add_u(r2, k4)));
-    const D i2 = sqr(invr);
-    D ia = invr, a3 = mul_u(i2, invr);
-    D Bc = mul_u(add_fast_u(1.5f, mul_u(i2, -3.0f)), a3);
-    uf_near_df(r2, invr, ia, a3, Bc);
-    const D u = sqr(s);
-    const D t = mul_u(u, s);
-    const D p = mul_u(t, u);
+    g.r2 = norm(add_u(sqr_u(dz), rho2));
+    g.invr = rsqrt_df(g.r2);
+    g.s = rsqrt_far_df(norm(ZPER ? add_u(rho2, sqr_u(Rz)) : add_u(g.r2, mul_u(h4, hj))));
+    g.i2 = sqr(g.invr);
+    g.u = sqr(g.s);
+    g.t = mul_u(g.u, g.s);
+    g.p = mul_u(g.t, g.u);
+    return g;
+}
+
+template <class D, bool ZPER = false>
+__device__ __forceinline__ UFBlockDF<D> uf_block_df(const PairGeoDF<D> &g, D dz, D Rz, D h4, D hj, D dw = D{})
+{
+    const D k4 = mul_u(h4, hj), s = g.s, u = g.u, t = g.t, p = g.p;
+    D ia = g.invr, a3 = mul_u(g.i2, g.invr);
+    D Bc = mul_u(add_fast_u(1.5f, mul_u(g.i2, -3.0f)), a3);
+    uf_near_df(g.r2, g.invr, ia, a3, Bc);
     const D z2 = sqr_u(Rz);
     const D E = mul_u(z2, u);
     const D w5 = add_fast_u(add_fast_u(mul_u(z2, 3.0f), 1.0f), mul_u(E, -5.0f));  // 1 + 3 Rz^2 - 5 E
@@ -278,9 +289,9 @@ __device__ __forceinline__ UFBlockDF<D> uf_block_df(D dx, D dy, D dz, D Rz, D h4
     D G = mul_u(dz, F);  // dz F
     D dG = mul_u(dz, G);  // dz^2 F
     if constexpr (ZPER) {
-        const D g = mul_u(dz, Bc), w = mul_u(mul_u(t, -1.5f), dw);
-        G = add_u(g, w);
-        dG = add_u(mul_u(dz, g), mul_u(dw, w));
+        const D x = mul_u(dz, Bc), w = mul_u(mul_u(t, -1.5f), dw);
+        G = add_u(x, w);
+        dG = add_u(mul_u(dz, x), mul_u(dw, w));
     }
     m.t3 = sub_u(G, X);
     m.t4 = add_u(G, X);
@@ -423,52 +434,49 @@ __device__ __forceinline__ void wt_near(df2 r2, df2 invr, df2 &A, df2 &Bc)
     }
 }
 
-// hi4 = 4 h_i
-__device__ __forceinline__ RotBlockDF2 rot_block_df(df2 dx, df2 dy, df2 dz, df2 Rz, df2 hi, df2 hi4, df2 hj)
+// UF32: the block times 3/2, as the UF block (for sums of both); the factor
+// only changes exact constants.
+template <bool UF32 = false>
+__device__ __forceinline__ RotBlockDF2 rot_block_df(const PairGeoDF<df2> &g, df2 dz, df2 Rz, df2 hi, df2 hj)
 {
-    const df2 r2 = norm(add_u(sqr_u(dz), add_u(sqr_u(dx), sqr_u(dy))));
-    const df2 invr = rsqrt_df(r2);
-    const df2 s = rsqrt_far_df(norm(add_u(r2, mul_u(hi4, hj))));
-    df2 c = mul_u(sqr(invr), invr);
-    rot_near_c(r2, invr, c);
-    const df2 u = sqr(s);
-    const df2 t = mul_u(u, s);
-    const df2 p = mul_u(t, u);
-    const df2 Ru = mul_u(Rz, u);
-    const df2 y = add_u(mul_u(mul_u(Rz, Ru), -10.0f), df2_dup(df_from(2.0f)));
+    constexpr float q = UF32 ? 1.5f : 1.0f;
+    df2 c = mul_u(g.i2, g.invr);
+    rot_near_c(g.r2, g.invr, c);
+    const df2 Ru = mul_u(Rz, g.u);
+    const df2 y = add_u(mul_u(mul_u(Rz, Ru), -10.0f * q), df2_dup(df_from(2.0f * q)));
     RotBlockDF2 k;
-    k.b = t - c;
-    const df2 m = mul_u(dz, k.b), n = scale2(mul_u(Rz, p), 2.0f);
+    k.b = g.t - c;
+    if constexpr (UF32) k.b = mul_u(k.b, 1.5f);
+    const df2 m = mul_u(dz, k.b), Rp = mul_u(Rz, g.p), n = UF32 ? mul_u(Rp, 3.0f) : scale2(Rp, 2.0f);
     k.a = sub_u(n, m);
     k.ar = add_u(n, m);
-    const df2 R10 = mul_u(Ru, 10.0f), R6 = mul_u(Rz, 6.0f);
-    k.ei = mul_u(p, sub_u(R10, mul_u(hi, 6.0f)));
-    k.ej = mul_u(p, sub_u(R10, mul_u(hj, 6.0f)));
-    k.wi = add_u(k.b, mul_u(p, add_u(y, mul_u(R6, hi))));
-    k.wj = add_u(k.b, mul_u(p, add_u(y, mul_u(R6, hj))));
+    const df2 R10 = mul_u(Ru, 10.0f * q), R6 = mul_u(Rz, 6.0f * q);
+    k.ei = mul_u(g.p, sub_u(R10, mul_u(hi, 6.0f * q)));
+    k.ej = mul_u(g.p, sub_u(R10, mul_u(hj, 6.0f * q)));
+    k.wi = add_u(k.b, mul_u(g.p, add_u(y, mul_u(R6, hi))));
+    k.wj = add_u(k.b, mul_u(g.p, add_u(y, mul_u(R6, hj))));
     return k;
 }
 
-__device__ __forceinline__ UFBlockDF<df2> wt_block_df(df2 dx, df2 dy, df2 dz, df2 Rz, df2 hi4, df2 hj)
+template <bool UF32 = false>
+__device__ __forceinline__ UFBlockDF<df2> wt_block_df(const PairGeoDF<df2> &g, df2 dz, df2 Rz)
 {
-    const df2 r2 = norm(add_u(sqr_u(dz), add_u(sqr_u(dx), sqr_u(dy))));
-    const df2 invr = rsqrt_df(r2);
-    const df2 s = rsqrt_far_df(norm(add_u(r2, mul_u(hi4, hj))));
-    const df2 i2 = sqr(invr);
-    const df2 i3 = mul_u(i2, invr);
-    df2 A = scale2(i3, -0.5f), Bc = mul_u(mul_u(i2, i3), 1.5f);
-    wt_near(r2, invr, A, Bc);
-    const df2 u = sqr(s);
-    const df2 t = mul_u(u, s);
-    const df2 p = mul_u(t, u);
-    const df2 Et = mul_u(mul_u(sqr_u(Rz), u), t);
+    constexpr float q = UF32 ? 1.5f : 1.0f;
+    const df2 i3 = mul_u(g.i2, g.invr);
+    df2 A = scale2(i3, -0.5f), Bc = mul_u(mul_u(g.i2, i3), 1.5f);
+    wt_near(g.r2, g.invr, A, Bc);
+    if constexpr (UF32) {
+        A = mul_u(A, q);
+        Bc = mul_u(Bc, q);
+    }
+    const df2 Et = mul_u(mul_u(sqr_u(Rz), g.u), g.t);
     UFBlockDF<df2> m;
-    m.Af = add_u(add_u(A, mul_u(t, 3.5f)), mul_u(Et, -6.0f));
-    m.b2 = add_u(Bc, mul_u(p, -4.5f));
-    const df2 D = mul_u(Bc, dz), X = mul_u(mul_u(p, Rz), 1.5f);
+    m.Af = add_u(add_u(A, mul_u(g.t, 3.5f * q)), mul_u(Et, -6.0f * q));
+    m.b2 = add_u(Bc, mul_u(g.p, -4.5f * q));
+    const df2 D = mul_u(Bc, dz), X = mul_u(mul_u(g.p, Rz), 1.5f * q);
     m.t3 = sub_u(D, X);
     m.t4 = add_u(D, X);
-    m.zz = add_u(add_u(A, scale2(t, 0.5f)), add_u(mul_u(Et, -1.5f), mul_u(D, dz)));
+    m.zz = add_u(add_u(A, mul_u(g.t, 0.5f * q)), add_u(mul_u(Et, -1.5f * q), mul_u(D, dz)));
     return m;
 }
 
@@ -556,7 +564,9 @@ __device__ __forceinline__ void pair_acc_df(df dx, df dy, df dz, df Rz, df hi, d
                                             df &uy, df &uz)
 {
     if (KIND == RMW_UF) {
-        const UFBlockDF<df> m = uf_block_df<df, ZPER>(dx, dy, dz, Rz, scale2(hi, 4.0f), hj, hi - hj);
+        const df h4 = scale2(hi, 4.0f);
+        const UFBlockDF<df> m =
+            uf_block_df<df, ZPER>(pair_geo_df<df, ZPER>(dx, dy, dz, Rz, h4, hj), dz, Rz, h4, hj, hi - hj);
         uf_block_acc_df(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
         return;
     }

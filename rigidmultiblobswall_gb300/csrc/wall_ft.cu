@@ -341,21 +341,43 @@ __global__ void __launch_bounds__(kFtThreads) ft_pair_df_kernel(const FtSrcDF *_
 }
 
 // ---------------------------------------------------------------------------
-// finalize: fixed-order chunk sum, FP64 self terms of the four blocks
-// (mobility/mobility_numba.py self terms), b_i and the scales
-__global__ void ft_finalize_kernel(const double *__restrict__ r, const double *__restrict__ F,
-                                   const double *__restrict__ T, const double *__restrict__ partial, int nchunks,
-                                   double *__restrict__ U, double *__restrict__ W, int n, double a, double nf)
+// finalize: fixed-order slot sum, FP64 self terms of the four blocks
+// (mobility/mobility_numba.py self terms), b_i and the scales.  A CTA takes
+// kFtFinBlobs blobs; thread (x, g) sums slots g, g + G, ... of component x
+// (coalesced), one thread per blob adds the G sums in order.  pair_scale: 2/3
+// where the slots hold 3/2 of the sums.
+constexpr int kFtFinBlobs = 32, kFtFinGroups = 8;
+__global__ void __launch_bounds__(3 * kFtFinBlobs * kFtFinGroups)
+    ft_finalize_kernel(const double *__restrict__ r, const double *__restrict__ F, const double *__restrict__ T,
+                       const double *__restrict__ partial, int nchunks, double *__restrict__ U,
+                       double *__restrict__ W, int n, double a, double nf, double pair_scale)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double u[3] = {0.0, 0.0, 0.0}, w[3] = {0.0, 0.0, 0.0};
-    for (int s = 0; s < nchunks; ++s) {
-        const double *p = partial + (size_t)s * 6 * n;
-        for (int c = 0; c < 3; ++c) {
-            u[c] += p[3 * (size_t)i + c];
-            w[c] += p[3 * (size_t)n + 3 * (size_t)i + c];
+    __shared__ double red[kFtFinGroups][2][3 * kFtFinBlobs];
+    const int x = threadIdx.x, g = threadIdx.y;
+    const long long e = 3LL * blockIdx.x * kFtFinBlobs + x;
+    if (e < 3LL * n) {
+        double su = 0.0, sw = 0.0;
+#pragma unroll 4
+        for (int s = g; s < nchunks; s += kFtFinGroups) {
+            const double *p = partial + (size_t)s * 6 * n + e;
+            su += p[0];
+            if (W) sw += p[3 * (size_t)n];
         }
+        red[g][0][x] = su;
+        red[g][1][x] = sw;
+    }
+    __syncthreads();
+    const int i = blockIdx.x * kFtFinBlobs + x;
+    if (g != 0 || x >= kFtFinBlobs || i >= n) return;
+    double u[3] = {0.0, 0.0, 0.0}, w[3] = {0.0, 0.0, 0.0};
+    for (int k = 0; k < kFtFinGroups; ++k)
+        for (int c = 0; c < 3; ++c) {
+            u[c] += red[k][0][3 * x + c];
+            w[c] += red[k][1][3 * x + c];
+        }
+    for (int c = 0; c < 3; ++c) {
+        u[c] *= pair_scale;
+        w[c] *= pair_scale;
     }
     const double z = r[3 * i + 2];
     const double b = (z < a) ? z / a : 1.0;
@@ -503,6 +525,253 @@ __global__ void __launch_bounds__(kFtSymTile) ft_sym_mixed_kernel(const FtSrcF *
     }
 }
 
+void ft_finalize(const double *r, const double *F, const double *T, const double *partial, int slots, double *U,
+                 double *W, int n, double eta, double a, double pair_scale, cudaStream_t st)
+{
+    ft_finalize_kernel<<<(n + kFtFinBlobs - 1) / kFtFinBlobs, dim3(3 * kFtFinBlobs, kFtFinGroups), 0, st>>>(
+        r, F, T, partial, slots, U, W, n, a, 1.0 / (8.0 * kPi * eta * a), pair_scale);
+}
+
+// ---------------------------------------------------------------------------
+// Symmetric FP64 and df64 force-torque kernels: the grid, pairing and split
+// (gridDim.y CTAs share a tile pair's steps) of the symmetric single products,
+// the four blocks of an unordered pair from one set of distances, reciprocal
+// roots and powers (about 150 of 600 + 500 + 500 + 500 FP32-pipe operations
+// in df64, 25 of 73 + 64 + 64 + 62 FP64 instructions), applied both ways;
+// every block times 3/2, undone by the finalize.  The sum of four symmetric
+// single products, which this replaces, read the blobs and formed the geometry
+// four times and needed a vector of scratch and two additions.  8,064 blobs,
+// [U; W]: df64 2.20 -> 1.51 ms (3.51 before the blocks were written out), four
+// CTAs of 255 registers per SM (six of 168 spill: 1.58 ms); FP64 10.6 ms.
+struct FtSteps {
+    int k0, k1, nsplit, split;
+    __device__ __forceinline__ size_t slot(int tile) const { return (size_t)tile * nsplit + split; }
+};
+__device__ __forceinline__ FtSteps ft_steps()
+{
+    const int m = gridDim.y, s = blockIdx.y;
+    return {kFtSymTile * s / m, kFtSymTile * (s + 1) / m, m, s};
+}
+
+template <bool WITH_W>
+__global__ void __launch_bounds__(kFtSymTile) ft_sym_fp64_kernel(const FtSrcD *__restrict__ src, int n, int nt,
+                                                                 double *__restrict__ partial)
+{
+    constexpr int NC = WITH_W ? 6 : 3;
+    __shared__ double sx[9][kFtSymTile];  // x y z f t
+    __shared__ double sacc[kFtSymWarps][NC][kFtSymTile];
+    int T, S;
+    sym_tile_pair(blockIdx.x, nt, T, S);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool diag = (T == S);
+    const int i = T * kFtSymTile + tid;
+    const bool valid_i = i < n;
+    // a target or source past the end is a dummy far above the wall with zero vectors
+    const FtSrcD dummy = {1.0e6, 1.0e6, 1.0e6, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    const FtSrcD me = valid_i ? src[i] : dummy;
+    {
+        const int j = S * kFtSymTile + tid;
+        const FtSrcD q = (j < n) ? src[j] : dummy;
+        const double c[9] = {q.x, q.y, q.z, q.fx, q.fy, q.fz, q.tx, q.ty, q.tz};
+        for (int k = 0; k < 9; ++k) sx[k][tid] = c[k];
+    }
+    for (int c = 0; c < NC; ++c)
+        for (int k = lane; k < kFtSymTile; k += 32) sacc[warp][c][k] = 0.0;
+    __syncthreads();
+    double u[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    auto step = [&](int k) {
+        const int j = (lane + k) & (kFtSymTile - 1);
+        const double zj = sx[2][j], dx = me.x - sx[0][j], dy = me.y - sx[1][j], dz = me.z - zj, Rz = me.z + zj;
+        const double fx = sx[3][j], fy = sx[4][j], fz = sx[5][j], tx = sx[6][j], ty = sx[7][j], tz = sx[8][j];
+        double w[NC];
+        for (int c = 0; c < NC; ++c) w[c] = sacc[warp][c][j];
+        const PairGeoD g = pair_geo_d<false>(dx, dy, dz, Rz, me.z, zj);
+        {
+            const UFBlockD m = uf_block_d<false>(g, dz, Rz, me.z, zj);
+            uf_block_acc_d(m, m.t3, m.t4, dx, dy, fx, fy, fz, u[0], u[1], u[2]);
+            uf_block_acc_d(m, m.t4, m.t3, dx, dy, me.fx, me.fy, me.fz, w[0], w[1], w[2]);
+        }
+        const RotBlockD k2 = rot_block_d<true>(g, dz, Rz, me.z, zj);
+        ut_acc_d(k2, dx, dy, tx, ty, tz, me.tx, me.ty, me.tz, u[0], u[1], u[2], w[0], w[1], w[2]);
+        if constexpr (WITH_W) {
+            wf_acc_d(k2, dx, dy, fx, fy, fz, me.fx, me.fy, me.fz, u[3], u[4], u[5], w[3], w[4], w[5]);
+            const UFBlockD m = wt_block_d<true>(g, dz, Rz);
+            uf_block_acc_d(m, m.t3, m.t4, dx, dy, tx, ty, tz, u[3], u[4], u[5]);
+            uf_block_acc_d(m, m.t4, m.t3, dx, dy, me.tx, me.ty, me.tz, w[3], w[4], w[5]);
+        }
+        for (int c = 0; c < NC; ++c) sacc[warp][c][j] = w[c];
+    };
+    const FtSteps sp = ft_steps();
+    for (int k = sp.k0; k < sp.k1; ++k) {
+        __syncwarp();
+        const int off = (k - 32 * warp) & (kFtSymTile - 1);  // (source - target) mod 128, warp-uniform
+        if (diag && (off == 0 || off > kFtSymTile / 2 || (off == kFtSymTile / 2 && warp >= kFtSymWarps / 2))) continue;
+        step(k);
+    }
+    __syncthreads();
+    const int j = S * kFtSymTile + tid;
+    for (int c = 0; c < NC; ++c) {
+        double q = 0.0;
+        for (int w = 0; w < kFtSymWarps; ++w) q += sacc[w][c][tid];
+        const size_t comp = (c / 3) * 3 * (size_t)n + c % 3;
+        if (valid_i) partial[sp.slot(diag ? T : S) * 6 * n + 3 * (size_t)i + comp] = diag ? u[c] + q : u[c];
+        if (!diag && j < n) partial[sp.slot(T) * 6 * n + 3 * (size_t)j + comp] = q;
+    }
+}
+
+// df64: two targets per thread in packed lanes, as wall_uf_df_sym_kernel
+constexpr int kFtF2Threads = kFtSymTile / 2;
+
+struct FtTarget {
+    df2 x, y, z, h4, f[3], t[3];
+};
+
+template <bool DIAG, bool WITH_W>
+__device__ __forceinline__ void ft_f2_step(const FtTarget &me, int ja, int jb, const float4 (*tile)[kFtSymTile],
+                                           float4 (*sacc)[kFtSymTile], df2 (&u)[6])
+{
+    constexpr int NC = WITH_W ? 6 : 3;
+    df2 v[3][3];  // position, F, T of the sources
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const float4 h = tile[2 * q][ja], l = tile[2 * q + 1][ja];
+        float4 h1 = h, l1 = l;
+        if (DIAG) {
+            h1 = tile[2 * q][jb];
+            l1 = tile[2 * q + 1][jb];
+        }
+        v[q][0] = {make_float2(h.x, h1.x), make_float2(l.x, l1.x)};
+        v[q][1] = {make_float2(h.y, h1.y), make_float2(l.y, l1.y)};
+        v[q][2] = {make_float2(h.z, h1.z), make_float2(l.z, l1.z)};
+    }
+    const df2 dx = me.x - v[0][0], dy = me.y - v[0][1], dz = me.z - v[0][2], zj = v[0][2], Rz = add_u(me.z, zj);
+    const PairGeoDF<df2> g = pair_geo_df<df2>(dx, dy, dz, Rz, me.h4, zj);
+    auto load = [&](int c) -> df2 {
+        const float4 a = sacc[c][ja];
+        if (!DIAG) return {make_float2(a.x, a.y), make_float2(a.z, a.w)};
+        const float4 b = sacc[c][jb];
+        return {make_float2(a.x, b.y), make_float2(a.z, b.w)};
+    };
+    auto store = [&](int c, const df2 &w) {
+        if (!DIAG) {
+            sacc[c][ja] = make_float4(w.hi.x, w.hi.y, w.lo.x, w.lo.y);
+        } else {
+            float *a = (float *)&sacc[c][ja], *b = (float *)&sacc[c][jb];
+            a[0] = w.hi.x; a[2] = w.lo.x;
+            b[1] = w.hi.y; b[3] = w.lo.y;
+        }
+    };
+    df2 wx = load(0), wy = load(1), wz = load(2);
+    {
+        const UFBlockDF<df2> m = uf_block_df<df2>(g, dz, Rz, me.h4, zj);
+        uf_block_acc_df(m, m.t3, m.t4, dx, dy, v[1][0], v[1][1], v[1][2], u[0], u[1], u[2]);
+        uf_block_acc_df(m, m.t4, m.t3, dx, dy, me.f[0], me.f[1], me.f[2], wx, wy, wz);
+    }
+    const RotBlockDF2 k = rot_block_df<true>(g, dz, Rz, me.z, zj);
+    ut_acc_df(k, dx, dy, v[2][0], v[2][1], v[2][2], me.t[0], me.t[1], me.t[2], u[0], u[1], u[2], wx, wy, wz);
+    store(0, wx); store(1, wy); store(2, wz);
+    if constexpr (WITH_W) {
+        wx = load(NC - 3); wy = load(NC - 2); wz = load(NC - 1);
+        wf_acc_df(k, dx, dy, v[1][0], v[1][1], v[1][2], me.f[0], me.f[1], me.f[2], u[3], u[4], u[5], wx, wy, wz);
+        const UFBlockDF<df2> m = wt_block_df<true>(g, dz, Rz);
+        uf_block_acc_df(m, m.t3, m.t4, dx, dy, v[2][0], v[2][1], v[2][2], u[3], u[4], u[5]);
+        uf_block_acc_df(m, m.t4, m.t3, dx, dy, me.t[0], me.t[1], me.t[2], wx, wy, wz);
+        store(NC - 3, wx); store(NC - 2, wy); store(NC - 1, wz);
+    }
+}
+
+template <bool WITH_W>
+__global__ void __launch_bounds__(kFtF2Threads, 4) ft_sym_df_kernel(const FtSrcDF *__restrict__ src, int n, int nt,
+                                                                    double *__restrict__ partial)
+{
+    constexpr int NC = WITH_W ? 6 : 3;
+    __shared__ float4 tile[6][kFtSymTile];  // hi, lo, fhi, flo, thi, tlo
+    __shared__ float4 sacc[kFtF2Threads / 32][NC][kFtSymTile];
+    int T, S;
+    sym_tile_pair(blockIdx.x, nt, T, S);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool diag = (T == S);
+    const int i0 = T * kFtSymTile + tid, i1 = i0 + kFtF2Threads;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const FtSrcDF dummy = {make_float4(1.0e6f, 1.0e6f, 1.0e6f, 0.f), zero, zero, zero, zero, zero};
+    FtTarget me;
+    {
+        const FtSrcDF a = i0 < n ? src[i0] : dummy, b = i1 < n ? src[i1] : dummy;
+        me.x = df2_pack({a.hi.x, a.lo.x}, {b.hi.x, b.lo.x});
+        me.y = df2_pack({a.hi.y, a.lo.y}, {b.hi.y, b.lo.y});
+        me.z = df2_pack({a.hi.z, a.lo.z}, {b.hi.z, b.lo.z});
+        me.h4 = scale2(me.z, 4.0f);
+        me.f[0] = df2_pack({a.fhi.x, a.flo.x}, {b.fhi.x, b.flo.x});
+        me.f[1] = df2_pack({a.fhi.y, a.flo.y}, {b.fhi.y, b.flo.y});
+        me.f[2] = df2_pack({a.fhi.z, a.flo.z}, {b.fhi.z, b.flo.z});
+        me.t[0] = df2_pack({a.thi.x, a.tlo.x}, {b.thi.x, b.tlo.x});
+        me.t[1] = df2_pack({a.thi.y, a.tlo.y}, {b.thi.y, b.tlo.y});
+        me.t[2] = df2_pack({a.thi.z, a.tlo.z}, {b.thi.z, b.tlo.z});
+    }
+    for (int k = tid; k < kFtSymTile; k += kFtF2Threads) {
+        const int j = S * kFtSymTile + k;
+        const FtSrcDF q = (j < n) ? src[j] : dummy;
+        tile[0][k] = q.hi; tile[1][k] = q.lo;
+        tile[2][k] = q.fhi; tile[3][k] = q.flo;
+        tile[4][k] = q.thi; tile[5][k] = q.tlo;
+    }
+    for (int c = 0; c < NC; ++c)
+        for (int k = lane; k < kFtSymTile; k += 32) sacc[warp][c][k] = zero;
+    __syncthreads();
+    df2 u[6];
+    for (int c = 0; c < 6; ++c) u[c] = df2_zero();
+    const FtSteps sp = ft_steps();
+    auto renorm = [&](int k) {
+        if (k & 7) return;
+        for (int c = 0; c < NC; ++c) u[c] = norm(u[c]);
+    };
+    if (diag) {
+        // offsets (source - target) 1..63, and 64 for lane x alone (lane y's pairs are lane x's)
+        for (int o = 1 + sp.k0 / 2; o < 1 + sp.k1 / 2; ++o) {
+            __syncwarp();
+            const int ja = (tid + o) & (kFtSymTile - 1), jb = (tid + kFtF2Threads + o) & (kFtSymTile - 1);
+            if (o < kFtSymTile / 2) {
+                ft_f2_step<true, WITH_W>(me, ja, jb, tile, sacc[warp], u);
+            } else {
+                FtTarget half = me;
+                for (int c = 0; c < 3; ++c)
+                    half.f[c].hi.y = half.f[c].lo.y = half.t[c].hi.y = half.t[c].lo.y = 0.f;
+                df2 v[6];
+                for (int c = 0; c < 6; ++c) v[c] = u[c];
+                ft_f2_step<true, WITH_W>(half, ja, jb, tile, sacc[warp], v);
+                for (int c = 0; c < NC; ++c) {
+                    u[c].hi.x = v[c].hi.x;
+                    u[c].lo.x = v[c].lo.x;
+                }
+            }
+            renorm(o);
+        }
+    } else {
+#pragma unroll 1
+        for (int k = sp.k0; k < sp.k1; ++k) {
+            __syncwarp();
+            const int j = (lane + k) & (kFtSymTile - 1);
+            ft_f2_step<false, WITH_W>(me, j, j, tile, sacc[warp], u);
+            renorm(k);
+        }
+    }
+    __syncthreads();
+    for (int half = 0; half < 2; ++half) {
+        const int l = tid + half * kFtF2Threads, i = T * kFtSymTile + l, j = S * kFtSymTile + l;
+        for (int c = 0; c < NC; ++c) {
+            const df t = half ? df{u[c].hi.y, u[c].lo.y} : df{u[c].hi.x, u[c].lo.x};
+            df q = df_from(0.f);
+            for (int w = 0; w < kFtF2Threads / 32; ++w) {
+                const float4 f = sacc[w][c][l];
+                q = q + (df{f.x, f.z} + df{f.y, f.w});
+            }
+            const size_t comp = (c / 3) * 3 * (size_t)n + c % 3;
+            if (i < n) partial[sp.slot(diag ? T : S) * 6 * n + 3 * (size_t)i + comp] = to_double(diag ? t + q : t);
+            if (!diag && j < n) partial[sp.slot(T) * 6 * n + 3 * (size_t)j + comp] = to_double(q);
+        }
+    }
+}
+
 __global__ void ft_add_kernel(const double *__restrict__ x, double *__restrict__ y, long long m)
 {
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -510,8 +779,9 @@ __global__ void ft_add_kernel(const double *__restrict__ x, double *__restrict__
 }
 
 // U (and W) as sums of single products, each through the symmetric kernel
-// (every unordered pair once per block): in FP64 and df64 faster than the
-// fused one-sided pass wherever the symmetric kernels apply.
+// (every unordered pair once per block): faster than the fused one-sided pass
+// (10,752 blobs df64 3.7 against 7.6 ms), with half the partial sums of the
+// fused symmetric kernel.
 int ft_by_symmetric_products(const double *r, const double *F, const double *T, double *U, double *W, int n,
                              double eta, double a, int mode, cudaStream_t st)
 {
@@ -528,6 +798,41 @@ int ft_by_symmetric_products(const double *r, const double *F, const double *T, 
         ft_add_kernel<<<g, 256, 0, st>>>(t, W, 3LL * n);
     }
     RMW_CHECK_LAUNCH("force-torque through symmetric products");
+    return RMW_OK;
+}
+
+// FP64 and df64, not periodic: the fused symmetric product.  RMW_ERR_ALLOC:
+// its partial sums do not fit (the caller takes the one-sided pass).
+int ft_symmetric(const double *r, const double *F, const double *T, double *U, double *W, int n, double eta, double a,
+                 int mode, cudaStream_t st)
+{
+    const int nt = (n + kFtSymTile - 1) / kFtSymTile, nsplit = wall_sym_split(mode, n);
+    const size_t rec = mode == RMW_MODE_DF64 ? sizeof(FtSrcDF) : sizeof(FtSrcD);
+    const size_t packed = ((rec * (size_t)n + 255) / 256) * 256;
+    const size_t part = sizeof(double) * 6 * (size_t)n * nt * nsplit;
+    void *ws = nullptr;
+    if (part > wall_sym_partial_budget()) return RMW_ERR_ALLOC;
+    if (scratch(SCRATCH_PAIR, packed + part, &ws, st) != RMW_OK) {
+        cudaGetLastError();
+        return RMW_ERR_ALLOC;
+    }
+    double *partial = (double *)((char *)ws + packed);
+    const int pb = 64, pg = (n + pb - 1) / pb;
+    if (mode == RMW_MODE_FP64) ft_pack_fp64_kernel<<<pg, pb, 0, st>>>(r, F, T, (FtSrcD *)ws, n, a);
+    else ft_pack_df_kernel<<<pg, pb, 0, st>>>(r, F, T, (FtSrcDF *)ws, n, a);
+    const dim3 grid((unsigned)((long long)nt * (nt + 1) / 2), nsplit);
+    void *tok = nullptr;
+    if (int rc = trace_begin(TRACE_PAIR, st, &tok)) return rc;
+    if (mode == RMW_MODE_FP64) {
+        if (W) ft_sym_fp64_kernel<true><<<grid, kFtSymTile, 0, st>>>((const FtSrcD *)ws, n, nt, partial);
+        else ft_sym_fp64_kernel<false><<<grid, kFtSymTile, 0, st>>>((const FtSrcD *)ws, n, nt, partial);
+    } else {
+        if (W) ft_sym_df_kernel<true><<<grid, kFtF2Threads, 0, st>>>((const FtSrcDF *)ws, n, nt, partial);
+        else ft_sym_df_kernel<false><<<grid, kFtF2Threads, 0, st>>>((const FtSrcDF *)ws, n, nt, partial);
+    }
+    if (int rc = trace_end(tok, st)) return rc;
+    ft_finalize(r, F, T, partial, nt * nsplit, U, W, n, eta, a, kUFCoeffScale, st);
+    RMW_CHECK_LAUNCH("symmetric force-torque wall product");
     return RMW_OK;
 }
 
@@ -584,14 +889,17 @@ int wall_force_torque(const double *r, const double *F, const double *T, double 
             if (W) ft_sym_mixed_kernel<true><<<ncta, kFtSymTile, 0, st>>>((const FtSrcF *)ws, N, nt, partial);
             else ft_sym_mixed_kernel<false><<<ncta, kFtSymTile, 0, st>>>((const FtSrcF *)ws, N, nt, partial);
             if (int rc = trace_end(tok, st)) return rc;
-            ft_finalize_kernel<<<pg, pb, 0, st>>>(r, F, T, partial, nt, U, W, N, a, 1.0 / (8.0 * kPi * eta * a));
+            ft_finalize(r, F, T, partial, nt, U, W, N, eta, a, 1.0, st);
             RMW_CHECK_LAUNCH("symmetric force-torque wall product");
             return RMW_OK;
         }
     }
-    // FP64 and df64: the four symmetric products (at 10,752 blobs FP64 39.4 vs
-    // 49.5 ms for the one-sided fused pass, df64 5.9 vs 7.6 ms)
-    if (!per && (mode == RMW_MODE_FP64 || mode == RMW_MODE_DF64)) {
+    // FP64 and df64 from 256 blobs: the fused symmetric kernel, where its
+    // partial sums fit; where they do not, four symmetric single products (whose
+    // sums are half as large, or banded), else the one-sided fused pass
+    if (!per && (mode == RMW_MODE_FP64 || mode == RMW_MODE_DF64) && N >= 2 * kFtSymTile) {
+        const int rc = ft_symmetric(r, F, T, U, W, N, eta, a, mode, st);
+        if (rc != RMW_ERR_ALLOC) return rc;
         bool sym = true;
         for (int kind : {RMW_UF, RMW_UT, RMW_WF, RMW_WT})
             sym = sym && wall_chunks(kind, mode, N) == kSymChunks && wall_sym_applicable(kind, mode, N, nullptr);
@@ -621,7 +929,7 @@ int wall_force_torque(const double *r, const double *F, const double *T, double 
         else ft_launch<false, false>(mode, grid, st, ws, N, chunk, P, partial);
     }
     if (int rc = trace_end(tok, st)) return rc;
-    ft_finalize_kernel<<<pg, pb, 0, st>>>(r, F, T, partial, nchunks, U, W, N, a, 1.0 / (8.0 * kPi * eta * a));
+    ft_finalize(r, F, T, partial, nchunks, U, W, N, eta, a, 1.0, st);
     RMW_CHECK_LAUNCH("force-torque wall product");
     return RMW_OK;
 }

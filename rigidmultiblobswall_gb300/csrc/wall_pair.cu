@@ -356,18 +356,21 @@ __device__ __forceinline__ void df_f2_step(const F2Target &me, int ja, int jb, c
     const df2 dx = me.x - xj, dy = me.y - yj, dz = me.z - zj;
     if constexpr (NOWALL) {
         rpy_acc_df<KIND>(dx, dy, dz, vx, vy, vz, me.qx, me.qy, me.qz, ux, uy, uz, wx, wy, wz);
-    } else if constexpr (KIND == RMW_UF || KIND == RMW_WT) {
-        const df2 Rz = add_u(me.z, zj);
-        UFBlockDF<df2> m;
-        if constexpr (KIND == RMW_UF) m = uf_block_df<df2>(dx, dy, dz, Rz, me.h4, zj);
-        else m = wt_block_df(dx, dy, dz, Rz, me.h4, zj);
-        uf_block_acc_df(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);           // M_ij v_j
-        uf_block_acc_df(m, m.t4, m.t3, dx, dy, me.qx, me.qy, me.qz, wx, wy, wz);  // M_ij^T v_i
     } else {
-        const RotBlockDF2 k = rot_block_df(dx, dy, dz, add_u(me.z, zj), me.z, me.h4, zj);
-        if constexpr (KIND == RMW_UT)
-            ut_acc_df(k, dx, dy, vx, vy, vz, me.qx, me.qy, me.qz, ux, uy, uz, wx, wy, wz);
-        else wf_acc_df(k, dx, dy, vx, vy, vz, me.qx, me.qy, me.qz, ux, uy, uz, wx, wy, wz);
+        const df2 Rz = add_u(me.z, zj);
+        const PairGeoDF<df2> g = pair_geo_df<df2>(dx, dy, dz, Rz, me.h4, zj);
+        if constexpr (KIND == RMW_UF || KIND == RMW_WT) {
+            UFBlockDF<df2> m;
+            if constexpr (KIND == RMW_UF) m = uf_block_df<df2>(g, dz, Rz, me.h4, zj);
+            else m = wt_block_df(g, dz, Rz);
+            uf_block_acc_df(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);           // M_ij v_j
+            uf_block_acc_df(m, m.t4, m.t3, dx, dy, me.qx, me.qy, me.qz, wx, wy, wz);  // M_ij^T v_i
+        } else {
+            const RotBlockDF2 k = rot_block_df(g, dz, Rz, me.z, zj);
+            if constexpr (KIND == RMW_UT)
+                ut_acc_df(k, dx, dy, vx, vy, vz, me.qx, me.qy, me.qz, ux, uy, uz, wx, wy, wz);
+            else wf_acc_df(k, dx, dy, vx, vy, vz, me.qx, me.qy, me.qz, ux, uy, uz, wx, wy, wz);
+        }
     }
     if (DIAG) {
         float *s = reinterpret_cast<float *>(sacc);
@@ -829,7 +832,7 @@ __device__ __forceinline__ void pair_acc_d(double dx, double dy, double dz, doub
                                            double vy, double vz, double &ux, double &uy, double &uz)
 {
     if constexpr (KIND == RMW_UF) {
-        const UFBlockD m = uf_block_d<ZPER>(dx, dy, dz, Rz, hi, hj);
+        const UFBlockD m = uf_block_d<ZPER>(pair_geo_d<ZPER>(dx, dy, dz, Rz, hi, hj), dz, Rz, hi, hj);
         uf_block_acc_d(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
     } else {
         pair_contrib<KIND, double>(dx, dy, dz, Rz, hi, hj, vx, vy, vz, ux, uy, uz);
@@ -887,13 +890,20 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
             const double dz = zi - zj, Rz = zi + zj;
             if constexpr (NOWALL) {
                 pair_rpy_sym<double, KIND>(dx, dy, dz, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
-            } else if constexpr (KIND == RMW_UF) {
-                const UFBlockD m = uf_block_d<false>(dx, dy, dz, Rz, zi, zj);
-                uf_block_acc_d(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
-                uf_block_acc_d(m, m.t4, m.t3, dx, dy, me.vx, me.vy, me.vz, wx, wy, wz);
             } else {
-                pair_rot_sym_d<KIND>(dx, dy, dz, Rz, zi, zj, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy,
-                                     wz);
+                const PairGeoD g = pair_geo_d<false>(dx, dy, dz, Rz, zi, zj);
+                if constexpr (KIND == RMW_UF || KIND == RMW_WT) {
+                    UFBlockD m;
+                    if constexpr (KIND == RMW_UF) m = uf_block_d<false>(g, dz, Rz, zi, zj);
+                    else m = wt_block_d(g, dz, Rz);
+                    uf_block_acc_d(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
+                    uf_block_acc_d(m, m.t4, m.t3, dx, dy, me.vx, me.vy, me.vz, wx, wy, wz);
+                } else {
+                    const RotBlockD k = rot_block_d(g, dz, Rz, zi, zj);
+                    if constexpr (KIND == RMW_UT)
+                        ut_acc_d(k, dx, dy, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
+                    else wf_acc_d(k, dx, dy, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
+                }
             }
         };
         if constexpr (PER) {
