@@ -3,10 +3,11 @@
 #include <cstring>
 
 #include "krylov_device.cuh"
+#include "pair_math.cuh"
 
 namespace rmw {
 
-// spins of a grid barrier before it gives up (about 0.3 s with the 64 ns sleeps)
+// polls of a grid barrier before it gives up (one L2 read each, 2 to 3 s in all)
 constexpr unsigned kBarrierSpins = 1u << 22;
 // tridiagonal matrices up to this size are diagonalised in shared memory
 constexpr int kLzShared = 256;
@@ -40,30 +41,108 @@ __device__ __forceinline__ double warp_sum8(const double a[8], int lane)
     return d;
 }
 
-// Grid barrier of a cooperative launch: generation counter, bounded spin.
-__device__ void grid_barrier(GridBar *b)
+// sqrt(x) and 1/sqrt(x).  The step kernels below are bound by FP64 issue: the
+// chip has two FP64 lanes per SM, a warp waits about 64 cycles for each of its
+// FP64 instructions, and the library's square root, division and hypot take
+// some 10, 10 and 25 of them.  Within the range where x and its square root
+// are far from overflow and underflow both come from rsqrt64 and one Newton
+// correction of the root (8 instructions); outside it (zero, subnormal,
+// non-finite x) from the library.
+struct RootInv {
+    double root, inv;
+};
+// 2^-930 <= x < 2^930, from the exponent bits: no FP64 instruction
+__device__ __forceinline__ bool mid_range(double x)
+{
+    return (unsigned)__double2hiint(x) - (93u << 20) < (1860u << 20);
+}
+__device__ __forceinline__ RootInv root_inv(double x)
+{
+    if (mid_range(x)) {
+        const double y = rsqrt64(x), r = x * y;
+        return {fma(fma(-r, r, x), 0.5 * y, r), y};
+    }
+    const double r = sqrt(x);
+    return {r, (r > 0.0) ? 1.0 / r : 0.0};
+}
+
+// Rotation (c, s) with c a + s b = r = |(a, b)|, -s a + c b = 0
+struct Rot {
+    double c, s, r;
+    bool zero;  // r == 0
+};
+__device__ __forceinline__ Rot plane_rotation(double a, double b)
+{
+    const double r2 = fma(a, a, b * b);
+    if (mid_range(r2)) {
+        const double y = rsqrt64(r2);
+        return {a * y, b * y, r2 * y, false};
+    }
+    const double r = hypot(a, b);
+    if (r == 0.0) return {1.0, 0.0, 0.0, true};
+    return {a / r, b / r, r, false};
+}
+
+// sqrt(a^2 + b^2)
+__device__ __forceinline__ double root_or_hypot(double a, double b)
+{
+    const double r2 = fma(a, a, b * b);
+    return mid_range(r2) ? r2 * rsqrt64(r2) : hypot(a, b);
+}
+
+// The first jobs of a CTA with their segments' job ranges, read once: after a
+// grid barrier every one of these reads goes to L2 again.
+constexpr int kJobCache = 8;
+struct JobCache {
+    KJob jb[kJobCache];
+    int s0[kJobCache], s1[kJobCache];
+};
+struct JobInfo {
+    KJob jb;
+    int s0, s1;
+};
+__device__ __forceinline__ JobInfo job_read(const KJob *jobs, const int *sjob, int job)
+{
+    const KJob jb = jobs[job];
+    return {jb, sjob[jb.seg], sjob[jb.seg + 1]};
+}
+__device__ __forceinline__ void job_cache_fill(JobCache &C, const KJob *jobs, const int *sjob, int jb0, int jb1)
+{
+    const int t = threadIdx.x;
+    if (t < kJobCache && jb0 + t < jb1) {
+        const JobInfo f = job_read(jobs, sjob, jb0 + t);
+        C.jb[t] = f.jb;
+        C.s0[t] = f.s0;
+        C.s1[t] = f.s1;
+    }
+}
+__device__ __forceinline__ JobInfo job_info(const JobCache &C, const KJob *jobs, const int *sjob, int jb0, int job)
+{
+    const int t = job - jb0;
+    if (t < kJobCache) return {C.jb[t], C.s0[t], C.s1[t]};
+    return job_read(jobs, sjob, job);
+}
+
+// Grid barrier of a cooperative launch, bounded spin.  The launch's barriers
+// count up on one word (goal: the barrier's number times the CTAs); the last
+// CTA of the launch sets it back.  One atomic and the waiters' polls of it,
+// instead of a second round trip for the last arrival to publish a
+// generation.
+__device__ void grid_barrier(GridBar *b, unsigned goal)
 {
     __syncthreads();
     if (threadIdx.x == 0) {
-        volatile unsigned *vgen = &b->gen;
-        const unsigned gen = *vgen;
         __threadfence();
-        const unsigned arrived = atomicAdd(&b->count, 1u);
-        if (arrived == gridDim.x - 1) {
-            atomicExch(&b->count, 0u);
-            __threadfence();
-            atomicAdd(&b->gen, 1u);
-        } else {
-            unsigned spins = 0;
-            while (*vgen == gen) {
-                if (++spins > kBarrierSpins) {
-                    atomicExch(&b->err, 1);
-                    break;
-                }
-                __nanosleep(64);
+        atomicAdd(&b->count, 1u);
+        unsigned spins = 0, seen;
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&b->count) : "memory");
+            if (seen >= goal) break;
+            if (++spins > kBarrierSpins) {
+                atomicExch(&b->err, 1);
+                break;
             }
         }
-        __threadfence();
     }
     __syncthreads();
 }
@@ -102,7 +181,7 @@ __device__ void job_dots_w(const double *__restrict__ V, long long ldv, int k, c
             for (int u = 0; u < 8; ++u)
                 if (u < nq) a[u] = fma(V0[(long long)u * ldv + i], wi, a[u]);
         }
-        const double sum = warp_sum8(a, lane);
+        const double sum = (nq == 1) ? warp_sum(a[0]) : warp_sum8(a, lane);
         const int u = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
         if ((lane & 3) == 0 && u < nq) red[(q0 + u) * 32 + wid] = sum;
     }
@@ -175,52 +254,63 @@ struct StepArgs {
 // One Arnoldi step of every segment: CGS2 against V_0..V_j, V_{j+1} = w/|w|
 // (also written to xin, the operator's next input), the Givens update of the
 // Hessenberg column and the stopping test.  Cooperative launch, one CTA per
-// SM at most; CTA b works on the jobs [bjob[b], bjob[b+1]).
+// SM at most; CTA b works on the jobs [bjob[b], bjob[b+1]).  Bound by latency
+// (three grid barriers, the dependent L2 reads between them) and FP64 issue:
+// 31 us a step at 32,000 unknowns and 36 at 43,000 with library roots,
+// generation-counting barriers and job tables read after each barrier; 24 and
+// 30 us now (serialised, cold caches).
 __global__ void __launch_bounds__(kKdThreads, 1) arnoldi_step_kernel(StepArgs A)
 {
     __shared__ double red[kKdMaxBasis * 32];
     __shared__ double hs[kKdMaxBasis];
+    __shared__ JobCache jc;
     const int j = *(volatile int *)&A.st->j;
     const int k = j + 1;
     const int jb0 = A.bjob[blockIdx.x], jb1 = A.bjob[blockIdx.x + 1];
+    job_cache_fill(jc, A.jobs, A.sjob, jb0, jb1);
+    __syncthreads();
     // pass 1: partial dots V^T w
-    for (int job = jb0; job < jb1; ++job) job_dots(A.V, A.ldv, k, A.w, A.jobs[job], A.partA, A.KP, job, red);
-    grid_barrier(&A.st->bar);
+    for (int job = jb0; job < jb1; ++job)
+        job_dots(A.V, A.ldv, k, A.w, job_info(jc, A.jobs, A.sjob, jb0, job).jb, A.partA, A.KP, job, red);
+    grid_barrier(&A.st->bar, gridDim.x);
     // pass 2: w -= V h1, partial dots V^T w again
     for (int job = jb0; job < jb1; ++job) {
-        const KJob jb = A.jobs[job];
-        reduce_segment(A.partA, A.KP, A.sjob[jb.seg], A.sjob[jb.seg + 1], k, hs);
-        if (job == A.sjob[jb.seg])
+        const JobInfo f = job_info(jc, A.jobs, A.sjob, jb0, job);
+        const KJob jb = f.jb;
+        reduce_segment(A.partA, A.KP, f.s0, f.s1, k, hs);
+        if (job == f.s0)
             for (int q = threadIdx.x; q < k; q += blockDim.x) A.hc1[(long long)jb.seg * A.KP + q] = hs[q];
         job_update(A.V, A.ldv, k, hs, A.w, jb);
         __syncthreads();
         job_dots(A.V, A.ldv, k, A.w, jb, A.partB, A.KP, job, red);
     }
-    grid_barrier(&A.st->bar);
+    grid_barrier(&A.st->bar, 2 * gridDim.x);
     // pass 3: w -= V h2, partial |w|^2
     for (int job = jb0; job < jb1; ++job) {
-        const KJob jb = A.jobs[job];
-        reduce_segment(A.partB, A.KP, A.sjob[jb.seg], A.sjob[jb.seg + 1], k, hs);
-        if (job == A.sjob[jb.seg])
+        const JobInfo f = job_info(jc, A.jobs, A.sjob, jb0, job);
+        const KJob jb = f.jb;
+        reduce_segment(A.partB, A.KP, f.s0, f.s1, k, hs);
+        if (job == f.s0)
             for (int q = threadIdx.x; q < k; q += blockDim.x) A.hc2[(long long)jb.seg * A.KP + q] = hs[q];
         const double nrm = job_update(A.V, A.ldv, k, hs, A.w, jb);
         __syncthreads();
         job_norm_partial(nrm, A.partC, A.KP, job, red);
     }
-    grid_barrier(&A.st->bar);
+    grid_barrier(&A.st->bar, 3 * gridDim.x);
     // pass 4: V_{j+1} = w / |w| (zero vector for |w| = 0); Givens by the CTA owning the segment's first job
     for (int job = jb0; job < jb1; ++job) {
-        const KJob jb = A.jobs[job];
-        reduce_segment(A.partC, A.KP, A.sjob[jb.seg], A.sjob[jb.seg + 1], 1, hs);
-        const double nw = hs[0];
-        const double inv = (nw > 0.0) ? 1.0 / sqrt(nw) : 0.0;
+        const JobInfo f = job_info(jc, A.jobs, A.sjob, jb0, job);
+        const KJob jb = f.jb;
+        reduce_segment(A.partC, A.KP, f.s0, f.s1, 1, hs);
+        const RootInv nw = root_inv(hs[0]);
+        const double inv = nw.inv;
         double *Vn = A.V + (long long)(j + 1) * A.ldv;
         for (long long i = jb.b + threadIdx.x; i < jb.e; i += blockDim.x) {
             const double v = A.w[i] * inv;
             Vn[i] = v;
             A.xin[i] = v;
         }
-        if (job == A.sjob[jb.seg]) {  // uniform over the CTA: it owns this segment's Givens update
+        if (job == f.s0) {  // uniform over the CTA: it owns this segment's Givens update
             const int s = jb.seg, R = A.R;
             double *col = red, *cq = red + kKdMaxBasis + 2, *sq = cq + kKdMaxBasis;  // shared scratch
             double *h = A.H + ((long long)s * R + j) * (R + 1);
@@ -234,7 +324,7 @@ __global__ void __launch_bounds__(kKdThreads, 1) arnoldi_step_kernel(StepArgs A)
             }
             __syncthreads();
             if (threadIdx.x == 0 && run) {
-                const double hn = sqrt(nw);
+                const double hn = nw.root;
                 col[j + 1] = hn;
                 int stop = 0;
                 if (!isfinite(hn)) {
@@ -246,12 +336,11 @@ __global__ void __launch_bounds__(kKdThreads, 1) arnoldi_step_kernel(StepArgs A)
                         col[q + 1] = -sq[q] * col[q] + cq[q] * col[q + 1];
                         col[q] = t;
                     }
-                    const double den = hypot(col[j], col[j + 1]);
-                    const double cj = (den == 0.0) ? 1.0 : col[j] / den;
-                    const double sj = (den == 0.0) ? 0.0 : col[j + 1] / den;
+                    const Rot rot = plane_rotation(col[j], col[j + 1]);
+                    const double cj = rot.c, sj = rot.s;
                     c[j] = cj;
                     sv[j] = sj;
-                    col[j] = cj * col[j] + sj * col[j + 1];
+                    col[j] = rot.r;
                     col[j + 1] = 0.0;
                     const double gj = gs[j];
                     gs[j + 1] = -sj * gj;
@@ -288,8 +377,8 @@ __global__ void __launch_bounds__(kKdThreads, 1) arnoldi_step_kernel(StepArgs A)
             A.st->j = jn;
             A.st->active = 0;
             A.st->more = more;
-            atomicExch(&A.st->bar.done, 0u);
-            __threadfence();
+            A.st->bar.count = 0;
+            A.st->bar.done = 0;
             if (A.use_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)A.cond, (unsigned)more);
         }
     }
@@ -356,6 +445,7 @@ __global__ void cycle_state_kernel(const double *__restrict__ beta, const double
         st->j = 0;
         st->active = 0;
         st->bar.done = 0;
+        st->bar.count = 0;
         st->more = 1;
     }
 }
@@ -408,9 +498,12 @@ __global__ void kd_axpby_kernel(const double *__restrict__ x, double *__restrict
 // Symmetric tridiagonal eigen-decomposition by implicit QL (the classical
 // algorithm of Bowdler, Martin, Reinsch and Wilkinson, as the host routine of
 // the library), run by one warp: every lane carries the scalar recurrence
-// (identical values, so each lane reads back its own writes of d and e) and
-// lane l applies the rotations to rows l, l+32, ... of z (k x k,
-// column-major).  On exit d holds the eigenvalues.
+// (identical values and identical writes of d and e), lane l tests entry
+// l, l+32, ... for the split and applies the rotations to rows l, l+32, ... of
+// z (k x k, column-major).  On exit d holds the eigenvalues.  The chain of
+// dependent FP64 instructions is the cost (about 64 cycles each): a rotation
+// takes some 25 with plane_rotation instead of 60 with hypot and two
+// divisions.
 __device__ bool tridiag_eigen_warp(double *d, double *e, double *z, int k, int lane)
 {
     for (int q = lane; q < k; q += 32)
@@ -419,30 +512,40 @@ __device__ bool tridiag_eigen_warp(double *d, double *e, double *z, int k, int l
     for (int l = 0; l < k; ++l) {
         int iter = 0, m;
         do {
-            for (m = l; m < k - 1; ++m) {
-                const double dd = fabs(d[m]) + fabs(d[m + 1]);
-                if (fabs(e[m]) <= 1e-16 * dd) break;
+            // first m >= l with a negligible e[m] (k - 1 if there is none)
+            __syncwarp();
+            m = k - 1;
+            for (int q0 = l; q0 < k - 1; q0 += 32) {
+                const int q = q0 + lane;
+                const bool small = q < k - 1 && fabs(e[q]) <= 1e-16 * (fabs(d[q]) + fabs(d[q + 1]));
+                const unsigned ball = __ballot_sync(0xffffffffu, small);
+                if (ball) {
+                    m = q0 + __ffs(ball) - 1;
+                    break;
+                }
             }
             if (m != l) {
                 if (++iter > 60) return false;
-                double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
-                double r = hypot(g, 1.0);
-                g = d[m] - d[l] + e[l] / (g + (g >= 0 ? fabs(r) : -fabs(r)));
+                // shift: d[l] less 2 e^2 / (p + sign(p) sqrt(p^2 + 4 e^2)), p = d[l+1] - d[l]
+                const double el = e[l], dl = d[l], pd = d[l + 1] - dl, e2 = 2.0 * el;
+                const double h = root_or_hypot(pd, e2);
+                double g = d[m] - dl + el * (e2 / (pd + copysign(h, pd)));
                 double s = 1.0, c = 1.0, p = 0.0;
-                int i;
-                for (i = m - 1; i >= l; --i) {
+                bool cut = false;
+                for (int i = m - 1; i >= l; --i) {
                     const double f = s * e[i], b = c * e[i];
-                    r = hypot(f, g);
-                    e[i + 1] = r;
-                    if (r == 0.0) {
+                    const Rot rot = plane_rotation(g, f);
+                    e[i + 1] = rot.r;
+                    if (rot.zero) {
                         d[i + 1] -= p;
                         e[m] = 0.0;
+                        cut = true;
                         break;
                     }
-                    s = f / r;
-                    c = g / r;
+                    s = rot.s;
+                    c = rot.c;
                     g = d[i + 1] - p;
-                    r = (d[i] - g) * s + 2.0 * c * b;
+                    const double r = (d[i] - g) * s + 2.0 * c * b;
                     p = s * r;
                     d[i + 1] = g + p;
                     g = c * r - b;
@@ -453,13 +556,14 @@ __device__ bool tridiag_eigen_warp(double *d, double *e, double *z, int k, int l
                         *z0 = c * *z0 - s * t;
                     }
                 }
-                if (r == 0.0 && i >= l) continue;
+                if (cut) continue;
                 d[l] -= p;
                 e[l] = g;
                 e[m] = 0.0;
             }
         } while (m != l);
     }
+    __syncwarp();
     return true;
 }
 
@@ -488,25 +592,28 @@ struct LzArgs {
 // warp, forms the coefficients c of the noise |z| factor V^T Q sqrt(L) Q^T e1
 // and applies the stopping test |c - c_old| < tol |c_old|.  A segment that
 // stopped at the previous iteration is frozen (its w and next vector zero).
+// At 36,864 unknowns 32 us for iteration 0 and 126 us for iteration 5 before
+// root_inv, plane_rotation and the single-word barrier; 27 and 80 us with them.
 __global__ void __launch_bounds__(kKdThreads, 3) lanczos_step_kernel(LzArgs A)
 {
     __shared__ double red[kKdMaxBasis * 32];
     __shared__ double hsh[kKdMaxBasis];
     __shared__ double tdg[kLzShared], tsd[kLzShared];  // the owner warp's tridiagonal matrix
-    __shared__ int actv[8];
+    __shared__ JobCache jc;
+    __shared__ int actv[kJobCache];
     const int i = *(volatile int *)&A.st->i;
     const int k = i + 1;
     double *const V = *(double *volatile *)&A.st->V;
     const long long ldv = A.st->ldv;
     const int jb0 = A.bjob[blockIdx.x], jb1 = A.bjob[blockIdx.x + 1];
     // frozen segments: read once, before any owner can change them (owners write after the last barrier)
-    for (int job = jb0; job < jb1 && job - jb0 < 8; ++job)
-        if (threadIdx.x == 0) actv[job - jb0] = A.cyc[A.jobs[job].seg];
+    job_cache_fill(jc, A.jobs, A.sjob, jb0, jb1);
+    if (threadIdx.x < kJobCache && jb0 + (int)threadIdx.x < jb1) actv[threadIdx.x] = A.cyc[jc.jb[threadIdx.x].seg];
     __syncthreads();
     // pass 1: w -= hs[i-1] V_{i-1} (frozen: w = 0) and, in the same pass, partial <w, V_i>
     for (int job = jb0; job < jb1; ++job) {
-        const KJob jb = A.jobs[job];
-        const bool on = (job - jb0 < 8) ? actv[job - jb0] != 0 : A.cyc[jb.seg] != 0;
+        const KJob jb = job_info(jc, A.jobs, A.sjob, jb0, job).jb;
+        const bool on = (job - jb0 < kJobCache) ? actv[job - jb0] != 0 : A.cyc[jb.seg] != 0;
         const double hp = (i > 0) ? A.hs[(long long)jb.seg * A.kcap + i - 1] : 0.0;
         const double *Vp = V + (long long)(i > 0 ? i - 1 : 0) * ldv;
         double *w = A.w;
@@ -516,25 +623,27 @@ __global__ void __launch_bounds__(kKdThreads, 3) lanczos_step_kernel(LzArgs A)
             return x;
         });
     }
-    grid_barrier(&A.st->bar);
+    grid_barrier(&A.st->bar, gridDim.x);
     // pass 2: hd = <w, V_i>; w -= hd V_i; partial |w|^2
     for (int job = jb0; job < jb1; ++job) {
-        const KJob jb = A.jobs[job];
-        reduce_segment(A.partA, A.KP, A.sjob[jb.seg], A.sjob[jb.seg + 1], 1, hsh);
+        const JobInfo f = job_info(jc, A.jobs, A.sjob, jb0, job);
+        const KJob jb = f.jb;
+        reduce_segment(A.partA, A.KP, f.s0, f.s1, 1, hsh);
         const double nrm = job_update(V + (long long)i * ldv, ldv, 1, hsh, A.w, jb);
-        if (job == A.sjob[jb.seg] && threadIdx.x == 0) A.dt[(long long)jb.seg * A.kcap] = hsh[0];  // hd[i], kept below
+        if (job == f.s0 && threadIdx.x == 0) A.dt[(long long)jb.seg * A.kcap] = hsh[0];  // hd[i], kept below
         __syncthreads();
         job_norm_partial(nrm, A.partC, A.KP, job, red);
     }
-    grid_barrier(&A.st->bar);
+    grid_barrier(&A.st->bar, 2 * gridDim.x);
     // pass 3: hs = |w|; w /= hs (0 on an exact breakdown) during the first pass of the partial
     // reorthogonalisation dots V_q^T w
     for (int job = jb0; job < jb1; ++job) {
-        const KJob jb = A.jobs[job];
-        reduce_segment(A.partC, A.KP, A.sjob[jb.seg], A.sjob[jb.seg + 1], 1, hsh);
-        const double wn = sqrt(hsh[0]);
-        const double inv = (wn > 0.0) ? 1.0 / wn : 0.0;
-        if (job == A.sjob[jb.seg] && threadIdx.x == 0) A.et[(long long)jb.seg * A.kcap] = wn;
+        const JobInfo f = job_info(jc, A.jobs, A.sjob, jb0, job);
+        const KJob jb = f.jb;
+        reduce_segment(A.partC, A.KP, f.s0, f.s1, 1, hsh);
+        const RootInv wn = root_inv(hsh[0]);
+        const double inv = wn.inv;
+        if (job == f.s0 && threadIdx.x == 0) A.et[(long long)jb.seg * A.kcap] = wn.root;
         __syncthreads();
         double *w = A.w;
         for (int q0 = 0; q0 < k; q0 += kKdMaxBasis)
@@ -548,21 +657,22 @@ __global__ void __launch_bounds__(kKdThreads, 3) lanczos_step_kernel(LzArgs A)
                            return w[e];
                        });
     }
-    grid_barrier(&A.st->bar);
+    grid_barrier(&A.st->bar, 3 * gridDim.x);
     // pass 4: w -= V h; V_{i+1} = w; owners: tridiagonal eigen-problem, coefficients, stopping test
     for (int job = jb0; job < jb1; ++job) {
-        const KJob jb = A.jobs[job];
+        const JobInfo f = job_info(jc, A.jobs, A.sjob, jb0, job);
+        const KJob jb = f.jb;
         double *Vn = V + (long long)(i + 1) * ldv;
         for (int q0 = 0; q0 < k; q0 += kKdMaxBasis) {
             const int kc = min(kKdMaxBasis, k - q0);
-            reduce_segment(A.partB + q0, A.KP, A.sjob[jb.seg], A.sjob[jb.seg + 1], kc, hsh);
+            reduce_segment(A.partB + q0, A.KP, f.s0, f.s1, kc, hsh);
             // the last group's pass also writes V_{i+1} and the operator's next input
             const bool last = q0 + kc >= k;
             job_update(V + (long long)q0 * ldv, ldv, kc, hsh, A.w, jb, last ? Vn : nullptr, last ? A.xin : nullptr);
             __syncthreads();
         }
         const int s = jb.seg;
-        if (job == A.sjob[s] && A.cyc[s] && threadIdx.x < 32) {
+        if (job == f.s0 && A.cyc[s] && threadIdx.x < 32) {
             const int lane = threadIdx.x;
             const long long so = (long long)s * A.kcap;
             const double hdi = A.dt[so], wn = A.et[so];
@@ -596,12 +706,14 @@ __global__ void __launch_bounds__(kKdThreads, 3) lanczos_step_kernel(LzArgs A)
                     double *cc = A.c + so, *co = A.cold + so;
                     const double sc = A.zn[s] * A.factor;
                     double dn = 0.0, on = 0.0;
+                    for (int jj = lane; jj < k; jj += 32) {  // ee is free: the factors of the rows' sums
+                        const double lam = d[jj] > 0.0 ? sqrt(d[jj]) : 0.0;
+                        ee[jj] = zz[(long long)k * jj] * lam * sc;
+                    }
+                    __syncwarp();
                     for (int q = lane; q < k; q += 32) {
                         double acc = 0.0;
-                        for (int jj = 0; jj < k; ++jj) {
-                            const double lam = d[jj] > 0.0 ? sqrt(d[jj]) : 0.0;
-                            acc += zz[q + (long long)k * jj] * (zz[(long long)k * jj] * lam * sc);
-                        }
+                        for (int jj = 0; jj < k; ++jj) acc += zz[q + (long long)k * jj] * ee[jj];
                         const double old = (q < i) ? co[q] : 0.0;
                         dn += (acc - old) * (acc - old);
                         on += old * old;
@@ -652,8 +764,8 @@ __global__ void __launch_bounds__(kKdThreads, 3) lanczos_step_kernel(LzArgs A)
                         A.mask[(long long)p * A.nsusp + u] = any;
                     }
             }
-            atomicExch(&A.st->bar.done, 0u);
-            __threadfence();
+            A.st->bar.count = 0;
+            A.st->bar.done = 0;
             if (A.use_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)A.cond, (unsigned)more);
         }
     }
@@ -999,6 +1111,7 @@ __global__ void lz_init_kernel(const double *__restrict__ nrm, int nseg, double 
         st->dev_k = kLzDeviceRows;
         st->host = 0;
         st->bar.done = 0;
+        st->bar.count = 0;
     }
 }
 

@@ -51,8 +51,7 @@ struct KJob {
 // grid barrier and last-CTA detection of one cooperative step kernel
 struct GridBar {
     unsigned done;  // CTAs finished with the step (last-CTA detection)
-    unsigned count;
-    unsigned gen;
+    unsigned count;  // arrivals at the launch's grid barriers
     int err;  // a grid barrier gave up waiting
 };
 
