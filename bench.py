@@ -63,7 +63,7 @@ DF64_UF_TRAFFIC_BYTES = {"symmetric": 744960, "standard": 710400}
 # counted twice as above ((smsp__inst_executed.sum 17,258,189,476 + packed 12,838,677,918) * 32 / (N^2 * 16),
 # 60,000 blobs)
 MULTI16_INST_PER_PAIR_RHS = 16.72
-DF64_UF_KERNEL_SOURCE_SHA = "0522c35e6745d2292d11f52dc3a84740a01081013519f7a092067f2e8417876d"
+DF64_UF_KERNEL_SOURCE_SHA = "080da48b09099f70d1748cd44e2c15685534fe86c7ad374b1a391062ed4bc5da"
 
 
 def df64_uf_kernel_source_sha():

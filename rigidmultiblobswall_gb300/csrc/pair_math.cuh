@@ -144,8 +144,7 @@ __device__ __forceinline__ void pair_contrib(T dx, T dy, T dz, T Rz, T hi, T hj,
 // finalize kernels multiply the pair sums by 2/3 in FP64), for the FP32 pair
 // kernels:  (3/2) M v = Af v + (Bc (d.v) + c2 W + c3 vz) (dx, dy, .) ...
 // with W = dx vx + dy vy + Rz vz (see uf_apply).  The 3/2 turns the RPY and
-// Swan-Brady constants into the small integers and halves below; the same
-// coefficients as the double-float pair_uf_sym_df:
+// Swan-Brady constants into the small integers and halves below:
 //   (3/2) A  = 3/(2r) + 1/r^3,          (3/2) Bc = (3/2 - 3/r^2) / r^3
 //   (3/2) f1 = -(3/2 + 3 hh) s - [(1 - 3E) t - (1 - 5E) p]
 //   (3/2) f2 = -(3/2 - 9 hh) s + 3 (1 - 5E) t - 5 (1 - 7E) p
@@ -155,62 +154,64 @@ __device__ __forceinline__ void pair_contrib(T dx, T dy, T dz, T Rz, T hi, T hj,
 // with t = s^3, p = s^5, E = (Rz s)^2, hh = h_i h_j s^2; for r <= 2
 // (3/2) A = 2 (1 - 9r/32), (3/2) Bc = 3 / (16 r).
 constexpr double kUFCoeffScale = 2.0 / 3.0;  // undoes the 3/2
-template <typename T> struct UFCoeffs {
-    T Af, Bc, c2, c3, c4, Af5;  // Af5 = Af + f5, the zz diagonal
+struct UFCoeffs {
+    float Af, Bc, c2, c3, c4, Af5;  // Af5 = Af + f5, the zz diagonal
 };
 
-template <typename T>
-__device__ __forceinline__ UFCoeffs<T> uf_coeffs(T dx, T dy, T dz, T Rz, T hi, T hj)
+__device__ __forceinline__ UFCoeffs uf_coeffs(float dx, float dy, float dz, float Rz, float hi, float hj)
 {
-    const T rho2 = dx * dx + dy * dy;
-    const T r2 = rho2 + dz * dz;
-    const T invr = rsq<T>(r2);
-    const T Rz2 = Rz * Rz;
-    const T s = rsq<T>(rho2 + Rz2);
-    const T u = s * s;
-    const T t = u * s;
-    const T p = t * u;
-    const T E = Rz2 * u;
-    const T invr2 = invr * invr;
-    const T invr3 = invr2 * invr;
-    T A = T(1.5) * invr + invr3;
-    T Bc = (T(1.5) - T(3) * invr2) * invr3;
-    const bool near = !(r2 > T(4));  // r <= 2
+    const float rho2 = dx * dx + dy * dy;
+    const float r2 = rho2 + dz * dz;
+    const float invr = rsqrt_approx(r2);
+    const float Rz2 = Rz * Rz;
+    const float s = rsqrt_approx(rho2 + Rz2);
+    const float u = s * s;
+    const float t = u * s;
+    const float p = t * u;
+    const float E = Rz2 * u;
+    const float invr2 = invr * invr;
+    const float invr3 = invr2 * invr;
+    float A = 1.5f * invr + invr3;
+    float Bc = (1.5f - 3.0f * invr2) * invr3;
+    const bool near = !(r2 > 4.0f);  // r <= 2
     if (__any_sync(__activemask(), near)) {
         if (near) {
-            const T r = r2 * invr;
-            A = T(2) - T(0.5625) * r;
-            Bc = T(0.1875) * invr;
+            const float r = r2 * invr;
+            A = 2.0f - 0.5625f * r;
+            Bc = 0.1875f * invr;
         }
     }
-    const T hh = hi * hj * u;
-    const T q5 = (T(1) - T(5) * E) * t;
-    const T Ru = Rz * u;
-    const T hjt3 = T(3) * hj * t;
-    const T f1 = -((T(1.5) + T(3) * hh) * s + ((T(1) - T(3) * E) * t - q5 * u));
-    const T f2 = T(3) * q5 - (T(1.5) - T(9) * hh) * s - T(5) * (T(1) - T(7) * E) * p;
-    const T c3 = hjt3 - T(18) * hh * Rz * t + Ru * (T(10) * (T(2) - T(7) * E) * p - T(6) * q5);
-    const T c4 = hjt3 - T(10) * Ru * p;
-    const T f5 = T(-2) * (T(3) * (hj * hj + E) * t + (T(2) - T(15) * E) * p);
-    const T Af = A + f1;
+    const float hh = hi * hj * u;
+    const float q5 = (1.0f - 5.0f * E) * t;
+    const float Ru = Rz * u;
+    const float hjt3 = 3.0f * hj * t;
+    const float f1 = -((1.5f + 3.0f * hh) * s + ((1.0f - 3.0f * E) * t - q5 * u));
+    const float f2 = 3.0f * q5 - (1.5f - 9.0f * hh) * s - 5.0f * (1.0f - 7.0f * E) * p;
+    const float c3 = hjt3 - 18.0f * hh * Rz * t + Ru * (10.0f * (2.0f - 7.0f * E) * p - 6.0f * q5);
+    const float c4 = hjt3 - 10.0f * Ru * p;
+    const float f5 = -2.0f * (3.0f * (hj * hj + E) * t + (2.0f - 15.0f * E) * p);
+    const float Af = A + f1;
     return {Af, Bc, f2 * u, c3, c4, Af + f5};
 }
 
-template <typename T>
-__device__ __forceinline__ void uf_apply(const UFCoeffs<T> &c, T dx, T dy, T dz, T Rz, T vx, T vy, T vz, T &ux,
-                                         T &uy, T &uz)
+// (M v) of uf_coeffs: every term chained into the accumulator by an FMA (two plain
+// multiplies and one subtraction per application)
+__device__ __forceinline__ void uf_apply(const UFCoeffs &c, float dx, float dy, float dz, float Rz, float vx, float vy,
+                                         float vz, float &ux, float &uy, float &uz)
 {
-    const T Pxy = dx * vx + dy * vy;
-    const T Gr = c.Bc * (Pxy + dz * vz);
-    const T W = Pxy + Rz * vz;
-    const T Gw = c.c2 * W + c.c3 * vz;
-    const T G = Gr + Gw;
-    ux += c.Af * vx + G * dx;
-    uy += c.Af * vy + G * dy;
-    uz += c.Af5 * vz + Gr * dz + Gw * Rz + c.c4 * W;
+    // with dv = d.v, G = Bc dv + Gw and Rz - dz = 2 h_j:
+    // (M v)_z = Af5 vz + G dz + Gw (Rz - dz) + c4 W
+    const float h2 = Rz - dz;
+    const float dv = fmaf(dz, vz, fmaf(dy, vy, dx * vx));
+    const float W = fmaf(h2, vz, dv);
+    const float Gw = fmaf(c.c2, W, c.c3 * vz);
+    const float G = fmaf(c.Bc, dv, Gw);
+    ux = fmaf(c.Af, vx, fmaf(G, dx, ux));
+    uy = fmaf(c.Af, vy, fmaf(G, dy, uy));
+    uz = fmaf(c.Af5, vz, fmaf(G, dz, fmaf(Gw, h2, fmaf(c.c4, W, uz))));
 }
 
-// uf_coeffs<float> for two pairs in packed lanes: every operation written out
+// uf_coeffs for two pairs in packed lanes: every operation written out
 // with the contractions the compiler gives the scalar form (products that
 // feed a sum fused into it, the operands of other products rounded), so a
 // mixed product is the same to the bit whichever form forms its blocks.
@@ -271,7 +272,7 @@ __device__ __forceinline__ UFCoeffs2 uf_coeffs_f2(f2 dx, f2 dy, f2 dz, f2 Rz, f2
     return c;
 }
 
-// uf_apply<float> in packed lanes
+// uf_apply in packed lanes
 __device__ __forceinline__ void uf_apply_f2(const UFCoeffs2 &c, f2 c3, f2 c4, f2 dx, f2 dy, f2 dz, f2 h2, f2 vx, f2 vy,
                                             f2 vz, f2 &ux, f2 &uy, f2 &uz)
 {
@@ -312,24 +313,6 @@ __device__ __forceinline__ UFBlock2 uf_block_f2(const UFCoeffs2 &c, f2 dx, f2 dy
     m.zy = f2_mul(dy, t4);
     m.zz = f2_fma(f2_fma(c.c2, Rz, f2_add(c.c3, c.c4)), Rz, f2_fma(f2_mul(c.Bc, dz), dz, c.Af5));
     return m;
-}
-
-// FP32: every term chained into the accumulator by an FMA (two plain
-// multiplies and one subtraction per application)
-template <>
-__device__ __forceinline__ void uf_apply<float>(const UFCoeffs<float> &c, float dx, float dy, float dz, float Rz,
-                                                float vx, float vy, float vz, float &ux, float &uy, float &uz)
-{
-    // with dv = d.v, G = Bc dv + Gw and Rz - dz = 2 h_j:
-    // (M v)_z = Af5 vz + G dz + Gw (Rz - dz) + c4 W
-    const float h2 = Rz - dz;
-    const float dv = fmaf(dz, vz, fmaf(dy, vy, dx * vx));
-    const float W = fmaf(h2, vz, dv);
-    const float Gw = fmaf(c.c2, W, c.c3 * vz);
-    const float G = fmaf(c.Bc, dv, Gw);
-    ux = fmaf(c.Af, vx, fmaf(G, dx, ux));
-    uy = fmaf(c.Af, vy, fmaf(G, dy, uy));
-    uz = fmaf(c.Af5, vz, fmaf(G, dz, fmaf(Gw, h2, fmaf(c.c4, W, uz))));
 }
 
 // The explicit M_UF block in FP64, times 3/2: the formulas of uf_block_df
@@ -719,6 +702,5 @@ template <typename T> __device__ __forceinline__ T project(T d, T L)
     T s = (T)((d > T(0)) - (d < T(0)));
     return d - (T)(long long)(d / L + T(0.5) * s) * L;
 }
-
 
 }  // namespace rmw

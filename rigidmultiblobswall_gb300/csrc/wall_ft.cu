@@ -458,11 +458,11 @@ __global__ void __launch_bounds__(kFtSymTile) ft_sym_mixed_kernel(const FtSrcF *
         const float hj = sh.z + sl.z;
         const float Rz = hi + hj;
         float a0 = sacc[warp][0][jl], a1 = sacc[warp][1][jl], a2 = sacc[warp][2][jl];
-        UFCoeffs<float> c = uf_coeffs<float>(dx, dy, dz, Rz, hi, hj);
+        UFCoeffs c = uf_coeffs(dx, dy, dz, Rz, hi, hj);
         c.Af *= kThird2; c.Bc *= kThird2; c.c2 *= kThird2; c.c3 *= kThird2; c.c4 *= kThird2; c.Af5 *= kThird2;
-        uf_apply<float>(c, dx, dy, dz, Rz, sf.x, sf.y, sf.z, u0, u1, u2);
-        const UFCoeffs<float> ct = {c.Af, c.Bc, c.c2, c.c4, c.c3, c.Af5};  // M^T: f3 and f4 trade places
-        uf_apply<float>(ct, dx, dy, dz, Rz, me.f.x, me.f.y, me.f.z, a0, a1, a2);
+        uf_apply(c, dx, dy, dz, Rz, sf.x, sf.y, sf.z, u0, u1, u2);
+        const UFCoeffs ct = {c.Af, c.Bc, c.c2, c.c4, c.c3, c.Af5};  // M^T: f3 and f4 trade places
+        uf_apply(ct, dx, dy, dz, Rz, me.f.x, me.f.y, me.f.z, a0, a1, a2);
         pair_rot_sym<float, RMW_UT>(dx, dy, dz, Rz, hi, hj, st.x, st.y, st.z, me.t.x, me.t.y, me.t.z, u0, u1, u2, a0,
                                     a1, a2);
         sacc[warp][0][jl] = a0;
