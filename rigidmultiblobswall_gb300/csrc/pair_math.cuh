@@ -2,7 +2,10 @@
 // all-pairs product kernels and the dense per-body mobility of the
 // preconditioner).
 #pragma once
+#include <type_traits>
+
 #include "f32x2.cuh"
+#include "fp64_int.cuh"
 #include "rmw_common.cuh"
 
 namespace rmw {
@@ -323,30 +326,43 @@ __device__ __forceinline__ UFBlock2 uf_block_f2(const UFCoeffs2 &c, f2 dx, f2 dy
 struct PairGeoD {
     double r2, invr, i2, u, s, t, p;
 };
-template <bool ZPER>
-__device__ __forceinline__ PairGeoD pair_geo_d(double dx, double dy, double dz, double Rz, double hi, double hj)
+// MUL = MulInt needs r2 and R2 (the squared distances of a pair, the second to
+// the mirror image) within int_range.
+template <class MUL>
+__device__ __forceinline__ PairGeoD pair_geo_d(double r2, double R2)
 {
+    constexpr bool I = std::is_same<MUL, MulInt>::value;
     PairGeoD g;
-    const double rho2 = fma(dx, dx, dy * dy);
-    g.r2 = fma(dz, dz, rho2);
-    g.invr = rsqrt64(g.r2);
-    g.s = rsqrt64(ZPER ? fma(Rz, Rz, rho2) : fma(4.0 * hi, hj, g.r2));
-    g.i2 = g.invr * g.invr;
-    g.u = g.s * g.s;
-    g.t = g.u * g.s;
-    g.p = g.t * g.u;
+    g.r2 = r2;
+    g.invr = I ? int_rsqrt(r2) : rsqrt64(r2);
+    g.s = I ? int_rsqrt(R2) : rsqrt64(R2);
+    g.i2 = MUL::pos(g.invr, g.invr);
+    g.u = MUL::pos(g.s, g.s);
+    g.t = MUL::pos(g.u, g.s);
+    g.p = MUL::pos(g.t, g.u);
     return g;
+}
+// Squared distances and f(geometry, MUL()): the integer forms where every lane's pair allows them (all but dummies,
+// coincident blobs and distances beyond 2^32 radii), else the FP64 ones.  ZPER pairs (dz an image's) take the latter.
+template <bool ZPER, class F>
+__device__ __forceinline__ void with_pair_geo_d(double dx, double dy, double dz, double Rz, double hi, double hj, F &&f)
+{
+    const double rho2 = fma(dx, dx, dy * dy), r2 = fma(dz, dz, rho2);
+    const double R2 = ZPER ? fma(Rz, Rz, rho2) : fma(4.0 * hi, hj, r2);
+    if (!ZPER && __all_sync(__activemask(), int_range(r2) && int_range(R2))) f(pair_geo_d<MulInt>(r2, R2), MulInt());
+    else f(pair_geo_d<MulFp64>(r2, R2), MulFp64());
 }
 struct UFBlockD {
     double Af, b2, t3, t4, zz;
 };
-template <bool ZPER>
-__device__ __forceinline__ UFBlockD uf_block_d(const PairGeoD &g, double dz, double Rz, double hi, double hj)
+template <bool ZPER, class MUL = MulFp64>
+__device__ __forceinline__ UFBlockD uf_block_d(const PairGeoD &g, double dz, double Rz, double hi, double hj,
+                                               MUL = MUL())
 {
-    const double k = hi * hj, z2 = Rz * Rz;
-    double ia = g.invr, a3 = g.i2 * g.invr;
-    double Bc = fma(-3.0, g.i2, 1.5) * a3;
-    const bool near = !(g.r2 > 4.0);  // r <= 2
+    const double k1 = fma(3.0 * hi, hj, 1.0), z2 = MUL::pos(Rz, Rz);  // 3 h_i h_j + 1
+    double ia = g.invr, a3 = MUL::pos(g.i2, g.invr);
+    double Bc = MUL::pos(fma(-3.0, g.i2, 1.5), a3);  // positive where it is used (r > 2)
+    const bool near = MUL::le4(g.r2);                // r <= 2
     if (__any_sync(__activemask(), near)) {
         if (near) {
             ia = 0.0;
@@ -355,15 +371,15 @@ __device__ __forceinline__ UFBlockD uf_block_d(const PairGeoD &g, double dz, dou
         }
     }
     const double s = g.s, u = g.u, t = g.t, p = g.p;
-    const double E = z2 * u;
+    const double E = MUL::pos(z2, u);
     const double b1 = fma(3.0, z2, 1.0);
     const double w5 = fma(-5.0, E, b1), w7 = fma(-7.0, E, b1);
-    const double Y = fma(-5.0, u * w7, fma(9.0, k, 3.0));
+    const double Y = fma(-5.0, MUL::mul(u, w7), fma(9.0 * hi, hj, 3.0));
     const double Y10 = fma(-10.0, u, Y);
     const double Z = fma(z2, fma(-20.0, u, Y10) + 6.0, 4.0);
-    const double X = Rz * p * Y10;
+    const double X = MUL::mul(MUL::pos(Rz, p), Y10);
     UFBlockD m;
-    m.Af = fma(p, w5, fma(-fma(3.0, k, 1.0), t, fma(1.5, ia - s, a3)));
+    m.Af = fma(p, w5, fma(-k1, t, fma(1.5, ia - s, a3)));
     const double F = fma(-1.5, t, Bc);
     m.b2 = fma(p, Y, F);
     double G, dG;  // dz F, dz^2 F
@@ -372,8 +388,8 @@ __device__ __forceinline__ UFBlockD uf_block_d(const PairGeoD &g, double dz, dou
         G = x + w;
         dG = fma(dz, x, dw * w);
     } else {
-        G = dz * F;
-        dG = dz * G;
+        G = MUL::mul(dz, F);
+        dG = MUL::mul(dz, G);
     }
     m.t3 = G - X;
     m.t4 = G + X;
@@ -399,34 +415,35 @@ __device__ __forceinline__ void uf_block_acc_d(const UFBlockD &m, double t3, dou
 struct RotBlockD {
     double a, ar, b, ei, ej, wi, wj;
 };
-template <bool UF32 = false>
-__device__ __forceinline__ RotBlockD rot_block_d(const PairGeoD &g, double dz, double Rz, double hi, double hj)
+template <bool UF32 = false, class MUL = MulFp64>
+__device__ __forceinline__ RotBlockD rot_block_d(const PairGeoD &g, double dz, double Rz, double hi, double hj,
+                                                 MUL = MUL())
 {
     constexpr double f = UF32 ? 1.5 : 1.0;
-    double c = g.i2 * g.invr;
-    const bool near = !(g.r2 >= 4.0);  // r < 2
+    double c = MUL::pos(g.i2, g.invr);
+    const bool near = MUL::lt4(g.r2);  // r < 2
     if (__any_sync(__activemask(), near)) {
         if (near) c = fma(-0.1875, g.r2 * g.invr, 0.5);
     }
     RotBlockD k;
     k.b = UF32 ? 1.5 * (g.t - c) : g.t - c;
-    const double m = dz * k.b, Rp = Rz * g.p, Ru = Rz * g.u;
+    const double m = MUL::mul(dz, k.b), Rp = MUL::pos(Rz, g.p), Ru = MUL::pos(Rz, g.u);
     k.a = fma(2.0 * f, Rp, -m);
     k.ar = fma(2.0 * f, Rp, m);
     const double R10 = 10.0 * f * Ru, R6 = 6.0 * f * Rz, y = fma(-10.0 * f * Rz, Ru, 2.0 * f);
-    k.ei = g.p * fma(-6.0 * f, hi, R10);
-    k.ej = g.p * fma(-6.0 * f, hj, R10);
+    k.ei = MUL::mul(g.p, fma(-6.0 * f, hi, R10));
+    k.ej = MUL::mul(g.p, fma(-6.0 * f, hj, R10));
     k.wi = fma(g.p, fma(R6, hi, y), k.b);
     k.wj = fma(g.p, fma(R6, hj, y), k.b);
     return k;
 }
-template <bool UF32 = false>
-__device__ __forceinline__ UFBlockD wt_block_d(const PairGeoD &g, double dz, double Rz)
+template <bool UF32 = false, class MUL = MulFp64>
+__device__ __forceinline__ UFBlockD wt_block_d(const PairGeoD &g, double dz, double Rz, MUL = MUL())
 {
     constexpr double f = UF32 ? 1.5 : 1.0;
-    const double i3 = g.i2 * g.invr;
-    double A = -0.5 * f * i3, Bc = 1.5 * f * g.i2 * i3;
-    const bool near = !(g.r2 >= 4.0);
+    const double i3 = MUL::pos(g.i2, g.invr);
+    double A = -0.5 * f * i3, Bc = 1.5 * f * MUL::pos(g.i2, i3);
+    const bool near = MUL::lt4(g.r2);
     if (__any_sync(__activemask(), near)) {
         if (near) {
             const double r = g.r2 * g.invr;
@@ -434,7 +451,8 @@ __device__ __forceinline__ UFBlockD wt_block_d(const PairGeoD &g, double dz, dou
             Bc = f * fma(-0.046875, r, 0.28125 * g.invr);
         }
     }
-    const double Et = Rz * Rz * g.u * g.t, D = Bc * dz, X = 1.5 * f * g.p * Rz;
+    const double Ru = MUL::pos(Rz, g.u), Et = MUL::pos(MUL::pos(Rz, Ru), g.t);
+    const double D = MUL::mul(Bc, dz), X = 1.5 * f * MUL::pos(g.p, Rz);
     UFBlockD m;
     m.Af = fma(-6.0 * f, Et, fma(3.5 * f, g.t, A));
     m.b2 = fma(-4.5 * f, g.p, Bc);
@@ -587,15 +605,13 @@ __device__ __forceinline__ void pair_rot_sym(T dx, T dy, T dz, T Rz, T hi, T hj,
 // kernels): M_ji = M_ij(-d), so UF and WT (even in d) apply the same block to
 // the other vector and UT / WF (odd in d) its negative.  (ux, uy, uz) +=
 // M_ij v, (wx, wy, wz) += M_ji q.
-template <typename T, int KIND>
-__device__ __forceinline__ void pair_rpy_sym(T dx, T dy, T dz, T vx, T vy, T vz, T qx, T qy, T qz, T &ux, T &uy,
-                                             T &uz, T &wx, T &wy, T &wz)
+template <typename T, int KIND, class MUL>
+__device__ __forceinline__ void pair_rpy_sym_body(T r2, T invr, T dx, T dy, T dz, T vx, T vy, T vz, T qx, T qy, T qz,
+                                                  T &ux, T &uy, T &uz, T &wx, T &wy, T &wz)
 {
-    const T r2 = fm<T>(dx, dx, fm<T>(dy, dy, dz * dz));
-    const T invr = rsq<T>(r2);
     if (KIND == RMW_UT || KIND == RMW_WF) {
-        T c = invr * invr * invr;
-        const bool near = !(r2 >= T(4));  // r < 2
+        T c = MUL::pos(MUL::pos(invr, invr), invr);
+        const bool near = MUL::lt4(r2);  // r < 2
         if (__any_sync(__activemask(), near)) {
             if (near) c = T(0.5) * (T(1) - T(0.375) * (r2 * invr));
         }
@@ -607,12 +623,12 @@ __device__ __forceinline__ void pair_rpy_sym(T dx, T dy, T dz, T vx, T vy, T vz,
         wz = fm<T>(-c, fm<T>(dy, qx, -dx * qy), wz);
         return;
     }
-    const T invr2 = invr * invr;
+    const T invr2 = MUL::pos(invr, invr);
     T A, Bc;
     if (KIND == RMW_UF) {
-        A = (T(1) + T(2.0 / 3.0) * invr2) * invr;
-        Bc = (T(1) - T(2) * invr2) * invr2 * invr;
-        const bool near = !(r2 > T(4));  // r <= 2
+        A = MUL::pos(T(1) + T(2.0 / 3.0) * invr2, invr);
+        Bc = MUL::pos(MUL::pos(T(1) - T(2) * invr2, invr2), invr);  // positive where it is used
+        const bool near = MUL::le4(r2);  // r <= 2
         if (__any_sync(__activemask(), near)) {
             if (near) {
                 const T r = r2 * invr;
@@ -621,10 +637,10 @@ __device__ __forceinline__ void pair_rpy_sym(T dx, T dy, T dz, T vx, T vy, T vz,
             }
         }
     } else {  // RMW_WT
-        const T invr3 = invr2 * invr;
+        const T invr3 = MUL::pos(invr2, invr);
         A = T(-0.5) * invr3;
-        Bc = T(1.5) * invr2 * invr3;
-        const bool near = !(r2 >= T(4));
+        Bc = MUL::pos(T(1.5) * invr2, invr3);
+        const bool near = MUL::lt4(r2);
         if (__any_sync(__activemask(), near)) {
             if (near) {
                 const T r = r2 * invr;
@@ -641,6 +657,20 @@ __device__ __forceinline__ void pair_rpy_sym(T dx, T dy, T dz, T vx, T vy, T vz,
     wx = fm<T>(A, qx, fm<T>(Gq, dx, wx));
     wy = fm<T>(A, qy, fm<T>(Gq, dy, wy));
     wz = fm<T>(A, qz, fm<T>(Gq, dz, wz));
+}
+template <typename T, int KIND>
+__device__ __forceinline__ void pair_rpy_sym(T dx, T dy, T dz, T vx, T vy, T vz, T qx, T qy, T qz, T &ux, T &uy,
+                                             T &uz, T &wx, T &wy, T &wz)
+{
+    const T r2 = fm<T>(dx, dx, fm<T>(dy, dy, dz * dz));
+    if constexpr (std::is_same<T, double>::value) {
+        if (__all_sync(__activemask(), int_range(r2))) {  // as with_pair_geo_d
+            pair_rpy_sym_body<T, KIND, MulInt>(r2, int_rsqrt(r2), dx, dy, dz, vx, vy, vz, qx, qy, qz, ux, uy, uz, wx,
+                                               wy, wz);
+            return;
+        }
+    }
+    pair_rpy_sym_body<T, KIND, MulPipe<T>>(r2, rsq<T>(r2), dx, dy, dz, vx, vy, vz, qx, qy, qz, ux, uy, uz, wx, wy, wz);
 }
 
 // Free-space RPY blocks (no wall): the RPY parts of pair_contrib, for the

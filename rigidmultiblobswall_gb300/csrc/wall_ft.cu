@@ -585,20 +585,22 @@ __global__ void __launch_bounds__(kFtSymTile) ft_sym_fp64_kernel(const FtSrcD *_
         const double fx = sx[3][j], fy = sx[4][j], fz = sx[5][j], tx = sx[6][j], ty = sx[7][j], tz = sx[8][j];
         double w[NC];
         for (int c = 0; c < NC; ++c) w[c] = sacc[warp][c][j];
-        const PairGeoD g = pair_geo_d<false>(dx, dy, dz, Rz, me.z, zj);
-        {
-            const UFBlockD m = uf_block_d<false>(g, dz, Rz, me.z, zj);
-            uf_block_acc_d(m, m.t3, m.t4, dx, dy, fx, fy, fz, u[0], u[1], u[2]);
-            uf_block_acc_d(m, m.t4, m.t3, dx, dy, me.fx, me.fy, me.fz, w[0], w[1], w[2]);
-        }
-        const RotBlockD k2 = rot_block_d<true>(g, dz, Rz, me.z, zj);
-        ut_acc_d(k2, dx, dy, tx, ty, tz, me.tx, me.ty, me.tz, u[0], u[1], u[2], w[0], w[1], w[2]);
-        if constexpr (WITH_W) {
-            wf_acc_d(k2, dx, dy, fx, fy, fz, me.fx, me.fy, me.fz, u[3], u[4], u[5], w[3], w[4], w[5]);
-            const UFBlockD m = wt_block_d<true>(g, dz, Rz);
-            uf_block_acc_d(m, m.t3, m.t4, dx, dy, tx, ty, tz, u[3], u[4], u[5]);
-            uf_block_acc_d(m, m.t4, m.t3, dx, dy, me.tx, me.ty, me.tz, w[3], w[4], w[5]);
-        }
+        with_pair_geo_d<false>(dx, dy, dz, Rz, me.z, zj, [&](const PairGeoD &g, auto mul) {
+            using MUL = decltype(mul);
+            {
+                const UFBlockD m = uf_block_d<false, MUL>(g, dz, Rz, me.z, zj);
+                uf_block_acc_d(m, m.t3, m.t4, dx, dy, fx, fy, fz, u[0], u[1], u[2]);
+                uf_block_acc_d(m, m.t4, m.t3, dx, dy, me.fx, me.fy, me.fz, w[0], w[1], w[2]);
+            }
+            const RotBlockD k2 = rot_block_d<true, MUL>(g, dz, Rz, me.z, zj);
+            ut_acc_d(k2, dx, dy, tx, ty, tz, me.tx, me.ty, me.tz, u[0], u[1], u[2], w[0], w[1], w[2]);
+            if constexpr (WITH_W) {
+                wf_acc_d(k2, dx, dy, fx, fy, fz, me.fx, me.fy, me.fz, u[3], u[4], u[5], w[3], w[4], w[5]);
+                const UFBlockD m = wt_block_d<true, MUL>(g, dz, Rz);
+                uf_block_acc_d(m, m.t3, m.t4, dx, dy, tx, ty, tz, u[3], u[4], u[5]);
+                uf_block_acc_d(m, m.t4, m.t3, dx, dy, me.tx, me.ty, me.tz, w[3], w[4], w[5]);
+            }
+        });
         for (int c = 0; c < NC; ++c) sacc[warp][c][j] = w[c];
     };
     const FtSteps sp = ft_steps();

@@ -832,8 +832,10 @@ __device__ __forceinline__ void pair_acc_d(double dx, double dy, double dz, doub
                                            double vy, double vz, double &ux, double &uy, double &uz)
 {
     if constexpr (KIND == RMW_UF) {
-        const UFBlockD m = uf_block_d<ZPER>(pair_geo_d<ZPER>(dx, dy, dz, Rz, hi, hj), dz, Rz, hi, hj);
-        uf_block_acc_d(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
+        with_pair_geo_d<ZPER>(dx, dy, dz, Rz, hi, hj, [&](const PairGeoD &g, auto mul) {
+            const UFBlockD m = uf_block_d<ZPER, decltype(mul)>(g, dz, Rz, hi, hj);
+            uf_block_acc_d(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
+        });
     } else {
         pair_contrib<KIND, double>(dx, dy, dz, Rz, hi, hj, vx, vy, vz, ux, uy, uz);
     }
@@ -891,19 +893,21 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
             if constexpr (NOWALL) {
                 pair_rpy_sym<double, KIND>(dx, dy, dz, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
             } else {
-                const PairGeoD g = pair_geo_d<false>(dx, dy, dz, Rz, zi, zj);
-                if constexpr (KIND == RMW_UF || KIND == RMW_WT) {
-                    UFBlockD m;
-                    if constexpr (KIND == RMW_UF) m = uf_block_d<false>(g, dz, Rz, zi, zj);
-                    else m = wt_block_d(g, dz, Rz);
-                    uf_block_acc_d(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
-                    uf_block_acc_d(m, m.t4, m.t3, dx, dy, me.vx, me.vy, me.vz, wx, wy, wz);
-                } else {
-                    const RotBlockD k = rot_block_d(g, dz, Rz, zi, zj);
-                    if constexpr (KIND == RMW_UT)
-                        ut_acc_d(k, dx, dy, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
-                    else wf_acc_d(k, dx, dy, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
-                }
+                with_pair_geo_d<false>(dx, dy, dz, Rz, zi, zj, [&](const PairGeoD &g, auto mul) {
+                    using MUL = decltype(mul);
+                    if constexpr (KIND == RMW_UF || KIND == RMW_WT) {
+                        UFBlockD m;
+                        if constexpr (KIND == RMW_UF) m = uf_block_d<false, MUL>(g, dz, Rz, zi, zj);
+                        else m = wt_block_d<false, MUL>(g, dz, Rz);
+                        uf_block_acc_d(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
+                        uf_block_acc_d(m, m.t4, m.t3, dx, dy, me.vx, me.vy, me.vz, wx, wy, wz);
+                    } else {
+                        const RotBlockD k = rot_block_d<false, MUL>(g, dz, Rz, zi, zj);
+                        if constexpr (KIND == RMW_UT)
+                            ut_acc_d(k, dx, dy, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
+                        else wf_acc_d(k, dx, dy, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
+                    }
+                });
             }
         };
         if constexpr (PER) {
