@@ -81,17 +81,55 @@ __device__ __forceinline__ double int_rsqrt(double x)
     return __hiloint2double((int)((uint32_t)(m >> 32) + ((uint32_t)(1021 - h) << 20)), (int)(uint32_t)m);
 }
 
+// a b + c of non-negative numbers below 2^400 in magnitude (signs ignored; zero allowed), a b and c not both 0: factors
+// or addends 2^62 below the other term count as zero.  0.51 ulp.
+__device__ __forceinline__ double int_fma_pos(double a, double b, double c)
+{
+    uint32_t ah, al, bh, bl, ch, cl;
+    int_significand(a, ah, al);
+    int_significand(b, bh, bl);
+    int_significand(c, ch, cl);
+    const int ec = (__double2hiint(c) & 0x7fffffff) >> 20;
+    const int ep = ((__double2hiint(a) & 0x7fffffff) >> 20) + ((__double2hiint(b) & 0x7fffffff) >> 20) - 1023;
+    const uint64_t p = int_mulhi(ah, al, bh, bl) >> 1, s = u64_of(ch, cl) >> 2;  // units 2^-61 of their exponents
+    const int d = ep - ec;
+    const uint64_t big = d >= 0 ? p : s, small = d >= 0 ? s : p;
+    const uint64_t t = big + (small >> min(abs(d), 63));  // in [2^61, 2^64)
+    const int z = __clz((int)(t >> 32));                  // 0 to 2
+    const uint64_t q = t << z, m = (q >> 11) + ((q >> 10) & 1);
+    const uint32_t hi = (uint32_t)(m >> 32) + ((uint32_t)(max(ep, ec) + 1 - z) << 20);
+    return __hiloint2double((int)hi, (int)(uint32_t)m);
+}
+
 // x in [2^-64, 2^64): what the pair kernels' integer forms ask of the squared distances
 __device__ __forceinline__ bool int_range(double x)
 {
     return (uint32_t)__double2hiint(x) - (959u << 20) < (128u << 20);
 }
 
+// |d| < 2^32, for separations (false for NaN and infinities)
+__device__ __forceinline__ bool int_range_sep(double dx, double dy, double dz)
+{
+    const uint32_t a = (uint32_t)__double2hiint(dx) & 0x7fffffffu, b = (uint32_t)__double2hiint(dy) & 0x7fffffffu;
+    return max(max(a, b), (uint32_t)__double2hiint(dz) & 0x7fffffffu) < (1055u << 20);
+}
+// zero or 2^-300 <= |v| < 2^300, for vectors: their products with separations and blocks stay normal
+__device__ __forceinline__ bool int_range_vec(double v)
+{
+    return ((uint32_t)__double2hiint(v) & 0x7fffffffu) - (723u << 20) < (600u << 20) || v == 0.0;
+}
+__device__ __forceinline__ bool int_range_vec(double x, double y, double z)
+{
+    return int_range_vec(x) && int_range_vec(y) && int_range_vec(z);
+}
+
 // Products of the pair blocks in plain arithmetic (MulPipe) or on the integer
-// pipes (MulInt).  pos: both factors positive; mul: any sign.
+// pipes (MulInt).  pos: both factors positive; mul: any sign; fma_pos: a b + c
+// of non-negative terms.
 template <typename T> struct MulPipe {
     static __device__ __forceinline__ T pos(T a, T b) { return a * b; }
     static __device__ __forceinline__ T mul(T a, T b) { return a * b; }
+    static __device__ __forceinline__ T fma_pos(T a, T b, T c) { return fma(a, b, c); }
     static __device__ __forceinline__ bool le4(T x) { return !(x > T(4)); }
     static __device__ __forceinline__ bool lt4(T x) { return !(x >= T(4)); }
 };
@@ -99,6 +137,7 @@ using MulFp64 = MulPipe<double>;
 struct MulInt {
     static __device__ __forceinline__ double pos(double a, double b) { return int_mul(a, b); }
     static __device__ __forceinline__ double mul(double a, double b) { return int_mul_signed(a, b); }
+    static __device__ __forceinline__ double fma_pos(double a, double b, double c) { return int_fma_pos(a, b, c); }
     static __device__ __forceinline__ bool le4(double x) { return __double_as_longlong(x) <= 0x4010000000000000ll; }
     static __device__ __forceinline__ bool lt4(double x) { return __double_as_longlong(x) < 0x4010000000000000ll; }
 };

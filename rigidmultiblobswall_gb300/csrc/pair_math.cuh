@@ -342,15 +342,22 @@ __device__ __forceinline__ PairGeoD pair_geo_d(double r2, double R2)
     g.p = MUL::pos(g.t, g.u);
     return g;
 }
-// Squared distances and f(geometry, MUL()): the integer forms where every lane's pair allows them (all but dummies,
-// coincident blobs and distances beyond 2^32 radii), else the FP64 ones.  ZPER pairs (dz an image's) take the latter.
+// Squared distances and f(geometry, MUL()): the integer forms where allow is set and every lane's pair permits them (all
+// but dummies, coincident blobs and distances beyond 2^32 radii), else the FP64 ones.  ZPER pairs (dz an image's) take
+// the latter.
 template <bool ZPER, class F>
-__device__ __forceinline__ void with_pair_geo_d(double dx, double dy, double dz, double Rz, double hi, double hj, F &&f)
+__device__ __forceinline__ void with_pair_geo_d(double dx, double dy, double dz, double Rz, double hi, double hj,
+                                                bool allow, F &&f)
 {
+    if (!ZPER && allow) {
+        const double q2 = int_fma_pos(dz, dz, int_fma_pos(dx, dx, int_mul_signed(dy, dy)));
+        if (__all_sync(__activemask(), int_range_sep(dx, dy, Rz) && int_range(q2))) {
+            f(pair_geo_d<MulInt>(q2, int_fma_pos(4.0 * hi, hj, q2)), MulInt());
+            return;
+        }
+    }
     const double rho2 = fma(dx, dx, dy * dy), r2 = fma(dz, dz, rho2);
-    const double R2 = ZPER ? fma(Rz, Rz, rho2) : fma(4.0 * hi, hj, r2);
-    if (!ZPER && __all_sync(__activemask(), int_range(r2) && int_range(R2))) f(pair_geo_d<MulInt>(r2, R2), MulInt());
-    else f(pair_geo_d<MulFp64>(r2, R2), MulFp64());
+    f(pair_geo_d<MulFp64>(r2, ZPER ? fma(Rz, Rz, rho2) : fma(4.0 * hi, hj, r2)), MulFp64());
 }
 struct UFBlockD {
     double Af, b2, t3, t4, zz;
@@ -359,7 +366,7 @@ template <bool ZPER, class MUL = MulFp64>
 __device__ __forceinline__ UFBlockD uf_block_d(const PairGeoD &g, double dz, double Rz, double hi, double hj,
                                                MUL = MUL())
 {
-    const double k1 = fma(3.0 * hi, hj, 1.0), z2 = MUL::pos(Rz, Rz);  // 3 h_i h_j + 1
+    const double k1 = MUL::fma_pos(3.0 * hi, hj, 1.0), z2 = MUL::pos(Rz, Rz);  // 3 h_i h_j + 1
     double ia = g.invr, a3 = MUL::pos(g.i2, g.invr);
     double Bc = MUL::pos(fma(-3.0, g.i2, 1.5), a3);  // positive where it is used (r > 2)
     const bool near = MUL::le4(g.r2);                // r <= 2
@@ -372,9 +379,9 @@ __device__ __forceinline__ UFBlockD uf_block_d(const PairGeoD &g, double dz, dou
     }
     const double s = g.s, u = g.u, t = g.t, p = g.p;
     const double E = MUL::pos(z2, u);
-    const double b1 = fma(3.0, z2, 1.0);
+    const double b1 = MUL::fma_pos(z2, 3.0, 1.0);
     const double w5 = fma(-5.0, E, b1), w7 = fma(-7.0, E, b1);
-    const double Y = fma(-5.0, MUL::mul(u, w7), fma(9.0 * hi, hj, 3.0));
+    const double Y = fma(-5.0, MUL::mul(u, w7), MUL::fma_pos(9.0 * hi, hj, 3.0));
     const double Y10 = fma(-10.0, u, Y);
     const double Z = fma(z2, fma(-20.0, u, Y10) + 6.0, 4.0);
     const double X = MUL::mul(MUL::pos(Rz, p), Y10);
@@ -396,12 +403,14 @@ __device__ __forceinline__ UFBlockD uf_block_d(const PairGeoD &g, double dz, dou
     m.zz = fma(-p, Z, m.Af + dG);
     return m;
 }
-// (ux, uy, uz) += (3/2) M v; with t3 and t4 exchanged, the transposed block
+// (ux, uy, uz) += (3/2) M v; with t3 and t4 exchanged, the transposed block.
+// V: MulInt where all vectors are within int_range_vec.
+template <class V>
 __device__ __forceinline__ void uf_block_acc_d(const UFBlockD &m, double t3, double t4, double dx, double dy,
                                                double vx, double vy, double vz, double &ux, double &uy, double &uz)
 {
-    const double P = fma(dy, vy, dx * vx);
-    const double G = fma(t3, vz, m.b2 * P);
+    const double P = fma(dy, vy, V::mul(dx, vx));
+    const double G = fma(t3, vz, V::mul(m.b2, P));
     ux = fma(G, dx, fma(m.Af, vx, ux));
     uy = fma(G, dy, fma(m.Af, vy, uy));
     uz = fma(t4, P, fma(m.zz, vz, uz));
@@ -461,12 +470,13 @@ __device__ __forceinline__ UFBlockD wt_block_d(const PairGeoD &g, double dz, dou
     m.zz = fma(D, dz, fma(-1.5 * f, Et, fma(0.5 * f, g.t, A)));
     return m;
 }
+template <class V>
 __device__ __forceinline__ void ut_acc_d(const RotBlockD &k, double dx, double dy, double vx, double vy, double vz,
                                          double qx, double qy, double qz, double &ux, double &uy, double &uz,
                                          double &wx, double &wy, double &wz)
 {
-    const double Q = fma(dy, vx, -dx * vy), Qq = fma(dy, qx, -dx * qy);
-    const double bv = k.b * vz, eQ = k.ei * Q, bq = k.b * qz, eq = k.ej * Qq;
+    const double Q = fma(dy, vx, -V::mul(dx, vy)), Qq = fma(dy, qx, -V::mul(dx, qy));
+    const double bv = V::mul(k.b, vz), eQ = V::mul(k.ei, Q), bq = V::mul(k.b, qz), eq = V::mul(k.ej, Qq);
     ux = fma(k.a, vy, fma(bv, dy, fma(eQ, dx, ux)));
     uy = fma(-k.a, vx, fma(-bv, dx, fma(eQ, dy, uy)));
     uz = fma(-k.wi, Q, uz);
@@ -474,12 +484,14 @@ __device__ __forceinline__ void ut_acc_d(const RotBlockD &k, double dx, double d
     wy = fma(-k.ar, qx, fma(bq, dx, fma(eq, dy, wy)));
     wz = fma(k.wj, Qq, wz);
 }
+template <class V>
 __device__ __forceinline__ void wf_acc_d(const RotBlockD &k, double dx, double dy, double vx, double vy, double vz,
                                          double qx, double qy, double qz, double &ux, double &uy, double &uz,
                                          double &wx, double &wy, double &wz)
 {
-    const double Q = fma(dy, vx, -dx * vy), Qq = fma(dy, qx, -dx * qy);
-    const double H = fma(k.ej, fma(dy, vy, dx * vx), k.wj * vz), Hq = fma(k.ei, fma(dy, qy, dx * qx), -k.wi * qz);
+    const double Q = fma(dy, vx, -V::mul(dx, vy)), Qq = fma(dy, qx, -V::mul(dx, qy));
+    const double H = fma(k.ej, fma(dy, vy, V::mul(dx, vx)), V::mul(k.wj, vz));
+    const double Hq = fma(k.ei, fma(dy, qy, V::mul(dx, qx)), -V::mul(k.wi, qz));
     ux = fma(-k.ar, vy, fma(H, dy, ux));
     uy = fma(k.ar, vx, fma(-H, dx, uy));
     uz = fma(-k.b, Q, uz);
@@ -615,12 +627,12 @@ __device__ __forceinline__ void pair_rpy_sym_body(T r2, T invr, T dx, T dy, T dz
         if (__any_sync(__activemask(), near)) {
             if (near) c = T(0.5) * (T(1) - T(0.375) * (r2 * invr));
         }
-        ux = fm<T>(c, fm<T>(vy, dz, -vz * dy), ux);
-        uy = fm<T>(c, fm<T>(vz, dx, -vx * dz), uy);
-        uz = fm<T>(c, fm<T>(dy, vx, -dx * vy), uz);
-        wx = fm<T>(-c, fm<T>(qy, dz, -qz * dy), wx);
-        wy = fm<T>(-c, fm<T>(qz, dx, -qx * dz), wy);
-        wz = fm<T>(-c, fm<T>(dy, qx, -dx * qy), wz);
+        ux = fm<T>(c, fm<T>(vy, dz, -MUL::mul(vz, dy)), ux);
+        uy = fm<T>(c, fm<T>(vz, dx, -MUL::mul(vx, dz)), uy);
+        uz = fm<T>(c, fm<T>(dy, vx, -MUL::mul(dx, vy)), uz);
+        wx = fm<T>(-c, fm<T>(qy, dz, -MUL::mul(qz, dy)), wx);
+        wy = fm<T>(-c, fm<T>(qz, dx, -MUL::mul(qx, dz)), wy);
+        wz = fm<T>(-c, fm<T>(dy, qx, -MUL::mul(dx, qy)), wz);
         return;
     }
     const T invr2 = MUL::pos(invr, invr);
@@ -649,8 +661,8 @@ __device__ __forceinline__ void pair_rpy_sym_body(T r2, T invr, T dx, T dy, T dz
             }
         }
     }
-    const T G = Bc * fm<T>(dx, vx, fm<T>(dy, vy, dz * vz));
-    const T Gq = Bc * fm<T>(dx, qx, fm<T>(dy, qy, dz * qz));
+    const T G = MUL::mul(Bc, fm<T>(dx, vx, fm<T>(dy, vy, MUL::mul(dz, vz))));
+    const T Gq = MUL::mul(Bc, fm<T>(dx, qx, fm<T>(dy, qy, MUL::mul(dz, qz))));
     ux = fm<T>(A, vx, fm<T>(G, dx, ux));
     uy = fm<T>(A, vy, fm<T>(G, dy, uy));
     uz = fm<T>(A, vz, fm<T>(G, dz, uz));
@@ -660,16 +672,19 @@ __device__ __forceinline__ void pair_rpy_sym_body(T r2, T invr, T dx, T dy, T dz
 }
 template <typename T, int KIND>
 __device__ __forceinline__ void pair_rpy_sym(T dx, T dy, T dz, T vx, T vy, T vz, T qx, T qy, T qz, T &ux, T &uy,
-                                             T &uz, T &wx, T &wy, T &wz)
+                                             T &uz, T &wx, T &wy, T &wz, bool allow = false)
 {
-    const T r2 = fm<T>(dx, dx, fm<T>(dy, dy, dz * dz));
     if constexpr (std::is_same<T, double>::value) {
-        if (__all_sync(__activemask(), int_range(r2))) {  // as with_pair_geo_d
-            pair_rpy_sym_body<T, KIND, MulInt>(r2, int_rsqrt(r2), dx, dy, dz, vx, vy, vz, qx, qy, qz, ux, uy, uz, wx,
-                                               wy, wz);
-            return;
+        if (allow) {  // as with_pair_geo_d
+            const double q2 = int_fma_pos(dx, dx, int_fma_pos(dy, dy, int_mul_signed(dz, dz)));
+            if (__all_sync(__activemask(), int_range_sep(dx, dy, dz) && int_range(q2))) {
+                pair_rpy_sym_body<T, KIND, MulInt>(q2, int_rsqrt(q2), dx, dy, dz, vx, vy, vz, qx, qy, qz, ux, uy, uz,
+                                                   wx, wy, wz);
+                return;
+            }
         }
     }
+    const T r2 = fm<T>(dx, dx, fm<T>(dy, dy, dz * dz));
     pair_rpy_sym_body<T, KIND, MulPipe<T>>(r2, rsq<T>(r2), dx, dy, dz, vx, vy, vz, qx, qy, qz, ux, uy, uz, wx, wy, wz);
 }
 

@@ -569,15 +569,17 @@ __global__ void __launch_bounds__(kFtSymTile) ft_sym_fp64_kernel(const FtSrcD *_
     // a target or source past the end is a dummy far above the wall with zero vectors
     const FtSrcD dummy = {1.0e6, 1.0e6, 1.0e6, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     const FtSrcD me = valid_i ? src[i] : dummy;
+    bool in_range = int_range_vec(me.fx, me.fy, me.fz) && int_range_vec(me.tx, me.ty, me.tz);
     {
         const int j = S * kFtSymTile + tid;
         const FtSrcD q = (j < n) ? src[j] : dummy;
         const double c[9] = {q.x, q.y, q.z, q.fx, q.fy, q.fz, q.tx, q.ty, q.tz};
         for (int k = 0; k < 9; ++k) sx[k][tid] = c[k];
+        in_range = in_range && int_range_vec(q.fx, q.fy, q.fz) && int_range_vec(q.tx, q.ty, q.tz);
     }
     for (int c = 0; c < NC; ++c)
         for (int k = lane; k < kFtSymTile; k += 32) sacc[warp][c][k] = 0.0;
-    __syncthreads();
+    const bool allow = __syncthreads_and(in_range);  // the integer forms, for every vector of the tile pair
     double u[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     auto step = [&](int k) {
         const int j = (lane + k) & (kFtSymTile - 1);
@@ -585,20 +587,20 @@ __global__ void __launch_bounds__(kFtSymTile) ft_sym_fp64_kernel(const FtSrcD *_
         const double fx = sx[3][j], fy = sx[4][j], fz = sx[5][j], tx = sx[6][j], ty = sx[7][j], tz = sx[8][j];
         double w[NC];
         for (int c = 0; c < NC; ++c) w[c] = sacc[warp][c][j];
-        with_pair_geo_d<false>(dx, dy, dz, Rz, me.z, zj, [&](const PairGeoD &g, auto mul) {
+        with_pair_geo_d<false>(dx, dy, dz, Rz, me.z, zj, allow, [&](const PairGeoD &g, auto mul) {
             using MUL = decltype(mul);
             {
                 const UFBlockD m = uf_block_d<false, MUL>(g, dz, Rz, me.z, zj);
-                uf_block_acc_d(m, m.t3, m.t4, dx, dy, fx, fy, fz, u[0], u[1], u[2]);
-                uf_block_acc_d(m, m.t4, m.t3, dx, dy, me.fx, me.fy, me.fz, w[0], w[1], w[2]);
+                uf_block_acc_d<MUL>(m, m.t3, m.t4, dx, dy, fx, fy, fz, u[0], u[1], u[2]);
+                uf_block_acc_d<MUL>(m, m.t4, m.t3, dx, dy, me.fx, me.fy, me.fz, w[0], w[1], w[2]);
             }
             const RotBlockD k2 = rot_block_d<true, MUL>(g, dz, Rz, me.z, zj);
-            ut_acc_d(k2, dx, dy, tx, ty, tz, me.tx, me.ty, me.tz, u[0], u[1], u[2], w[0], w[1], w[2]);
+            ut_acc_d<MUL>(k2, dx, dy, tx, ty, tz, me.tx, me.ty, me.tz, u[0], u[1], u[2], w[0], w[1], w[2]);
             if constexpr (WITH_W) {
-                wf_acc_d(k2, dx, dy, fx, fy, fz, me.fx, me.fy, me.fz, u[3], u[4], u[5], w[3], w[4], w[5]);
+                wf_acc_d<MUL>(k2, dx, dy, fx, fy, fz, me.fx, me.fy, me.fz, u[3], u[4], u[5], w[3], w[4], w[5]);
                 const UFBlockD m = wt_block_d<true, MUL>(g, dz, Rz);
-                uf_block_acc_d(m, m.t3, m.t4, dx, dy, tx, ty, tz, u[3], u[4], u[5]);
-                uf_block_acc_d(m, m.t4, m.t3, dx, dy, me.tx, me.ty, me.tz, w[3], w[4], w[5]);
+                uf_block_acc_d<MUL>(m, m.t3, m.t4, dx, dy, tx, ty, tz, u[3], u[4], u[5]);
+                uf_block_acc_d<MUL>(m, m.t4, m.t3, dx, dy, me.tx, me.ty, me.tz, w[3], w[4], w[5]);
             }
         });
         for (int c = 0; c < NC; ++c) sacc[warp][c][j] = w[c];

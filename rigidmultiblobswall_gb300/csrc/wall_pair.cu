@@ -832,9 +832,9 @@ __device__ __forceinline__ void pair_acc_d(double dx, double dy, double dz, doub
                                            double vy, double vz, double &ux, double &uy, double &uz)
 {
     if constexpr (KIND == RMW_UF) {
-        with_pair_geo_d<ZPER>(dx, dy, dz, Rz, hi, hj, [&](const PairGeoD &g, auto mul) {
+        with_pair_geo_d<ZPER>(dx, dy, dz, Rz, hi, hj, true, [&](const PairGeoD &g, auto mul) {
             const UFBlockD m = uf_block_d<ZPER, decltype(mul)>(g, dz, Rz, hi, hj);
-            uf_block_acc_d(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
+            uf_block_acc_d<MulFp64>(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
         });
     } else {
         pair_contrib<KIND, double>(dx, dy, dz, Rz, hi, hj, vx, vy, vz, ux, uy, uz);
@@ -869,6 +869,7 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
     const SrcD me = valid_i ? src[i] : dummy;
     // in radii; PER: x and y as given, scaled after the image shift
     const double xi = PER ? me.x : me.x * inva, yi = PER ? me.y : me.y * inva, zi = me.z * inva;
+    bool in_range = int_range_vec(me.vx, me.vy, me.vz);
     {
         const int j = S * kTile + tid;
         const SrcD sj = (j < n) ? src[j] : dummy;
@@ -878,10 +879,11 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
         tvx[tid] = sj.vx;
         tvy[tid] = sj.vy;
         tvz[tid] = sj.vz;
+        in_range = in_range && int_range_vec(sj.vx, sj.vy, sj.vz);
     }
     for (int c = 0; c < 3; ++c)
         for (int k = lane; k < kTile; k += 32) sacc[warp][c][k] = 0.0;
-    __syncthreads();
+    const bool allow = __syncthreads_and(in_range);  // the integer forms, for every vector of the tile pair
     double ux = 0.0, uy = 0.0, uz = 0.0;
     auto step = [&](int k) {
         const int jl = (lane + k) & (kTile - 1);
@@ -891,21 +893,22 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
         auto pair = [&](double dx, double dy) {
             const double dz = zi - zj, Rz = zi + zj;
             if constexpr (NOWALL) {
-                pair_rpy_sym<double, KIND>(dx, dy, dz, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
+                pair_rpy_sym<double, KIND>(dx, dy, dz, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz,
+                                           allow);
             } else {
-                with_pair_geo_d<false>(dx, dy, dz, Rz, zi, zj, [&](const PairGeoD &g, auto mul) {
+                with_pair_geo_d<false>(dx, dy, dz, Rz, zi, zj, allow, [&](const PairGeoD &g, auto mul) {
                     using MUL = decltype(mul);
                     if constexpr (KIND == RMW_UF || KIND == RMW_WT) {
                         UFBlockD m;
                         if constexpr (KIND == RMW_UF) m = uf_block_d<false, MUL>(g, dz, Rz, zi, zj);
                         else m = wt_block_d<false, MUL>(g, dz, Rz);
-                        uf_block_acc_d(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
-                        uf_block_acc_d(m, m.t4, m.t3, dx, dy, me.vx, me.vy, me.vz, wx, wy, wz);
+                        uf_block_acc_d<MUL>(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
+                        uf_block_acc_d<MUL>(m, m.t4, m.t3, dx, dy, me.vx, me.vy, me.vz, wx, wy, wz);
                     } else {
                         const RotBlockD k = rot_block_d<false, MUL>(g, dz, Rz, zi, zj);
                         if constexpr (KIND == RMW_UT)
-                            ut_acc_d(k, dx, dy, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
-                        else wf_acc_d(k, dx, dy, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
+                            ut_acc_d<MUL>(k, dx, dy, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
+                        else wf_acc_d<MUL>(k, dx, dy, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
                     }
                 });
             }

@@ -24,7 +24,9 @@ static double __hiloint2double(int h, int l)
 static uint32_t __umulhi(uint32_t a, uint32_t b) { return (uint32_t)(((uint64_t)a * b) >> 32); }
 static int __mulhi(int a, int b) { return (int)(((int64_t)a * b) >> 32); }
 static uint32_t __float2uint_rn(float x) { return x >= 4294967296.f ? 0xffffffffu : (uint32_t)std::nearbyint((double)x); }
+using std::max;
 using std::min;
+static int __clz(int x) { return x ? __builtin_clz((unsigned)x) : 32; }
 namespace rmw {
 static float rsqrt_approx(float x) { return (float)((1.0 / std::sqrt((double)x)) * (1.0 + seed_error)); }
 }
@@ -45,7 +47,7 @@ int main()
         default: return p * (1.0 + u(g));
         }
     };
-    double em = 0, es = 0, er = 0;
+    double ef = 0, em = 0, es = 0, er = 0;
     int bad = 0;
     for (int it = 0; it < 3000000; ++it) {
         const double a = number(200), b = number(200);
@@ -55,6 +57,17 @@ int main()
         es = std::max(es, (double)std::fabs(int_mul_signed(sa, sb) - (long double)sa * sb) / ulp(sa * sb));
         sa = (it & 1) ? -0.0 : ((it & 2) ? 0.0 : 3e-310);
         bad += int_mul_signed(sa, sb) != 0.0 || int_mul_signed(sb, sa) != 0.0;
+        {
+            const double fb = number(60), fa = it % 7 == 0 ? 0.0 : (it % 5 == 0 ? fb : number(60));
+            double fc = it % 3 == 0 ? fa * fb * std::ldexp(1.0, (int)(g() % 9) - 4) : number(100);
+            if (it % 11 == 0 && fa != 0.0) fc = 0.0;
+            if (fa != 0.0 || fc != 0.0) {
+                const long double w = (long double)fa * fb + fc;
+                ef = std::max(ef, (double)(std::fabs(w - (long double)int_fma_pos((g() & 1) ? -fa : fa, fb, fc)) /
+                                           ulp((double)w)));
+            }
+            bad += !(std::fabs(int_fma_pos(0.0, 0.0, -0.0)) < 1e-300);
+        }
         seed_error = (u(g) - 0.5) * std::ldexp(1.0, -21);
         const double x = number(64);
         const long double y = 1.0L / std::sqrt((long double)x);
@@ -66,6 +79,9 @@ int main()
     const double lo = std::ldexp(1.0, -64), hi = std::ldexp(1.0, 64), inf = INFINITY;
     bad += !int_range(lo) || int_range(std::nextafter(lo, 0.0)) || int_range(hi) || !int_range(std::nextafter(hi, 0.0));
     bad += int_range(0.0) || int_range(inf) || int_range(NAN) || int_range(-1.0) || int_range(-NAN) || int_range(1e-310);
-    std::printf("%.6f %.6f %.6f %d\n", em, es, er, bad);
+    for (double v : {0.0, -0.0, std::ldexp(1.0, -300), -std::nextafter(std::ldexp(1.0, 300), 0.0)}) bad += !int_range_vec(v);
+    for (double v : {3e-310, std::ldexp(1.0, -301), std::ldexp(1.0, 300), -inf, (double)NAN}) bad += int_range_vec(v);
+    bad += !int_range_sep(-4e9, 0.0, 1e-310) || int_range_sep(0.0, 4.3e9, 0.0) || int_range_sep(0.0, 0.0, NAN);
+    std::printf("%.6f %.6f %.6f %.6f %d\n", ef, em, es, er, bad);
     return 0;
 }

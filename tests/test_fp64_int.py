@@ -21,8 +21,10 @@ def test_integer_forms_on_the_host(tmp_path):
     exe = tmp_path / "host"
     subprocess.run(["g++", "-O2", "-std=c++17", "-fwrapv", f'-DFP64_INT_HEADER="{header}"',
                     os.path.join(ROOT, "tests", "fp64_int_host.cpp"), "-o", str(exe)], check=True)
-    mul, signed, rsqrt, bad = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
-    # half an ulp, and what is left out: 3 units of the 64-bit product, 2^-10 .. 2^-9 ulp each; six of 2^-7 ulp
+    fma, mul, signed, rsqrt, bad = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
+    # half an ulp, and what is left out: 3 units of the 64-bit product, 2^-10 .. 2^-9 ulp each, and one of the smaller
+    # term of a sum, 2^-8; six of 2^-7 ulp
+    assert float(fma) <= 0.5 + 3 * 2.0 ** -9 + 2.0 ** -8
     assert float(mul) <= 0.5 + 3 * 2.0 ** -9 and float(signed) <= 0.5 + 3 * 2.0 ** -9
     assert float(rsqrt) <= 0.5 + 6 * 2.0 ** -7
     assert int(bad) == 0
@@ -73,3 +75,16 @@ def test_non_finite_vectors_and_positions_reach_the_result(cuda_device, n, bad):
     s[8, 0] = bad
     out = np.asarray(mob.wall_product("uf", s, v, 1.0, A, mode="fp64")).reshape(-1, 3)
     assert not np.isfinite(out[8]).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["uf", "wf"])
+@pytest.mark.parametrize("exponent", [-600, -290, 250, 700])
+def test_scale_of_the_vector(cuda_device, kind, exponent):
+    """Vectors within and beyond the integer forms' range: products are linear in a power of two."""
+    from rigidmultiblobswall_gb300 import mobility as mob
+    r, v = _blobs(300, 3)
+    v[7] = 0.0
+    ref = mob.wall_product(kind, r, v, 1.0, A, mode="fp64")
+    got = mob.wall_product(kind, r, v * 2.0 ** exponent, 1.0, A, mode="fp64")
+    assert rel_err(np.asarray(got) * 2.0 ** -exponent, ref) <= 1e-14
