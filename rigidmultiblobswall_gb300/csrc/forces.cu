@@ -13,19 +13,21 @@
 //   bit of the sum (the largest term's own rounding is 2^-53).  An optional
 //   cutoff restricts the sum to pairs within it (the reference's
 //   neighbour-list variant uses 2a + 30 b, multi_bodies/forces_numba.py:228-270).
-//   Two FP32 passes over all pairs (nearest blob, candidates; two sources in
-//   packed lanes, 60 us each at 12,288 blobs) and the FP64 work of about 25
-//   candidates per blob (150 us: lanes of a warp have lists of different
-//   lengths), several source chunks per target tile so that the GPU is full.
+//   r_min is an upper bound from the blobs around i in memory, which only
+//   moves the line outwards.  One FP32 pass over all pairs (candidates; two
+//   sources in packed lanes, 60 us at 12,288 blobs) and the FP64 work of about
+//   25 candidates per blob (lanes of a warp have lists of different lengths),
+//   several source chunks per target tile so that the GPU is full.
 //   1,024 shells of 12 blobs with the wall and body reduction, Debye length
-//   0.1a: 19.2 -> 0.29 ms (before: FP64 for a fifth of all pairs, lanes waiting
-//   for each other's, on 96 CTAs); 0.5a 25.4 -> 1.5 ms; 1a 24.6 -> 3.6 ms;
-//   172,032 blobs, 0.1a 195 -> 29 ms, 1a 2,818 -> 74 ms.
+//   0.1a: 19.2 -> 0.21 ms (before: FP64 for a fifth of all pairs, lanes waiting
+//   for each other's, on 96 CTAs); 0.5a 25.4 -> 0.90 ms; 1a 24.6 -> 2.4 ms;
+//   172,032 blobs, 0.1a 195 -> 19 ms.
 // * external blob forces (multi_bodies_functions.py:153-189): gravity
 //   -g m e_z and the wall repulsion (e/b) exp(-(h - a)/b) (e/b for h <= a).
 // The body reduction [F_b, T_b] = K^T f is rmw_rigid_KT_mult.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "pair_math.cuh"
 #include "rmw_common.cuh"
@@ -34,12 +36,12 @@ namespace rmw {
 
 namespace {
 
-constexpr int kFThreads = 128;
-
 // Pair lists of the FP64 work: kPend candidates per thread in shared memory,
 // evaluated together when some lane's list is full, so the lanes of a warp
-// work on different pairs instead of waiting for each other's.
-constexpr int kPend = 16;
+// work on different pairs instead of waiting for each other's.  32 rather
+// than 16: the blobs of three shells share a warp and meet their neighbours
+// at different times (12,288 blobs, Debye length 0.5a: 1.22 -> 0.90 ms).
+constexpr int kPend = 32;
 
 // FP32 coordinates relative to the CTA's first target (absolute if that is not
 // finite) in units of 2a + b, and the error bound of a distance to them: with
@@ -60,10 +62,11 @@ struct Screen {
     float ext;      // largest |coordinate| of the CTA's targets
 };
 
+template <int NT>
 __device__ __forceinline__ Screen screen_setup(const double *__restrict__ r, int n, const Box &L, unsigned *bits)
 {
     Screen s;
-    const int i0 = blockIdx.x * kFThreads, i = min(i0 + (int)threadIdx.x, n - 1);
+    const int i0 = blockIdx.x * NT, i = min(i0 + (int)threadIdx.x, n - 1);
     if (threadIdx.x == 0) *bits = 0u;
     for (int c = 0; c < 3; ++c) {
         s.x0[c] = r[3 * i0 + c];
@@ -120,25 +123,31 @@ __device__ __forceinline__ f2 screen_r2(const Screen &s, const Box &L, float4 a,
     return f2_fma(ex, ex, f2_fma(ey, ey, f2_mul(ez, ez)));
 }
 
-// nearest[i] = min over this CTA's sources of an upper bound on the distance
-// to blob i (bit pattern of a positive float: atomicMin keeps it independent
-// of the order); blobs that may coincide with i, which exert no force, do not
-// count.
-template <bool PER>
-__global__ void __launch_bounds__(kFThreads) nearest_kernel(const double *__restrict__ r, int n, int chunk, Box L,
+// nearest[i] = min over the kNearWindow sources around blob i's tile of an upper
+// bound on the distance to blob i (bit pattern of a positive float: atomicMin
+// keeps it independent of the order); blobs that may coincide with i, which
+// exert no force, do not count.  Any blob's distance bounds the largest term
+// from below, so a window is as valid as all sources.  A shell's blobs are
+// neighbours in memory, so theirs is the nearest blob; n free blobs in random
+// order have about n / kNearWindow candidates more each, whose FP64 work is
+// below that of the FP32 scan of the sources left out.
+constexpr int kNearWindow = 1024, kNearSplit = 4;
+template <int NT, bool PER>
+__global__ void __launch_bounds__(NT) nearest_kernel(const double *__restrict__ r, int n, Box L,
                                                              unsigned *__restrict__ nearest)
 {
-    __shared__ float4 tile[kFThreads];
+    __shared__ float4 tile[NT];
     __shared__ unsigned bits;
-    const Screen s = screen_setup(r, n, L, &bits);
-    const int i = blockIdx.x * kFThreads + threadIdx.x;
-    const int j0 = blockIdx.y * chunk, j1 = min(n, j0 + chunk);
+    const Screen s = screen_setup<NT>(r, n, L, &bits);
+    const int i = blockIdx.x * NT + threadIdx.x;
+    const int w0 = max(0, min((int)blockIdx.x * NT - kNearWindow / 2, n - kNearWindow));
+    const int j0 = w0 + blockIdx.y * (kNearWindow / kNearSplit), j1 = min(n, j0 + kNearWindow / kNearSplit);
     float best = 3.0e38f, err = 0.f;
-    for (int t0 = j0; t0 < j1; t0 += kFThreads) {
+    for (int t0 = j0; t0 < j1; t0 += NT) {
         __syncthreads();
         screen_tile(r, s, L, t0 + threadIdx.x, j1, tile);
         __syncthreads();
-        const int cnt = min(kFThreads, j1 - t0);
+        const int cnt = min(NT, j1 - t0);
 #pragma unroll 4
         for (int k = 0; k < cnt; k += 2) {
             const float4 a = tile[k], b = tile[k + 1];
@@ -160,19 +169,19 @@ __global__ void __launch_bounds__(kFThreads) nearest_kernel(const double *__rest
 // NULL: within max(2a, r_min) + reach; always within rc = rcut units), FP64
 // evaluates them.
 // Partial sums to part[blockIdx.y][3n], or (part = NULL, one chunk) straight to f.
-template <bool PER>
-__global__ void __launch_bounds__(kFThreads) blob_blob_kernel(const double *__restrict__ r, double *__restrict__ f,
+template <int NT, bool PER>
+__global__ void __launch_bounds__(NT) blob_blob_kernel(const double *__restrict__ r, double *__restrict__ f,
                                                                double *__restrict__ part, int n, int chunk,
                                                                double eps_over_b, double inv_b, double two_a,
                                                                double rc, float rcut,
                                                                const unsigned *__restrict__ nearest, float reach,
                                                                Box L, int accumulate)
 {
-    __shared__ float4 tile[kFThreads];
-    __shared__ int pend[kPend][kFThreads];
+    __shared__ float4 tile[NT];
+    __shared__ int pend[kPend][NT];
     __shared__ unsigned bits;
-    const Screen s = screen_setup(r, n, L, &bits);
-    const int tid = threadIdx.x, i = blockIdx.x * kFThreads + tid;
+    const Screen s = screen_setup<NT>(r, n, L, &bits);
+    const int tid = threadIdx.x, i = blockIdx.x * NT + tid;
     const bool valid = i < n;
     const int ii = valid ? i : n - 1;
     const double xi = r[3 * (size_t)ii], yi = r[3 * (size_t)ii + 1], zi = r[3 * (size_t)ii + 2];
@@ -195,9 +204,10 @@ __global__ void __launch_bounds__(kFThreads) blob_blob_kernel(const double *__re
                 if (L.y > 0) dy = project(dy, L.y);
                 if (L.z > 0) dz = project(dz, L.z);
             }
-            // 1/r by rsqrt64, r = r^2 / r with one Newton correction (nine FP64 instructions instead of
+            // 1/r on the integer pipes, r = r^2 / r with one Newton correction (four FP64 instructions instead of
             // the library's square root and division, about 35)
-            const double r2 = dx * dx + dy * dy + dz * dz, invr = rsqrt64(r2), r0 = r2 * invr;
+            const double r2 = dx * dx + dy * dy + dz * dz, invr = int_range(r2) ? int_rsqrt(r2) : rsqrt64(r2);
+            const double r0 = r2 * invr;
             const double rn = fma(fma(-r0, r0, r2), 0.5 * invr, r0);
             if (!(rn > 0.0) || rn > rc) continue;  // coincident: no direction; beyond rc: exactly zero
             const double g = (rn > two_a) ? exp(-(rn - two_a) * inv_b) : 1.0;
@@ -209,11 +219,11 @@ __global__ void __launch_bounds__(kFThreads) blob_blob_kernel(const double *__re
         np = 0;
     };
     const int j0 = blockIdx.y * chunk, j1 = min(n, j0 + chunk);
-    for (int t0 = j0; t0 < j1; t0 += kFThreads) {
+    for (int t0 = j0; t0 < j1; t0 += NT) {
         __syncthreads();
         screen_tile(r, s, L, t0 + tid, j1, tile);
         __syncthreads();
-        const int cnt = min(kFThreads, j1 - t0);
+        const int cnt = min(NT, j1 - t0);
         for (int k0 = 0; k0 < cnt; k0 += kPend / 2) {
             const int k1 = min(cnt, k0 + kPend / 2);
             for (int k = k0; k < k1; k += 2) {
@@ -269,14 +279,14 @@ __global__ void external_force_kernel(const double *__restrict__ r, double *__re
     }
 }
 
-template <bool PER>
+template <int NT, bool PER>
 int blob_blob_launch(const double *r, double *f, int n, double eps_over_b, double b, double two_a, double rc,
                      const Box &L, int accumulate, cudaStream_t st)
 {
-    const int tiles = (n + kFThreads - 1) / kFThreads;
+    const int tiles = (n + NT - 1) / NT;
     // enough CTAs for eight per SM, no chunk below two tiles of sources
-    const int want = std::min((152 * 8 + tiles - 1) / tiles, std::max(1, n / (2 * kFThreads)));
-    const int chunk = (((n + want - 1) / want + kFThreads - 1) / kFThreads) * kFThreads;
+    const int want = std::min((152 * 8 + tiles - 1) / tiles, std::max(1, n / (2 * NT)));
+    const int chunk = (((n + want - 1) / want + NT - 1) / NT) * NT;
     const int nchunks = (n + chunk - 1) / chunk;
     const size_t head = ((sizeof(unsigned) * (size_t)n + 255) / 256) * 256;
     const size_t bytes = head + (nchunks > 1 ? sizeof(double) * 3 * (size_t)n * nchunks : 0);
@@ -288,7 +298,7 @@ int blob_blob_launch(const double *r, double *f, int n, double eps_over_b, doubl
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
         scratch(SCRATCH_FORCES, bytes, &ws, st) != RMW_OK) {
         cudaGetLastError();
-        blob_blob_kernel<PER><<<tiles, kFThreads, 0, st>>>(r, f, nullptr, n, n, eps_over_b, 1.0 / b, two_a, rc, rcut,
+        blob_blob_kernel<NT, PER><<<tiles, NT, 0, st>>>(r, f, nullptr, n, n, eps_over_b, 1.0 / b, two_a, rc, rcut,
                                                            nullptr, 0.f, L, accumulate);
         RMW_CHECK_LAUNCH("blob-blob forces");
         return RMW_OK;
@@ -297,9 +307,9 @@ int blob_blob_launch(const double *r, double *f, int n, double eps_over_b, doubl
     double *part = nchunks > 1 ? (double *)((char *)ws + head) : nullptr;
     const dim3 grid(tiles, nchunks);
     RMW_CUDA(cudaMemsetAsync(nearest, 0x7f, sizeof(unsigned) * (size_t)n, st));  // 3.4e38
-    nearest_kernel<PER><<<grid, kFThreads, 0, st>>>(r, n, chunk, L, nearest);
+    nearest_kernel<NT, PER><<<dim3(tiles, kNearSplit), NT, 0, st>>>(r, n, L, nearest);
     const float reach = (float)(b / (two_a + b) * (65.0 * 0.69314718055994531 + std::log((double)n)) * 1.000001);
-    blob_blob_kernel<PER><<<grid, kFThreads, 0, st>>>(r, f, part, n, chunk, eps_over_b, 1.0 / b, two_a, rc, rcut,
+    blob_blob_kernel<NT, PER><<<grid, NT, 0, st>>>(r, f, part, n, chunk, eps_over_b, 1.0 / b, two_a, rc, rcut,
                                                       nearest, reach, L, accumulate);
     if (part) force_sum_kernel<<<(3 * n + 255) / 256, 256, 0, st>>>(part, f, 3 * n, nchunks, accumulate);
     RMW_CHECK_LAUNCH("blob-blob forces");
@@ -315,8 +325,21 @@ static int blob_blob(const double *r, double *f, int n, double eps_over_b, doubl
     auto inv = [unit](double L) { return L > 0 ? (float)(1.0 / (L * unit)) : 0.f; };
     const Box L = {Lx, Ly, Lz, (float)(Lx * unit), (float)(Ly * unit), (float)(Lz * unit), inv(Lx), inv(Ly), inv(Lz),
                    (float)(unit * std::max(0.0, std::max(Lx, std::max(Ly, Lz)))), (float)unit};
-    if (Lx > 0 || Ly > 0 || Lz > 0) return blob_blob_launch<true>(r, f, n, eps_over_b, b, two_a, rc, L, accumulate, st);
-    return blob_blob_launch<false>(r, f, n, eps_over_b, b, two_a, rc, L, accumulate, st);
+    const bool per = Lx > 0 || Ly > 0 || Lz > 0;
+    auto launch = [&](auto nt) {
+        constexpr int NT = decltype(nt)::value;
+        return per ? blob_blob_launch<NT, true>(r, f, n, eps_over_b, b, two_a, rc, L, accumulate, st)
+                   : blob_blob_launch<NT, false>(r, f, n, eps_over_b, b, two_a, rc, L, accumulate, st);
+    };
+    // Targets per CTA.  A tile's FP64 work falls to the one CTA whose sources
+    // are its neighbours, so small suspensions take tiles small enough to
+    // reach every SM; large ones the tile that reads sources least often.
+    // 32 / 64 / 128 targets, Debye length 0.4a: 600 blobs 123 / 201 / 344 us,
+    // 4,200 387 / 401 / 542, 9,600 541 / 529 / 552, 12,288 720 / 689 / 652;
+    // 0.1a: 4,200 175 / 205 / 248, 12,288 244 / 219 / 215.
+    if (n <= 6000) return launch(std::integral_constant<int, 32>());
+    if (n <= 11000) return launch(std::integral_constant<int, 64>());
+    return launch(std::integral_constant<int, 128>());
 }
 
 }  // namespace rmw

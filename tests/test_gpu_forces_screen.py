@@ -94,3 +94,25 @@ def test_captured_forces_match_oracle(cuda_device):
     graph.replay()
     torch.cuda.synchronize()
     _check(r, 0.7, 0.05, 0.4, got=out.cpu().numpy())
+
+
+@pytest.mark.parametrize("n", [6000, 6001, 11000, 11003])
+@pytest.mark.parametrize("b,L", [(0.02, 0.0), (0.2, 70.0)])
+def test_tile_widths_and_distant_nearest_blobs(cuda_device, n, b, L):
+    """Every tile width against an FP64 sum over all pairs; blobs in random order, so that the nearest blob is
+    seldom among the sources next to it in memory."""
+    import torch
+    r = torch.tensor(_slab(n, n, 1.2 * np.sqrt(n), 4.0), device=cuda_device)
+    a, eps = 0.4, 0.7
+    got = F.calc_blob_blob_forces_pycuda(r, periodic_length=np.array([L, L, 0.0]), repulsion_strength=eps,
+                                         debye_length=b, blob_radius=a).reshape(-1, 3)
+    ref, mag = torch.zeros_like(r), torch.zeros(n, dtype=torch.float64, device=cuda_device)
+    for i in torch.arange(n, device=cuda_device).split(1000):
+        d = r[None] - r[i, None]
+        if L > 0:
+            d[..., :2] -= L * torch.trunc(d[..., :2] / L + 0.5 * torch.sign(d[..., :2]))
+        rn = d.norm(dim=2)
+        g = torch.where(rn > 0, torch.exp(-(rn - 2 * a).clamp(min=0) / b), torch.zeros_like(rn)) * eps / b
+        mag[i] = g.sum(1)
+        ref[i] = -(g / rn.clamp(min=1e-300))[..., None].mul(d).sum(1)
+    assert (((got - ref).norm(dim=1)) <= TOL * mag + 1e-300).all()
