@@ -13,11 +13,12 @@
 //   bit of the sum (the largest term's own rounding is 2^-53).  An optional
 //   cutoff restricts the sum to pairs within it (the reference's
 //   neighbour-list variant uses 2a + 30 b, multi_bodies/forces_numba.py:228-270).
-//   r_min is an upper bound from the blobs around i in memory, which only
-//   moves the line outwards.  One FP32 pass over all pairs (candidates; two
-//   sources in packed lanes, 60 us at 12,288 blobs) and the FP64 work of about
-//   25 candidates per blob (lanes of a warp have lists of different lengths),
-//   several source chunks per target tile so that the GPU is full.
+//   Any blob's distance may stand for r_min, which only moves the line
+//   outwards: the nearest of the 1,024 blobs around i in memory does.  One
+//   FP32 pass over all pairs (candidates; two sources in packed lanes, 60 us
+//   at 12,288 blobs) and the FP64 work of about 25 candidates per blob (lanes
+//   of a warp have lists of different lengths), several source chunks per
+//   target tile so that the GPU is full.
 //   1,024 shells of 12 blobs with the wall and body reduction, Debye length
 //   0.1a: 19.2 -> 0.21 ms (before: FP64 for a fifth of all pairs, lanes waiting
 //   for each other's, on 96 CTAs); 0.5a 25.4 -> 0.90 ms; 1a 24.6 -> 2.4 ms;

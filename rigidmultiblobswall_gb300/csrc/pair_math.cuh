@@ -319,10 +319,12 @@ __device__ __forceinline__ UFBlock2 uf_block_f2(const UFCoeffs2 &c, f2 dx, f2 dy
 }
 
 // The explicit M_UF block in FP64, times 3/2: the formulas of uf_block_df
-// (pair_math_df.cuh), where they are derived.  73 FP64 instructions a pair,
-// both ways, against 93 of uf_coeffs / uf_apply: the FP64 pipe bounds the
-// kernels that use it (1/64 of the FP32 rate).  ZPER: dz is an image's and
-// not h_i - h_j.
+// (pair_math_df.cuh), where they are derived.  73 operations a pair, both
+// ways, against 93 of uf_coeffs / uf_apply: the FP64 pipe (1/64 of the FP32
+// rate) bounds the kernels that use it, so MulInt takes 35 of them to the
+// integer pipes (fp64_int.cuh): the products and positive sums of the
+// geometry and the products with the vectors.  10,752 blobs 8.1 -> 4.36 ms.
+// ZPER: dz is an image's and not h_i - h_j.
 struct PairGeoD {
     double r2, invr, i2, u, s, t, p;
 };
@@ -418,9 +420,9 @@ __device__ __forceinline__ void uf_block_acc_d(const UFBlockD &m, double t3, dou
 
 // UT, WF and WT for both orders of a pair in FP64, the formulas of
 // rot_block_df and wt_block_df (pair_math_df.cuh), where they are derived: 64
-// (UT, WF) and 62 (WT) FP64 instructions a pair against 91 and 74 of the
-// tensor forms.  10,752 blobs: UT 9.82 -> 7.01 ms, WF 9.97 -> 7.01, WT 8.08 ->
-// 7.06.  UF32: the blocks times 3/2, as the UF block (for sums of both).
+// (UT, WF) and 62 (WT) operations a pair against 91 and 74 of the tensor
+// forms, about half of them on the integer pipes (MulInt).  10,752 blobs: UT
+// 9.82 -> 3.96 ms, WF 9.97 -> 4.09, WT 8.08 -> 3.78.  UF32: the blocks times 3/2, as the UF block (for sums of both).
 struct RotBlockD {
     double a, ar, b, ei, ej, wi, wj;
 };

@@ -537,12 +537,13 @@ void ft_finalize(const double *r, const double *F, const double *T, const double
 // (gridDim.y CTAs share a tile pair's steps) of the symmetric single products,
 // the four blocks of an unordered pair from one set of distances, reciprocal
 // roots and powers (about 150 of 600 + 500 + 500 + 500 FP32-pipe operations
-// in df64, 25 of 73 + 64 + 64 + 62 FP64 instructions), applied both ways;
+// in df64, 25 of 73 + 64 + 64 + 62 operations in FP64), applied both ways;
 // every block times 3/2, undone by the finalize.  The sum of four symmetric
 // single products, which this replaces, read the blobs and formed the geometry
 // four times and needed a vector of scratch and two additions.  8,064 blobs,
 // [U; W]: df64 2.20 -> 1.51 ms (3.51 before the blocks were written out), four
-// CTAs of 255 registers per SM (six of 168 spill: 1.58 ms); FP64 10.6 ms.
+// CTAs of 255 registers per SM (six of 168 spill: 1.58 ms); FP64
+// 23.0 -> 7.35 ms (10.6 with every operation on the FP64 pipe).
 struct FtSteps {
     int k0, k1, nsplit, split;
     __device__ __forceinline__ size_t slot(int tile) const { return (size_t)tile * nsplit + split; }

@@ -843,9 +843,12 @@ __device__ __forceinline__ void pair_acc_d(double dx, double dy, double dz, doub
 // Symmetric FP64 kernel of any kind: the same grid, pairing and partial-sum
 // slots, FP64 pair arithmetic (the FP64 pipe bounds it, so halving the
 // coefficient work per ordered pair is the gain); source-side sums per warp
-// in FP64 shared memory.  UF through the explicit block of uf_block_d: the
-// 10,752-blob product 11.6 -> 8.1 ms, 73 FP64 instructions per pair at 98 %
-// of the pipe's measured rate (0.53 T instructions/s).
+// in FP64 shared memory.  UF through the explicit block of uf_block_d with
+// what can leave the FP64 pipe on the integer pipes: the 10,752-blob product
+// 11.6 -> 4.36 ms, 38 FP64 instructions per pair at 97 % of the pipe's measured
+// rate (0.53 T instructions/s).  Additions on the integer pipes too (dx, dy,
+// dz, Rz: 34 left) measured 4.31 ms, and free-space and periodic products 2 to
+// 5 % slower: the integer pipes are then the bound.
 // PER (periodic in x and / or y): a pair is its minimum image and the
 // neighbour boxes' images, each both ways (the reverse separations are the
 // negatives of the same set); a blob's own images are added once, to the
