@@ -7,7 +7,6 @@
 #include <cstring>
 #include <random>
 
-#define RMW_COMMON_STUB
 static double seed_error;  // relative error given to the FP32 estimate of 1/sqrt
 static uint64_t bits(double x) { uint64_t u; std::memcpy(&u, &x, 8); return u; }
 static uint32_t __funnelshift_l(uint32_t lo, uint32_t hi, uint32_t s) { return s &= 31, s ? (hi << s) | (lo >> (32 - s)) : hi; }
