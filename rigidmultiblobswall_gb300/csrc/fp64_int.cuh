@@ -8,7 +8,7 @@
 // halves (22 to 28 integer instructions) and 1/sqrt as one third-order Newton
 // step in fixed point (about 45).  M_UF at 10,752 blobs 8.1 -> 5.5 ms with
 // products and roots, 4.36 ms with multiply-adds of positive terms and the
-// products with the vectors; 2,048 blobs 353 -> 212 us.
+// products with the vectors, 3.69 ms with seven of mixed signs.
 //
 // Error bounds, tested against exact arithmetic: int_mul 0.504 ulp (the
 // product of the low halves, below 2^-62 of the result, and the order of ties
@@ -103,6 +103,32 @@ __device__ __forceinline__ double int_fma_pos(double a, double b, double c)
     return __hiloint2double((int)hi, (int)(uint32_t)m);
 }
 
+// a b + c of finite numbers below 2^400 in magnitude; terms below 2^-400 count
+// as zero.  0.51 ulp where the terms do not cancel, 2^-59 of it
+// where they do.
+__device__ __forceinline__ double int_fma(double a, double b, double c)
+{
+    const uint32_t ha = (uint32_t)__double2hiint(a), hb = (uint32_t)__double2hiint(b), hc = (uint32_t)__double2hiint(c);
+    uint32_t ah, al, bh, bl, ch, cl;
+    int_significand(a, ah, al);
+    int_significand(b, bh, bl);
+    int_significand(c, ch, cl);
+    const int ec = (int)(hc >> 20 & 0x7ffu), ep = (int)(ha >> 20 & 0x7ffu) + (int)(hb >> 20 & 0x7ffu) - 1023;
+    const int d = ep - ec;
+    const bool sw = d < 0;
+    const uint64_t p = int_mulhi(ah, al, bh, bl) >> 2, s = u64_of(ch, cl) >> 3;  // units 2^-60 of their exponents
+    const int64_t big = (int64_t)(sw ? s : p), small = (int64_t)((sw ? p : s) >> min(abs(d), 63));
+    const uint32_t sp = ha ^ hb;
+    const int64_t t = (int32_t)(sp ^ hc) < 0 ? big - small : big + small;
+    const uint64_t m0 = (uint64_t)(t < 0 ? -t : t);
+    const int z = __clzll((long long)m0);
+    const uint64_t q = m0 << (z & 63), m = (q >> 11) + ((q >> 10) & 1);
+    const uint32_t sign = ((sw ? hc : sp) ^ (uint32_t)(t >> 32)) & 0x80000000u;
+    const int e = max(ep, ec) + 2 - z;
+    const uint32_t hi = (uint32_t)(m >> 32) + ((uint32_t)e << 20) + sign;
+    return t == 0 || e < 560 ? 0.0 : __hiloint2double((int)hi, (int)(uint32_t)m);
+}
+
 // x in [2^-64, 2^64): what the pair kernels' integer forms ask of the squared distances
 __device__ __forceinline__ bool int_range(double x)
 {
@@ -127,11 +153,12 @@ __device__ __forceinline__ bool int_range_vec(double x, double y, double z)
 
 // Products of the pair blocks in plain arithmetic (MulPipe) or on the integer
 // pipes (MulInt).  pos: both factors positive; mul: any sign; fma_pos: a b + c
-// of non-negative terms.
+// of non-negative terms; fma_any: of any sign.
 template <typename T> struct MulPipe {
     static __device__ __forceinline__ T pos(T a, T b) { return a * b; }
     static __device__ __forceinline__ T mul(T a, T b) { return a * b; }
     static __device__ __forceinline__ T fma_pos(T a, T b, T c) { return fma(a, b, c); }
+    static __device__ __forceinline__ T fma_any(T a, T b, T c) { return fma(a, b, c); }
     static __device__ __forceinline__ bool le4(T x) { return !(x > T(4)); }
     static __device__ __forceinline__ bool lt4(T x) { return !(x >= T(4)); }
 };
@@ -140,6 +167,7 @@ struct MulInt {
     static __device__ __forceinline__ double pos(double a, double b) { return int_mul(a, b); }
     static __device__ __forceinline__ double mul(double a, double b) { return int_mul_signed(a, b); }
     static __device__ __forceinline__ double fma_pos(double a, double b, double c) { return int_fma_pos(a, b, c); }
+    static __device__ __forceinline__ double fma_any(double a, double b, double c) { return int_fma(a, b, c); }
     static __device__ __forceinline__ bool le4(double x) { return __double_as_longlong(x) <= 0x4010000000000000ll; }
     static __device__ __forceinline__ bool lt4(double x) { return __double_as_longlong(x) < 0x4010000000000000ll; }
 };

@@ -321,9 +321,10 @@ __device__ __forceinline__ UFBlock2 uf_block_f2(const UFCoeffs2 &c, f2 dx, f2 dy
 // The explicit M_UF block in FP64, times 3/2: the formulas of uf_block_df
 // (pair_math_df.cuh), where they are derived.  73 operations a pair, both
 // ways, against 93 of uf_coeffs / uf_apply: the FP64 pipe (1/64 of the FP32
-// rate) bounds the kernels that use it, so MulInt takes 35 of them to the
+// rate) bounds the kernels that use it, so MulInt takes 42 of them to the
 // integer pipes (fp64_int.cuh): the products and positive sums of the
-// geometry and the products with the vectors.  10,752 blobs 8.1 -> 4.36 ms.
+// geometry, seven multiply-adds of mixed signs and the products with the
+// vectors.  10,752 blobs 8.1 -> 3.69 ms.
 // ZPER: dz is an image's and not h_i - h_j.
 struct PairGeoD {
     double r2, invr, i2, u, s, t, p;
@@ -370,7 +371,7 @@ __device__ __forceinline__ UFBlockD uf_block_d(const PairGeoD &g, double dz, dou
 {
     const double k1 = MUL::fma_pos(3.0 * hi, hj, 1.0), z2 = MUL::pos(Rz, Rz);  // 3 h_i h_j + 1
     double ia = g.invr, a3 = MUL::pos(g.i2, g.invr);
-    double Bc = MUL::pos(fma(-3.0, g.i2, 1.5), a3);  // positive where it is used (r > 2)
+    double Bc = MUL::pos(MUL::fma_any(g.i2, -3.0, 1.5), a3);  // positive where it is used (r > 2)
     const bool near = MUL::le4(g.r2);                // r <= 2
     if (__any_sync(__activemask(), near)) {
         if (near) {
@@ -382,15 +383,15 @@ __device__ __forceinline__ UFBlockD uf_block_d(const PairGeoD &g, double dz, dou
     const double s = g.s, u = g.u, t = g.t, p = g.p;
     const double E = MUL::pos(z2, u);
     const double b1 = MUL::fma_pos(z2, 3.0, 1.0);
-    const double w5 = fma(-5.0, E, b1), w7 = fma(-7.0, E, b1);
-    const double Y = fma(-5.0, MUL::mul(u, w7), MUL::fma_pos(9.0 * hi, hj, 3.0));
-    const double Y10 = fma(-10.0, u, Y);
+    const double w5 = MUL::fma_any(E, -5.0, b1), w7 = MUL::fma_any(E, -7.0, b1);
+    const double Y = MUL::fma_any(MUL::mul(u, w7), -5.0, MUL::fma_pos(9.0 * hi, hj, 3.0));
+    const double Y10 = MUL::fma_any(u, -10.0, Y);
     const double Z = fma(z2, fma(-20.0, u, Y10) + 6.0, 4.0);
     const double X = MUL::mul(MUL::pos(Rz, p), Y10);
     UFBlockD m;
     m.Af = fma(p, w5, fma(-k1, t, fma(1.5, ia - s, a3)));
-    const double F = fma(-1.5, t, Bc);
-    m.b2 = fma(p, Y, F);
+    const double F = MUL::fma_any(t, -1.5, Bc);
+    m.b2 = MUL::fma_any(p, Y, F);
     double G, dG;  // dz F, dz^2 F
     if constexpr (ZPER) {
         const double dw = hi - hj, x = dz * Bc, w = -1.5 * t * dw;

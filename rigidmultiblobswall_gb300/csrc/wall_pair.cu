@@ -845,10 +845,10 @@ __device__ __forceinline__ void pair_acc_d(double dx, double dy, double dz, doub
 // coefficient work per ordered pair is the gain); source-side sums per warp
 // in FP64 shared memory.  UF through the explicit block of uf_block_d with
 // what can leave the FP64 pipe on the integer pipes: the 10,752-blob product
-// 11.6 -> 4.36 ms, 38 FP64 instructions per pair at 97 % of the pipe's measured
-// rate (0.53 T instructions/s; 33 % of the issue slots).  Additions on the
-// integer pipes too (dx, dy, dz, Rz: 34 left) measured 4.31 ms, and free-space
-// and periodic products 2 to 5 % slower; five or six CTAs per SM change nothing.
+// 11.6 -> 3.69 ms, 31 FP64 instructions per pair.  Measured beside it: three
+// more multiply-adds on the integer pipes 3.87 ms; from 38 instructions and
+// 4.36 ms, additions there (dx, dy, dz, Rz) 4.31 ms, and free-space and periodic
+// products 2 to 5 % slower; five or six CTAs per SM no change.
 // PER (periodic in x and / or y): a pair is its minimum image and the
 // neighbour boxes' images, each both ways (the reverse separations are the
 // negatives of the same set); a blob's own images are added once, to the

@@ -25,6 +25,7 @@ static int __mulhi(int a, int b) { return (int)(((int64_t)a * b) >> 32); }
 static uint32_t __float2uint_rn(float x) { return x >= 4294967296.f ? 0xffffffffu : (uint32_t)std::nearbyint((double)x); }
 using std::max;
 using std::min;
+static int __clzll(long long x) { return x ? __builtin_clzll((unsigned long long)x) : 64; }
 static int __clz(int x) { return x ? __builtin_clz((unsigned)x) : 32; }
 namespace rmw {
 static float rsqrt_approx(float x) { return (float)((1.0 / std::sqrt((double)x)) * (1.0 + seed_error)); }
@@ -46,7 +47,7 @@ int main()
         default: return p * (1.0 + u(g));
         }
     };
-    double ef = 0, em = 0, es = 0, er = 0;
+    double ea = 0, ef = 0, em = 0, es = 0, er = 0;
     int bad = 0;
     for (int it = 0; it < 3000000; ++it) {
         const double a = number(200), b = number(200);
@@ -67,6 +68,21 @@ int main()
             }
             bad += !(std::fabs(int_fma_pos(0.0, 0.0, -0.0)) < 1e-300);
         }
+        {
+            double fa = number(60), fb = number(60), fc = number(100);
+            if (it % 3 == 0) fc = fa * fb * std::ldexp(1.0 + 1e-3 * u(g), (int)(g() % 9) - 4);
+            if (it % 7 == 0) fa = 0.0;
+            else if (it % 11 == 0) fc = 0.0;
+            if (g() & 1) fa = -fa;
+            if (g() & 1) fb = -fb;
+            if (g() & 1) fc = -fc;
+            const long double p = (long double)fa * fb, w = p + fc;
+            const long double larger = std::max(std::fabs(p), (long double)std::fabs(fc));
+            // half an ulp of the result, 2^-59 of the larger term
+            const long double tol = 0.5L * ulp((double)(w == 0 ? larger : w)) + std::ldexp(larger, -59);
+            ea = std::max(ea, (double)(std::fabs(w - (long double)int_fma(fa, fb, fc)) / tol));
+            bad += int_fma(0.0, fb, 0.0) != 0.0 || int_fma(fa, -1.5, 1.5 * fa) > 1e-15 * std::fabs(fa);
+        }
         seed_error = (u(g) - 0.5) * std::ldexp(1.0, -21);
         const double x = number(64);
         const long double y = 1.0L / std::sqrt((long double)x);
@@ -81,6 +97,6 @@ int main()
     for (double v : {0.0, -0.0, std::ldexp(1.0, -300), -std::nextafter(std::ldexp(1.0, 300), 0.0)}) bad += !int_range_vec(v);
     for (double v : {3e-310, std::ldexp(1.0, -301), std::ldexp(1.0, 300), -inf, (double)NAN}) bad += int_range_vec(v);
     bad += !int_range_sep(-4e9, 0.0, 1e-310) || int_range_sep(0.0, 4.3e9, 0.0) || int_range_sep(0.0, 0.0, NAN);
-    std::printf("%.6f %.6f %.6f %.6f %d\n", ef, em, es, er, bad);
+    std::printf("%.6f %.6f %.6f %.6f %.6f %d\n", ea, ef, em, es, er, bad);
     return 0;
 }

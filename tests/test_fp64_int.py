@@ -21,12 +21,13 @@ def test_integer_forms_on_the_host(tmp_path):
     exe = tmp_path / "host"
     subprocess.run(["g++", "-O2", "-std=c++17", "-fwrapv", f'-DFP64_INT_HEADER="{header}"',
                     os.path.join(ROOT, "tests", "fp64_int_host.cpp"), "-o", str(exe)], check=True)
-    fma, mul, signed, rsqrt, bad = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
+    any_sign, fma, mul, signed, rsqrt, bad = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
     # half an ulp, and what is left out: 3 units of the 64-bit product, 2^-10 .. 2^-9 ulp each, and one of the smaller
     # term of a sum, 2^-8; six of 2^-7 ulp
     assert float(fma) <= 0.5 + 3 * 2.0 ** -9 + 2.0 ** -8
     assert float(mul) <= 0.5 + 3 * 2.0 ** -9 and float(signed) <= 0.5 + 3 * 2.0 ** -9
     assert float(rsqrt) <= 0.5 + 6 * 2.0 ** -7
+    assert float(any_sign) <= 1.0
     assert int(bad) == 0
 
 
