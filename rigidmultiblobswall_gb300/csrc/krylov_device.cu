@@ -497,10 +497,13 @@ __global__ void kd_axpby_kernel(const double *__restrict__ x, double *__restrict
 
 // Symmetric tridiagonal eigen-decomposition by implicit QL (the classical
 // algorithm of Bowdler, Martin, Reinsch and Wilkinson, as the host routine of
-// the library), run by one warp: every lane carries the scalar recurrence
-// (identical values and identical writes of d and e), lane l tests entry
-// l, l+32, ... for the split and applies the rotations to rows l, l+32, ... of
-// z (k x k, column-major).  On exit d holds the eigenvalues.  The chain of
+// the library), run by one warp: every lane carries the scalar recurrence, lane
+// 0 stores d and e, lane l tests entry l, l+32, ... for the split and applies
+// the rotations to rows l, l+32, ... of z (k x k, column-major).  The lanes
+// are not in step between two synchronisations (their row counts differ), so
+// an entry is stored only after the __syncwarp that follows every lane's read
+// of it: rotation i reads d[i] and e[i], then synchronises, then stores
+// d[i + 1] and e[i + 1].  On exit d holds the eigenvalues.  The chain of
 // dependent FP64 instructions is the cost (about 64 cycles each): a rotation
 // takes some 25 with plane_rotation instead of 60 with hypot and two
 // divisions.
@@ -508,7 +511,7 @@ __device__ bool tridiag_eigen_warp(double *d, double *e, double *z, int k, int l
 {
     for (int q = lane; q < k; q += 32)
         for (int c = 0; c < k; ++c) z[q + (long long)k * c] = (q == c) ? 1.0 : 0.0;
-    e[k - 1] = 0.0;
+    if (lane == 0) e[k - 1] = 0.0;
     for (int l = 0; l < k; ++l) {
         int iter = 0, m;
         do {
@@ -528,27 +531,33 @@ __device__ bool tridiag_eigen_warp(double *d, double *e, double *z, int k, int l
                 if (++iter > 60) return false;
                 // shift: d[l] less 2 e^2 / (p + sign(p) sqrt(p^2 + 4 e^2)), p = d[l+1] - d[l]
                 const double el = e[l], dl = d[l], pd = d[l + 1] - dl, e2 = 2.0 * el;
+                double dn = d[m];  // d[i + 1] of the next rotation
                 const double h = root_or_hypot(pd, e2);
-                double g = d[m] - dl + el * (e2 / (pd + copysign(h, pd)));
+                double g = dn - dl + el * (e2 / (pd + copysign(h, pd)));
                 double s = 1.0, c = 1.0, p = 0.0;
                 bool cut = false;
                 for (int i = m - 1; i >= l; --i) {
-                    const double f = s * e[i], b = c * e[i];
+                    const double ei = e[i], di = d[i];
+                    __syncwarp();
+                    const double f = s * ei, b = c * ei;
                     const Rot rot = plane_rotation(g, f);
-                    e[i + 1] = rot.r;
+                    if (lane == 0) e[i + 1] = rot.r;
                     if (rot.zero) {
-                        d[i + 1] -= p;
-                        e[m] = 0.0;
+                        if (lane == 0) {
+                            d[i + 1] = dn - p;
+                            e[m] = 0.0;
+                        }
                         cut = true;
                         break;
                     }
                     s = rot.s;
                     c = rot.c;
-                    g = d[i + 1] - p;
-                    const double r = (d[i] - g) * s + 2.0 * c * b;
+                    g = dn - p;
+                    const double r = (di - g) * s + 2.0 * c * b;
                     p = s * r;
-                    d[i + 1] = g + p;
+                    if (lane == 0) d[i + 1] = g + p;
                     g = c * r - b;
+                    dn = di;
                     for (int q = lane; q < k; q += 32) {
                         double *z1 = z + q + (long long)k * (i + 1), *z0 = z + q + (long long)k * i;
                         const double t = *z1;
@@ -557,9 +566,11 @@ __device__ bool tridiag_eigen_warp(double *d, double *e, double *z, int k, int l
                     }
                 }
                 if (cut) continue;
-                d[l] -= p;
-                e[l] = g;
-                e[m] = 0.0;
+                if (lane == 0) {
+                    d[l] = dn - p;
+                    e[l] = g;
+                    e[m] = 0.0;
+                }
             }
         } while (m != l);
     }
