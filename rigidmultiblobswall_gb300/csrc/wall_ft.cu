@@ -588,7 +588,8 @@ __global__ void __launch_bounds__(kFtSymTile) ft_sym_fp64_kernel(const FtSrcD *_
         const double fx = sx[3][j], fy = sx[4][j], fz = sx[5][j], tx = sx[6][j], ty = sx[7][j], tz = sx[8][j];
         double w[NC];
         for (int c = 0; c < NC; ++c) w[c] = sacc[warp][c][j];
-        with_pair_geo_d<false>(dx, dy, dz, Rz, me.z, zj, allow, [&](const PairGeoD &g, auto mul) {
+        with_pair_geo_d<false, false>(dx, dy, dz, 1.0, Rz, me.z, zj, allow,
+                                      [&](const PairGeoD &g, double, double, double, auto mul) {
             using MUL = decltype(mul);
             {
                 const UFBlockD m = uf_block_d<false, MUL>(g, dz, Rz, me.z, zj);

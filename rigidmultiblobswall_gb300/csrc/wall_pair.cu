@@ -832,7 +832,8 @@ __device__ __forceinline__ void pair_acc_d(double dx, double dy, double dz, doub
                                            double vy, double vz, double &ux, double &uy, double &uz)
 {
     if constexpr (KIND == RMW_UF) {
-        with_pair_geo_d<ZPER>(dx, dy, dz, Rz, hi, hj, true, [&](const PairGeoD &g, auto mul) {
+        with_pair_geo_d<ZPER, false>(dx, dy, dz, 1.0, Rz, hi, hj, true,
+                                     [&](const PairGeoD &g, double, double, double, auto mul) {
             const UFBlockD m = uf_block_d<ZPER, decltype(mul)>(g, dz, Rz, hi, hj);
             uf_block_acc_d<MulFp64>(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
         });
@@ -845,8 +846,9 @@ __device__ __forceinline__ void pair_acc_d(double dx, double dy, double dz, doub
 // coefficient work per ordered pair is the gain); source-side sums per warp
 // in FP64 shared memory.  UF through the explicit block of uf_block_d with
 // what can leave the FP64 pipe on the integer pipes: the 10,752-blob product
-// 11.6 -> 3.69 ms, 31 FP64 instructions per pair.  Measured beside it: three
-// more multiply-adds on the integer pipes 3.87 ms; from 38 instructions and
+// 11.6 -> 3.77 ms, 31 FP64 instructions per pair.  Measured beside it (at
+// 3.69 ms, positions scaled when packed): three more multiply-adds on the
+// integer pipes 3.87 ms; from 38 instructions and
 // 4.36 ms, additions there (dx, dy, dz, Rz) 4.31 ms, and free-space and periodic
 // products 2 to 5 % slower; five or six CTAs per SM no change.
 // PER (periodic in x and / or y): a pair is its minimum image and the
@@ -859,7 +861,7 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
                                               double *__restrict__ partial, const SymJob *__restrict__ jobs,
                                               const Periodic P = Periodic{0.0, 0.0, 0.0})
 {
-    __shared__ double tx[kTile], ty[kTile], tz[kTile], tvx[kTile], tvy[kTile], tvz[kTile];
+    __shared__ double tx[kTile], ty[kTile], tz[kTile], th[kTile], tvx[kTile], tvy[kTile], tvz[kTile];
     __shared__ double sacc[kSymWarps][3][kTile];
     int T, S;
     sym_cta<SEG>(jobs, n, nt, T, S, src, partial);
@@ -870,15 +872,15 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
     // a target or source past the end is a dummy far above the wall with a zero vector
     const SrcD dummy = {1.0e6, 1.0e6, 1.0e6, 0.0, 0.0, 0.0, 0.0, 0.0};
     const SrcD me = valid_i ? src[i] : dummy;
-    // in radii; PER: x and y as given, scaled after the image shift
-    const double xi = PER ? me.x : me.x * inva, yi = PER ? me.y : me.y * inva, zi = me.z * inva;
+    const double hi = me.z * inva;  // the height in radii (free space: inva = 1, positions over a)
     bool in_range = int_range_vec(me.vx, me.vy, me.vz);
     {
         const int j = S * kTile + tid;
         const SrcD sj = (j < n) ? src[j] : dummy;
-        tx[tid] = PER ? sj.x : sj.x * inva;
-        ty[tid] = PER ? sj.y : sj.y * inva;
-        tz[tid] = sj.z * inva;
+        tx[tid] = sj.x;
+        ty[tid] = sj.y;
+        tz[tid] = sj.z;
+        if constexpr (!NOWALL) th[tid] = sj.z * inva;
         tvx[tid] = sj.vx;
         tvy[tid] = sj.vy;
         tvz[tid] = sj.vz;
@@ -886,29 +888,31 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
     }
     for (int c = 0; c < 3; ++c)
         for (int k = lane; k < kTile; k += 32) sacc[warp][c][k] = 0.0;
-    const bool allow = __syncthreads_and(in_range);  // the integer forms, for every vector of the tile pair
+    // the integer forms, for every vector of the tile pair
+    const bool allow = __syncthreads_and(in_range && int_range(inva));
     double ux = 0.0, uy = 0.0, uz = 0.0;
     auto step = [&](int k) {
         const int jl = (lane + k) & (kTile - 1);
-        const double zj = tz[jl];
         const double vx = tvx[jl], vy = tvy[jl], vz = tvz[jl];
         double wx = sacc[warp][0][jl], wy = sacc[warp][1][jl], wz = sacc[warp][2][jl];
-        auto pair = [&](double dx, double dy) {
-            const double dz = zi - zj, Rz = zi + zj;
+        auto pair = [&](double ex, double ey) {
+            const double ez = me.z - tz[jl];
             if constexpr (NOWALL) {
-                pair_rpy_sym<double, KIND>(dx, dy, dz, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz,
+                pair_rpy_sym<double, KIND>(ex, ey, ez, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz,
                                            allow);
             } else {
-                with_pair_geo_d<false>(dx, dy, dz, Rz, zi, zj, allow, [&](const PairGeoD &g, auto mul) {
+                const double hj = th[jl], Rz = hi + hj;
+                with_pair_geo_d<false, true>(ex, ey, ez, inva, Rz, hi, hj, allow,
+                                             [&](const PairGeoD &g, double dx, double dy, double dz, auto mul) {
                     using MUL = decltype(mul);
                     if constexpr (KIND == RMW_UF || KIND == RMW_WT) {
                         UFBlockD m;
-                        if constexpr (KIND == RMW_UF) m = uf_block_d<false, MUL>(g, dz, Rz, zi, zj);
+                        if constexpr (KIND == RMW_UF) m = uf_block_d<false, MUL>(g, dz, Rz, hi, hj);
                         else m = wt_block_d<false, MUL>(g, dz, Rz);
                         uf_block_acc_d<MUL>(m, m.t3, m.t4, dx, dy, vx, vy, vz, ux, uy, uz);
                         uf_block_acc_d<MUL>(m, m.t4, m.t3, dx, dy, me.vx, me.vy, me.vz, wx, wy, wz);
                     } else {
-                        const RotBlockD k = rot_block_d<false, MUL>(g, dz, Rz, zi, zj);
+                        const RotBlockD k = rot_block_d<false, MUL>(g, dz, Rz, hi, hj);
                         if constexpr (KIND == RMW_UT)
                             ut_acc_d<MUL>(k, dx, dy, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
                         else wf_acc_d<MUL>(k, dx, dy, vx, vy, vz, me.vx, me.vy, me.vz, ux, uy, uz, wx, wy, wz);
@@ -917,14 +921,14 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
             }
         };
         if constexpr (PER) {
-            double rx = xi - tx[jl], ry = yi - ty[jl];
+            double rx = me.x - tx[jl], ry = me.y - ty[jl];
             if (P.Lx > 0) rx = project(rx, P.Lx);
             if (P.Ly > 0) ry = project(ry, P.Ly);
             const int px = P.Lx > 0, py = P.Ly > 0;
             for (int bx = -px; bx <= px; ++bx)
-                for (int by = -py; by <= py; ++by) pair((rx + bx * P.Lx) * inva, (ry + by * P.Ly) * inva);
+                for (int by = -py; by <= py; ++by) pair(rx + bx * P.Lx, ry + by * P.Ly);
         } else {
-            pair(xi - tx[jl], yi - ty[jl]);
+            pair(me.x - tx[jl], me.y - ty[jl]);
         }
         sacc[warp][0][jl] = wx;
         sacc[warp][1][jl] = wy;
@@ -944,7 +948,7 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
                 for (int bx = -px; bx <= px; ++bx)
                     for (int by = -py; by <= py; ++by)
                         if (bx || by)
-                            pair_acc_d<KIND, true>(bx * P.Lx * inva, by * P.Ly * inva, 0.0, 2.0 * zi, zi, zi, me.vx,
+                            pair_acc_d<KIND, true>(bx * P.Lx * inva, by * P.Ly * inva, 0.0, 2.0 * hi, hi, hi, me.vx,
                                                    me.vy, me.vz, ux, uy, uz);
             }
         }
