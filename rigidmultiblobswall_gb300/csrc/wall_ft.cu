@@ -900,16 +900,20 @@ int wall_force_torque(const double *r, const double *F, const double *T, double 
             return RMW_OK;
         }
     }
-    // FP64 and df64 from 256 blobs: the fused symmetric kernel, where its
-    // partial sums fit; where they do not, four symmetric single products (whose
-    // sums are half as large, or banded), else the one-sided fused pass
+    // FP64 and df64 where all four products prefer the symmetric kernel (untuned: from 256 blobs; a tuned or pinned
+    // source split keeps the one-sided pass and its small scratch): the fused symmetric kernel, where its partial sums
+    // fit; where they do not, four symmetric single products, whose sums are half as large; else the one-sided pass
     if (!per && (mode == RMW_MODE_FP64 || mode == RMW_MODE_DF64) && N >= 2 * kFtSymTile) {
-        const int rc = ft_symmetric(r, F, T, U, W, N, eta, a, mode, st);
-        if (rc != RMW_ERR_ALLOC) return rc;
-        bool sym = true;
-        for (int kind : {RMW_UF, RMW_UT, RMW_WF, RMW_WT})
-            sym = sym && wall_chunks(kind, mode, N) == kSymChunks && wall_sym_applicable(kind, mode, N, nullptr);
-        if (sym) return ft_by_symmetric_products(r, F, T, U, W, N, eta, a, mode, st);
+        bool prefer = true, applies = true;
+        for (int kind : {RMW_UF, RMW_UT, RMW_WF, RMW_WT}) {
+            prefer = prefer && wall_prefers_sym(kind, mode, N);
+            applies = applies && wall_sym_applicable(kind, mode, N, nullptr);
+        }
+        if (prefer) {
+            const int rc = ft_symmetric(r, F, T, U, W, N, eta, a, mode, st);
+            if (rc != RMW_ERR_ALLOC) return rc;
+            if (applies) return ft_by_symmetric_products(r, F, T, U, W, N, eta, a, mode, st);
+        }
     }
     const int nchunks = wall_default_chunks(N);
     void *ws = nullptr;
