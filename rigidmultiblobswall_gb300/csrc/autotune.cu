@@ -123,7 +123,7 @@ int rmw_wall_autotune(int kind, int mode, int64_t n, int reps, void *stream, int
     if (std::find(cand.begin(), cand.end(), def) == cand.end()) cand.push_back(def);
     const bool try_sym = rmw::wall_sym_applicable(kind, mode, N, nullptr);
     if (try_sym) cand.push_back(rmw::kSymChunks);
-    const int nsplit = try_sym ? rmw::wall_sym_split(mode, N) : 1;
+    const int nsplit = try_sym ? rmw::wall_sym_split(mode, N, rmw::wall_scratch_bytes(N, mode, 0)) : 1;
     const int cmax = std::max(*std::max_element(cand.begin(), cand.end()), try_sym ? rmw::wall_sym_slots(N, nsplit) : 1);
     const size_t vec = sizeof(double) * 3 * (size_t)N;
     const size_t ws_bytes = rmw::wall_scratch_bytes(N, mode, cmax);

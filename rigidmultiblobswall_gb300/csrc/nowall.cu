@@ -306,13 +306,19 @@ int nowall_product(int kind, const double *r, const double *v, double *out, int6
     // in FP64 and df64 and 8,192 in mixed, as the wall products' untuned rule
     bool sym = !per && N >= (mode == RMW_MODE_MIXED ? 8192 : 256) &&
                wall_sym_applicable(kind, mode, N, nullptr);
-    const int nsplit = sym ? wall_sym_split(mode, N) : 1;
-    int nchunks = sym ? wall_sym_slots(N, nsplit) : wall_default_chunks(mode, N);
     const size_t rec = (mode == RMW_MODE_FP64) ? sizeof(NwSrcD) : (mode == RMW_MODE_DF64 ? sizeof(NwSrcDF)
                                                                                           : sizeof(NwSrcF));
     const size_t packed = ((rec * (size_t)N + 255) / 256) * 256;
+    int nsplit = sym ? wall_sym_split(mode, N, packed) : 1;
+    int nchunks = sym ? wall_sym_slots(N, nsplit) : wall_default_chunks(mode, N);
     void *ws = nullptr;
     int src = scratch(SCRATCH_PAIR, packed + sizeof(double) * 3 * (size_t)N * nchunks, &ws, st);
+    if (src && sym && nsplit > 1) {  // memory pressure: whole tile pairs need the least
+        cudaGetLastError();
+        nsplit = 1;
+        nchunks = wall_sym_slots(N, 1);
+        src = scratch(SCRATCH_PAIR, packed + sizeof(double) * 3 * (size_t)N * nchunks, &ws, st);
+    }
     if (src && (sym || nchunks > wall_default_chunks(N))) {
         // the symmetric partial sums did not fit next to the caller's
         // allocations (or above rmw_set_scratch_limit): the one-sided kernels

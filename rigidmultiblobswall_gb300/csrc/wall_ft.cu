@@ -812,13 +812,19 @@ int ft_by_symmetric_products(const double *r, const double *F, const double *T, 
 int ft_symmetric(const double *r, const double *F, const double *T, double *U, double *W, int n, double eta, double a,
                  int mode, cudaStream_t st)
 {
-    const int nt = (n + kFtSymTile - 1) / kFtSymTile, nsplit = wall_sym_split(mode, n);
+    const int nt = (n + kFtSymTile - 1) / kFtSymTile;
     const size_t rec = mode == RMW_MODE_DF64 ? sizeof(FtSrcDF) : sizeof(FtSrcD);
-    const size_t packed = ((rec * (size_t)n + 255) / 256) * 256;
-    const size_t part = sizeof(double) * 6 * (size_t)n * nt * nsplit;
+    const size_t packed = ((rec * (size_t)n + 255) / 256) * 256, slot = sizeof(double) * 6 * (size_t)n * nt;
+    int nsplit = wall_sym_split(mode, n, packed, false, 6);
     void *ws = nullptr;
-    if (part > wall_sym_partial_budget()) return RMW_ERR_ALLOC;
-    if (scratch(SCRATCH_PAIR, packed + part, &ws, st) != RMW_OK) {
+    if (slot > wall_sym_partial_budget()) return RMW_ERR_ALLOC;
+    int rc = scratch(SCRATCH_PAIR, packed + slot * nsplit, &ws, st);
+    if (rc && nsplit > 1) {  // memory pressure: whole tile pairs need the least
+        cudaGetLastError();
+        nsplit = 1;
+        rc = scratch(SCRATCH_PAIR, packed + slot, &ws, st);
+    }
+    if (rc) {
         cudaGetLastError();
         return RMW_ERR_ALLOC;
     }

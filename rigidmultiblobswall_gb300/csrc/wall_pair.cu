@@ -34,6 +34,7 @@
 
 #include "pair_math.cuh"
 #include "pair_math_df.cuh"
+#include "product_plan.h"
 #include "rmw_common.cuh"
 #include "wall_pair.cuh"
 
@@ -1022,8 +1023,6 @@ __global__ void __launch_bounds__(kThreads) nowall_fp64_sym_kernel(const SrcD *_
     fp64_sym_body<false, KIND, true>(src, n, nt, 1.0, partial, nullptr);
 }
 
-static int sym_tiles(int n) { return (n + kTile - 1) / kTile; }
-
 template <int KIND>
 static void nowall_sym_launch_kind(int mode, const void *src, int n, int nt, double *partial, cudaStream_t st,
                                    int nsplit)
@@ -1663,9 +1662,6 @@ size_t wall_sym_partial_budget()
     return cap ? std::min(b, cap) : b;
 }
 
-constexpr int kSplitMax = 64;
-constexpr double kSplitBytes = 64e6;  // partial sums of a split product: they stay in L2
-
 // periodic in x and / or y only: the FP64 kernel has a symmetric form
 static bool per_sym(int mode, const double *L)
 {
@@ -1683,46 +1679,15 @@ bool wall_sym_applicable(int kind, int mode, int n, const double *L)
     return nt * 3.0 * (double)n * sizeof(double) <= (double)wall_sym_partial_budget();
 }
 
-// How many CTAs share the steps of a tile pair.  Below about 4,000 blobs the
-// tile pairs alone leave SMs idle (2,048 blobs: 136 of them); the split fills
-// the GPU with the symmetric kernel's work per pair where the one-sided kernel
-// used to do each pair twice (2,048 blobs: FP64 UF 961 -> 364 us, df64 181 ->
-// 70).  With P tile pairs, s CTAs each and a CTA's start and end worth e steps,
-// an SM takes (P s / 152 + d)(128 / s + e) step times, d the uneven end of the
-// grid: least at s = sqrt(152 * 128 d / (e P)).  Measured by s: df64 UF 2,048
-// blobs 8: 72, 16: 74, 32: 81 us; 5,003 blobs 2: 275, 4: 259, 8: 279 us; FP64
-// UF 10,752 blobs 1: 8.24, 2: 8.08 ms; FP64 periodic 4,800 blobs 2: 15.2,
-// 8: 14.8 ms, which K = 13,000 (df64), 40,000 (FP64) and 160,000 (periodic
-// FP64, whose steps are nine times as long) in s = sqrt(K / P) reproduce.
-// Where even 64 CTAs per pair are fewer than 16 per SM, the split whose
-// busiest SM has least to do (504 blobs FP64: 43, 48 us; 32: 54 us).  Mixed
-// products keep whole tile pairs: their FP32 sums would change with the split.
-int wall_sym_split(int mode, int n, bool periodic)
+// Mixed products keep whole tile pairs: their FP32 sums would change with the split.
+int wall_sym_split(int mode, int n, size_t packed, bool periodic, int comps)
 {
     if (mode == RMW_MODE_MIXED) return 1;
-    const bool fp64 = mode == RMW_MODE_FP64;
-    const double nt = (double)sym_tiles(n), pairs = 0.5 * nt * (nt + 1);
-    const double slot = nt * 3.0 * (double)n * sizeof(double);
-    const double bytes = std::min((double)wall_sym_partial_budget(), kSplitBytes);
-    int s = 1;
-    if (pairs * kSplitMax < 16 * 152.0) {
-        const double ends = periodic ? 0.05 : fp64 ? 0.4 : 1.2, fill = fp64 ? 2.0 : 6.0;
-        double cost = 0.0;
-        for (int c = 1; c <= kSplitMax; ++c) {
-            const double t = std::max(std::ceil(pairs * c / 152.0), fill) * (std::ceil((double)kTile / c) + ends);
-            if (c == 1 || t < 0.99 * cost) {
-                cost = t;
-                s = c;
-            }
-        }
-    } else {
-        s = (int)std::min((double)kSplitMax, std::sqrt((periodic ? 160000.0 : fp64 ? 40000.0 : 13000.0) / pairs) +
-                                                     (fp64 ? 0.5 : 0.05));  // whole df64 pairs have constant bounds
-    }
-    while (s > 1 && slot * s > bytes) --s;
-    return std::max(1, s);
+    return sym_split(mode == RMW_MODE_FP64, periodic, n, comps, (double)packed, (double)wall_sym_partial_budget(),
+                     (double)scratch_limit());
 }
 
+static_assert(kTile == kPlanTile, "the plan counts the kernels' tiles");
 int wall_sym_slots(int n, int nsplit) { return sym_tiles(n) * nsplit; }
 
 // the symmetric kernel and finalize of one kind: the UF kernels sum (3/2) M v
@@ -1920,7 +1885,7 @@ int wall_product(int kind, const double *r, const double *v, double *out, int64_
     int nchunks = wall_prefers_sym(kind, mode, (int)n) ? kSymChunks : wall_chunks(kind, mode, (int)n);
     bool sym = nchunks == kSymChunks && wall_sym_applicable(kind, mode, (int)n, L);
     const bool periodic = L && (L[0] > 0 || L[1] > 0 || L[2] > 0);
-    const int nsplit = sym ? wall_sym_split(mode, (int)n, periodic) : 1;
+    int nsplit = sym ? wall_sym_split(mode, (int)n, wall_scratch_bytes((int)n, mode, 0), periodic) : 1;
     void *ws = nullptr;
     if (nchunks == kSymChunks && !sym && mode == RMW_MODE_DF64 && !periodic && n >= 2 * kTile) {
         // too many tiles for one partial-sum slot per tile: the symmetric kernel band by band
@@ -1931,6 +1896,11 @@ int wall_product(int kind, const double *r, const double *v, double *out, int64_
     if (nchunks == kSymChunks && !sym) nchunks = wall_default_chunks(mode, (int)n);
     rc = scratch(SCRATCH_PAIR, wall_scratch_bytes((int)n, mode, sym ? wall_sym_slots((int)n, nsplit) : nchunks), &ws,
                  st);
+    if (rc && sym && nsplit > 1) {  // memory pressure: whole tile pairs need the least
+        cudaGetLastError();
+        nsplit = 1;
+        rc = scratch(SCRATCH_PAIR, wall_scratch_bytes((int)n, mode, wall_sym_slots((int)n, 1)), &ws, st);
+    }
     if (rc && sym) {
         // the symmetric kernel's partial sums did not fit next to the caller's
         // allocations: the standard kernel needs far less scratch

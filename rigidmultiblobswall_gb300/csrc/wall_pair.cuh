@@ -86,8 +86,9 @@ constexpr size_t kSymMaxPartialBytes = size_t(6) << 30;  // up to ~185,000 blobs
 // given n does not depend on what else is allocated.
 size_t wall_sym_partial_budget();
 bool wall_sym_applicable(int kind, int mode, int n, const double *L);
-// CTAs per tile pair of the symmetric kernels, and their partial-sum slots
-int wall_sym_split(int mode, int n, bool periodic = false);
+// CTAs per tile pair of the symmetric kernels beside `packed` bytes of records (product_plan.h), for `comps` doubles
+// of partial sums a blob and tile, and their partial-sum slots
+int wall_sym_split(int mode, int n, size_t packed, bool periodic = false, int comps = 3);
 int wall_sym_slots(int n, int nsplit);
 // banded symmetric df64 product (above the partial-sum budget): tile rows per band, its scratch
 int wall_sym_band_rows(int n);
