@@ -312,7 +312,8 @@ int nowall_product(int kind, const double *r, const double *v, double *out, int6
     int nsplit = sym ? wall_sym_split(mode, N, packed) : 1;
     int nchunks = sym ? wall_sym_slots(N, nsplit) : wall_default_chunks(mode, N);
     void *ws = nullptr;
-    int src = scratch(SCRATCH_PAIR, packed + sizeof(double) * 3 * (size_t)N * nchunks, &ws, st);
+    int src = scratch(SCRATCH_PAIR, packed + sizeof(double) * 3 * (size_t)N * nchunks, &ws, st,
+                      wall_reserve_bytes(mode, N, packed, sym));
     if (src && sym && nsplit > 1) {  // memory pressure: whole tile pairs need the least
         cudaGetLastError();
         nsplit = 1;

@@ -64,4 +64,54 @@ inline int sym_split(bool fp64, bool periodic, int n, int comps, double packed, 
     return std::max(1, s);
 }
 
+// Partial sums that a symmetric product's buffer has room for: at least what
+// any smaller product takes, whose split may be finer (df64: 22 MB at 10,752
+// blobs, 38 MB at 10,000), so that a buffer that served n blobs serves every
+// smaller n, also where it must not grow (a stream capture).
+inline double sym_reserve_bytes(int n, int comps)
+{
+    const double slot = sym_slot_bytes(n, comps);
+    return std::max(slot, std::min(kSplitBytes * comps / 3, kSplitMax * slot));
+}
+
+// The one-sided kernels' source chunks: enough CTAs to fill the 152 SMs
+// several times over, at least 256 sources each.
+inline int coarse_chunks(int n)
+{
+    const int tiles = sym_tiles(n);
+    const int s = std::min((152 * 8 + tiles - 1) / tiles, std::max(1, n / 256));
+    return std::max(1, std::min(s, kSplitMax));
+}
+
+// The same in FP64 and df64 (periodic products, fewer than 256 blobs): the
+// split whose busiest SM has the least to do, counting a tile's staging as two
+// sources; an SM needs about two FP64 or four df64 CTAs to keep its pipe busy.
+// coarse_chunks left 1,500 periodic blobs on 60 CTAs.  Finer than that only
+// while the partial sums stay within kSplitBytes and, with the packed records,
+// within the scratch cap (0 = none).
+inline int fine_chunks(bool fp64, int n, double packed, double cap)
+{
+    const int base = coarse_chunks(n), tiles = sym_tiles(n), fill = fp64 ? 2 : 4;
+    const double one = 3.0 * (double)n * sizeof(double);
+    int best = base;
+    long long cost = -1;
+    for (int c = 1; c <= kSplitMax && c <= std::max(base, n / 8); ++c) {
+        if (c > base && (one * c > kSplitBytes || (cap > 0 && packed + one * c > cap))) break;
+        const long long ctas = ((long long)tiles * c + 151) / 152;
+        const long long t = std::max<long long>(ctas, fill) * ((n + c - 1) / c + 2);
+        if (cost < 0 || t < cost) {
+            cost = t;
+            best = c;
+        }
+    }
+    return best;
+}
+
+// as sym_reserve_bytes, for fine_chunks
+inline double fine_reserve_bytes(int n)
+{
+    const double one = 3.0 * (double)n * sizeof(double);
+    return std::max(one * coarse_chunks(n), std::min(kSplitBytes, kSplitMax * one));
+}
+
 }  // namespace rmw

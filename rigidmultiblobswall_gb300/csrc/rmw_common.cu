@@ -148,7 +148,7 @@ int pool_retain()
     return RMW_OK;
 }
 
-int scratch(ScratchSlot slot, size_t bytes, void **ptr, cudaStream_t st)
+int scratch(ScratchSlot slot, size_t bytes, void **ptr, cudaStream_t st, size_t keep)
 {
     int dev = 0;
     RMW_CUDA(cudaGetDevice(&dev));
@@ -170,9 +170,19 @@ int scratch(ScratchSlot slot, size_t bytes, void **ptr, cudaStream_t st)
             b.bytes = 0;
         }
         // headroom so that slowly growing sizes reallocate rarely (none above 1 GiB, and never past the cap)
-        size_t want = bytes + (bytes >= ((size_t)1 << 30) ? 0 : bytes / 4) + 4096;
-        if (cap && want > cap) want = bytes;
-        RMW_CUDA(cudaMalloc(&b.ptr, want));
+        size_t want = std::max(bytes, keep);
+        want += (want >= ((size_t)1 << 30) ? 0 : want / 4) + 4096;
+        if (cap && want > cap) want = std::max(bytes, std::min(keep, cap));
+        cudaError_t e = cudaMalloc(&b.ptr, want);
+        if (e != cudaSuccess && want > bytes) {  // a nearly full device: what the call needs
+            cudaGetLastError();
+            want = bytes;
+            e = cudaMalloc(&b.ptr, want);
+        }
+        if (e != cudaSuccess) {
+            b.ptr = nullptr;
+            return cuda_fail(e, "cudaMalloc (scratch)");
+        }
         b.bytes = want;
     }
     *ptr = b.ptr;

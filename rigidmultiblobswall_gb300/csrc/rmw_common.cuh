@@ -29,9 +29,10 @@ int cuda_fail(cudaError_t e, const char *where);
 // A grow-only device buffer per (device, stream, slot).  Calls on the same
 // device, stream and slot share it (they are ordered by the stream); a call that
 // needs more frees the old buffer (cudaFree synchronises the device, so no
-// kernel still reads it) and allocates anew.
+// kernel still reads it) and allocates anew, with room for `keep` bytes where
+// the limit and the device's free memory allow it.
 enum ScratchSlot { SCRATCH_PAIR = 0, SCRATCH_HOST_STAGING = 1, SCRATCH_FT_TERM = 2, SCRATCH_FORCES = 3, SCRATCH_SLOTS = 4 };
-int scratch(ScratchSlot slot, size_t bytes, void **ptr, cudaStream_t st);
+int scratch(ScratchSlot slot, size_t bytes, void **ptr, cudaStream_t st, size_t keep = 0);
 // frees the current device's scratch buffers (deferred while graphs are alive)
 int scratch_release_all();
 // requests above `bytes` fail with RMW_ERR_ALLOC without touching the device (0 = no cap)

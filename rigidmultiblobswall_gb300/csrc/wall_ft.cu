@@ -818,7 +818,7 @@ int ft_symmetric(const double *r, const double *F, const double *T, double *U, d
     int nsplit = wall_sym_split(mode, n, packed, false, 6);
     void *ws = nullptr;
     if (slot > wall_sym_partial_budget()) return RMW_ERR_ALLOC;
-    int rc = scratch(SCRATCH_PAIR, packed + slot * nsplit, &ws, st);
+    int rc = scratch(SCRATCH_PAIR, packed + slot * nsplit, &ws, st, wall_reserve_bytes(mode, n, packed, true, 6));
     if (rc && nsplit > 1) {  // memory pressure: whole tile pairs need the least
         cudaGetLastError();
         nsplit = 1;

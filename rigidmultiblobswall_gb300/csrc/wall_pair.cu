@@ -1518,41 +1518,18 @@ __global__ void __launch_bounds__(3 * kFinBlobs * 8) wall_finalize_kernel(
 
 // ---------------------------------------------------------------------------
 // host side
-static int choose_chunks(int n)
-{
-    const int tiles = (n + kThreads - 1) / kThreads;
-    const int want = 152 * 8;  // CTAs to fill the 152 SMs several times over
-    int s = (want + tiles - 1) / tiles;
-    s = std::min(s, std::max(1, n / 256));  // keep each chunk >= 256 sources
-    return std::max(1, std::min(s, 64));
-}
+int wall_default_chunks(int n) { return coarse_chunks(n); }
 
-int wall_default_chunks(int n) { return choose_chunks(n); }
-
-// The one-sided kernels' source split in FP64 and df64 (periodic products,
-// fewer than 256 blobs): the split whose busiest SM has the least to do,
-// counting a tile's staging as two sources; an SM needs about two FP64 or
-// four df64 CTAs to keep its pipe busy.  choose_chunks keeps 256 sources per
-// chunk, which left 1,500 periodic blobs on 60 CTAs.  Where the partial sums
-// of the finer split would exceed the scratch limit, the coarser one stands.
 int wall_default_chunks(int mode, int n)
 {
-    const int base = choose_chunks(n);
-    if (mode == RMW_MODE_MIXED) return base;
-    const int tiles = (n + kThreads - 1) / kThreads, fill = mode == RMW_MODE_FP64 ? 2 : 4;
-    const size_t cap = scratch_limit();
-    int best = base;
-    long long cost = -1;
-    for (int c = 1; c <= 64 && c <= std::max(base, n / 8); ++c) {
-        if (c > base && cap && wall_scratch_bytes(n, mode, c) > cap) break;
-        const long long ctas = ((long long)tiles * c + 151) / 152;
-        const long long t = std::max<long long>(ctas, fill) * ((n + c - 1) / c + 2);
-        if (cost < 0 || t < cost) {
-            cost = t;
-            best = c;
-        }
-    }
-    return best;
+    if (mode == RMW_MODE_MIXED) return coarse_chunks(n);
+    return fine_chunks(mode == RMW_MODE_FP64, n, (double)wall_scratch_bytes(n, mode, 0), (double)scratch_limit());
+}
+
+size_t wall_reserve_bytes(int mode, int n, size_t packed, bool sym, int comps)
+{
+    if (mode == RMW_MODE_MIXED) return 0;
+    return packed + (size_t)(sym ? sym_reserve_bytes(n, comps) : fine_reserve_bytes(n));
 }
 
 size_t wall_scratch_bytes(int n, int mode, int nchunks)
@@ -1894,8 +1871,9 @@ int wall_product(int kind, const double *r, const double *v, double *out, int64_
         cudaGetLastError();
     }
     if (nchunks == kSymChunks && !sym) nchunks = wall_default_chunks(mode, (int)n);
+    const size_t packed = wall_scratch_bytes((int)n, mode, 0);
     rc = scratch(SCRATCH_PAIR, wall_scratch_bytes((int)n, mode, sym ? wall_sym_slots((int)n, nsplit) : nchunks), &ws,
-                 st);
+                 st, wall_reserve_bytes(mode, (int)n, packed, sym));
     if (rc && sym && nsplit > 1) {  // memory pressure: whole tile pairs need the least
         cudaGetLastError();
         nsplit = 1;
@@ -2053,7 +2031,7 @@ int wall_uf_multi(const double *r, const double *V, long long ldv, double *Y, lo
 {
     if (!B) active = nullptr;
     if (nrhs <= 0 || n <= 0) return RMW_OK;
-    const int nchunks = B ? B->max_slots : choose_chunks(n);
+    const int nchunks = B ? B->max_slots : coarse_chunks(n);
     const int wmax = nrhs > 8 ? kMultiPass : 8;
     const size_t pos = ((sizeof(SrcF) * (size_t)n + 255) / 256) * 256;
     const size_t vecb = ((sizeof(float) * 3 * (size_t)n * wmax + 255) / 256) * 256;

@@ -99,6 +99,9 @@ int wall_product_sym_with_scratch(int kind, const double *r, const double *v, do
 // no-wall product (layouts of SrcD / SrcDF / SrcF, positions over a); writes
 // wall_sym_slots(n, nsplit) partial-sum slots of 3n doubles.
 int nowall_sym_launch(int kind, int mode, const void *src, int n, double *partial, cudaStream_t st, int nsplit);
+// Bytes that the scratch buffer of a product beside `packed` bytes of records keeps room for, so that it serves every
+// smaller product of that route too (0: what the product needs): sym_reserve_bytes, fine_reserve_bytes.
+size_t wall_reserve_bytes(int mode, int n, size_t packed, bool sym, int comps = 3);
 // Source-chunk count the standard entry points use: the autotuned choice of
 // (kind, mode, n's size bucket) on the current device if there is one
 // (autotune.cu; kSymChunks = the symmetric kernel), else the built-in rule.
