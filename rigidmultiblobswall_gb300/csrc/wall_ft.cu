@@ -693,6 +693,7 @@ __global__ void __launch_bounds__(kFtF2Threads, 4) ft_sym_df_kernel(const FtSrcD
     constexpr int NC = WITH_W ? 6 : 3;
     __shared__ float4 tile[6][kFtSymTile];  // hi, lo, fhi, flo, thi, tlo
     __shared__ float4 sacc[kFtF2Threads / 32][NC][kFtSymTile];
+    __shared__ double tacc[2][NC][kFtF2Threads];  // the targets' FP64 sums
     int T, S;
     sym_tile_pair(blockIdx.x, nt, T, S);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -723,6 +724,7 @@ __global__ void __launch_bounds__(kFtF2Threads, 4) ft_sym_df_kernel(const FtSrcD
     }
     for (int c = 0; c < NC; ++c)
         for (int k = lane; k < kFtSymTile; k += 32) sacc[warp][c][k] = zero;
+    for (int c = 0; c < NC; ++c) tacc[0][c][tid] = tacc[1][c][tid] = 0.0;
     __syncthreads();
     df2 u[6];
     for (int c = 0; c < 6; ++c) u[c] = df2_zero();
@@ -730,6 +732,13 @@ __global__ void __launch_bounds__(kFtF2Threads, 4) ft_sym_df_kernel(const FtSrcD
     auto renorm = [&](int k) {
         if (k & 7) return;
         for (int c = 0; c < NC; ++c) u[c] = norm(u[c]);
+    };
+    auto fold = [&]() {
+        for (int c = 0; c < NC; ++c) {
+            tacc[0][c][tid] += to_double(df{u[c].hi.x, u[c].lo.x});
+            tacc[1][c][tid] += to_double(df{u[c].hi.y, u[c].lo.y});
+            u[c] = df2_zero();
+        }
     };
     if (diag) {
         // offsets (source - target) 1..63, and 64 for lane x alone (lane y's pairs are lane x's)
@@ -751,6 +760,7 @@ __global__ void __launch_bounds__(kFtF2Threads, 4) ft_sym_df_kernel(const FtSrcD
                 }
             }
             renorm(o);
+            if (!(o & (kFtDfGroup - 1))) fold();
         }
     } else {
 #pragma unroll 1
@@ -758,22 +768,24 @@ __global__ void __launch_bounds__(kFtF2Threads, 4) ft_sym_df_kernel(const FtSrcD
             __syncwarp();
             const int j = (lane + k) & (kFtSymTile - 1);
             ft_f2_step<false, WITH_W>(me, j, j, tile, sacc[warp], u);
-            renorm(k);
+            renorm(k + 1);
+            if (!((k + 1) & (kFtDfGroup - 1))) fold();
         }
     }
+    fold();
     __syncthreads();
     for (int half = 0; half < 2; ++half) {
         const int l = tid + half * kFtF2Threads, i = T * kFtSymTile + l, j = S * kFtSymTile + l;
         for (int c = 0; c < NC; ++c) {
-            const df t = half ? df{u[c].hi.y, u[c].lo.y} : df{u[c].hi.x, u[c].lo.x};
-            df q = df_from(0.f);
+            const double t = tacc[half][c][tid];
+            double q = 0.0;
             for (int w = 0; w < kFtF2Threads / 32; ++w) {
                 const float4 f = sacc[w][c][l];
-                q = q + (df{f.x, f.z} + df{f.y, f.w});
+                q += to_double(df{f.x, f.z}) + to_double(df{f.y, f.w});
             }
             const size_t comp = (c / 3) * 3 * (size_t)n + c % 3;
-            if (i < n) partial[sp.slot(diag ? T : S) * 6 * n + 3 * (size_t)i + comp] = to_double(diag ? t + q : t);
-            if (!diag && j < n) partial[sp.slot(T) * 6 * n + 3 * (size_t)j + comp] = to_double(q);
+            if (i < n) partial[sp.slot(diag ? T : S) * 6 * n + 3 * (size_t)i + comp] = diag ? t + q : t;
+            if (!diag && j < n) partial[sp.slot(T) * 6 * n + 3 * (size_t)j + comp] = q;
         }
     }
 }

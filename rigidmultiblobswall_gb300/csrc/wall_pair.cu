@@ -313,7 +313,9 @@ __device__ __forceinline__ void sym_band_pair(long long b, int nt, const SymBand
 // the explicit block (uf_block_df) takes 30 % of the arithmetic.  The
 // source-side sums are float4 (hi x, hi y, lo x, lo y) per warp, component
 // and source; the target-side ones are renormalised every kF2Group steps and
-// stay on the FP32 pipe.
+// folded into FP64 sums (in shared memory) every kDfGroup, and the warps'
+// source-side sums are added in FP64 (0.4 % of the time; double-float sums of
+// the whole tile: error 5.64e-14 instead of 5.57e-14 at 10,752 blobs).
 // Measured (pair kernel): 10,752 blobs 1.63 -> 0.99 ms, FMA pipe 86 % active,
 // issue 48 %; the product at 172,032 blobs 400 -> 240 ms.  128 registers (8 CTAs per SM) are
 // 2 % faster than the 158 that one CTA takes unbounded.
@@ -395,6 +397,7 @@ __device__ __forceinline__ void df_f2_body(const SrcDF *__restrict__ src, int n,
 {
     __shared__ float4 thi[kTile], tlo[kTile], tvh[kTile], tvl[kTile];
     __shared__ float4 sacc[kF2Threads / 32][3][kTile];
+    __shared__ double tacc[2][3][kF2Threads];  // the targets' FP64 sums
     int T, S;
     if constexpr (BAND) sym_band_pair(blockIdx.x, nt, bd, T, S);
     else sym_cta<SEG>(jobs, n, nt, T, S, src, partial);
@@ -425,8 +428,18 @@ __device__ __forceinline__ void df_f2_body(const SrcDF *__restrict__ src, int n,
     }
     for (int c = 0; c < 3; ++c)
         for (int k = lane; k < kTile; k += 32) sacc[warp][c][k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int c = 0; c < 3; ++c) tacc[0][c][tid] = tacc[1][c][tid] = 0.0;
     __syncthreads();
     df2 ux = df2_zero(), uy = df2_zero(), uz = df2_zero();
+    auto fold = [&]() {
+        const df2 uu[3] = {ux, uy, uz};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            tacc[0][c][tid] += to_double(df{uu[c].hi.x, uu[c].lo.x});
+            tacc[1][c][tid] += to_double(df{uu[c].hi.y, uu[c].lo.y});
+        }
+        ux = uy = uz = df2_zero();
+    };
     const SymSteps sp = sym_steps<WHOLE>();
     if (diag) {
         // offsets 1..64 (source - target): each unordered pair once; 64 pairs up targets 0..63 with
@@ -446,7 +459,9 @@ __device__ __forceinline__ void df_f2_body(const SrcDF *__restrict__ src, int n,
                 uz.hi.x = vz.hi.x; uz.lo.x = vz.lo.x;
             }
             if (!(o & (kF2Group - 1))) { ux = norm(ux); uy = norm(uy); uz = norm(uz); }
+            if (!(o & (kDfGroup - 1))) fold();
         }
+        fold();
     } else {
         for (int g = sp.k0; g < sp.k1;) {
             const int e = min(g + kF2Group, sp.k1);
@@ -459,28 +474,27 @@ __device__ __forceinline__ void df_f2_body(const SrcDF *__restrict__ src, int n,
             ux = norm(ux);
             uy = norm(uy);
             uz = norm(uz);
+            if (!((g - sp.k0) & (kDfGroup - 1))) fold();
         }
+        fold();
     }
     __syncthreads();
     const size_t stride = 3 * (size_t)n;
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         const int l = tid + half * kF2Threads;  // blob l of the tile
-        // source role of blob S*128 + l (dummy pairs contributed exact zeros): four double-float sums, on the
-        // FP32 pipe (an FP64 add costs as much as 64 FP32 ones), one FP64 value per component at the end
-        const df2 uu[3] = {ux, uy, uz};
+        // source role of blob S*128 + l (dummy pairs contributed exact zeros): four double-float sums
         double own[3], s[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const df t = half ? df{uu[c].hi.y, uu[c].lo.y} : df{uu[c].hi.x, uu[c].lo.x};
-            df q = df_from(0.f);
+            double q = 0.0;
 #pragma unroll
             for (int w = 0; w < kF2Threads / 32; ++w) {
                 const float4 f = sacc[w][c][l];
-                q = q + (df{f.x, f.z} + df{f.y, f.w});
+                q += to_double(df{f.x, f.z}) + to_double(df{f.y, f.w});
             }
-            own[c] = to_double(diag ? t + q : t);
-            s[c] = diag ? 0.0 : to_double(q);
+            own[c] = tacc[half][c][tid] + (diag ? q : 0.0);
+            s[c] = q;
         }
         if constexpr (BAND) {
             const int W = nt - bd.t0, C = bd.t1 - bd.t0;
