@@ -48,22 +48,22 @@ NF_ALL_EXACT_R = NF_CUTOFF_R
 # instruction counted as the two lanes' operations it does on the FMA pipe
 # (which takes it two clocks).  Symmetric kernel (each unordered pair once,
 # two targets per thread in packed lanes): smsp__inst_executed.sum
-# 587,491,408 + packed (pipe_fmaheavy + pipe_fmalite - pipe_fma) 512,310,398
-# = 1,099,801,806 warp instructions * 32 / 10752^2 = 304.4; one-sided kernel
-# (source split 15) 1,804,025,700 * 32 / 10752^2 = 499.4.  The FP32 pipe takes
+# 589,297,576 + packed (pipe_fmaheavy + pipe_fmalite - pipe_fma) 514,116,734
+# = 1,103,414,310 warp instructions * 32 / 10752^2 = 305.4; one-sided kernel
+# (source split 15) 1,811,251,044 * 32 / 10752^2 = 501.4.  The FP32 pipe takes
 # at most one thread instruction per lane per clock, the rate the FMA-chain
 # probe measures (FLOP/s / 2), so achieved / peak is the fraction of that
 # capacity used.  The constants hold for the kernel sources whose hash is
 # DF64_UF_KERNEL_SOURCE_SHA (tests/test_bench_constants.py fails when the
 # kernel changes without a new capture).
-DF64_UF_INST_PER_PAIR = {"symmetric": 1099801806.0 * 32 / 10752 ** 2, "standard": 1804025700.0 * 32 / 10752 ** 2}
+DF64_UF_INST_PER_PAIR = {"symmetric": 1103414310.0 * 32 / 10752 ** 2, "standard": 1811251044.0 * 32 / 10752 ** 2}
 # dram__bytes_read.sum + dram__bytes_write.sum per launch, same captures
-DF64_UF_TRAFFIC_BYTES = {"symmetric": 759296, "standard": 719616}
+DF64_UF_TRAFFIC_BYTES = {"symmetric": 759552, "standard": 717824}
 # FP32-issue slots per pair and right-hand side of the 16-wide multi-RHS M_UF kernel, packed instructions
 # counted twice as above ((smsp__inst_executed.sum 17,258,189,476 + packed 12,838,677,918) * 32 / (N^2 * 16),
 # 60,000 blobs)
 MULTI16_INST_PER_PAIR_RHS = 16.72
-DF64_UF_KERNEL_SOURCE_SHA = "8ea76f8caa84ffaee71a11c1b92ac68fc006087f7c2a7d17befec2700226c35a"
+DF64_UF_KERNEL_SOURCE_SHA = "b66356df218e39bc68f5d92067a96c5fea16d68b3d3ea26dc294e5bd3808fbc9"
 
 
 def df64_uf_kernel_source_sha():

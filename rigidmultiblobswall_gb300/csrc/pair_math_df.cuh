@@ -207,6 +207,9 @@ __device__ __forceinline__ void pair_rpy_df(df dx, df dy, df dz, df vx, df vy, d
 // r = 2 .. 350 a).  Bounds used by the
 // ordered sums: heights >= 1 (clamped by the wall regularisation), so k >= 1,
 // Rz >= 2, u <= 1/4, E <= 1.
+// p is held times kDfP and its partners (Y, Z, w5, ...) by 1 / kDfP, both
+// exact: s^5 loses its low part 10^6 radii above the wall and vanishes at
+// 10^8, while p Z and p w5 stay of the order of s and s^3.
 template <class D> struct UFBlockDF {
     D Af, b2, t3, t4, zz;
 };
@@ -249,8 +252,9 @@ __device__ __forceinline__ void uf_near_df(df2 r2, df2 invr, df2 &ia, df2 &a3, d
 // h4 = 4 h_i, hj, Rz = h_i + h_j (may be unnormalised).  ZPER: dz is an
 // image's and not h_i - h_j (= dw), so R^2 and the wall parts of G and zz are
 // formed from the heights.
+constexpr float kDfP = 0x1p64f;
 template <class D> struct PairGeoDF {
-    D r2, invr, i2, s, u, t, p;
+    D r2, invr, i2, s, u, t, p;  // p = kDfP s^5
 };
 template <class D, bool ZPER = false>
 __device__ __forceinline__ PairGeoDF<D> pair_geo_df(D dx, D dy, D dz, D Rz, D h4, D hj)
@@ -263,7 +267,7 @@ __device__ __forceinline__ PairGeoDF<D> pair_geo_df(D dx, D dy, D dz, D Rz, D h4
     g.i2 = sqr(g.invr);
     g.u = sqr(g.s);
     g.t = mul_u(g.u, g.s);
-    g.p = mul_u(g.t, g.u);
+    g.p = mul_u(g.t, scale2(g.u, kDfP));
     return g;
 }
 
@@ -276,15 +280,16 @@ __device__ __forceinline__ UFBlockDF<D> uf_block_df(const PairGeoDF<D> &g, D dz,
     uf_near_df(g.r2, g.invr, ia, a3, Bc);
     const D z2 = sqr_u(Rz);
     const D E = mul_u(z2, u);
-    const D w5 = add_fast_u(add_fast_u(mul_u(z2, 3.0f), 1.0f), mul_u(E, -5.0f));  // 1 + 3 Rz^2 - 5 E
-    const D w7 = add_fast_u(w5, scale2(E, -2.0f));
+    constexpr float P = 1.0f / kDfP;
+    const D w5 = add_fast_u(add_fast_u(mul_u(z2, 3.0f * P), P), mul_u(E, -5.0f * P));  // P (1 + 3 Rz^2 - 5 E)
+    const D w7 = add_fast_u(w5, scale2(E, -2.0f * P));
     const D al = add_fast_u(mul_u(k4, 0.75f), 1.0f);  // 1 + 3 k
     UFBlockDF<D> m;
     m.Af = add_u(add_u(mul_u(sub_u(ia, s), 1.5f), a3), sub_u(mul_u(p, w5), mul_u(al, t)));
     const D F = add_u(Bc, mul_u(t, -1.5f));
-    const D Y = add_fast_u(mul_u(al, 3.0f), mul_u(mul_u(u, w7), -5.0f));
+    const D Y = add_fast_u(mul_u(al, 3.0f * P), mul_u(mul_u(u, w7), -5.0f));  // P times Y, and so on
     m.b2 = add_u(F, mul_u(p, Y));
-    const D Y10 = add_fast_u(Y, mul_u(u, -10.0f));
+    const D Y10 = add_fast_u(Y, mul_u(u, -10.0f * P));
     const D X = mul_u(mul_u(Rz, p), Y10);
     D G = mul_u(dz, F);  // dz F
     D dG = mul_u(dz, G);  // dz^2 F
@@ -295,7 +300,7 @@ __device__ __forceinline__ UFBlockDF<D> uf_block_df(const PairGeoDF<D> &g, D dz,
     }
     m.t3 = sub_u(G, X);
     m.t4 = add_u(G, X);
-    const D Z = add_fast_u(mul_u(z2, add_u(add_fast_u(6.0f, mul_u(u, -20.0f)), Y10)), 4.0f);
+    const D Z = add_fast_u(mul_u(z2, add_u(add_fast_u(6.0f * P, mul_u(u, -20.0f * P)), Y10)), 4.0f * P);
     m.zz = sub_u(add_u(m.Af, dG), mul_u(p, Z));
     return m;
 }
@@ -439,20 +444,20 @@ __device__ __forceinline__ void wt_near(df2 r2, df2 invr, df2 &A, df2 &Bc)
 template <bool UF32 = false>
 __device__ __forceinline__ RotBlockDF2 rot_block_df(const PairGeoDF<df2> &g, df2 dz, df2 Rz, df2 hi, df2 hj)
 {
-    constexpr float q = UF32 ? 1.5f : 1.0f;
+    constexpr float q = UF32 ? 1.5f : 1.0f, P = 1.0f / kDfP;  // y, R6, R10 times P
     df2 c = mul_u(g.i2, g.invr);
     rot_near_c(g.r2, g.invr, c);
     const df2 Ru = mul_u(Rz, g.u);
-    const df2 y = add_u(mul_u(mul_u(Rz, Ru), -10.0f * q), df2_dup(df_from(2.0f * q)));
+    const df2 y = add_u(mul_u(mul_u(Rz, Ru), -10.0f * q * P), df2_dup(df_from(2.0f * q * P)));
     RotBlockDF2 k;
     k.b = g.t - c;
     if constexpr (UF32) k.b = mul_u(k.b, 1.5f);
-    const df2 m = mul_u(dz, k.b), Rp = mul_u(Rz, g.p), n = UF32 ? mul_u(Rp, 3.0f) : scale2(Rp, 2.0f);
+    const df2 m = mul_u(dz, k.b), Rp = mul_u(Rz, g.p), n = UF32 ? mul_u(Rp, 3.0f * P) : scale2(Rp, 2.0f * P);
     k.a = sub_u(n, m);
     k.ar = add_u(n, m);
-    const df2 R10 = mul_u(Ru, 10.0f * q), R6 = mul_u(Rz, 6.0f * q);
-    k.ei = mul_u(g.p, sub_u(R10, mul_u(hi, 6.0f * q)));
-    k.ej = mul_u(g.p, sub_u(R10, mul_u(hj, 6.0f * q)));
+    const df2 R10 = mul_u(Ru, 10.0f * q * P), R6 = mul_u(Rz, 6.0f * q * P);
+    k.ei = mul_u(g.p, sub_u(R10, mul_u(hi, 6.0f * q * P)));
+    k.ej = mul_u(g.p, sub_u(R10, mul_u(hj, 6.0f * q * P)));
     k.wi = add_u(k.b, mul_u(g.p, add_u(y, mul_u(R6, hi))));
     k.wj = add_u(k.b, mul_u(g.p, add_u(y, mul_u(R6, hj))));
     return k;
@@ -461,7 +466,7 @@ __device__ __forceinline__ RotBlockDF2 rot_block_df(const PairGeoDF<df2> &g, df2
 template <bool UF32 = false>
 __device__ __forceinline__ UFBlockDF<df2> wt_block_df(const PairGeoDF<df2> &g, df2 dz, df2 Rz)
 {
-    constexpr float q = UF32 ? 1.5f : 1.0f;
+    constexpr float q = UF32 ? 1.5f : 1.0f, P = 1.0f / kDfP;
     const df2 i3 = mul_u(g.i2, g.invr);
     df2 A = scale2(i3, -0.5f), Bc = mul_u(mul_u(g.i2, i3), 1.5f);
     wt_near(g.r2, g.invr, A, Bc);
@@ -472,8 +477,8 @@ __device__ __forceinline__ UFBlockDF<df2> wt_block_df(const PairGeoDF<df2> &g, d
     const df2 Et = mul_u(mul_u(sqr_u(Rz), g.u), g.t);
     UFBlockDF<df2> m;
     m.Af = add_u(add_u(A, mul_u(g.t, 3.5f * q)), mul_u(Et, -6.0f * q));
-    m.b2 = add_u(Bc, mul_u(g.p, -4.5f * q));
-    const df2 D = mul_u(Bc, dz), X = mul_u(mul_u(g.p, Rz), 1.5f * q);
+    m.b2 = add_u(Bc, mul_u(g.p, -4.5f * q * P));
+    const df2 D = mul_u(Bc, dz), X = mul_u(mul_u(g.p, Rz), 1.5f * q * P);
     m.t3 = sub_u(D, X);
     m.t4 = add_u(D, X);
     m.zz = add_u(add_u(A, mul_u(g.t, 0.5f * q)), add_u(mul_u(Et, -1.5f * q), mul_u(D, dz)));
