@@ -567,8 +567,9 @@ __global__ void __launch_bounds__(kFtSymTile) ft_sym_fp64_kernel(const FtSrcD *_
     const bool diag = (T == S);
     const int i = T * kFtSymTile + tid;
     const bool valid_i = i < n;
-    // a target or source past the end is a dummy far above the wall with zero vectors
-    const FtSrcD dummy = {1.0e6, 1.0e6, 1.0e6, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    // a target or source past the end is a dummy with zero vectors half a radius above the wall, where no blob is
+    // (heights are at least 1; a dummy on a blob's place would make its products NaN)
+    const FtSrcD dummy = {0.0, 0.0, 0.5, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     const FtSrcD me = valid_i ? src[i] : dummy;
     bool in_range = int_range_vec(me.fx, me.fy, me.fz) && int_range_vec(me.tx, me.ty, me.tz);
     {
@@ -700,7 +701,7 @@ __global__ void __launch_bounds__(kFtF2Threads, 4) ft_sym_df_kernel(const FtSrcD
     const bool diag = (T == S);
     const int i0 = T * kFtSymTile + tid, i1 = i0 + kFtF2Threads;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    const FtSrcDF dummy = {make_float4(1.0e6f, 1.0e6f, 1.0e6f, 0.f), zero, zero, zero, zero, zero};
+    const FtSrcDF dummy = {make_float4(0.f, 0.f, 0.5f, 0.f), zero, zero, zero, zero, zero};
     FtTarget me;
     {
         const FtSrcDF a = i0 < n ? src[i0] : dummy, b = i1 < n ? src[i1] : dummy;

@@ -322,6 +322,9 @@ __device__ __forceinline__ void sym_band_pair(long long b, int nt, const SymBand
 constexpr int kF2Threads = kTile / 2;
 constexpr int kF2Group = 8;
 
+// where no user puts a blob: three coordinates in radii, exact in FP32
+__device__ constexpr float kFreeDummy[3] = {1048603.375f, -1047481.125f, 1049887.625f};
+
 struct F2Target {
     df2 x, y, z, h4, qx, qy, qz;  // positions, 4 z, b v of both targets
 };
@@ -404,9 +407,12 @@ __device__ __forceinline__ void df_f2_body(const SrcDF *__restrict__ src, int n,
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool diag = (T == S);
     const int i0 = T * kTile + tid, i1 = i0 + kF2Threads;
-    // a target or source past the end is a dummy far above the wall with a zero vector
-    const SrcDF dummy = {make_float4(1.0e6f, 1.0e6f, 1.0e6f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f),
-                         make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+    // a target or source past the end is a dummy with a zero vector, half a radius above the wall, where no blob is
+    // (heights are at least 1; a dummy on a blob's place would make its products NaN); without a wall, somewhere
+    const SrcDF dummy = {NOWALL ? make_float4(kFreeDummy[0], kFreeDummy[1], kFreeDummy[2], 0.f)
+                                : make_float4(0.f, 0.f, 0.5f, 0.f),
+                         make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f),
+                         make_float4(0.f, 0.f, 0.f, 0.f)};
     F2Target me;
     {
         const SrcDF a = i0 < n ? src[i0] : dummy, b = i1 < n ? src[i1] : dummy;
@@ -884,8 +890,9 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
     const bool diag = (T == S);
     const int i = T * kTile + tid;
     const bool valid_i = i < n;
-    // a target or source past the end is a dummy far above the wall with a zero vector
-    const SrcD dummy = {1.0e6, 1.0e6, 1.0e6, 0.0, 0.0, 0.0, 0.0, 0.0};
+    // a target or source past the end is a dummy with a zero vector (as in df_f2_body)
+    const SrcD dummy = {NOWALL ? kFreeDummy[0] : 0.0, NOWALL ? kFreeDummy[1] : 0.0,
+                        NOWALL ? kFreeDummy[2] : 0.5 / inva, 0.0, 0.0, 0.0, 0.0, 0.0};
     const SrcD me = valid_i ? src[i] : dummy;
     const double hi = me.z * inva;  // the height in radii (free space: inva = 1, positions over a)
     bool in_range = int_range_vec(me.vx, me.vy, me.vz);

@@ -1,0 +1,27 @@
+"""GPU: products that do not fill their last tile of 128 blobs, with a blob at a round position far from the others:
+nothing that stands in for the missing blobs may meet it."""
+import numpy as np
+import pytest
+
+from conftest import rel_err
+from oracle import wall as owall
+from rigidmultiblobswall_gb300 import mobility as mob
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("mode", ["fp64", "df64"])
+@pytest.mark.parametrize("at", [(1e6, 1e6, 1e6), (0.0, 0.0, 0.5), (0.0, 0.0, 1.0)])
+def test_blob_at_a_round_position(cuda_device, mode, at):
+    n, a = 300, 1.0
+    rng = np.random.default_rng(6)
+    r = np.column_stack([rng.uniform(5, 60, n), rng.uniform(5, 60, n), rng.uniform(1.0, 9.0, n)])
+    r[17] = at
+    v, t = rng.standard_normal(3 * n), rng.standard_normal(3 * n)
+    for kind in ("uf", "ut", "wf", "wt"):
+        ref = owall.wall_product(kind, r, v, 1.0, a)
+        assert rel_err(mob.wall_product(kind, r, v, 1.0, a, mode=mode), ref) <= 1e-12
+        ref = owall.no_wall_product(kind, r, v, 1.0, a)
+        assert rel_err(mob.no_wall_product(kind, r, v, 1.0, a, mode=mode), ref) <= 1e-12
+    for got, ref in zip(mob.wall_force_torque(r, v, t, 1.0, a, mode=mode), owall.force_torque(r, v, t, 1.0, a)):
+        assert rel_err(got, ref) <= 1e-12
