@@ -148,14 +148,21 @@ __device__ __forceinline__ bool int_range_sep(double dx, double dy, double dz)
     const uint32_t a = (uint32_t)__double2hiint(dx) & 0x7fffffffu, b = (uint32_t)__double2hiint(dy) & 0x7fffffffu;
     return max(max(a, b), (uint32_t)__double2hiint(dz) & 0x7fffffffu) < (1055u << 20);
 }
-// zero or 2^-300 <= |v| < 2^300, for vectors: their products with separations and blocks stay normal
-__device__ __forceinline__ bool int_range_vec(double v)
+// zero or 2^-E <= |v| < 2^300.  Factors below 2^-400 count as zero, so what the pair kernels multiply has to stay above:
+// coordinates (E = 130) differ by nothing or by 2^-182, separations in radii are 2^-246 at least, their products
+// with vectors (E = 150) 2^-396.
+template <int E = 300> __device__ __forceinline__ bool int_range_vec(double v)
 {
-    return ((uint32_t)__double2hiint(v) & 0x7fffffffu) - (723u << 20) < (600u << 20) || v == 0.0;
+    return ((uint32_t)__double2hiint(v) & 0x7fffffffu) - ((uint32_t)(1023 - E) << 20) < ((uint32_t)(300 + E) << 20) ||
+           v == 0.0;
 }
-__device__ __forceinline__ bool int_range_vec(double x, double y, double z)
+template <int E = 300> __device__ __forceinline__ bool int_range_vec(double x, double y, double z)
 {
-    return int_range_vec(x) && int_range_vec(y) && int_range_vec(z);
+    return int_range_vec<E>(x) && int_range_vec<E>(y) && int_range_vec<E>(z);
+}
+__device__ __forceinline__ bool int_range_blob(double x, double y, double z, double vx, double vy, double vz)
+{
+    return int_range_vec<130>(x, y, z) && int_range_vec<150>(vx, vy, vz);
 }
 
 // Products of the pair blocks in plain arithmetic (MulPipe) or on the integer

@@ -571,17 +571,18 @@ __global__ void __launch_bounds__(kFtSymTile) ft_sym_fp64_kernel(const FtSrcD *_
     // (heights are at least 1; a dummy on a blob's place would make its products NaN)
     const FtSrcD dummy = {0.0, 0.0, 0.5, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     const FtSrcD me = valid_i ? src[i] : dummy;
-    bool in_range = int_range_vec(me.fx, me.fy, me.fz) && int_range_vec(me.tx, me.ty, me.tz);
+    bool in_range = int_range_blob(me.x, me.y, me.z, me.fx, me.fy, me.fz) && int_range_vec<150>(me.tx, me.ty, me.tz);
     {
         const int j = S * kFtSymTile + tid;
         const FtSrcD q = (j < n) ? src[j] : dummy;
         const double c[9] = {q.x, q.y, q.z, q.fx, q.fy, q.fz, q.tx, q.ty, q.tz};
         for (int k = 0; k < 9; ++k) sx[k][tid] = c[k];
-        in_range = in_range && int_range_vec(q.fx, q.fy, q.fz) && int_range_vec(q.tx, q.ty, q.tz);
+        in_range = in_range && int_range_blob(q.x, q.y, q.z, q.fx, q.fy, q.fz) &&
+                   int_range_vec<150>(q.tx, q.ty, q.tz);
     }
     for (int c = 0; c < NC; ++c)
         for (int k = lane; k < kFtSymTile; k += 32) sacc[warp][c][k] = 0.0;
-    const bool allow = __syncthreads_and(in_range);  // the integer forms, for every vector of the tile pair
+    const bool allow = __syncthreads_and(in_range);  // the integer forms, for every blob of the tile pair
     double u[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     auto step = [&](int k) {
         const int j = (lane + k) & (kFtSymTile - 1);

@@ -895,7 +895,7 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
                         NOWALL ? kFreeDummy[2] : 0.5 / inva, 0.0, 0.0, 0.0, 0.0, 0.0};
     const SrcD me = valid_i ? src[i] : dummy;
     const double hi = me.z * inva;  // the height in radii (free space: inva = 1, positions over a)
-    bool in_range = int_range_vec(me.vx, me.vy, me.vz);
+    bool in_range = int_range_blob(me.x, me.y, me.z, me.vx, me.vy, me.vz);
     {
         const int j = S * kTile + tid;
         const SrcD sj = (j < n) ? src[j] : dummy;
@@ -906,11 +906,11 @@ __device__ __forceinline__ void fp64_sym_body(const SrcD *__restrict__ src, int 
         tvx[tid] = sj.vx;
         tvy[tid] = sj.vy;
         tvz[tid] = sj.vz;
-        in_range = in_range && int_range_vec(sj.vx, sj.vy, sj.vz);
+        in_range = in_range && int_range_blob(sj.x, sj.y, sj.z, sj.vx, sj.vy, sj.vz);
     }
     for (int c = 0; c < 3; ++c)
         for (int k = lane; k < kTile; k += 32) sacc[warp][c][k] = 0.0;
-    // the integer forms, for every vector of the tile pair
+    // the integer forms, for every blob of the tile pair
     const bool allow = __syncthreads_and(in_range && int_range(inva));
     double ux = 0.0, uy = 0.0, uz = 0.0;
     auto step = [&](int k) {
