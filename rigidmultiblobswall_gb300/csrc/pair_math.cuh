@@ -350,7 +350,8 @@ __device__ __forceinline__ PairGeoD pair_geo_d(double r2, double R2)
 // but dummies, coincident blobs and distances beyond 2^32 radii), else the FP64 ones.  ZPER pairs (dz an image's) take
 // the latter.  SCALE: positions are subtracted before they are scaled to radii, so that blobs near each other and far
 // from the origin keep their separation to the last bit (scaled first, it would carry the rounding of x / a); false:
-// scale is 1.  allow also stands for a scale within 2^+-64.  Three integer products a pair: M_UF of 10,752 blobs 3.77 ms,
+// scale is 1.  Every lane of the warp calls this together (the choice of the form is the warp's, and with it the
+// rounding: it must not depend on which lanes happen to run in step).  allow also stands for a scale within 2^+-64.  Three integer products a pair: M_UF of 10,752 blobs 3.77 ms,
 // 4.03 with FP64 multiplies, 3.69 scaled first.
 template <bool ZPER, bool SCALE, class F>
 __device__ __forceinline__ void with_pair_geo_d(double ex, double ey, double ez, double scale, double Rz, double hi,
@@ -360,7 +361,7 @@ __device__ __forceinline__ void with_pair_geo_d(double ex, double ey, double ez,
         const double dx = SCALE ? int_mul_signed(ex, scale) : ex, dy = SCALE ? int_mul_signed(ey, scale) : ey,
                      dz = SCALE ? int_mul_signed(ez, scale) : ez;
         const double q2 = int_fma_pos(dz, dz, int_fma_pos(dx, dx, int_mul_signed(dy, dy)));
-        if (__all_sync(__activemask(), int_range_mag(ex, ey, ez) && int_range_sep(Rz, Rz, Rz) && int_range(q2))) {
+        if (__all_sync(0xffffffffu, int_range_mag(ex, ey, ez) && int_range_sep(Rz, Rz, Rz) && int_range(q2))) {
             f(pair_geo_d<MulInt>(q2, int_fma_pos(4.0 * hi, hj, q2)), dx, dy, dz, MulInt());
             return;
         }
@@ -685,9 +686,9 @@ __device__ __forceinline__ void pair_rpy_sym(T dx, T dy, T dz, T vx, T vy, T vz,
                                              T &uz, T &wx, T &wy, T &wz, bool allow = false)
 {
     if constexpr (std::is_same<T, double>::value) {
-        if (allow) {  // as with_pair_geo_d
+        if (allow) {  // as with_pair_geo_d, by whole warps too
             const double q2 = int_fma_pos(dx, dx, int_fma_pos(dy, dy, int_mul_signed(dz, dz)));
-            if (__all_sync(__activemask(), int_range_sep(dx, dy, dz) && int_range(q2))) {
+            if (__all_sync(0xffffffffu, int_range_sep(dx, dy, dz) && int_range(q2))) {
                 pair_rpy_sym_body<T, KIND, MulInt>(q2, int_rsqrt(q2), dx, dy, dz, vx, vy, vz, qx, qy, qz, ux, uy, uz,
                                                    wx, wy, wz);
                 return;
