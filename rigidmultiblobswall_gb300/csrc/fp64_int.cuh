@@ -13,7 +13,11 @@
 //
 // Error bounds, tested against exact arithmetic: int_mul 0.504 ulp (the
 // product of the low halves, below 2^-62 of the result, and the order of ties
-// are left out), int_fma_pos 0.51 ulp, int_rsqrt 0.51 ulp (the FP64 sequence of rsqrt64: 1 ulp).
+// are left out; the FP64 pipe's 0.5), int_fma_pos 0.51 ulp, int_fma half an
+// ulp and 2^-59 of the larger term (the pipe's: half an ulp, also where the
+// terms cancel; their own roundings are 2^-53 of them), int_rsqrt 0.51 ulp
+// (rsqrt64 1 ulp).  The products' errors against 64 bits are no larger than
+// with the pipe's operations alone.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -62,6 +66,17 @@ __device__ __forceinline__ double int_mul_signed(double a, double b)
     return min(ea, eb) < (623u << 20) ? 0.0 : p;
 }
 
+// 1/sqrt(x) in FP64 from an estimate y of relative error below 2^-20: one
+// third-order Householder step, y + y e (1/2 + 3 e / 8) with e = 1 - x y^2.
+// What the step leaves out is 5/16 e^3 < 2^-57.  The rounding of y^2 moves e by 2^-53 and
+// the result by half an ulp at most, the last fma rounds by another half:
+// 1 ulp, as the library's rsqrt.
+__device__ __forceinline__ double rsqrt64_step(double x, double y)
+{
+    const double e = fma(-x, y * y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
 // 1/sqrt(x) of a positive normal x.  m = x 4^-h in [1, 4); y0 = 1/sqrt(m) to
 // 2^-22 in units 2^-31, e = 1 - m y0^2 and y0 (1 + e/2 + 3 e^2/8), rounded once.
 __device__ __forceinline__ double int_rsqrt(double x)
@@ -84,8 +99,9 @@ __device__ __forceinline__ double int_rsqrt(double x)
     return __hiloint2double((int)((uint32_t)(m >> 32) + ((uint32_t)(1021 - h) << 20)), (int)(uint32_t)m);
 }
 
-// a b + c of non-negative numbers below 2^400 in magnitude (signs ignored; zero allowed), a b and c not both 0: factors
-// or addends 2^62 below the other term count as zero.  0.51 ulp.
+// a b + c of non-negative numbers below 2^400 in magnitude (signs ignored; zero allowed): factors or addends 2^62 below
+// the other term count as zero.  0.51 ulp; 0 0 + 0 is 0 (squares of stacked blobs' separations), and the sum of two
+// zero terms otherwise below 2^-600.
 __device__ __forceinline__ double int_fma_pos(double a, double b, double c)
 {
     uint32_t ah, al, bh, bl, ch, cl;
@@ -105,8 +121,8 @@ __device__ __forceinline__ double int_fma_pos(double a, double b, double c)
 }
 
 // a b + c of finite numbers below 2^400 in magnitude; terms below 2^-400 count
-// as zero.  0.51 ulp where the terms do not cancel, 2^-59 of it
-// where they do.
+// as zero.  Half an ulp and 2^-59 of the larger term, which counts where the
+// terms cancel.
 __device__ __forceinline__ double int_fma(double a, double b, double c)
 {
     const uint32_t ha = (uint32_t)__double2hiint(a), hb = (uint32_t)__double2hiint(b), hc = (uint32_t)__double2hiint(c);

@@ -11,16 +11,14 @@
 namespace rmw {
 
 // 1/sqrt(x) in FP64: the hardware's estimate (relative error below 2^-20) and
-// one third-order Householder step, y + y e (1/2 + 3 e / 8) with
-// e = 1 - x y^2: five FP64 instructions and no special-case branch (zero,
+// rsqrt64_step, five FP64 instructions and no special-case branch (zero,
 // infinite and subnormal x give non-finite values; no pair of distinct blobs
 // has one).
 __device__ __forceinline__ double rsqrt64(double x)
 {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y * y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
+    return rsqrt64_step(x, y);
 }
 
 // pair math.  (dx,dy,dz) = (r_i - r_j)/a; Rz = (z_i + z_j)/a; hi = z_i/a; hj = z_j/a.
