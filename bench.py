@@ -60,9 +60,9 @@ DF64_UF_INST_PER_PAIR = {"symmetric": 1103357190.0 * 32 / 10752 ** 2, "standard"
 # dram__bytes_read.sum + dram__bytes_write.sum per launch, same captures
 DF64_UF_TRAFFIC_BYTES = {"symmetric": 771584, "standard": 711168}
 # FP32-issue slots per pair and right-hand side of the 16-wide multi-RHS M_UF kernel, packed instructions
-# counted twice as above ((smsp__inst_executed.sum 17,258,189,476 + packed 12,838,677,918) * 32 / (N^2 * 16),
+# counted twice as above ((smsp__inst_executed.sum 17,225,517,484 + packed 12,782,367,918) * 32 / (N^2 * 16),
 # 60,000 blobs)
-MULTI16_INST_PER_PAIR_RHS = 16.72
+MULTI16_INST_PER_PAIR_RHS = 16.67
 DF64_UF_KERNEL_SOURCE_SHA = "57e3f9b2d1ec21db37a9843619c3b783ea039af8bc6ce46ea81bb5cba1b92f6b"
 
 

@@ -220,7 +220,6 @@ __device__ __forceinline__ void uf_apply(const UFCoeffs &c, float dx, float dy, 
 // the scalar form came out as in every second step of an unrolled loop.
 struct UFCoeffs2 {
     f2 Af, Bc, c2, c3, c4, Af5;
-    f2 g, u;  // c2 = g u
 };
 __device__ __forceinline__ f2 f2_c(float a, f2 b, f2 c) { return f2_fma(f2_dup(a), b, c); }  // a b + c
 __device__ __forceinline__ f2 f2_c(float a, f2 b, float c) { return f2_fma(f2_dup(a), b, f2_dup(c)); }
@@ -264,12 +263,10 @@ __device__ __forceinline__ UFCoeffs2 uf_coeffs_f2(f2 dx, f2 dy, f2 dz, f2 Rz, f2
     UFCoeffs2 c;
     c.Af = f2_sub(A, g1);
     c.Bc = Bc;
-    c.c2 = f2_mul(f2c, u);
+    c.c2 = f2_mulr(f2c, u);
     c.c3 = f2_fma(Ru, in, f2_fma(f2_neg(f2_mul(f2_s(18.0f, hh), Rz)), t, hjt3));
     c.c4 = f2_fma(f2_neg(f2_s(10.0f, Ru)), p, hjt3);
     c.Af5 = f2_c(-2.0f, f5, c.Af);
-    c.g = f2c;
-    c.u = u;
     return c;
 }
 
@@ -292,15 +289,14 @@ __device__ __forceinline__ void uf_apply_f2(const UFCoeffs2 &c, f2 c3, f2 c4, f2
 //   M = Af I + Bc d d^T + c2 e e^T + c3 e z^T + c4 z e^T + f5 z z^T,
 // so M_xy = M_yx = (Bc + c2) dx dy, M_xz = dx t3, M_zx = dx t4 with
 // t3,4 = Bc dz + c2 Rz + c3,4, and M_zz = Af + f5 + Bc dz^2 + (c2 Rz + c3 + c4) Rz.
-// Two pairs (sources) in packed lanes; Bc + c2 with c2's product fused into it.
+// Two pairs (sources) in packed lanes.
 struct UFBlock2 {
     f2 xx, xy, xz, yy, yz, zx, zy, zz;  // M_yx = M_xy
 };
 
-template <bool FUSED_B>
 __device__ __forceinline__ UFBlock2 uf_block_f2(const UFCoeffs2 &c, f2 dx, f2 dy, f2 dz, f2 Rz)
 {
-    const f2 b2 = FUSED_B ? f2_fma(c.g, c.u, c.Bc) : f2_add(c.Bc, f2_mulr(c.g, c.u));
+    const f2 b2 = f2_add(c.Bc, c.c2);
     const f2 t = f2_fma(c.Bc, dz, f2_mul(c.c2, Rz));
     const f2 t3 = f2_add(t, c.c3), t4 = f2_add(t, c.c4);
     const f2 px = f2_mul(b2, dx);

@@ -1260,12 +1260,12 @@ __global__ void pack_multi_kernel(const double *__restrict__ r, const double *__
 // tile may contain the target itself, whose pair block is zeroed (the self
 // term is added by the finalize kernel).  The positions of sources k, k + 1
 // are three float4: hx hx' hy hy', hz hz' lx lx', ly ly' lz lz'.
-// FUSED_R2 / FUSED_B: uf_coeffs_f2, uf_block_f2 (the operations of the scalar
-// kernel this replaced, in its order: the same products to the bit).
+// The operations of the scalar kernel this replaced, in its order: the same
+// products to the bit.
 // Measured, 30,000 blobs x 16: 8.18 -> 7.51 ms, 20,000 x 8: 2.54 -> 2.30 ms;
 // issue slots bounded the scalar form (79 % active), the FMA pipe this one
 // (76 %, three-operand 64-bit reads).
-template <bool DIAG, int NR, bool FUSED_R2, bool FUSED_B>
+template <bool DIAG, int NR>
 __device__ __forceinline__ void multi_tile(const float4 *tpos, const float4 *tvec, int cnt, int t0, int i, float4 mh,
                                            float4 ml, float hi, f2 (&acc)[NR / 2][3])
 {
@@ -1278,12 +1278,12 @@ __device__ __forceinline__ void multi_tile(const float4 *tpos, const float4 *tve
         const f2 dz = f2_add(f2_sub(f2_dup(mh.z), hz), f2_sub(f2_dup(ml.z), lz));
         const f2 hj = f2_add(hz, lz);
         const f2 Rz = f2_add(f2_dup(hi), hj);
-        UFCoeffs2 c = uf_coeffs_f2<FUSED_R2>(dx, dy, dz, Rz, f2_dup(hi), hj);
+        UFCoeffs2 c = uf_coeffs_f2<false>(dx, dy, dz, Rz, f2_dup(hi), hj);
         if (DIAG) {  // finite inputs
-            if (t0 + k == i) c.Af.x = c.Bc.x = c.c2.x = c.c3.x = c.c4.x = c.Af5.x = c.g.x = 0.f;
-            if (t0 + k + 1 == i) c.Af.y = c.Bc.y = c.c2.y = c.c3.y = c.c4.y = c.Af5.y = c.g.y = 0.f;
+            if (t0 + k == i) c.Af.x = c.Bc.x = c.c2.x = c.c3.x = c.c4.x = c.Af5.x = 0.f;
+            if (t0 + k + 1 == i) c.Af.y = c.Bc.y = c.c2.y = c.c3.y = c.c4.y = c.Af5.y = 0.f;
         }
-        const UFBlock2 m = uf_block_f2<FUSED_B>(c, dx, dy, dz, Rz);
+        const UFBlock2 m = uf_block_f2(c, dx, dy, dz, Rz);
         const float4 *vk = tvec + k * (3 * NR / 4);
         auto apply = [&](const UFBlock2 &w, const float4 *v) {
             // z, then y, then x terms of every right-hand side: consecutive FMAs share the block's entry
@@ -1371,8 +1371,8 @@ __global__ void __launch_bounds__(kThreads, 3) wall_pair_multi_kernel(const SrcF
         for (int q = 0; q < NR / 2; ++q) acc2[q][0] = acc2[q][1] = acc2[q][2] = f2_dup(0.f);
         // only a tile that overlaps the CTA's targets can hold a self pair
         if (t0 < pr.tend && t0 + cnt > pr.tbeg)
-            multi_tile<true, NR, false, false>(tpos, tvec, cnt, t0, i, mh, ml, hi, acc2);
-        else multi_tile<false, NR, false, false>(tpos, tvec, cnt, t0, i, mh, ml, hi, acc2);
+            multi_tile<true, NR>(tpos, tvec, cnt, t0, i, mh, ml, hi, acc2);
+        else multi_tile<false, NR>(tpos, tvec, cnt, t0, i, mh, ml, hi, acc2);
 #pragma unroll
         for (int q = 0; q < NR; ++q)
 #pragma unroll
