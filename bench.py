@@ -48,22 +48,22 @@ NF_ALL_EXACT_R = NF_CUTOFF_R
 # instruction counted as the two lanes' operations it does on the FMA pipe
 # (which takes it two clocks).  Symmetric kernel (each unordered pair once,
 # two targets per thread in packed lanes): smsp__inst_executed.sum
-# 589,269,016 + packed (pipe_fmaheavy + pipe_fmalite - pipe_fma) 514,088,174
-# = 1,103,357,190 warp instructions * 32 / 10752^2 = 305.4; one-sided kernel
+# 589,061,956 + packed (pipe_fmaheavy + pipe_fmalite - pipe_fma) 514,088,174
+# = 1,103,150,130 warp instructions * 32 / 10752^2 = 305.4; one-sided kernel
 # (source split 15) 1,811,251,044 * 32 / 10752^2 = 501.4.  The FP32 pipe takes
 # at most one thread instruction per lane per clock, the rate the FMA-chain
 # probe measures (FLOP/s / 2), so achieved / peak is the fraction of that
 # capacity used.  The constants hold for the kernel sources whose hash is
 # DF64_UF_KERNEL_SOURCE_SHA (tests/test_bench_constants.py fails when the
 # kernel changes without a new capture).
-DF64_UF_INST_PER_PAIR = {"symmetric": 1103357190.0 * 32 / 10752 ** 2, "standard": 1811251044.0 * 32 / 10752 ** 2}
+DF64_UF_INST_PER_PAIR = {"symmetric": 1103150130.0 * 32 / 10752 ** 2, "standard": 1811251044.0 * 32 / 10752 ** 2}
 # dram__bytes_read.sum + dram__bytes_write.sum per launch, same captures
-DF64_UF_TRAFFIC_BYTES = {"symmetric": 771584, "standard": 711168}
+DF64_UF_TRAFFIC_BYTES = {"symmetric": 758784, "standard": 710912}
 # FP32-issue slots per pair and right-hand side of the 16-wide multi-RHS M_UF kernel, packed instructions
 # counted twice as above ((smsp__inst_executed.sum 17,225,517,484 + packed 12,782,367,918) * 32 / (N^2 * 16),
 # 60,000 blobs)
 MULTI16_INST_PER_PAIR_RHS = 16.67
-DF64_UF_KERNEL_SOURCE_SHA = "57e3f9b2d1ec21db37a9843619c3b783ea039af8bc6ce46ea81bb5cba1b92f6b"
+DF64_UF_KERNEL_SOURCE_SHA = "9c7434a56055c983c69002d3d3fdeeeabbba395778a782db36f8f7934762ba57"
 
 
 def df64_uf_kernel_source_sha():

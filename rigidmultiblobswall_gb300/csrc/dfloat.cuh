@@ -283,6 +283,21 @@ __device__ __forceinline__ bool operator>=(df a, float b) { return a.hi > b || (
 
 __device__ __forceinline__ double to_double(df a) { return (double)a.hi + (double)a.lo; }
 
+// a + b + c + d in FP64: the high parts' exact sum and its three errors with
+// the low parts in double-float, on the FP32 pipe, so that only three
+// conversions and two additions take the FP64 pipe (15 as four to_double).
+__device__ __forceinline__ double sum4_to_double(df a, df b, df c, df d)
+{
+    const df p = two_sum_df(a.hi, b.hi), q = two_sum_df(c.hi, d.hi), s = two_sum_df(p.hi, q.hi);
+    df r = two_sum_df(p.lo, q.lo);
+    acc_add(r, df_from(s.lo));
+    acc_add(r, df_from(a.lo));
+    acc_add(r, df_from(b.lo));
+    acc_add(r, df_from(c.lo));
+    acc_add(r, df_from(d.lo));
+    return (double)s.hi + ((double)r.hi + (double)r.lo);
+}
+
 // double -> double-float (round hi, exact remainder in lo)
 __device__ __forceinline__ df df_of_double(double d)
 {

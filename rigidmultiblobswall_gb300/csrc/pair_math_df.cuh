@@ -318,13 +318,9 @@ __device__ __forceinline__ void uf_block_acc_df(const UFBlockDF<D> &m, D t3, D t
 }
 
 // ---------------------------------------------------------------------------
-// Symmetric forms of the rotation blocks.  With d = r_i - r_j, M_ji is the
-// same formula as M_ij with d -> -d and h_i <-> h_j (the grand mobility is
-// symmetric, M_ji = M_ij^T): the WT coefficients do not involve the heights,
-// so its reverse block only flips d; the UT and WF coefficients depend on one
-// height (UT: the target's, WF: the source's), so both height sets are formed
-// and the reverse block uses the other one.  Shared per pair: the distances,
-// both reciprocal square roots and the powers of s = 1/|R|.
+// The rotation blocks in tensor form, for the one-sided kernels: the UT
+// coefficients take the target's height, the WF ones the source's, WT has
+// none.
 
 // The height-dependent coefficients of UT / WF for height h (unnormalised
 // where only a sum consumes them).
@@ -398,7 +394,7 @@ __device__ __forceinline__ void wt_apply_df(df Af, df Bc, df s5, df dx, df dy, d
 //   Af = A + 7t/2 - 6 E t,  b2 = Bc - 9p/2,  t3,4 = Bc dz -+ 3/2 p Rz,
 //   zz = A + t/2 - 3/2 E t + Bc dz^2     (A = -1/(2 r^3), Bc = 3/(2 r^5)).
 // About 500 FP32-pipe operations a pair against 720 (WT) and 840 (UT, WF) of
-// the tensor forms below.
+// the tensor forms above applied both ways.
 struct RotBlockDF2 {
     df2 a, ar, b, ei, ej, wi, wj;
 };

@@ -780,11 +780,9 @@ __global__ void __launch_bounds__(kFtF2Threads, 4) ft_sym_df_kernel(const FtSrcD
         const int l = tid + half * kFtF2Threads, i = T * kFtSymTile + l, j = S * kFtSymTile + l;
         for (int c = 0; c < NC; ++c) {
             const double t = tacc[half][c][tid];
-            double q = 0.0;
-            for (int w = 0; w < kFtF2Threads / 32; ++w) {
-                const float4 f = sacc[w][c][l];
-                q += to_double(df{f.x, f.z}) + to_double(df{f.y, f.w});
-            }
+            static_assert(kFtF2Threads == 64, "two warps' sums, two lanes each");
+            const float4 f = sacc[0][c][l], g = sacc[1][c][l];
+            const double q = sum4_to_double({f.x, f.z}, {f.y, f.w}, {g.x, g.z}, {g.y, g.w});
             const size_t comp = (c / 3) * 3 * (size_t)n + c % 3;
             if (i < n) partial[sp.slot(diag ? T : S) * 6 * n + 3 * (size_t)i + comp] = diag ? t + q : t;
             if (!diag && j < n) partial[sp.slot(T) * 6 * n + 3 * (size_t)j + comp] = q;

@@ -314,8 +314,8 @@ __device__ __forceinline__ void sym_band_pair(long long b, int nt, const SymBand
 // source-side sums are float4 (hi x, hi y, lo x, lo y) per warp, component
 // and source; the target-side ones are renormalised every kF2Group steps and
 // folded into FP64 sums (in shared memory) every kDfGroup, and the warps'
-// source-side sums are added in FP64 (0.4 % of the time; double-float sums of
-// the whole tile: error 5.64e-14 instead of 5.57e-14 at 10,752 blobs).
+// source-side sums are added to FP64 accuracy (0.4 % of the time; double-float
+// sums of the whole tile: error 5.64e-14 instead of 5.57e-14 at 10,752 blobs).
 // Measured (pair kernel): 10,752 blobs 1.63 -> 0.99 ms, FMA pipe 86 % active,
 // issue 48 %; the product at 172,032 blobs 400 -> 240 ms.  128 registers (8 CTAs per SM) are
 // 2 % faster than the 158 that one CTA takes unbounded.
@@ -493,12 +493,15 @@ __device__ __forceinline__ void df_f2_body(const SrcDF *__restrict__ src, int n,
         double own[3], s[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            double q = 0.0;
-#pragma unroll
-            for (int w = 0; w < kF2Threads / 32; ++w) {
-                const float4 f = sacc[w][c][l];
-                q += to_double(df{f.x, f.z}) + to_double(df{f.y, f.w});
-            }
+            static_assert(kF2Threads == 64, "two warps' sums, two lanes each");
+            const float4 f = sacc[0][c][l], g = sacc[1][c][l];
+            double q;
+            // split tile pairs end often (1,000 blobs 51 -> 40 us); whole ones keep the form their loop schedules
+            // best with (10,752 blobs M_UF 1,008 us, 1,039 with the other)
+            if constexpr (WHOLE)
+                q = to_double(df{f.x, f.z}) + to_double(df{f.y, f.w}) +
+                    (to_double(df{g.x, g.z}) + to_double(df{g.y, g.w}));
+            else q = sum4_to_double({f.x, f.z}, {f.y, f.w}, {g.x, g.z}, {g.y, g.w});
             own[c] = tacc[half][c][tid] + (diag ? q : 0.0);
             s[c] = q;
         }
@@ -1749,8 +1752,9 @@ static void launch_sym_finalize(const double *r, const double *v, const double *
 }
 
 // The FP64 product periodic in x and / or y through the symmetric kernel.
-// Measured, M_UF of 1,500 blobs in a square box: one-sided 2.94, symmetric
-// 1.62 ms (FP64 pipe floor 1.5); the images of a pair share its minimum-image division.
+// M_UF of 1,500 blobs in a square box: one-sided 2.94, symmetric 1.62 ms with
+// every operation on the FP64 pipe, 0.92 with the integer forms; the images of
+// a pair share its minimum-image division.
 template <int KIND>
 static int per_sym_product(const double *r, const double *v, double *out, int n, double a, double nf, const double *L,
                            cudaStream_t st, void *scratch_ptr, int nsplit)
