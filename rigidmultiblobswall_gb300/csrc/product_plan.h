@@ -20,34 +20,38 @@ inline double sym_slot_bytes(int n, int comps) { return (double)sym_tiles(n) * c
 // How many CTAs share the steps of a tile pair.  Below about 4,000 blobs the
 // tile pairs alone leave SMs idle (2,048 blobs: 136 of them); the split fills
 // the GPU with the symmetric kernel's work per pair where the one-sided kernel
-// used to do each pair twice (2,048 blobs: FP64 UF 961 -> 364 us, df64 181 ->
-// 70).  With P tile pairs, s CTAs each and a CTA's start and end worth e steps,
+// used to do each pair twice (2,048 blobs: FP64 UF 961 -> 189 us, df64 181 ->
+// 71).  With P tile pairs, s CTAs each and a CTA's start and end worth e steps,
 // an SM takes (P s / 152 + d)(128 / s + e) step times, d the uneven end of the
-// grid: least at s = sqrt(152 * 128 d / (e P)).  Measured by s: df64 UF 2,048
-// blobs 8: 72, 16: 74, 32: 81 us; 5,003 blobs 2: 275, 4: 259, 8: 279 us; FP64
-// UF 10,752 blobs 1: 8.24, 2: 8.08 ms; FP64 periodic 4,800 blobs 2: 15.2,
-// 8: 14.8 ms, which K = 13,000 (df64), 40,000 (FP64) and 160,000 (periodic
-// FP64, whose steps are nine times as long) in s = sqrt(K / P) reproduce.
-// Where even 64 CTAs per pair are fewer than 16 per SM, the split whose
-// busiest SM has least to do (504 blobs FP64: 43, 48 us; 32: 54 us).
+// grid: least at s = sqrt(152 * 128 d / (e P)) = sqrt(K / P).  Measured by s,
+// us: FP64 UF 2,048 blobs 8: 191, 10: 189, 12: 192, 17: 199; 3,000 4: 372,
+// 6: 370, 8: 374, 12: 383; 5,003 3: 942, 4: 929, 6: 940, 7: 948; 10,752
+// 1: 3,769, 2: 3,735, 3: 3,732.  df64 UF 1,000 blobs 8: 38, 16: 39, 22: 44,
+// 32: 50; 2,048 4: 69, 9: 71, 16: 77; 5,003 2: 281, 3: 270, 4: 266, 6: 270;
+// 10,752 1: 1,009, 2: 1,027.  FP64 periodic, whose steps are nine times as
+// long: 1,500 blobs 16: 957, 32: 910, 43: 906, 64: 923; 4,800 4: 7,961,
+// 8: 7,830, 14: 7,836.  K = 13,000, periodic 145,000, reproduces them.
+// Where even 64 CTAs per pair are fewer than 16 per SM (up to 1,024 blobs), in
+// FP64 the split whose busiest SM has least to do (504 blobs 26: 41.5,
+// 32: 43.0, 43: 38.8, 64: 48.0; 1,000 8: 75, 16: 71, 32: 80).
 inline int sym_split_rule(bool fp64, bool periodic, int n)
 {
     const double nt = (double)sym_tiles(n), pairs = 0.5 * nt * (nt + 1);
     int s = 1;
-    if (pairs * kSplitMax < 16 * 152.0) {
-        const double ends = periodic ? 0.05 : fp64 ? 0.4 : 1.2, fill = fp64 ? 2.0 : 6.0;
+    if (fp64 && pairs * kSplitMax < 16 * 152.0) {
+        const double ends = periodic ? 0.05 : 0.4;
         double cost = 0.0;
         for (int c = 1; c <= kSplitMax; ++c) {
             const double t =
-                std::max(std::ceil(pairs * c / 152.0), fill) * (std::ceil((double)kPlanTile / c) + ends);
+                std::max(std::ceil(pairs * c / 152.0), 2.0) * (std::ceil((double)kPlanTile / c) + ends);
             if (c == 1 || t < 0.99 * cost) {
                 cost = t;
                 s = c;
             }
         }
     } else {
-        s = (int)std::min((double)kSplitMax, std::sqrt((periodic ? 160000.0 : fp64 ? 40000.0 : 13000.0) / pairs) +
-                                                     (fp64 ? 0.5 : 0.05));  // whole df64 pairs have constant bounds
+        s = (int)std::min((double)kSplitMax, std::sqrt((periodic ? 145000.0 : 13000.0) / pairs) +
+                                                 (fp64 ? 0.5 : 0.05));  // whole df64 pairs have constant bounds
     }
     return s;
 }
