@@ -489,11 +489,15 @@ int rmw_wall_product_noalloc(int kind, const double *r, const double *v, double 
  * rmw_release_scratch, so a process holds at most a few such buffers per
  * stream it calls the library on.  The symmetric pair kernels need
  * ceil(n/128) * 3n doubles of partial sums (21.7 MB at 10,752 blobs, 5.5 GB at
- * 172,032); buffers of 1 GiB and more are allocated without headroom.
- * rmw_set_scratch_limit caps one buffer at `bytes` (0 = no cap): a product
- * whose symmetric partial sums would exceed it runs the one-sided kernels,
- * whose scratch is a few hundred bytes per blob, and a request still above the
- * cap returns RMW_ERR_ALLOC.  rmw_release_scratch frees the current device's
+ * 172,032; twice that for [U; W]), times the CTAs that share a tile pair below
+ * some 10,000 blobs in FP64 and df64.  A buffer of these modes keeps room for
+ * any smaller product of the same kind: up to 64 MB of partial sums (128 MB for
+ * [U; W]) where a product's own are less.  Buffers of 1 GiB and more are
+ * allocated without headroom.  rmw_set_scratch_limit caps one buffer at `bytes`
+ * (0 = no cap): fewer CTAs share a tile pair then, a product whose unsplit
+ * partial sums would still exceed it runs the one-sided kernels, whose scratch
+ * is a few hundred bytes per blob, and a request above the cap even then
+ * returns RMW_ERR_ALLOC.  rmw_release_scratch frees the current device's
  * buffers (after the device is idle); buffers a live CUDA graph may use are
  * freed when the last graph is destroyed. */
 int rmw_set_scratch_limit(int64_t bytes);

@@ -73,11 +73,12 @@ int wall_product_batched(const WallBatch &B, int kind, const double *r, const do
 int wall_default_chunks(int n);
 // the same for a precision mode: finer in FP64 and df64 where few tiles would leave SMs idle
 int wall_default_chunks(int mode, int n);
-// Symmetric product of any kind (each unordered pair once, applied both ways),
-// df64 or mixed: selected when wall_chunks returns kSymChunks and
-// wall_sym_applicable holds (df64 or mixed, not periodic, n >= 256, ntiles x
-// 3n doubles of partial sums within wall_sym_partial_budget()).  Its scratch is
-// wall_scratch_bytes(n, mode, wall_sym_slots(n, nsplit)).
+// Symmetric product of any kind (each unordered pair once, applied both ways)
+// in any precision mode: selected when wall_prefers_sym and
+// wall_sym_applicable hold (n >= 256; not periodic, but for FP64 in x and / or
+// y; ntiles x 3n doubles of partial sums within wall_sym_partial_budget()).
+// Its scratch is wall_scratch_bytes(n, mode, wall_sym_slots(n, nsplit)), with
+// room for wall_reserve_bytes.
 constexpr int kSymChunks = -1;
 constexpr size_t kSymMaxPartialBytes = size_t(6) << 30;  // up to ~185,000 blobs (5.5 GB at 172,032)
 // The partial-sum budget of the current device: kSymMaxPartialBytes, or an
