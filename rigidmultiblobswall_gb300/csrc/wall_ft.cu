@@ -541,7 +541,7 @@ void ft_finalize(const double *r, const double *F, const double *T, const double
 // every block times 3/2, undone by the finalize.  The sum of four symmetric
 // single products, which this replaces, read the blobs and formed the geometry
 // four times and needed a vector of scratch and two additions.  8,064 blobs,
-// [U; W]: df64 2.20 -> 1.51 ms (3.51 before the blocks were written out), four
+// [U; W]: df64 2.20 -> 1.55 ms (3.51 before the blocks were written out), four
 // CTAs of 255 registers per SM (six of 168 spill: 1.58 ms); FP64
 // 23.0 -> 6.94 ms (10.6 with every operation on the FP64 pipe).
 struct FtSteps {
@@ -627,7 +627,10 @@ __global__ void __launch_bounds__(kFtSymTile) ft_sym_fp64_kernel(const FtSrcD *_
     }
 }
 
-// df64: two targets per thread in packed lanes, as wall_uf_df_sym_kernel
+// df64: two targets per thread in packed lanes, as wall_uf_df_sym_kernel.  An
+// accumulator takes the terms of two blocks a step, so both sides' sums are
+// renormalised every four steps: error at 8,064 blobs 9.46e-14, that of four
+// single products 9.50e-14 (9.57e-14 with the targets' every eight, 0.5 % faster).
 constexpr int kFtF2Threads = kFtSymTile / 2;
 
 struct FtTarget {
@@ -636,7 +639,7 @@ struct FtTarget {
 
 template <bool DIAG, bool WITH_W>
 __device__ __forceinline__ void ft_f2_step(const FtTarget &me, int ja, int jb, const float4 (*tile)[kFtSymTile],
-                                           float4 (*sacc)[kFtSymTile], df2 (&u)[6])
+                                           float4 (*sacc)[kFtSymTile], df2 (&u)[6], bool renorm)
 {
     constexpr int NC = WITH_W ? 6 : 3;
     df2 v[3][3];  // position, F, T of the sources
@@ -677,6 +680,7 @@ __device__ __forceinline__ void ft_f2_step(const FtTarget &me, int ja, int jb, c
     }
     const RotBlockDF2 k = rot_block_df<true>(g, dz, Rz, me.z, zj);
     ut_acc_df(k, dx, dy, v[2][0], v[2][1], v[2][2], me.t[0], me.t[1], me.t[2], u[0], u[1], u[2], wx, wy, wz);
+    if (renorm) { wx = norm(wx); wy = norm(wy); wz = norm(wz); }
     store(0, wx); store(1, wy); store(2, wz);
     if constexpr (WITH_W) {
         wx = load(NC - 3); wy = load(NC - 2); wz = load(NC - 1);
@@ -684,6 +688,7 @@ __device__ __forceinline__ void ft_f2_step(const FtTarget &me, int ja, int jb, c
         const UFBlockDF<df2> m = wt_block_df<true>(g, dz, Rz);
         uf_block_acc_df(m, m.t3, m.t4, dx, dy, v[2][0], v[2][1], v[2][2], u[3], u[4], u[5]);
         uf_block_acc_df(m, m.t4, m.t3, dx, dy, me.t[0], me.t[1], me.t[2], wx, wy, wz);
+        if (renorm) { wx = norm(wx); wy = norm(wy); wz = norm(wz); }
         store(NC - 3, wx); store(NC - 2, wy); store(NC - 1, wz);
     }
 }
@@ -732,7 +737,7 @@ __global__ void __launch_bounds__(kFtF2Threads, 4) ft_sym_df_kernel(const FtSrcD
     for (int c = 0; c < 6; ++c) u[c] = df2_zero();
     const FtSteps sp = ft_steps();
     auto renorm = [&](int k) {
-        if (k & 7) return;
+        if (k & 3) return;
         for (int c = 0; c < NC; ++c) u[c] = norm(u[c]);
     };
     auto fold = [&]() {
@@ -748,14 +753,14 @@ __global__ void __launch_bounds__(kFtF2Threads, 4) ft_sym_df_kernel(const FtSrcD
             __syncwarp();
             const int ja = (tid + o) & (kFtSymTile - 1), jb = (tid + kFtF2Threads + o) & (kFtSymTile - 1);
             if (o < kFtSymTile / 2) {
-                ft_f2_step<true, WITH_W>(me, ja, jb, tile, sacc[warp], u);
+                ft_f2_step<true, WITH_W>(me, ja, jb, tile, sacc[warp], u, !(o & 3));
             } else {
                 FtTarget half = me;
                 for (int c = 0; c < 3; ++c)
                     half.f[c].hi.y = half.f[c].lo.y = half.t[c].hi.y = half.t[c].lo.y = 0.f;
                 df2 v[6];
                 for (int c = 0; c < 6; ++c) v[c] = u[c];
-                ft_f2_step<true, WITH_W>(half, ja, jb, tile, sacc[warp], v);
+                ft_f2_step<true, WITH_W>(half, ja, jb, tile, sacc[warp], v, true);
                 for (int c = 0; c < NC; ++c) {
                     u[c].hi.x = v[c].hi.x;
                     u[c].lo.x = v[c].lo.x;
@@ -769,7 +774,7 @@ __global__ void __launch_bounds__(kFtF2Threads, 4) ft_sym_df_kernel(const FtSrcD
         for (int k = sp.k0; k < sp.k1; ++k) {
             __syncwarp();
             const int j = (lane + k) & (kFtSymTile - 1);
-            ft_f2_step<false, WITH_W>(me, j, j, tile, sacc[warp], u);
+            ft_f2_step<false, WITH_W>(me, j, j, tile, sacc[warp], u, !((k + 1) & 3));
             renorm(k + 1);
             if (!((k + 1) & (kFtDfGroup - 1))) fold();
         }
