@@ -63,7 +63,7 @@ DF64_UF_TRAFFIC_BYTES = {"symmetric": 758784, "standard": 710912}
 # counted twice as above ((smsp__inst_executed.sum 17,225,517,484 + packed 12,782,367,918) * 32 / (N^2 * 16),
 # 60,000 blobs)
 MULTI16_INST_PER_PAIR_RHS = 16.67
-DF64_UF_KERNEL_SOURCE_SHA = "9c7434a56055c983c69002d3d3fdeeeabbba395778a782db36f8f7934762ba57"
+DF64_UF_KERNEL_SOURCE_SHA = "b7e4e888c7f46a9a6bb39836fe53f0d372c5734ba0f5881141e7f14a97eb9bf1"
 
 
 def df64_uf_kernel_source_sha():

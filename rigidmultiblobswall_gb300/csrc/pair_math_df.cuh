@@ -209,7 +209,8 @@ __device__ __forceinline__ void pair_rpy_df(df dx, df dy, df dz, df vx, df vy, d
 // Rz >= 2, u <= 1/4, E <= 1.
 // p is held times kDfP and its partners (Y, Z, w5, ...) by 1 / kDfP, both
 // exact: s^5 loses its low part 10^6 radii above the wall and vanishes at
-// 10^8, while p Z and p w5 stay of the order of s and s^3.
+// 10^8, while p Z and p w5 stay of the order of s and s^3.  2^100 keeps every
+// term finite to 10^17 radii (2^64: to 10^14) and the low parts normal.
 template <class D> struct UFBlockDF {
     D Af, b2, t3, t4, zz;
 };
@@ -252,7 +253,7 @@ __device__ __forceinline__ void uf_near_df(df2 r2, df2 invr, df2 &ia, df2 &a3, d
 // h4 = 4 h_i, hj, Rz = h_i + h_j (may be unnormalised).  ZPER: dz is an
 // image's and not h_i - h_j (= dw), so R^2 and the wall parts of G and zz are
 // formed from the heights.
-constexpr float kDfP = 0x1p64f;
+constexpr float kDfP = 0x1p100f;
 template <class D> struct PairGeoDF {
     D r2, invr, i2, s, u, t, p;  // p = kDfP s^5
 };

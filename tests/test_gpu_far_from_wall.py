@@ -41,3 +41,16 @@ def test_rotations_far_from_the_wall(cuda_device, kind, n):
 def test_force_torque_far_from_the_wall(cuda_device):
     r, F = _blobs(300, 1e9)
     _check(mob.wall_force_torque(r, F, 0.0 * F, 1.0, A, mode="df64")[0], owall.force_torque(r, F, 0.0 * F, 1.0, A)[0])
+
+
+@pytest.mark.parametrize("n", [200, 300])
+@pytest.mark.parametrize("kind", ["uf", "ut", "wf", "wt"])
+def test_parked_blobs(cuda_device, kind, n):
+    """Blobs moved out of the way, 10^16 radii up and aside, leave the others' product as it is."""
+    rng = np.random.default_rng(n)
+    r = np.column_stack([rng.uniform(0, 60, n), rng.uniform(0, 60, n), rng.uniform(1.0, 9.0, n)])
+    r[::7] = rng.uniform(0.5, 1.5, (r[::7].shape[0], 3)) * 1e16
+    v = rng.standard_normal(3 * n)
+    got = np.asarray(mob.wall_product(kind, r, v, 1.0, A, mode="df64"))
+    ref = owall.wall_product(kind, r, v, 1.0, A)
+    assert np.linalg.norm(got - ref) <= 1e-12 * np.linalg.norm(ref)
