@@ -9,7 +9,7 @@
 // step in fixed point (about 45).  M_UF at 10,752 blobs 8.1 -> 5.5 ms with
 // products and roots, 4.36 ms with multiply-adds of positive terms and the
 // products with the vectors, 3.69 ms with seven of mixed signs
-// (3.77 with the scaling of the separations).
+// (3.73 with the scaling of the separations).
 //
 // Error bounds, tested against exact arithmetic: int_mul 0.504 ulp (the
 // product of the low halves, below 2^-62 of the result, and the order of ties

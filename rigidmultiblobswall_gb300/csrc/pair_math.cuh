@@ -318,7 +318,7 @@ __device__ __forceinline__ UFBlock2 uf_block_f2(const UFCoeffs2 &c, f2 dx, f2 dy
 // rate) bounds the kernels that use it, so MulInt takes 42 of them to the
 // integer pipes (fp64_int.cuh): the products and positive sums of the
 // geometry, seven multiply-adds of mixed signs and the products with the
-// vectors.  10,752 blobs 8.1 -> 3.77 ms.
+// vectors.  10,752 blobs 8.1 -> 3.73 ms.
 // ZPER: dz is an image's and not h_i - h_j.
 struct PairGeoD {
     double r2, invr, i2, u, s, t, p;
@@ -343,10 +343,11 @@ __device__ __forceinline__ PairGeoD pair_geo_d(double r2, double R2)
 // f(geometry, dx, dy, dz, MUL()): the integer forms where allow is set and every lane's pair permits them (all
 // but dummies, coincident blobs and distances beyond 2^32 radii), else the FP64 ones.  ZPER pairs (dz an image's) take
 // the latter.  SCALE: positions are subtracted before they are scaled to radii, so that blobs near each other and far
-// from the origin keep their separation to the last bit (scaled first, it would carry the rounding of x / a); false:
+// from the origin keep their separation to the last bit (scaled first, it would carry the rounding of x / a: at 504
+// blobs near the origin 5.4e-16 of M_UF against 2.3e-16, by extended precision); false:
 // scale is 1.  Every lane of the warp calls this together (the choice of the form is the warp's, and with it the
-// rounding: it must not depend on which lanes happen to run in step).  allow also stands for a scale within 2^+-64.  Three integer products a pair: M_UF of 10,752 blobs 3.77 ms,
-// 4.03 with FP64 multiplies, 3.69 scaled first.
+// rounding: it must not depend on which lanes happen to run in step).  allow also stands for a scale within 2^+-64.  Three integer products a pair: M_UF of 10,752 blobs
+// 3.69 -> 3.77 ms (4.03 with FP64 multiplies; 3.73 since the vote is the whole warp's).
 template <bool ZPER, bool SCALE, class F>
 __device__ __forceinline__ void with_pair_geo_d(double ex, double ey, double ez, double scale, double Rz, double hi,
                                                 double hj, bool allow, F &&f)
@@ -425,7 +426,7 @@ __device__ __forceinline__ void uf_block_acc_d(const UFBlockD &m, double t3, dou
 // rot_block_df and wt_block_df (pair_math_df.cuh), where they are derived: 64
 // (UT, WF) and 62 (WT) operations a pair against 91 and 74 of the tensor
 // forms, about half of them on the integer pipes (MulInt).  10,752 blobs: UT
-// 9.82 -> 3.96 ms, WF 9.97 -> 4.09, WT 8.08 -> 3.78.  UF32: the blocks times 3/2, as the UF block (for sums of both).
+// 9.82 -> 3.98 ms, WF 9.97 -> 4.10, WT 8.08 -> 3.80.  UF32: the blocks times 3/2, as the UF block (for sums of both).
 struct RotBlockD {
     double a, ar, b, ei, ej, wi, wj;
 };

@@ -543,7 +543,7 @@ void ft_finalize(const double *r, const double *F, const double *T, const double
 // four times and needed a vector of scratch and two additions.  8,064 blobs,
 // [U; W]: df64 2.20 -> 1.55 ms (3.51 before the blocks were written out), four
 // CTAs of 255 registers per SM (six of 168 spill: 1.58 ms); FP64
-// 23.0 -> 6.94 ms (10.6 with every operation on the FP64 pipe).
+// 23.0 -> 6.92 ms (10.6 with every operation on the FP64 pipe).
 struct FtSteps {
     int k0, k1, nsplit, split;
     __device__ __forceinline__ size_t slot(int tile) const { return (size_t)tile * nsplit + split; }

@@ -870,7 +870,7 @@ __device__ __forceinline__ void pair_acc_d(double dx, double dy, double dz, doub
 // coefficient work per ordered pair is the gain); source-side sums per warp
 // in FP64 shared memory.  UF through the explicit block of uf_block_d with
 // what can leave the FP64 pipe on the integer pipes: the 10,752-blob product
-// 11.6 -> 3.77 ms, 31 FP64 instructions per pair.  Measured beside it (at
+// 11.6 -> 3.73 ms, 31 FP64 instructions per pair.  Measured beside it (at
 // 3.69 ms, positions scaled when packed): three more multiply-adds on the
 // integer pipes 3.87 ms; from 38 instructions and
 // 4.36 ms, additions there (dx, dy, dz, Rz) 4.31 ms, and free-space and periodic
@@ -1753,7 +1753,7 @@ static void launch_sym_finalize(const double *r, const double *v, const double *
 
 // The FP64 product periodic in x and / or y through the symmetric kernel.
 // M_UF of 1,500 blobs in a square box: one-sided 2.94, symmetric 1.62 ms with
-// every operation on the FP64 pipe, 0.92 with the integer forms; the images of
+// every operation on the FP64 pipe, 0.90 with the integer forms; the images of
 // a pair share its minimum-image division.
 template <int KIND>
 static int per_sym_product(const double *r, const double *v, double *out, int n, double a, double nf, const double *L,
