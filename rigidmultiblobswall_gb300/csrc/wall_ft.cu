@@ -431,8 +431,8 @@ __global__ void __launch_bounds__(kFtSymTile) ft_sym_mixed_kernel(const FtSrcF *
     const bool diag = (T == S);
     const int i = T * kFtSymTile + tid;
     const bool valid_i = i < n;
-    // a target or source past the end is a dummy far above the wall with zero vectors
-    const FtSrcF dummy = {make_float4(1.0e6f, 1.0e6f, 1.0e6f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f),
+    // a target or source past the end is a dummy with zero vectors half a radius above the wall, where no blob is
+    const FtSrcF dummy = {make_float4(0.f, 0.f, 0.5f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f),
                           make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
     const FtSrcF me = valid_i ? src[i] : dummy;
     const float hi = me.hi.z + me.lo.z;

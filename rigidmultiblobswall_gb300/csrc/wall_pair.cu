@@ -613,8 +613,10 @@ __device__ __forceinline__ void mixed_sym_body(const SrcF *__restrict__ src, int
     const bool diag = (T == S);
     const int i = T * kTile + tid;
     const bool valid_i = i < n;
-    const SrcF dummy = {make_float4(1.0e6f, 1.0e6f, 1.0e6f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f),
-                        make_float4(0.f, 0.f, 0.f, 0.f)};
+    // a target or source past the end is a dummy with a zero vector (as in df_f2_body)
+    const SrcF dummy = {NOWALL ? make_float4(kFreeDummy[0], kFreeDummy[1], kFreeDummy[2], 0.f)
+                               : make_float4(0.f, 0.f, 0.5f, 0.f),
+                        make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
     const SrcF me = valid_i ? src[i] : dummy;
     const float hi = me.hi.z + me.lo.z;
     {
@@ -765,7 +767,8 @@ __global__ void __launch_bounds__(kF2Threads, 14) wall_uf_mixed_sym_kernel(const
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool diag = (T == S);
     const int i0 = T * kTile + tid, i1 = i0 + kF2Threads;
-    const SrcF dummy = {make_float4(1.0e6f, 1.0e6f, 1.0e6f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f),
+    // a target or source past the end is a dummy with a zero vector (as in df_f2_body)
+    const SrcF dummy = {make_float4(0.f, 0.f, 0.5f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f),
                         make_float4(0.f, 0.f, 0.f, 0.f)};
     MixTarget me;
     {
