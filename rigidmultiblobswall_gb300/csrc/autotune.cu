@@ -73,9 +73,6 @@ __global__ void synth_blobs_kernel(double *r, double *v, int n, double a, unsign
 
 }  // namespace
 
-// the built-in rule of the standard entry points: the symmetric kernel, where it applies
-static bool rule_prefers_sym(int mode, int n) { return n >= (mode == RMW_MODE_MIXED ? 8192 : 256); }
-
 int wall_chunks(int kind, int mode, int n)
 {
     {
@@ -100,7 +97,7 @@ bool wall_prefers_sym(int kind, int mode, int n)
         auto it = g_tuned.find(key_of(kind, mode, n));
         if (it != g_tuned.end()) return it->second == kSymChunks;
     }
-    return rule_prefers_sym(mode, n);
+    return n >= (mode == RMW_MODE_MIXED ? 8192 : 256);
 }
 
 }  // namespace rmw
@@ -122,12 +119,10 @@ int rmw_wall_autotune(int kind, int mode, int64_t n, int reps, void *stream, int
     std::vector<int> cand;
     for (int c : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64})
         if (c <= rmw::max_chunks(N)) cand.push_back(c);
-    const int split = rmw::wall_default_chunks(mode, N);
-    if (std::find(cand.begin(), cand.end(), split) == cand.end()) cand.push_back(split);
+    const int def = rmw::wall_default_chunks(mode, N);
+    if (std::find(cand.begin(), cand.end(), def) == cand.end()) cand.push_back(def);
     const bool try_sym = rmw::wall_sym_applicable(kind, mode, N, nullptr);
     if (try_sym) cand.push_back(rmw::kSymChunks);
-    // what an untuned product runs
-    const int def = try_sym && rmw::rule_prefers_sym(mode, N) ? rmw::kSymChunks : split;
     const int nsplit = try_sym ? rmw::wall_sym_split(mode, N, rmw::wall_scratch_bytes(N, mode, 0)) : 1;
     const int cmax = std::max(*std::max_element(cand.begin(), cand.end()), try_sym ? rmw::wall_sym_slots(N, nsplit) : 1);
     const size_t vec = sizeof(double) * 3 * (size_t)N;
