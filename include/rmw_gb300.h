@@ -194,8 +194,9 @@ int rmw_wall_force_torque(const double *r, const double *F, const double *T, dou
  * kernel, reported as nchunks = -1) on n synthetic blobs and caches the
  * fastest for (device, kind, mode, n's quarter-octave size bucket); the
  * product entry points above and the rigid-body operators then use it.
- * Synchronous.  best_ms / default_ms: mean time of the chosen split and of
- * the built-in rule's. */
+ * Synchronous.  best_ms: mean time of the chosen split or kernel; default_ms:
+ * of the one-sided kernel with its built-in split, also at sizes where an
+ * untuned product runs the symmetric kernel. */
 int rmw_wall_autotune(int kind, int mode, int64_t n, int reps, void *stream, int *best_nchunks, double *best_ms,
                       double *default_ms);
 /* The choice for (kind, mode, n): -1 the symmetric kernel, else the one-sided

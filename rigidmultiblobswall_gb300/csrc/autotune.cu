@@ -107,7 +107,7 @@ extern "C" {
 // Time every admissible source split of the `kind` product in `mode` on n
 // synthetic blobs (reps timed launches each, after one warm-up), cache the
 // fastest for n's size bucket on the current device and report it with its
-// time and the built-in rule's.  Synchronous.
+// time and that of the one-sided kernel's built-in split.  Synchronous.
 int rmw_wall_autotune(int kind, int mode, int64_t n, int reps, void *stream, int *best_nchunks, double *best_ms,
                       double *default_ms)
 {

@@ -251,7 +251,8 @@ def autotune(kind="uf", n=10752, mode="df64", reps=3, device=None):
     """Time every admissible source split of the `kind` product in `mode` on n
     synthetic blobs and cache the fastest for n's size bucket on the device;
     later products of that size use it.  Returns {"nchunks", "ms",
-    "default_ms"}."""
+    "default_ms"}, the last one the time of the one-sided kernel with its
+    built-in split."""
     import torch
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     best = ctypes.c_int(0)
